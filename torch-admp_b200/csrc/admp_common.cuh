@@ -90,6 +90,20 @@ __device__ __forceinline__ void load_box(const T* box, double* b) {
   for (int k = 0; k < 9; ++k) b[k] = (double)box[k];
 }
 
+// Minimum-image displacement in place (spatial.py:15-36, floor(f + 0.5)); nimg: the images taken off.
+__device__ __forceinline__ void min_image(const double* b, const double* bi, double* dr, double* nimg) {
+  double f[3];
+#pragma unroll
+  for (int e = 0; e < 3; ++e) f[e] = dr[0] * bi[0 * 3 + e] + dr[1] * bi[1 * 3 + e] + dr[2] * bi[2 * 3 + e];
+#pragma unroll
+  for (int e = 0; e < 3; ++e) {
+    nimg[e] = floor(f[e] + 0.5);
+    f[e] -= nimg[e];
+  }
+#pragma unroll
+  for (int e = 0; e < 3; ++e) dr[e] = f[0] * b[0 * 3 + e] + f[1] * b[1 * 3 + e] + f[2] * b[2 * 3 + e];
+}
+
 // Order-6 cardinal B-spline weights for fractional offset t in [0,1).
 // w[k] = M6(t + k), k = 0..5, built by the Cox-de Boor recursion
 // M_n(u) = u/(n-1) M_{n-1}(u) + (n-u)/(n-1) M_{n-1}(u-1);  d[k] = M6'(t+k)

@@ -191,20 +191,6 @@ __global__ void __launch_bounds__(512)
 }
 
 template <typename T>
-__device__ __forceinline__ void min_image(const double* b, const double* bi, double* dr, double* nimg) {
-  double f[3];
-#pragma unroll
-  for (int e = 0; e < 3; ++e) f[e] = dr[0] * bi[0 * 3 + e] + dr[1] * bi[1 * 3 + e] + dr[2] * bi[2 * 3 + e];
-#pragma unroll
-  for (int e = 0; e < 3; ++e) {
-    nimg[e] = floor(f[e] + 0.5);
-    f[e] -= nimg[e];
-  }
-#pragma unroll
-  for (int e = 0; e < 3; ++e) dr[e] = f[0] * b[0 * 3 + e] + f[1] * b[1 * 3 + e] + f[2] * b[2 * 3 + e];
-}
-
-template <typename T>
 __global__ void __launch_bounds__(256)
     pair_dist_kernel(int pbc, int N, long long P, const long long* __restrict__ pairs,
                      const T* __restrict__ pos, const T* __restrict__ box, T* __restrict__ ds,
@@ -226,7 +212,7 @@ __global__ void __launch_bounds__(256)
     double dr[3], n[3];
     if (pbc) {
       for (int e = 0; e < 3; ++e) dr[e] = (double)pos[3 * i + e] - (double)pos[3 * j + e];
-      min_image<T>(geo, geo + 9, dr, n);
+      min_image(geo, geo + 9, dr, n);
     } else {
       for (int e = 0; e < 3; ++e) dr[e] = (double)pos[3 * j + e] - (double)pos[3 * i + e];
     }
@@ -259,7 +245,7 @@ __global__ void __launch_bounds__(256)
     double dr[3], n[3] = {0, 0, 0};
     if (pbc) {
       for (int e = 0; e < 3; ++e) dr[e] = (double)pos[3 * i + e] - (double)pos[3 * j + e];
-      min_image<T>(geo, geo + 9, dr, n);
+      min_image(geo, geo + 9, dr, n);
     } else {
       for (int e = 0; e < 3; ++e) dr[e] = (double)pos[3 * j + e] - (double)pos[3 * i + e];
     }

@@ -96,6 +96,38 @@ DevError* scratch_error(cudaStream_t) {
   return g_err_ptr[dev];
 }
 
+// The thread's page-locked staging buffer: kept while the thread lives.
+struct PinnedBuf {
+  void* p = nullptr;
+  ~PinnedBuf() {
+    if (p) cudaFreeHost(p);
+  }
+};
+static thread_local PinnedBuf g_pin;
+
+static void* pinned() {
+  if (!g_pin.p) {
+    cudaError_t e = cudaHostAlloc(&g_pin.p, kReadBack, cudaHostAllocPortable);
+    if (e != cudaSuccess) {
+      g_pin.p = nullptr;
+      set_last_cuda_error(e, "cudaHostAlloc", __FILE__, __LINE__);
+    }
+  }
+  return g_pin.p;
+}
+
+const void* read_back(const void* dev, size_t bytes, cudaStream_t st) {
+  void* p = bytes <= kReadBack ? pinned() : nullptr;
+  if (!p) return nullptr;
+  cudaError_t e = cudaMemcpyAsync(p, dev, bytes, cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e != cudaSuccess) {
+    set_last_cuda_error(e, "read-back", __FILE__, __LINE__);
+    return nullptr;
+  }
+  return p;
+}
+
 static const char* where_name(int w) {
   switch (w) {
     case 1: return "pair energy";

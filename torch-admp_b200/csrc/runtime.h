@@ -15,6 +15,11 @@ DevError* scratch_error(cudaStream_t st);
 // the error word and turn it into a status.  Otherwise return ADMP_OK and
 // leave the error sticky for admp_check_errors().
 int check_error(DevError* err, cudaStream_t st);
+// Copy `bytes` (at most kReadBack) of device memory into a page-locked buffer
+// of the calling thread and wait for it; the result is valid until the
+// thread's next call.  nullptr on a CUDA error.
+constexpr size_t kReadBack = 64 * 1024;
+const void* read_back(const void* dev, size_t bytes, cudaStream_t st);
 // Record a message and return `code`.
 int fail(int code, const char* fmt, ...);
 bool sync_checks();
