@@ -9,6 +9,13 @@
 
 namespace admp {
 
+// Spread / gather kernels: four warps of eight atoms a block (eight warps were 10-20% slower up to 10,000
+// atoms and equal above).  The potential-only gather has so little work per atom that above kGatherRun
+// atoms its blocks take 256 atoms, each warp four groups in turn: 49 launches over 410,000 atoms 2,864 ->
+// 2,508 us (FP32); the other kernels lose 10-20% that way.
+constexpr int kStWarps = 4;
+constexpr int kGatherRun = 64000;
+
 struct SysSpec {
   int natoms;
   int atom_off;
@@ -35,6 +42,7 @@ struct RecipPlan {
   // (every K1, K2 <= kTcMaxK)
   bool tc_x = false;
   bool tc_y = false;
+  int blk_st[kMaxBatch];  // first block of each system in the spread / gather kernels
 };
 
 // The per-system table as one by-value parameter: the only launch of a call
@@ -77,6 +85,7 @@ inline Batch family_batch(const RecipPlan<T>& p, int F) {
                : F == F_XT ? d.blk_xt
                : F == F_YT ? d.blk_yt
                : F == F_ZT ? d.blk_zt
+               : F == F_ST ? p.blk_st[s]
                            : d.blk_slab;
   }
   return b;
@@ -91,6 +100,7 @@ inline int build_recip_plan(const SysSpec* sys, int nsys, RecipPlan<T>& p) {
   Batch& b = p.b;
   b.nsys = nsys;
   b.apb = 256;
+  b.aps = kStWarps * kPw;
   b.done = nullptr;
   b.done_stride = 0;
   b.status_off = 0;
@@ -121,7 +131,7 @@ inline int build_recip_plan(const SysSpec* sys, int nsys, RecipPlan<T>& p) {
   p.smem_x = (2 * (size_t)zb + 1) * maxK[0] * cs + ((size_t)maxK[0] + 2 * zb) * 8 + (size_t)zb * 16;
   if (p.smem_z > 227 * 1024 || p.smem_y > 227 * 1024 || p.smem_x > 227 * 1024)
     return fail(ADMP_ERR_MESH, "mesh %dx%dx%d too large for the shared-memory FFT", maxK[0], maxK[1], maxK[2]);
-  int ba = 0, bz = 0, by = 0, bx = 0, bxt = 0, byt = 0, bzt = 0;
+  int ba = 0, bst = 0, bz = 0, by = 0, bx = 0, bxt = 0, byt = 0, bzt = 0;
   size_t mo = 0, so = 0;
   for (int s = 0; s < nsys; ++s) {
     SysDesc& d = p.hs[s];
@@ -135,6 +145,7 @@ inline int build_recip_plan(const SysSpec* sys, int nsys, RecipPlan<T>& p) {
     d.box_idx = sys[s].box_idx;
     d.flags = 0;
     d.blk_atom = ba;
+    p.blk_st[s] = bst;
     d.blk_z = bz;
     d.blk_y = by;
     d.blk_x = bx;
@@ -146,6 +157,7 @@ inline int build_recip_plan(const SysSpec* sys, int nsys, RecipPlan<T>& p) {
     d.green_off = sys[s].green_off >= 0 ? (int64_t)sys[s].green_off : (int64_t)so;
     const int ncb = (d.K2h + zb - 1) / zb;
     ba += (d.natoms + b.apb - 1) / b.apb;
+    bst += (d.natoms + b.aps - 1) / b.aps;
     bz += ((d.K0 * d.K1 + 1) / 2 + lp - 1) / lp;
     by += d.K0 * ncb;
     bx += (d.K1 * d.K2h + zb - 1) / zb;  // x passes: runs of zb flattened (y, kz) columns
@@ -156,6 +168,7 @@ inline int build_recip_plan(const SysSpec* sys, int nsys, RecipPlan<T>& p) {
     so += align_up((size_t)d.K0 * d.K1 * d.K2h, 32);
   }
   b.nblk_atom = ba;
+  b.nblk_st = bst;
   b.nblk_xt = bxt;
   b.nblk_yt = byt;
   b.nblk_zt = bzt;
@@ -200,7 +213,7 @@ inline int launch_green_build(const RecipPlan<T>& p, const T* box, T* green, dou
 
 template <typename T>
 inline int launch_fft_green(const RecipPlan<T>& p, T* mesh, Cplx<T>* spec, const T* box, double* acc, double ke,
-                            cudaStream_t st, const T* green = nullptr) {
+                            cudaStream_t st, const T* green = nullptr, bool virial = false) {
   const Batch& b = p.b;
   const Batch bsl = family_batch(p, F_SLAB), bz = family_batch(p, F_Z), by = family_batch(p, F_Y),
               bx = family_batch(p, F_X);
@@ -208,7 +221,8 @@ inline int launch_fft_green(const RecipPlan<T>& p, T* mesh, Cplx<T>* spec, const
   ADMP_CUDA_TRY(ensure_smem(fft_z_inv_kernel<T>, p.smem_z));
   ADMP_CUDA_TRY(ensure_smem(fft_y_kernel<T, false>, p.smem_y));
   ADMP_CUDA_TRY(ensure_smem(fft_y_kernel<T, true>, p.smem_y));
-  ADMP_CUDA_TRY(ensure_smem(fft_x_green_kernel<T>, p.smem_x));
+  ADMP_CUDA_TRY(ensure_smem(fft_x_green_kernel<T, false>, p.smem_x));
+  ADMP_CUDA_TRY(ensure_smem(fft_x_green_kernel<T, true>, p.smem_x));
   ADMP_CUDA_TRY(ensure_smem(fft_x_apply_kernel<T>, p.smem_x));
   // algorithmic bytes: z passes read/write M reals + Mh complex, y/x passes Mh complex in and out
   const double rb = (double)p.mesh_elems * sizeof(T), cb = (double)p.spec_elems * sizeof(Cplx<T>);
@@ -265,8 +279,10 @@ inline int launch_fft_green(const RecipPlan<T>& p, T* mesh, Cplx<T>* spec, const
                                                           (const float*)green, tct);
     else if (green)
       fft_x_apply_kernel<T><<<b.nblk_x, 256, p.smem_x, st>>>(bx, spec, green);
+    else if (virial)
+      fft_x_green_kernel<T, true><<<b.nblk_x, 256, p.smem_x, st>>>(bx, spec, box, acc, ke);
     else
-      fft_x_green_kernel<T><<<b.nblk_x, 256, p.smem_x, st>>>(bx, spec, box, acc, ke);
+      fft_x_green_kernel<T, false><<<b.nblk_x, 256, p.smem_x, st>>>(bx, spec, box, acc, ke);
   }
   // spectrum in and out, plus the cached Green's function (one real per entry) when it is read
   prof_end(h, PK_FFT_X_GREEN, 2 * cb + (green ? (double)p.spec_elems * sizeof(T) : 0.0), st);
@@ -288,17 +304,6 @@ inline int launch_fft_green(const RecipPlan<T>& p, T* mesh, Cplx<T>* spec, const
   return ADMP_OK;
 }
 
-// Full reciprocal evaluation: spread q, FFT/Green, gather.
-// `dE_dq` receives the potential (dE/dq), `dE_dpos` the gradient; both accumulate.
-template <typename T>
-inline size_t spread_smem() {
-  return 8 * WarpStencil<T, false>::bytes();
-}
-template <typename T, bool F>
-inline size_t gather_smem() {
-  return 8 * WarpStencil<T, F>::bytes();
-}
-
 template <typename T>
 inline double plan_atoms(const RecipPlan<T>& p) {
   double n = 0;
@@ -307,40 +312,49 @@ inline double plan_atoms(const RecipPlan<T>& p) {
 }
 
 template <typename T>
-inline int launch_spread(const Batch& b, const T* pos, const T* box, const T* q, T* mesh, const int* order,
+inline int launch_spread(const RecipPlan<T>& p, const T* pos, const T* box, const T* q, T* mesh, const int* order,
                          cudaStream_t st) {
-  if (!b.nblk_atom) return ADMP_OK;
-  ADMP_CUDA_TRY(ensure_smem(spread_kernel<T>, spread_smem<T>()));
-  spread_kernel<T><<<b.nblk_atom, 256, spread_smem<T>(), st>>>(b, pos, box, q, mesh, order);
+  if (!p.b.nblk_st) return ADMP_OK;
+  constexpr size_t sm = kStWarps * WarpStencil<T, false>::bytes();
+  ADMP_CUDA_TRY(ensure_smem(spread_kernel<T>, sm));
+  spread_kernel<T><<<p.b.nblk_st, kStWarps * 32, sm, st>>>(family_batch(p, F_ST), pos, box, q, mesh, order);
   return ADMP_OK;
 }
 
-template <typename T, bool F>
-inline int launch_gather(const Batch& b, const T* pos, const T* box, const T* q, const T* phi, T* dE_dq,
+template <typename T, bool F, bool V>
+inline int launch_gather(const RecipPlan<T>& p, const T* pos, const T* box, const T* q, const T* phi, T* dE_dq,
                          T* dE_dpos, double* acc, const int* order, cudaStream_t st) {
-  if (!b.nblk_atom) return ADMP_OK;
-  ADMP_CUDA_TRY(ensure_smem(gather_kernel<T, F>, gather_smem<T, F>()));
-  gather_kernel<T, F><<<b.nblk_atom, 256, gather_smem<T, F>(), st>>>(b, pos, box, q, phi, dE_dq, dE_dpos, acc, T(1),
-                                                                     order);
+  if (!p.b.nblk_st) return ADMP_OK;
+  const bool run = !F && plan_atoms(p) > kGatherRun;
+  const int nw = run ? 8 : kStWarps;
+  const size_t sm = nw * WarpStencil<T, F>::bytes();
+  ADMP_CUDA_TRY(ensure_smem(gather_kernel<T, F, V>, sm));
+  Batch b = family_batch(p, run ? F_ATOM : F_ST);
+  if (run) b.aps = b.apb;
+  gather_kernel<T, F, V><<<run ? b.nblk_atom : b.nblk_st, nw * 32, sm, st>>>(b, pos, box, q, phi, dE_dq, dE_dpos, acc,
+                                                                            order);
   return ADMP_OK;
 }
 
+// Full reciprocal evaluation: spread q, FFT/Green, gather.
+// `dE_dq` receives the potential (dE/dq), `dE_dpos` the gradient; both accumulate.
+// `virial`: the accumulators get the virial terms too (dE/dbox is asked for).
 template <typename T>
 inline int launch_recip(const RecipPlan<T>& p, const T* pos, const T* box, const T* q, T* mesh, Cplx<T>* spec,
-                        double* acc, double ke, T* dE_dq, T* dE_dpos, cudaStream_t st,
+                        double* acc, double ke, T* dE_dq, T* dE_dpos, cudaStream_t st, bool virial,
                         const int* order = nullptr) {
-  const Batch& b = p.b;
   const double na = plan_atoms(p), mb = (double)p.mesh_elems * sizeof(T);
   ADMP_CUDA_TRY(cudaMemsetAsync(mesh, 0, p.mesh_elems * sizeof(T), st));
   int h = prof_begin(st);
-  int s = launch_spread<T>(b, pos, box, q, mesh, order, st);
+  int s = launch_spread<T>(p, pos, box, q, mesh, order, st);
   if (s) return s;
   prof_end(h, PK_SPREAD, na * 4 * sizeof(T) + mb, st);
   count_launches(1);
-  s = launch_fft_green<T>(p, mesh, spec, box, acc, ke, st);
+  s = launch_fft_green<T>(p, mesh, spec, box, acc, ke, st, nullptr, virial);
   if (s) return s;
   h = prof_begin(st);
-  s = launch_gather<T, true>(b, pos, box, q, mesh, dE_dq, dE_dpos, acc, order, st);
+  s = virial ? launch_gather<T, true, true>(p, pos, box, q, mesh, dE_dq, dE_dpos, acc, order, st)
+             : launch_gather<T, true, false>(p, pos, box, q, mesh, dE_dq, dE_dpos, acc, order, st);
   if (s) return s;
   prof_end(h, PK_GATHER, mb + na * 4 * sizeof(T) + na * 3 * sizeof(T), st);
   count_launches(1);
@@ -353,17 +367,16 @@ template <typename T>
 inline int launch_recip_potential(const RecipPlan<T>& p, const T* pos, const T* box, const T* v, T* mesh,
                                   Cplx<T>* spec, double* acc, double ke, T* pot, cudaStream_t st,
                                   const int* order = nullptr, const T* green = nullptr) {
-  const Batch& b = p.b;
   const double na = plan_atoms(p), mb = (double)p.mesh_elems * sizeof(T);
   ADMP_CUDA_TRY(cudaMemsetAsync(mesh, 0, p.mesh_elems * sizeof(T), st));
   int h = prof_begin(st);
-  int s = launch_spread<T>(b, pos, box, v, mesh, order, st);
+  int s = launch_spread<T>(p, pos, box, v, mesh, order, st);
   if (s) return s;
   prof_end(h, PK_SPREAD, na * 4 * sizeof(T) + mb, st);
   s = launch_fft_green<T>(p, mesh, spec, box, acc, ke, st, green);
   if (s) return s;
   h = prof_begin(st);
-  s = launch_gather<T, false>(b, pos, box, v, mesh, pot, nullptr, acc, order, st);
+  s = launch_gather<T, false, false>(p, pos, box, v, mesh, pot, nullptr, acc, order, st);
   if (s) return s;
   prof_end(h, PK_GATHER, mb + na * 4 * sizeof(T) + na * sizeof(T), st);
   count_launches(2);

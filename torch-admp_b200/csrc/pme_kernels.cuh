@@ -40,6 +40,7 @@ struct Batch {
   int nsys;
   int nblk_atom, nblk_z, nblk_y, nblk_x, nblk_slab, nblk_xt, nblk_yt, nblk_zt;
   int apb;  // atoms per block (atom kernels)
+  int nblk_st, aps;  // blocks and atoms per block of the spread / gather kernels
   int lp;   // line pairs per block (z passes)
   int zb;   // columns per block (y / x passes)
   int maxK0, maxK1, maxK2;
@@ -66,7 +67,7 @@ constexpr int kAccVk = 1;       // 9: dE/dB (B = box^-1) through k vectors
 constexpr int kAccWf = 10;      // 9: dE/dB through fractional coordinates
 constexpr int kAccSlots = 19;
 
-enum SysField { F_ATOM = 0, F_Z = 1, F_Y = 2, F_X = 3, F_SLAB = 4, F_XT = 5, F_YT = 6, F_ZT = 7 };
+enum SysField { F_ATOM = 0, F_Z = 1, F_Y = 2, F_X = 3, F_SLAB = 4, F_XT = 5, F_YT = 6, F_ZT = 7, F_ST = 8 };
 
 template <int F>
 __device__ __forceinline__ int blk_of(const SysDesc& d) {
@@ -83,7 +84,7 @@ __device__ __forceinline__ int blk_of(const SysDesc& d) {
 template <int F>
 __device__ __forceinline__ int find_sys(const Batch& b, int blk) {
   int lo = 0, hi = b.nsys - 1;
-  if (b.fam == F) {
+  if (F == F_ST || b.fam == F) {  // the stencil kernels' column is only in the parameter
     while (lo < hi) {
       const int mid = (lo + hi + 1) >> 1;
       if (b.blk[mid] <= blk)
@@ -151,112 +152,103 @@ __device__ __forceinline__ void load_geom(const T* box, int idx, Geom* g) {
   }
 }
 
-// Stencil of one atom: mesh indices per dim and weights (+derivatives).
-template <typename T>
-struct Stencil {
-  int ix[6], iy[6], iz[6];
-  T w[3][6];
-  T dw[3][6];
-};
+__device__ __forceinline__ int wrap_up(int i, int K) {
+  while (i >= K) i -= K;
+  return i;
+}
 
+// One axis of an atom's stencil: B-spline weights (and derivatives) of the six
+// mesh points and the wrapped index of the first.
 template <typename T>
-__device__ __forceinline__ void make_stencil(const T* r, const Geom& g, int K0, int K1, int K2,
-                                             Stencil<T>& st) {
-  const int K[3] = {K0, K1, K2};
-  const double x0 = r[0], x1 = r[1], x2 = r[2];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    // x_d = K_d * (r @ box_inv)_d  (recip.py:33, 61)
-    double x = (double)K[d] * (x0 * g.binv[0 * 3 + d] + x1 * g.binv[1 * 3 + d] + x2 * g.binv[2 * 3 + d]);
-    double m0 = ceil(x);             // recip.py:62
-    // u0 = m0 - x + 3 (recip.py:63); the stencil point s = k - 3 has u = (m0 - x) + k
-    const T t = (T)(m0 - x);
-    bspline6<T>(t, st.w[d], st.dw[d]);
-    int base = (int)m0 - 3;
-    int* idx = d == 0 ? st.ix : d == 1 ? st.iy : st.iz;
-#pragma unroll
-    for (int k = 0; k < 6; ++k) idx[k] = wrap_index(base + k, K[d]);
-  }
+__device__ __forceinline__ int stencil_axis(int d, int K, const T* r, const Geom& g, T* w, T* dw) {
+  // x_d = K_d * (r @ box_inv)_d  (recip.py:33, 61)
+  const double x = (double)K * ((double)r[0] * g.binv[0 * 3 + d] + (double)r[1] * g.binv[1 * 3 + d] +
+                                (double)r[2] * g.binv[2 * 3 + d]);
+  const double m0 = ceil(x);  // recip.py:62
+  // u0 = m0 - x + 3 (recip.py:63); the stencil point s = k - 3 has u = (m0 - x) + k
+  bspline6<T>((T)(m0 - x), w, dw);
+  return wrap_index((int)m0 - 3, K);
 }
 
 // ---------------------------------------------------------------------------
-// Warp-cooperative stencils: each lane builds the stencil of one atom (its
-// 3x6 B-spline weights, derivatives and wrapped mesh indices) into shared
-// memory, then the warp walks those 32 atoms with its lanes spread over the
-// 36 (y, z) stencil columns, each lane looping over the 6 x offsets.  The
-// optional `order` visits atoms in cell-sorted order so that neighbouring
-// atoms touch neighbouring mesh lines.
+// Warp-cooperative stencils: a warp takes eight atoms.  A lane builds one axis
+// of one atom (6 B-spline weights, derivatives, wrapped mesh indices) into
+// shared memory, then the warp walks the atoms with its lanes spread over the
+// first 32 of the 36 (y, z) stencil columns, each lane looping over the 6 x
+// offsets; the last four columns (y 5, z 2..5) of all eight atoms take one
+// further pass (lane -> atom lane / 4).  The optional `order` visits atoms in
+// cell-sorted order so that neighbouring atoms touch neighbouring mesh lines.
+//
+// Eight atoms a warp and not 32 (a lane building a whole atom): a launch of
+// 3,000 atoms has 375 warps instead of 94, and a third of the building chain.
+// Spread of 200 / 3,000 / 20,000 / 192,000 atoms (FP32): 13.2 / 15.8 / 16.4 /
+// 65.3 -> 5.1 / 5.2 / 10.4 / 58.8 us.
 // ---------------------------------------------------------------------------
-// Per-warp shared layout (dynamic shared memory): for 32 atoms, the 18
-// weights, optionally the 18 derivatives, x offsets ix*K1*K2 (6 ints), the
-// wrapped y / z stencil bases, the charge and the atom index.
+constexpr int kPw = 8;  // atoms per warp
+
+// Per-warp shared layout (dynamic shared memory): the 18 weights of each atom,
+// optionally the 18 derivatives, x offsets ix*K1*K2 (6 ints), the wrapped y / z
+// stencil bases, the charge and the atom index.
 template <typename T, bool DERIV>
 struct WarpStencil {
-  T* w;     // [32][18]
-  T* dw;    // [32][18]
-  int* ox;  // [32][6]
-  int* byz; // [32][2]
-  T* q;     // [32]
-  int* atom;// [32]
+  T* w;     // [kPw][18]
+  T* dw;    // [kPw][18]
+  int* ox;  // [kPw][6]
+  int* byz; // [kPw][2]
+  T* q;     // [kPw]
+  int* atom;// [kPw]
   __host__ __device__ static constexpr size_t bytes() {
-    return 32 * 18 * sizeof(T) * (DERIV ? 2 : 1) + 32 * 6 * sizeof(int) + 32 * 2 * sizeof(int) + 32 * sizeof(T) +
-           32 * sizeof(int) + 16;
+    return kPw * 18 * sizeof(T) * (DERIV ? 2 : 1) + kPw * 6 * sizeof(int) + kPw * 2 * sizeof(int) + kPw * sizeof(T) +
+           kPw * sizeof(int);
   }
   __device__ void carve(unsigned char* base) {
     w = reinterpret_cast<T*>(base);
-    T* e = w + 32 * 18;
+    T* e = w + kPw * 18;
     if (DERIV) {
       dw = e;
-      e += 32 * 18;
+      e += kPw * 18;
     } else {
       dw = nullptr;
     }
     q = e;
-    int* ip = reinterpret_cast<int*>(q + 32);
+    int* ip = reinterpret_cast<int*>(q + kPw);
     ox = ip;
-    byz = ox + 32 * 6;
-    atom = byz + 32 * 2;
+    byz = ox + kPw * 6;
+    atom = byz + kPw * 2;
   }
 };
 
+// Stencils of atoms a_first .. a_first + 7 (those below a_end) of a system.
 template <typename T, bool DERIV>
 __device__ __forceinline__ void warp_build_stencil(WarpStencil<T, DERIV>& ws, const SysDesc& d, const Geom& g,
                                                    const T* __restrict__ pos, const T* __restrict__ q,
                                                    const int* __restrict__ order, int a_first, int a_end, int lane) {
-  const int a = a_first + lane;
+  const int l = lane & (kPw - 1), ax = lane / kPw;
+  const int a = a_first + l;
   if (a < a_end) {
     const int ga = order ? order[d.atom_off + a] : d.atom_off + a;
-    T r[3] = {pos[3 * (size_t)ga], pos[3 * (size_t)ga + 1], pos[3 * (size_t)ga + 2]};
-    Stencil<T> st;
-    make_stencil<T>(r, g, d.K0, d.K1, d.K2, st);
-    T* w = ws.w + lane * 18;
+    if (ax < 3) {
+      const T r[3] = {pos[3 * (size_t)ga], pos[3 * (size_t)ga + 1], pos[3 * (size_t)ga + 2]};
+      const int n = ax == 0 ? d.K0 : ax == 1 ? d.K1 : d.K2;
+      T w[6], dw[6];
+      const int base = stencil_axis<T>(ax, n, r, g, w, dw);
 #pragma unroll
-    for (int k = 0; k < 6; ++k) {
-      w[k] = st.w[0][k];
-      w[6 + k] = st.w[1][k];
-      w[12 + k] = st.w[2][k];
-      ws.ox[lane * 6 + k] = st.ix[k] * d.K1 * d.K2;
-    }
-    if (DERIV) {
-      T* dw = ws.dw + lane * 18;
-#pragma unroll
-      for (int k = 0; k < 6; ++k) {
-        dw[k] = st.dw[0][k];
-        dw[6 + k] = st.dw[1][k];
-        dw[12 + k] = st.dw[2][k];
+      for (int p = 0; p < 6; ++p) {
+        ws.w[l * 18 + 6 * ax + p] = w[p];
+        if (DERIV) ws.dw[l * 18 + 6 * ax + p] = dw[p];
       }
+      if (ax == 0) {
+#pragma unroll
+        for (int p = 0; p < 6; ++p) ws.ox[l * 6 + p] = wrap_up(base + p, n) * d.K1 * d.K2;
+      } else {
+        ws.byz[l * 2 + ax - 1] = base;
+      }
+    } else {
+      ws.q[l] = q ? q[ga] : T(0);
+      ws.atom[l] = ga;
     }
-    ws.byz[lane * 2] = st.iy[0];
-    ws.byz[lane * 2 + 1] = st.iz[0];
-    ws.q[lane] = q ? q[ga] : T(0);
-    ws.atom[lane] = ga;
   }
   __syncwarp();
-}
-
-__device__ __forceinline__ int wrap_up(int i, int K) {
-  while (i >= K) i -= K;
-  return i;
 }
 
 // spread: q -> mesh (zeroed), atomic adds
@@ -267,50 +259,39 @@ __global__ void __launch_bounds__(256) spread_kernel(Batch b, const T* __restric
                                                      const int* __restrict__ order) {
   extern __shared__ __align__(16) unsigned char dsm[];
   __shared__ Geom g;
-  const int s = find_sys<F_ATOM>(b, blockIdx.x);
+  const int s = find_sys<F_ST>(b, blockIdx.x);
   if (skip_sys(b, s)) return;
   const SysDesc& d = b.s[s];  // a register copy would cost this kernel 10 registers
   load_geom(box, d.box_idx, &g);
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int nw = blockDim.x >> 5;
-  const int a_begin = (blockIdx.x - d.blk_atom) * b.apb;
-  const int a_end = min(a_begin + b.apb, d.natoms);
+  const int a0 = (blockIdx.x - b.blk[s]) * b.aps + warp * kPw;  // b.aps: eight atoms for each warp
+  const int na = min(kPw, d.natoms - a0);
   T* M = mesh + d.mesh_off;
   WarpStencil<T, false> ws;
   ws.carve(dsm + warp * WarpStencil<T, false>::bytes());
-  // columns 0..31 of an atom: lane = 6 y + z; the last four columns (y 5, z 2..5) of eight
-  // atoms at once: lane -> atom lane / 4, z 2 + lane % 4
   const int y0 = lane / 6, z0 = lane % 6, jt = lane >> 2, zt = 2 + (lane & 3);
-  for (int a0 = a_begin + warp * 32; a0 < a_end; a0 += nw * 32) {
-    warp_build_stencil<T, false>(ws, d, g, pos, q, order, a0, a_end, lane);
-    const int na = min(32, a_end - a0);
-    for (int j0 = 0; j0 < na; j0 += 8) {
-      const int j1 = min(j0 + 8, na);
-      for (int j = j0; j < j1; ++j) {
-        const T qa = ws.q[j];
-        if (qa == T(0)) continue;
-        const T* w = ws.w + j * 18;
-        const int* ox = ws.ox + j * 6;
-        const T wyz = qa * w[6 + y0] * w[12 + z0];
-        const int oyz = wrap_up(ws.byz[2 * j] + y0, d.K1) * d.K2 + wrap_up(ws.byz[2 * j + 1] + z0, d.K2);
+  warp_build_stencil<T, false>(ws, d, g, pos, q, order, a0, d.natoms, lane);
+  for (int j = 0; j < na; ++j) {
+    const T qa = ws.q[j];
+    if (qa == T(0)) continue;
+    const T* w = ws.w + j * 18;
+    const int* ox = ws.ox + j * 6;
+    const T wyz = qa * w[6 + y0] * w[12 + z0];
+    const int oyz = wrap_up(ws.byz[2 * j] + y0, d.K1) * d.K2 + wrap_up(ws.byz[2 * j + 1] + z0, d.K2);
 #pragma unroll
-        for (int dx = 0; dx < 6; ++dx) atomicAdd(M + ox[dx] + oyz, w[dx] * wyz);
-      }
-      const int j = j0 + jt;
-      if (j < j1) {
-        const T qa = ws.q[j];
-        if (qa != T(0)) {
-          const T* w = ws.w + j * 18;
-          const int* ox = ws.ox + j * 6;
-          const T wyz = qa * w[6 + 5] * w[12 + zt];
-          const int oyz = wrap_up(ws.byz[2 * j] + 5, d.K1) * d.K2 + wrap_up(ws.byz[2 * j + 1] + zt, d.K2);
+    for (int dx = 0; dx < 6; ++dx) atomicAdd(M + ox[dx] + oyz, w[dx] * wyz);
+  }
+  if (jt < na) {
+    const T qa = ws.q[jt];
+    if (qa != T(0)) {
+      const T* w = ws.w + jt * 18;
+      const int* ox = ws.ox + jt * 6;
+      const T wyz = qa * w[6 + 5] * w[12 + zt];
+      const int oyz = wrap_up(ws.byz[2 * jt] + 5, d.K1) * d.K2 + wrap_up(ws.byz[2 * jt + 1] + zt, d.K2);
 #pragma unroll
-          for (int dx = 0; dx < 6; ++dx) atomicAdd(M + ox[dx] + oyz, w[dx] * wyz);
-        }
-      }
+      for (int dx = 0; dx < 6; ++dx) atomicAdd(M + ox[dx] + oyz, w[dx] * wyz);
     }
-    __syncwarp();
   }
 }
 
@@ -394,13 +375,14 @@ __global__ void __launch_bounds__(256) fft_y_kernel(Batch b, Cplx<T>* __restrict
 // ---------------------------------------------------------------------------
 // x pass: forward FFT, Green's function (energy + virial), scale, inverse FFT
 // ---------------------------------------------------------------------------
-template <typename T>
+template <typename T, bool VIRIAL>
 __global__ void __launch_bounds__(256) fft_x_green_kernel(Batch b, Cplx<T>* __restrict__ spec,
                                                           const T* __restrict__ box,
                                                           double* __restrict__ acc, double ke) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ Geom g;
-  __shared__ double red[10 * 32];
+  constexpr int NV = VIRIAL ? 10 : 1;  // energy, and dE/d(box^-1) through the k vectors where it is asked for
+  __shared__ double red[NV * 32];
   const int s = find_sys<F_X>(b, blockIdx.x);
   if (skip_sys(b, s)) return;
   const SysDesc d = b.s[s];
@@ -448,9 +430,9 @@ __global__ void __launch_bounds__(256) fft_x_green_kernel(Batch b, Cplx<T>* __re
   const double kappa = d.kappa;
   const double inv4k2 = 1.0 / (4.0 * kappa * kappa);
   const double pref = ke * 2.0 * kPi / g.vol;
-  double v[10];
+  double v[NV];
 #pragma unroll
-  for (int k = 0; k < 10; ++k) v[k] = 0.0;
+  for (int k = 0; k < NV; ++k) v[k] = 0.0;
   for (int idx = threadIdx.x; idx < K0 * nz; idx += blockDim.x) {
     const int x = fdiv(idx, fdnz), c = idx - x * nz;
     // A half-spectrum entry p stands for p and its mirror pb = -p (mod K); both
@@ -484,20 +466,22 @@ __global__ void __launch_bounds__(256) fft_x_green_kernel(Batch b, Cplx<T>* __re
       Gs += 0.5 * mult * G;
       const double Ek = 0.5 * mult * w * G * s2;
       v[0] += Ek;
-      // dE/dB[a][e] = sum_k E_k (-(1/(4 kappa^2) + 1/k^2)) 2 k_e 2 pi n_a
-      const double f = -4.0 * kPi * (inv4k2 + 1.0 / ksq) * Ek;
-      const double nn[3] = {(double)a0, (double)a1, (double)a2};
+      if constexpr (VIRIAL) {
+        // dE/dB[a][e] = sum_k E_k (-(1/(4 kappa^2) + 1/k^2)) 2 k_e 2 pi n_a
+        const double f = -4.0 * kPi * (inv4k2 + 1.0 / ksq) * Ek;
+        const double nn[3] = {(double)a0, (double)a1, (double)a2};
 #pragma unroll
-      for (int a = 0; a < 3; ++a)
+        for (int a = 0; a < 3; ++a)
 #pragma unroll
-        for (int e = 0; e < 3; ++e) v[1 + a * 3 + e] += f * nn[a] * kv[e];
+          for (int e = 0; e < 3; ++e) v[1 + a * 3 + e] += f * nn[a] * kv[e];
+      }
     }
     // phi = dE/dQ = 2 * IFFT(Gs S)
     S.x = (T)(2.0 * Gs * (double)S.x);
     S.y = (T)(2.0 * Gs * (double)S.y);
     R[x * zb + c] = S;
   }
-  block_atomic_sum<10>(v, acc + (size_t)s * kAccStride + kAccErec, red);
+  block_atomic_sum<NV>(v, acc + (size_t)s * kAccStride + kAccErec, red);
   Cplx<T>* P = fft_lines<T, true, true>(R, F, nz, K0, 1, zb, W);
   for (int idx = threadIdx.x; idx < K0 * nz; idx += blockDim.x) {
     const int x = fdiv(idx, fdnz), c = idx - x * nz;
@@ -803,156 +787,177 @@ __global__ void __launch_bounds__(256) fft_z_inv_kernel(Batch b, const Cplx<T>* 
   }
 }
 
+// Sums of NV values over the warp, all at once: at every step half of a lane's
+// values go to its partner and the partner's other half comes back, so NV sums
+// take NV - 1 shuffles (plus one per remaining step) instead of 5 NV.  Lane l
+// gets the sum of value l >> (5 - log2 NV).
+template <int NV, typename T>
+__device__ __forceinline__ T warp_sum_each(T (&v)[NV], int lane) {
+  int m = 16;
+#pragma unroll
+  for (int h = NV / 2; h >= 1; h >>= 1) {
+    const bool up = (lane & m) != 0;
+#pragma unroll
+    for (int k = 0; k < h; ++k) {
+      const T send = up ? v[k] : v[k + h], keep = up ? v[k + h] : v[k];
+      v[k] = keep + __shfl_xor_sync(0xffffffffu, send, m);
+    }
+    m >>= 1;
+  }
+  T r = v[0];
+  for (; m >= 1; m >>= 1) r += __shfl_xor_sync(0xffffffffu, r, m);
+  return r;
+}
+
 // ---------------------------------------------------------------------------
 // gather: pot_i = sum phi theta; dE/du_d = q sum phi dtheta/du_d (warp-cooperative)
+//
+// The warp's eight atoms go in groups of GU: 6 GU mesh loads are issued before
+// their sums, and the group's sums over the 32 columns are taken together
+// (warp_sum_each).  At the end lane l holds quantity l % 4 (potential, three
+// derivatives) of atom l / 4, so the last four columns need three more
+// shuffles and each lane writes its own component.  VIRIAL: also the
+// fractional-coordinate virial into `acc` (only where dE/dbox is asked for).
+//
+// With a warp sum per atom and quantity (32 atoms a warp) 200 / 3,000 / 20,000 /
+// 192,000 atoms (FP32, forces) took 17.5 / 19.4 / 19.9 / 76.2 us, now 6.2 / 6.2 /
+// 10.3 / 51.6.
 // ---------------------------------------------------------------------------
-template <typename T, bool FORCES>
+template <typename T, bool FORCES, bool VIRIAL>
 __global__ void __launch_bounds__(256) gather_kernel(Batch b, const T* __restrict__ pos,
                                                      const T* __restrict__ box,
                                                      const T* __restrict__ q,
                                                      const T* __restrict__ phi,
                                                      T* __restrict__ dE_dq, T* __restrict__ dE_dpos,
-                                                     double* __restrict__ acc, T pot_scale,
-                                                     const int* __restrict__ order) {
+                                                     double* __restrict__ acc, const int* __restrict__ order) {
   extern __shared__ __align__(16) unsigned char dsm[];
   __shared__ Geom g;
-  __shared__ double red[9 * 32];
-  const int s = find_sys<F_ATOM>(b, blockIdx.x);
+  __shared__ double red[VIRIAL ? 8 : 1][9];
+  const int s = find_sys<F_ST>(b, blockIdx.x);
   if (skip_sys(b, s)) return;
   const SysDesc d = b.s[s];
   load_geom(box, d.box_idx, &g);
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int nw = blockDim.x >> 5;
-  const int a_begin = (blockIdx.x - d.blk_atom) * b.apb;
-  const int a_end = min(a_begin + b.apb, d.natoms);
+  const int a_begin = (blockIdx.x - b.blk[s]) * b.aps, a_end = min(a_begin + b.aps, d.natoms);
   const T* M = phi + d.mesh_off;
-  const int K[3] = {d.K0, d.K1, d.K2};
   WarpStencil<T, FORCES> ws;
   ws.carve(dsm + warp * WarpStencil<T, FORCES>::bytes());
-  // column mapping as in spread_kernel: columns 0..31 per atom, the last four of eight atoms at once
   const int y0 = lane / 6, z0 = lane % 6, jt = lane >> 2, zt = 2 + (lane & 3);
-  double wf[9];
-#pragma unroll
-  for (int k = 0; k < 9; ++k) wf[k] = 0.0;
-  for (int a0 = a_begin + warp * 32; a0 < a_end; a0 += nw * 32) {
+  constexpr int NQ = FORCES ? 4 : 1;                                    // quantities per atom
+  constexpr int GU = (sizeof(T) == 8 ? 2 : 4) * (FORCES ? 1 : 2);       // atoms per group
+  constexpr int kLanes = 32 / (GU * NQ);                                // lanes that share a group sum
+  double wf[3] = {0, 0, 0};  // virial row of this lane's component
+  for (int a0 = a_begin + warp * kPw; a0 < a_end; a0 += (blockDim.x >> 5) * kPw) {
+    const int na = min(kPw, a_end - a0);
     warp_build_stencil<T, FORCES>(ws, d, g, pos, FORCES ? q : nullptr, order, a0, a_end, lane);
-    const int na = min(32, a_end - a0);
-    T my_pot = 0, my_g0 = 0, my_g1 = 0, my_g2 = 0;
-    for (int j0 = 0; j0 < na; j0 += 8) {
-      const int j1 = min(j0 + 8, na);
-      // GU atoms at a time: their 6 GU mesh loads are issued before the first reduction
-      constexpr int GU = sizeof(T) == 8 ? 2 : 4;
-      for (int jb = j0; jb < j1; jb += GU) {
-        T fm[GU][6];
+    T mine = T(0);
 #pragma unroll
-        for (int u = 0; u < GU; ++u) {
-          const int j = jb + u;
-          if (j < j1) {
-            const int* ox = ws.ox + j * 6;
-            const int oyz = wrap_up(ws.byz[2 * j] + y0, d.K1) * d.K2 + wrap_up(ws.byz[2 * j + 1] + z0, d.K2);
+    for (int jb = 0; jb < kPw; jb += GU) {
+      if (jb >= na) break;
+      T fm[GU][6];
 #pragma unroll
-            for (int dx = 0; dx < 6; ++dx) fm[u][dx] = M[ox[dx] + oyz];
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < GU; ++u) {
-          const int j = jb + u;
-          if (j >= j1) break;
-          const T* w = ws.w + j * 18;
-          const T wy = w[6 + y0], wz = w[12 + z0];
-          T sw = 0, sdw = 0;
-#pragma unroll
-          for (int dx = 0; dx < 6; ++dx) {
-            sw += fm[u][dx] * w[dx];
-            if (FORCES) sdw += fm[u][dx] * ws.dw[j * 18 + dx];
-          }
-          T pot = sw * wy * wz, g0 = 0, g1 = 0, g2 = 0;
-          pot = warp_sum(pot);
-          if (FORCES) {
-            g0 = warp_sum(sdw * wy * wz);
-            g1 = warp_sum(sw * ws.dw[j * 18 + 6 + y0] * wz);
-            g2 = warp_sum(sw * wy * ws.dw[j * 18 + 12 + z0]);
-          }
-          if (lane == j) {
-            my_pot = pot;
-            my_g0 = g0;
-            my_g1 = g1;
-            my_g2 = g2;
-          }
-        }
-      }
-      // the last four columns of atoms j0 .. j1-1, reduced over each atom's four lanes
-      T pot = 0, g0 = 0, g1 = 0, g2 = 0;
-      const int j = j0 + jt;
-      if (j < j1) {
-        const T* w = ws.w + j * 18;
+      for (int u = 0; u < GU; ++u) {
+        const int j = min(jb + u, na - 1);
         const int* ox = ws.ox + j * 6;
-        const T wy = w[6 + 5], wz = w[12 + zt];
-        const int oyz = wrap_up(ws.byz[2 * j] + 5, d.K1) * d.K2 + wrap_up(ws.byz[2 * j + 1] + zt, d.K2);
+        const int oyz = wrap_up(ws.byz[2 * j] + y0, d.K1) * d.K2 + wrap_up(ws.byz[2 * j + 1] + z0, d.K2);
+#pragma unroll
+        for (int dx = 0; dx < 6; ++dx) fm[u][dx] = M[ox[dx] + oyz];
+      }
+      T v[GU * NQ];
+#pragma unroll
+      for (int u = 0; u < GU; ++u) {
+        const int j = min(jb + u, na - 1);
+        const T* w = ws.w + j * 18;
+        const T wy = w[6 + y0], wz = w[12 + z0];
         T sw = 0, sdw = 0;
 #pragma unroll
         for (int dx = 0; dx < 6; ++dx) {
-          const T f = M[ox[dx] + oyz];
-          sw += f * w[dx];
-          if (FORCES) sdw += f * ws.dw[j * 18 + dx];
+          sw += fm[u][dx] * w[dx];
+          if (FORCES) sdw += fm[u][dx] * ws.dw[j * 18 + dx];
         }
-        pot = sw * wy * wz;
+        v[u * NQ] = sw * wy * wz;
         if (FORCES) {
-          g0 = sdw * wy * wz;
-          g1 = sw * ws.dw[j * 18 + 6 + 5] * wz;
-          g2 = sw * wy * ws.dw[j * 18 + 12 + zt];
+          v[u * NQ + 1] = sdw * wy * wz;
+          v[u * NQ + 2] = sw * ws.dw[j * 18 + 6 + y0] * wz;
+          v[u * NQ + 3] = sw * wy * ws.dw[j * 18 + 12 + z0];
         }
       }
+      const T sum = warp_sum_each<GU * NQ>(v, lane);
+      // to the lanes of the group's atoms: lane l takes quantity l % 4 of atom l / 4
+      const int want = FORCES ? lane - 4 * jb : jt - jb;
+      const T got = __shfl_sync(0xffffffffu, sum, (want * kLanes) & 31);
+      if (want >= 0 && want < GU * NQ) mine = got;
+    }
+    // the last four columns of atom lane / 4
+    T left[NQ] = {};
+    if (jt < na) {
+      const T* w = ws.w + jt * 18;
+      const int* ox = ws.ox + jt * 6;
+      const T wy = w[6 + 5], wz = w[12 + zt];
+      const int oyz = wrap_up(ws.byz[2 * jt] + 5, d.K1) * d.K2 + wrap_up(ws.byz[2 * jt + 1] + zt, d.K2);
+      T sw = 0, sdw = 0;
 #pragma unroll
-      for (int o = 1; o < 4; o <<= 1) {
-        pot += __shfl_xor_sync(0xffffffffu, pot, o);
-        if (FORCES) {
-          g0 += __shfl_xor_sync(0xffffffffu, g0, o);
-          g1 += __shfl_xor_sync(0xffffffffu, g1, o);
-          g2 += __shfl_xor_sync(0xffffffffu, g2, o);
-        }
+      for (int dx = 0; dx < 6; ++dx) {
+        const T f = M[ox[dx] + oyz];
+        sw += f * w[dx];
+        if (FORCES) sdw += f * ws.dw[jt * 18 + dx];
       }
-      // lane j0 + k takes the sums of atom j0 + k from lane 4 k
-      const int src = 4 * ((lane - j0) & 7);
-      pot = __shfl_sync(0xffffffffu, pot, src);
-      if (FORCES) {
-        g0 = __shfl_sync(0xffffffffu, g0, src);
-        g1 = __shfl_sync(0xffffffffu, g1, src);
-        g2 = __shfl_sync(0xffffffffu, g2, src);
-      }
-      if (lane >= j0 && lane < j1) {
-        my_pot += pot;
-        my_g0 += g0;
-        my_g1 += g1;
-        my_g2 += g2;
+      left[0] = sw * wy * wz;
+      if constexpr (FORCES) {
+        left[1] = sdw * wy * wz;
+        left[2] = sw * ws.dw[jt * 18 + 6 + 5] * wz;
+        left[3] = sw * wy * ws.dw[jt * 18 + 12 + zt];
       }
     }
-    if (lane < na) {
-      const int ga = ws.atom[lane];
-      if (dE_dq) dE_dq[ga] += my_pot * pot_scale;
-      if (FORCES) {
-        const T qa = ws.q[lane];
-        // u = m0 - x + 3  ->  dE/dx_d = -q * dE/du_d ; x_d = K_d (r @ B)_d
-        const double gx[3] = {-(double)qa * my_g0 * K[0], -(double)qa * my_g1 * K[1], -(double)qa * my_g2 * K[2]};
-        if (dE_dpos) {
+    if constexpr (!FORCES) {
+      left[0] += __shfl_xor_sync(0xffffffffu, left[0], 1);
+      left[0] += __shfl_xor_sync(0xffffffffu, left[0], 2);
+      if (jt < na && (lane & 3) == 0 && dE_dq) dE_dq[ws.atom[jt]] += mine + left[0];
+    } else {
+      // four quantities over four lanes: lane c of the four ends with quantity c
+      const bool hi = (lane & 2) != 0, od = (lane & 1) != 0;
+      const T s0 = hi ? left[0] : left[2], s1 = hi ? left[1] : left[3];
+      const T k0 = (hi ? left[2] : left[0]) + __shfl_xor_sync(0xffffffffu, s0, 2);
+      const T k1 = (hi ? left[3] : left[1]) + __shfl_xor_sync(0xffffffffu, s1, 2);
+      mine += (od ? k1 : k0) + __shfl_xor_sync(0xffffffffu, od ? k0 : k1, 1);
+      const bool live = jt < na;
+      const int c = lane & 3, ga = live ? ws.atom[jt] : 0;
+      if (live && c == 0 && dE_dq) dE_dq[ga] += mine;
+      // u = m0 - x + 3  ->  dE/dx_d = -q * dE/du_d ; x_d = K_d (r @ B)_d
+      const int Kc = c == 1 ? d.K0 : c == 2 ? d.K1 : d.K2;
+      const double gc = live ? -(double)ws.q[jt] * mine * Kc : 0.0;
+      double gx[3];
 #pragma unroll
-          for (int e = 0; e < 3; ++e) {
-            const double v = gx[0] * g.binv[e * 3 + 0] + gx[1] * g.binv[e * 3 + 1] + gx[2] * g.binv[e * 3 + 2];
-            dE_dpos[3 * (size_t)ga + e] += (T)v;
-          }
-        }
-        const double r[3] = {(double)pos[3 * (size_t)ga], (double)pos[3 * (size_t)ga + 1],
-                             (double)pos[3 * (size_t)ga + 2]};
+      for (int e = 0; e < 3; ++e) gx[e] = __shfl_sync(0xffffffffu, gc, (lane & ~3) + 1 + e);
+      if (live && c && dE_dpos) {
+        const int e = c - 1;
+        const double f = gx[0] * g.binv[e * 3 + 0] + gx[1] * g.binv[e * 3 + 1] + gx[2] * g.binv[e * 3 + 2];
+        dE_dpos[3 * (size_t)ga + e] += (T)f;
+      }
+      if constexpr (VIRIAL) {
+        // lanes of component e: row e of sum r_e gx_c
+        const double r = live && c ? (double)pos[3 * (size_t)ga + c - 1] : 0.0;
 #pragma unroll
-        for (int e = 0; e < 3; ++e)
-#pragma unroll
-          for (int c = 0; c < 3; ++c) wf[e * 3 + c] += r[e] * gx[c];
+        for (int k = 0; k < 3; ++k) wf[k] += r * gx[k];
       }
     }
     __syncwarp();
   }
-  if (FORCES) block_atomic_sum<9>(wf, acc + (size_t)s * kAccStride + kAccWf, red);
+  if constexpr (VIRIAL) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+#pragma unroll
+      for (int m = 4; m < 32; m <<= 1) wf[k] += __shfl_xor_sync(0xffffffffu, wf[k], m);
+      if (lane >= 1 && lane < 4) red[warp][(lane - 1) * 3 + k] = wf[k];
+    }
+    __syncthreads();
+    if (threadIdx.x < 9) {
+      double t = 0.0;
+      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w][threadIdx.x];
+      if (t != 0.0) atomicAdd(acc + (size_t)s * kAccStride + kAccWf + threadIdx.x, t);
+    }
+  }
 }
 
 // ---------------------------------------------------------------------------

@@ -63,7 +63,7 @@ static int pme_recip_impl(int nf, int N, const int* kmesh, const T* pos, const T
     ADMP_CUDA_TRY(cudaMemsetAsync(acc, 0, sizeof(double) * ns * kAccStride, st));
     const size_t ao = (size_t)c0 * N;
     s = launch_recip<T>(p, pos + ao * 3, box + (size_t)c0 * 9, q + ao, mesh, spec, acc, ke, dq ? dq + ao : nullptr,
-                        dpos ? dpos + ao * 3 : nullptr, st);
+                        dpos ? dpos + ao * 3 : nullptr, st, dbox != nullptr);
     if (s) return s;
     recip_finalize_kernel<T><<<(ns + 127) / 128, 128, 0, st>>>(p.b, box + (size_t)c0 * 9, acc,
                                                                energy ? energy + c0 : nullptr,

@@ -208,7 +208,7 @@ static int serve_ef_impl(const admp_pools* P, const admp_sys* sys, int nsys, dou
   count_launches(6);
   ADMP_CUDA_TRY(cudaMemsetAsync(P->acc, 0, sizeof(double) * kAccStride * nsys, st));
   s = launch_recip<T>(plan, (const T*)P->pos, (const T*)P->box, (const T*)P->q, (T*)P->mesh, (Cplx<T>*)P->spec,
-                      P->acc, ke, nullptr, (T*)P->force, st, P->sorted);
+                      P->acc, ke, nullptr, (T*)P->force, st, false, P->sorted);
   if (s) return s;
   recip_finalize_kernel<T><<<(nsys + 127) / 128, 128, 0, st>>>(b, (const T*)P->box, P->acc, P->energy, nullptr);
   sys_terms_kernel<T><<<nsys, 512, 0, st>>>(b, ss, (const T*)P->q, (const T*)P->chi, (const T*)P->hardness,

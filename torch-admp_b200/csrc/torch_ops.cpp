@@ -92,7 +92,7 @@ class CoulombPBC : public torch::autograd::Function<CoulombPBC> {
     Tensor gpos, gbox, gds, gq;
     if (need) {
       gpos = torch::zeros_like(pos);
-      gbox = torch::zeros_like(box);
+      if (box.requires_grad()) gbox = torch::zeros_like(box);
       gds = torch::zeros_like(ds);
       gq = torch::zeros_like(q);
     }
@@ -135,7 +135,7 @@ class CoulombPBC : public torch::autograd::Function<CoulombPBC> {
     if (gE.defined() && s[3].defined()) {
       const Tensor w = gE.to(s[3].scalar_type());
       out_pos = s[0] * w.view({-1, 1, 1});
-      out_box = s[1] * w.view({-1, 1, 1});
+      if (s[1].defined()) out_box = s[1] * w.view({-1, 1, 1});
       out_ds = s[2] * w.view({-1, 1});
       out_q = s[3] * w.view({-1, 1});
     }
