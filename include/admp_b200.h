@@ -150,6 +150,26 @@ int admp_atom_terms(int dtype, int flags, int nframes, int natoms, const void* p
                     void* stream);
 
 /* ------------------------------------------------------------------------ */
+/* The whole Coulomb energy of nframes periodic systems (pme.py:261-310):    */
+/* real-space sum over the pairs (flag ADMP_QEQ_RSPACE), reciprocal part      */
+/* (ADMP_QEQ_KSPACE, required), self, non-neutral and (ADMP_QEQ_SLAB, axis in */
+/* bits 8..9) slab terms.  Unlike the entry points above, outputs are         */
+/* WRITTEN: energy [nframes] dtype, comps [nframes, 5] double (real,          */
+/* reciprocal, self, non-neutral, slab) and, where not NULL, the gradients    */
+/* (dE_dbox without the part that flows through ds).  Workspace as            */
+/* admp_pme_recip.  Waits for the pair kernel only (bad pair indices).        */
+/* ------------------------------------------------------------------------ */
+int admp_coulomb_pbc(int dtype, int flags, int nframes, int natoms, const int* kmesh,
+                     const void* pos, const void* box, long long npairs, const long long* pairs,
+                     const void* ds, const void* buffer_scales, const void* q, double kappa,
+                     double ke, void* energy, double* comps, void* dE_dpos, void* dE_dq,
+                     void* dE_dbox, void* dE_dds, void* workspace, size_t workspace_bytes,
+                     void* stream);
+/* Copies up to 64 KiB of device memory to `host` through page-locked staging */
+/* and waits for it.                                                          */
+int admp_read_back(const void* dev, size_t bytes, void* host, void* stream);
+
+/* ------------------------------------------------------------------------ */
 /* Pair distances ds = |pbc_shift(r_i - r_j)| (nblist.py:517-551,            */
 /* spatial.py:15-36) or |r_j - r_i| without a box (pbc = 0), and their       */
 /* backward (gradient of a loss w.r.t. positions and box given dL/dds).       */
@@ -159,6 +179,15 @@ int admp_pair_distances(int dtype, int pbc, int natoms, long long npairs, const 
 int admp_pair_distances_backward(int dtype, int pbc, int natoms, long long npairs,
                                  const long long* pairs, const void* pos, const void* box,
                                  const void* grad_ds, void* grad_pos, void* grad_box, void* stream);
+
+/* The backward over nframes frames of one atom count (pairs [nframes,       */
+/* npairs, 2] with frame-local indices); rows with i == j contribute nothing. */
+/* It does not wait for the device: a bad index is skipped and left in the    */
+/* error word for the next checked call or admp_check_errors.                 */
+int admp_pair_distances_frames_backward(int dtype, int pbc, int nframes, int natoms,
+                                        long long npairs, const long long* pairs, const void* pos,
+                                        const void* box, const void* grad_ds, void* grad_pos,
+                                        void* grad_box, void* stream);
 
 /* ------------------------------------------------------------------------ */
 /* Cell-list neighbour list: TorchNeighborList.forward (nblist.py:304-445,   */
@@ -176,6 +205,21 @@ int admp_nblist_count(int dtype, int pbc, int natoms, const void* pos, const voi
 int admp_nblist_fill(int dtype, int pbc, int natoms, const void* pos, const void* box,
                      double cutoff, void* workspace, size_t workspace_bytes, long long* pairs,
                      long long* buffer_scales, long long capacity, void* stream);
+/* The same over nframes (at most ADMP_NBLIST_MAX_FRAMES) frames of one atom  */
+/* count: npairs is HOST [nframes]; the fill writes slices of `stride` rows   */
+/* (at least the longest frame's count) to pairs [nframes, stride, 2],        */
+/* buffer_scales [nframes, stride] and, if given, the pair distances ds       */
+/* [nframes, stride]; rows past a frame's own pairs are (0, 0), scale 0,      */
+/* distance 1.  It does not wait for the device.                              */
+#define ADMP_NBLIST_MAX_FRAMES 4096
+size_t admp_nblist_frames_workspace_size(int nframes, int natoms);
+int admp_nblist_frames_count(int dtype, int pbc, int nframes, int natoms, const void* pos,
+                             const void* box, double cutoff, void* workspace,
+                             size_t workspace_bytes, long long* npairs, void* stream);
+int admp_nblist_frames_fill(int dtype, int pbc, int nframes, int natoms, const void* pos,
+                            double cutoff, void* workspace, size_t workspace_bytes,
+                            long long stride, long long* pairs, long long* buffer_scales, void* ds,
+                            void* stream);
 
 /* ------------------------------------------------------------------------ */
 /* Neighbour list over periodic images for any cutoff, including rc above   */

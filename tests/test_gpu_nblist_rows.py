@@ -83,3 +83,36 @@ def test_nonfinite_position_is_refused_and_the_next_call_runs(cuda):
     with pytest.raises(L.AdmpError):
         TorchNeighborList(5.0)(bad, box)
     assert TorchNeighborList(5.0)(pos, box).shape[0] > 0
+
+
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+@pytest.mark.parametrize("n", [1, 40, 8300])
+def test_frames_equal_single_lists(cuda, n, dtype):
+    """Frames with different pair counts (different boxes) against one list per
+    frame: rows, padding, distances and their gradients."""
+    from admp_b200.nblist import TorchNeighborList, frame_pair_lists
+    rng = np.random.default_rng(n)
+    sizes = [13.0, 15.0, 14.0] if n < 8000 else [44.0, 46.0, 45.0]
+    box = T(np.stack([np.diag([s] * 3) + np.array([[0, 0, 0], [0.3, 0, 0], [0, 0.2, 0]]) for s in sizes]), cuda, dtype,
+            grad=True)
+    pos = T(rng.random((3, n, 3)) * 40.0, cuda, dtype, grad=True)
+    pairs, ds, bs = frame_pair_lists(pos, box, 5.0)
+    w = torch.linspace(0.5, 1.5, max(ds.shape[1], 1), dtype=dtype, device=cuda)[:ds.shape[1]]
+    gpos, gbox = torch.autograd.grad((ds * w).sum(), [pos, box])
+    counts = []
+    for f in range(3):
+        nb = TorchNeighborList(5.0)
+        p1, b1 = pos[f].detach().requires_grad_(True), box[f].detach().requires_grad_(True)
+        one = nb(p1, b1)
+        k = one.shape[0]
+        counts.append(k)
+        assert torch.equal(pairs[f, :k], one) and torch.equal(bs[f, :k], nb.get_buffer_scales())
+        assert torch.equal(ds[f, :k], nb.get_ds())
+        assert not pairs[f, k:].any() and not bs[f, k:].any() and bool((ds[f, k:] == 1).all())
+        if k:
+            g1, g2 = torch.autograd.grad((nb.get_ds() * w[:k]).sum(), [p1, b1])
+            # the same terms summed by atomics in another order: 1e-15 (FP64) / 1e-6 (FP32) of ~100 terms
+            tol = 1e-12 if dtype == torch.float64 else 1e-4
+            assert float((gpos[f] - g1).abs().max()) < tol * max(1.0, float(g1.abs().max()))
+            assert float((gbox[f] - g2).abs().max()) < tol * max(1.0, float(g2.abs().max()))
+    assert pairs.shape[1] == max(counts)

@@ -17,7 +17,10 @@ from typing import Optional
 import torch
 
 from . import _lib as L
-from .ops import ImagePairDistanceFn, PairDistanceFn, image_neighbor_pairs, neighbor_pairs
+from .ops import ImagePairDistanceFn, PairDistanceFn, image_neighbor_pairs
+
+L.load_torch_ops()  # torch.ops.admp_b200.neighbor_list
+_MAX_FRAMES = 4096  # frames per call of the frame lists
 
 
 def check_cutoff(box: torch.Tensor, cutoff: float) -> None:
@@ -42,16 +45,15 @@ class TorchNeighborList(torch.nn.Module):
 
     def forward(self, positions: torch.Tensor, box: Optional[torch.Tensor] = None) -> torch.Tensor:
         L.require_cuda(positions, "positions")
-        pos_c = positions.detach().contiguous()
-        box_c = box.detach().to(positions.dtype).contiguous() if box is not None else None
-        try:
-            pairs, bs = neighbor_pairs(pos_c, box_c, self.cutoff)
-        except AssertionError:
+        L.dtype_code(positions.dtype)
+        b = box.to(positions.dtype) if box is not None else None
+        status, pairs, bs, ds = torch.ops.admp_b200.neighbor_list(positions, b, float(self.cutoff), 1)
+        if status == L.CUTOFF:
             check_cutoff(box, self.cutoff)
-            raise
+        L.check(status, "neighbour list")
         self.pairs = pairs
         self.buffer_scales = bs
-        self.ds = self.pairs_ds(positions, pairs, box, box is not None)
+        self.ds = ds
         return pairs
 
     @staticmethod
@@ -145,17 +147,26 @@ def frame_pair_lists(positions: torch.Tensor, box: torch.Tensor, cutoff: float):
     respect to positions [nf, N, 3] and box [nf, 3, 3]) and buffer_scales
     [nf, P], with P the longest frame's list; the rows past a frame's own
     pairs hold (0, 0) with distance 1 and scale 0, which every kernel skips."""
-    nf = positions.shape[0]
-    lists = []
-    for f in range(nf):
-        nb = TorchNeighborList(cutoff)
-        pr = nb(positions[f], box[f])
-        lists.append((pr, nb.get_ds(), nb.get_buffer_scales()))
-    P = max(int(p.shape[0]) for p, _, _ in lists)
-    pairs, ds, bs = [], [], []
-    for pr, d, s in lists:
-        pad = P - int(pr.shape[0])
-        pairs.append(torch.cat([pr, pr.new_zeros(pad, 2)]))
-        ds.append(torch.cat([d, d.new_ones(pad)]))
-        bs.append(torch.cat([s, s.new_zeros(pad)]))
-    return torch.stack(pairs), torch.stack(ds), torch.stack(bs)
+    nf, na = positions.shape[0], positions.shape[1]
+    L.require_cuda(positions, "positions")
+    L.dtype_code(positions.dtype)
+    if nf == 0:
+        raise ValueError("frame_pair_lists needs at least one frame")
+    b = box.to(positions.dtype)
+    parts = []
+    for f0 in range(0, nf, _MAX_FRAMES):
+        n = min(_MAX_FRAMES, nf - f0)
+        status, *rows = torch.ops.admp_b200.neighbor_list(positions[f0:f0 + n].reshape(n * na, 3), b[f0:f0 + n],
+                                                          float(cutoff), n)
+        if status == L.CUTOFF:
+            for f in range(f0, f0 + n):
+                check_cutoff(box[f], cutoff)
+        L.check(status, "neighbour list")
+        P = rows[0].shape[0] // n
+        parts.append((rows[0].reshape(n, P, 2), rows[1].reshape(n, P), rows[2].reshape(n, P)))
+    if len(parts) == 1:
+        return parts[0][0], parts[0][2], parts[0][1]
+    P = max(p.shape[1] for p, _, _ in parts)
+    pad = lambda t, v: torch.cat([t, t.new_full((t.shape[0], P - t.shape[1]) + t.shape[2:], v)], 1)  # noqa: E731
+    return (torch.cat([pad(p, 0) for p, _, _ in parts]), torch.cat([pad(d, 1) for _, _, d in parts]),
+            torch.cat([pad(s, 0) for _, s, _ in parts]))

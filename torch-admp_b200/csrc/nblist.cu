@@ -557,16 +557,31 @@ __device__ __forceinline__ void nb_order(const int* row, int n, int* out) {
 struct NbOut {
   long long* pairs;
   long long* bscale;
+  void* ds;            // distances in the positions' type, or null
   long long stride;    // rows of one frame's slice
   long long cap;       // rows that may be written in it
 };
 
 // Filling pass: a warp per atom orders its neighbours by index (bitonic sort
 // in registers: about 260 instructions for 128 values, against 900 for ranking
-// each value against all others) and writes the row, whole and coalesced.
-static __global__ void __launch_bounds__(256) nb_fill_kernel(int pbc, int N, int mc, double rc, NbWS w0, NbOut o) {
+// each value against all others) and writes the row, whole and coalesced, with
+// the pair distances (admp_pair_distances) if they are asked for.  The rows of
+// a frame's slice past its own pairs become (0, 0), distance 1, scale 0.
+template <typename T>
+__global__ void __launch_bounds__(256) nb_fill_kernel(int pbc, int N, int mc, double rc, NbWS w0,
+                                                      const T* __restrict__ pos, NbOut o) {
   __shared__ __align__(16) int ord_sh[8][kNbRow];
   const int f = blockIdx.y;
+  if (o.stride) {
+    const NbResult* r = w0.res + f;
+    for (long long k = r->npairs + blockIdx.x * (long long)blockDim.x + threadIdx.x; k < o.stride;
+         k += (long long)gridDim.x * blockDim.x) {
+      const size_t p = (size_t)f * o.stride + k;
+      reinterpret_cast<longlong2*>(o.pairs)[p] = make_longlong2(0, 0);
+      if (o.bscale) o.bscale[p] = 0;
+      if (o.ds) reinterpret_cast<T*>(o.ds)[p] = T(1);
+    }
+  }
   const NbWS w = nb_frame(w0, f, N, mc);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int at = blockIdx.x * (blockDim.x >> 5) + warp;
@@ -576,9 +591,20 @@ static __global__ void __launch_bounds__(256) nb_fill_kernel(int pbc, int N, int
   if (n == 0 || base + n > o.cap) return;
   const size_t out = (size_t)f * o.stride + base;
   int* ord = ord_sh[warp];
+  const NbMeta* __restrict__ m = w.meta;
+  const T* ps = o.ds ? pos + (size_t)f * N * 3 : nullptr;
+  double ri[3] = {0.0, 0.0, 0.0};
+  if (o.ds)
+    for (int e = 0; e < 3; ++e) ri[e] = (double)ps[3 * (size_t)i + e];
   auto emit = [&](int k, int j) {
     reinterpret_cast<longlong2*>(o.pairs)[out + k] = make_longlong2(i, j);
     if (o.bscale) o.bscale[out + k] = i < j ? 1 : 0;
+    if (o.ds) {
+      double dr[3], n[3];
+      for (int e = 0; e < 3; ++e) dr[e] = ri[e] - (double)ps[3 * (size_t)j + e];
+      if (pbc) min_image(m->b, m->bi, dr, n);
+      reinterpret_cast<T*>(o.ds)[out + k] = (T)sqrt(dr[0] * dr[0] + dr[1] * dr[1] + dr[2] * dr[2]);
+    }
   };
   if (n <= kNbRow) {
     const int* row = w.kept + (size_t)at * kNbKeep;
@@ -672,8 +698,10 @@ static int nblist_count_impl(int pbc, int nf, int N, const T* pos, const T* box,
   return ecode ? check_error(err, st) : ADMP_OK;
 }
 
-static int nblist_fill_impl(int pbc, int nf, int N, double rc, const NbWS& w, const NbOut& o, cudaStream_t st) {
-  nb_fill_kernel<<<dim3((N + 7) / 8, nf), 256, 0, st>>>(pbc, N, max_cells(N), rc, w, o);
+template <typename T>
+static int nblist_fill_impl(int pbc, int nf, int N, double rc, const NbWS& w, const T* pos, const NbOut& o,
+                            cudaStream_t st) {
+  nb_fill_kernel<T><<<dim3((N + 7) / 8, nf), 256, 0, st>>>(pbc, N, max_cells(N), rc, w, pos, o);
   ADMP_CUDA_TRY(cudaGetLastError());
   return ADMP_OK;
 }
@@ -688,19 +716,50 @@ extern "C" size_t admp_nblist_workspace_size(int natoms) {
   return need;
 }
 
-extern "C" int admp_nblist_count(int dtype, int pbc, int natoms, const void* pos, const void* box, double cutoff,
-                                 void* workspace, size_t workspace_bytes, long long* npairs, void* stream) {
+extern "C" size_t admp_nblist_frames_workspace_size(int nframes, int natoms) {
+  size_t need;
+  carve_nb(nullptr, 0, nframes < 0 ? 0 : nframes, natoms < 0 ? 0 : natoms, &need);
+  return need;
+}
+
+extern "C" int admp_nblist_frames_count(int dtype, int pbc, int nframes, int natoms, const void* pos, const void* box,
+                                        double cutoff, void* workspace, size_t workspace_bytes, long long* npairs,
+                                        void* stream) {
   if (!npairs) return fail(ADMP_ERR_BAD_ARG, "npairs is null");
-  *npairs = 0;
-  if (natoms == 0) return ADMP_OK;
+  if (nframes < 0 || nframes > ADMP_NBLIST_MAX_FRAMES)
+    return fail(ADMP_ERR_BAD_ARG, "admp_nblist_count: %d frames (0..%d)", nframes, ADMP_NBLIST_MAX_FRAMES);
+  for (int f = 0; f < nframes; ++f) npairs[f] = 0;
+  if (natoms == 0 || nframes == 0) return ADMP_OK;
   if (natoms < 0 || !pos || (pbc && !box) || !(cutoff > 0)) return fail(ADMP_ERR_BAD_ARG, "admp_nblist_count: args");
   cudaStream_t st = (cudaStream_t)stream;
   if (dtype == ADMP_F64)
-    return nblist_count_impl<double>(pbc, 1, natoms, (const double*)pos, (const double*)box, cutoff, workspace,
+    return nblist_count_impl<double>(pbc, nframes, natoms, (const double*)pos, (const double*)box, cutoff, workspace,
                                      workspace_bytes, npairs, st);
   if (dtype == ADMP_F32)
-    return nblist_count_impl<float>(pbc, 1, natoms, (const float*)pos, (const float*)box, cutoff, workspace,
+    return nblist_count_impl<float>(pbc, nframes, natoms, (const float*)pos, (const float*)box, cutoff, workspace,
                                     workspace_bytes, npairs, st);
+  return fail(ADMP_ERR_BAD_ARG, "bad dtype");
+}
+
+extern "C" int admp_nblist_count(int dtype, int pbc, int natoms, const void* pos, const void* box, double cutoff,
+                                 void* workspace, size_t workspace_bytes, long long* npairs, void* stream) {
+  return admp_nblist_frames_count(dtype, pbc, 1, natoms, pos, box, cutoff, workspace, workspace_bytes, npairs, stream);
+}
+
+extern "C" int admp_nblist_frames_fill(int dtype, int pbc, int nframes, int natoms, const void* pos, double cutoff,
+                                       void* workspace, size_t workspace_bytes, long long stride, long long* pairs,
+                                       long long* buffer_scales, void* ds, void* stream) {
+  if (nframes < 0 || nframes > ADMP_NBLIST_MAX_FRAMES || natoms < 0 || stride < 0)
+    return fail(ADMP_ERR_BAD_ARG, "admp_nblist_frames_fill: args");
+  if (natoms == 0 || nframes == 0 || stride == 0) return ADMP_OK;
+  if (!pos || !pairs) return fail(ADMP_ERR_BAD_ARG, "admp_nblist_frames_fill: args");
+  size_t need;
+  const NbWS w = carve_nb(workspace, workspace_bytes, nframes, natoms, &need);
+  if (need > workspace_bytes || !workspace) return fail(ADMP_ERR_WORKSPACE, "nblist workspace too small");
+  const NbOut o{pairs, buffer_scales, ds, stride, stride};
+  cudaStream_t st = (cudaStream_t)stream;
+  if (dtype == ADMP_F64) return nblist_fill_impl<double>(pbc, nframes, natoms, cutoff, w, (const double*)pos, o, st);
+  if (dtype == ADMP_F32) return nblist_fill_impl<float>(pbc, nframes, natoms, cutoff, w, (const float*)pos, o, st);
   return fail(ADMP_ERR_BAD_ARG, "bad dtype");
 }
 
@@ -722,5 +781,6 @@ extern "C" int admp_nblist_fill(int dtype, int pbc, int natoms, const void* pos,
   if (total > capacity)
     return fail(ADMP_ERR_CAPACITY, "neighbour list: %lld pairs exceed capacity %lld", total, capacity);
   if (total == 0) return ADMP_OK;
-  return nblist_fill_impl(pbc, 1, natoms, cutoff, w, NbOut{pairs, buffer_scales, 0, capacity}, st);
+  return nblist_fill_impl<double>(pbc, 1, natoms, cutoff, w, nullptr, NbOut{pairs, buffer_scales, nullptr, 0, capacity},
+                                  st);
 }

@@ -5,7 +5,7 @@
 //                         qeq.py:121-126 (damping self), qeq.py:159-209 (site)
 //   admp_pair_distances   nblist.py:517-551 with spatial.py:15-36
 #include "admp_common.cuh"
-#include "runtime.h"
+#include "pair_terms.h"
 
 namespace admp {
 
@@ -13,8 +13,8 @@ template <typename T, int MODE>
 __global__ void __launch_bounds__(256)
     pair_list_kernel(int N, long long P, const long long* __restrict__ pairs, const T* __restrict__ ds,
                      const T* __restrict__ bs, const T* __restrict__ q, const T* __restrict__ eta, T kappa,
-                     T ke, double* __restrict__ energy, T* __restrict__ dE_dds, T* __restrict__ dE_dq,
-                     T* __restrict__ dE_deta, DevError* err) {
+                     T ke, double* __restrict__ energy, int estride, int put, T* __restrict__ dE_dds,
+                     T* __restrict__ dE_dq, T* __restrict__ dE_deta, DevError* err) {
   __shared__ double red[32];
   const int f = blockIdx.y;
   pairs += (size_t)f * P * 2;
@@ -32,6 +32,7 @@ __global__ void __launch_bounds__(256)
     const long long i = pairs[2 * p], j = pairs[2 * p + 1];
     if (i < 0 || i >= N || j < 0 || j >= N) {
       report_error(err, ADMP_ERR_BAD_INDEX, 1, p);
+      if (put && dE_dds) dE_dds[p] = T(0);
       continue;
     }
     const T d = ds[p], s = bs[p];
@@ -68,14 +69,14 @@ __global__ void __launch_bounds__(256)
       }
     }
     e += (double)ep;
-    if (dE_dds) dE_dds[p] += dd;
+    if (dE_dds) dE_dds[p] = put ? dd : dE_dds[p] + dd;
     if (dE_dq && c != T(0)) {
       atomicAdd(dE_dq + i, c * qj);
       atomicAdd(dE_dq + j, c * qi);
     }
   }
   double v[1] = {e};
-  if (energy) block_atomic_sum<1>(v, energy + f, red);
+  if (energy) block_atomic_sum<1>(v, energy + (size_t)f * estride, red);
 }
 
 template <typename T>
@@ -227,6 +228,13 @@ __global__ void __launch_bounds__(256)
                          T* __restrict__ gpos, T* __restrict__ gbox, DevError* err) {
   __shared__ double geo[18];
   __shared__ double red[9 * 32];
+  const int f = blockIdx.y;
+  pairs += (size_t)f * P * 2;
+  g += (size_t)f * P;
+  pos += (size_t)f * N * 3;
+  if (box) box += (size_t)f * 9;
+  if (gpos) gpos += (size_t)f * N * 3;
+  if (gbox) gbox += (size_t)f * 9;
   if (threadIdx.x == 0 && pbc) {
     load_box(box, geo);
     inv3(geo, geo + 9);
@@ -273,6 +281,30 @@ __global__ void __launch_bounds__(256)
 }
 
 // ------------------------------------------------------------------ host side
+// energy[f estride] += E of frame f; dE/dds is added to, or with `put` written.
+template <typename T>
+int launch_pair_energy(int mode, int nf, int N, long long P, const long long* pairs, const T* ds, const T* bs,
+                       const T* q, const T* eta, double kappa, double ke, double* energy, int estride, bool put, T* dds,
+                       T* dq, T* deta, DevError* err, cudaStream_t st) {
+  if (P == 0 || nf == 0) return ADMP_OK;
+  long long blocks = (P + 255) / 256;
+  if (blocks > 4096) blocks = 4096;
+  const dim3 grid((unsigned)blocks, (unsigned)nf);
+  auto* k = mode == ADMP_PAIR_EWALD ? pair_list_kernel<T, ADMP_PAIR_EWALD>
+            : mode == ADMP_PAIR_OBC ? pair_list_kernel<T, ADMP_PAIR_OBC>
+                                    : pair_list_kernel<T, ADMP_PAIR_DAMPING>;
+  k<<<grid, 256, 0, st>>>(N, P, pairs, ds, bs, q, eta, (T)kappa, (T)ke, energy, estride, put ? 1 : 0, dds, dq, deta,
+                          err);
+  ADMP_CUDA_TRY(cudaGetLastError());
+  return ADMP_OK;
+}
+template int launch_pair_energy<float>(int, int, int, long long, const long long*, const float*, const float*,
+                                       const float*, const float*, double, double, double*, int, bool, float*, float*,
+                                       float*, DevError*, cudaStream_t);
+template int launch_pair_energy<double>(int, int, int, long long, const long long*, const double*, const double*,
+                                        const double*, const double*, double, double, double*, int, bool, double*,
+                                        double*, double*, DevError*, cudaStream_t);
+
 template <typename T>
 static int pair_energy_impl(int mode, int nf, int N, long long P, const long long* pairs, const void* ds,
                             const void* bs, const void* q, const void* eta, double kappa, double ke,
@@ -280,28 +312,9 @@ static int pair_energy_impl(int mode, int nf, int N, long long P, const long lon
   if (P == 0 || nf == 0) return ADMP_OK;
   DevError* err = scratch_error(st);
   if (!err) return ADMP_ERR_CUDA;
-  long long blocks = (P + 255) / 256;
-  if (blocks > 4096) blocks = 4096;
-  dim3 grid((unsigned)blocks, (unsigned)nf);
-  const T* tds = (const T*)ds;
-  const T* tbs = (const T*)bs;
-  const T* tq = (const T*)q;
-  const T* te = (const T*)eta;
-  switch (mode) {
-    case ADMP_PAIR_EWALD:
-      pair_list_kernel<T, ADMP_PAIR_EWALD><<<grid, 256, 0, st>>>(N, P, pairs, tds, tbs, tq, te, (T)kappa, (T)ke,
-                                                                  energy, (T*)dds, (T*)dq, (T*)deta, err);
-      break;
-    case ADMP_PAIR_OBC:
-      pair_list_kernel<T, ADMP_PAIR_OBC><<<grid, 256, 0, st>>>(N, P, pairs, tds, tbs, tq, te, (T)kappa, (T)ke,
-                                                                energy, (T*)dds, (T*)dq, (T*)deta, err);
-      break;
-    default:
-      pair_list_kernel<T, ADMP_PAIR_DAMPING><<<grid, 256, 0, st>>>(N, P, pairs, tds, tbs, tq, te, (T)kappa,
-                                                                    (T)ke, energy, (T*)dds, (T*)dq, (T*)deta, err);
-  }
-  ADMP_CUDA_TRY(cudaGetLastError());
-  return check_error(err, st);
+  const int s = launch_pair_energy<T>(mode, nf, N, P, pairs, (const T*)ds, (const T*)bs, (const T*)q, (const T*)eta,
+                                      kappa, ke, energy, 1, false, (T*)dds, (T*)dq, (T*)deta, err, st);
+  return s ? s : check_error(err, st);
 }
 
 }  // namespace admp
@@ -378,6 +391,25 @@ extern "C" int admp_pair_distances(int dtype, int pbc, int natoms, long long npa
   return check_error(err, st);
 }
 
+static int pair_dist_bwd(int dtype, int pbc, int nf, int natoms, long long npairs, const long long* pairs,
+                         const void* pos, const void* box, const void* grad_ds, void* grad_pos, void* grad_box,
+                         DevError* err, cudaStream_t st) {
+  long long blocks = (npairs + 255) / 256;
+  if (blocks > 4096) blocks = 4096;
+  const dim3 grid((unsigned)blocks, (unsigned)nf);
+  if (dtype == ADMP_F64)
+    pair_dist_bwd_kernel<double><<<grid, 256, 0, st>>>(pbc, natoms, npairs, pairs, (const double*)pos,
+                                                       (const double*)box, (const double*)grad_ds, (double*)grad_pos,
+                                                       (double*)grad_box, err);
+  else if (dtype == ADMP_F32)
+    pair_dist_bwd_kernel<float><<<grid, 256, 0, st>>>(pbc, natoms, npairs, pairs, (const float*)pos, (const float*)box,
+                                                      (const float*)grad_ds, (float*)grad_pos, (float*)grad_box, err);
+  else
+    return fail(ADMP_ERR_BAD_ARG, "bad dtype");
+  ADMP_CUDA_TRY(cudaGetLastError());
+  return ADMP_OK;
+}
+
 extern "C" int admp_pair_distances_backward(int dtype, int pbc, int natoms, long long npairs,
                                             const long long* pairs, const void* pos, const void* box,
                                             const void* grad_ds, void* grad_pos, void* grad_box, void* stream) {
@@ -386,18 +418,18 @@ extern "C" int admp_pair_distances_backward(int dtype, int pbc, int natoms, long
   cudaStream_t st = (cudaStream_t)stream;
   DevError* err = scratch_error(st);
   if (!err) return ADMP_ERR_CUDA;
-  long long blocks = (npairs + 255) / 256;
-  if (blocks > 4096) blocks = 4096;
-  if (dtype == ADMP_F64)
-    pair_dist_bwd_kernel<double><<<(unsigned)blocks, 256, 0, st>>>(pbc, natoms, npairs, pairs, (const double*)pos,
-                                                                   (const double*)box, (const double*)grad_ds,
-                                                                   (double*)grad_pos, (double*)grad_box, err);
-  else if (dtype == ADMP_F32)
-    pair_dist_bwd_kernel<float><<<(unsigned)blocks, 256, 0, st>>>(pbc, natoms, npairs, pairs, (const float*)pos,
-                                                                  (const float*)box, (const float*)grad_ds,
-                                                                  (float*)grad_pos, (float*)grad_box, err);
-  else
-    return fail(ADMP_ERR_BAD_ARG, "bad dtype");
-  ADMP_CUDA_TRY(cudaGetLastError());
-  return check_error(err, st);
+  const int s = pair_dist_bwd(dtype, pbc, 1, natoms, npairs, pairs, pos, box, grad_ds, grad_pos, grad_box, err, st);
+  return s ? s : check_error(err, st);
+}
+
+extern "C" int admp_pair_distances_frames_backward(int dtype, int pbc, int nframes, int natoms, long long npairs,
+                                                   const long long* pairs, const void* pos, const void* box,
+                                                   const void* grad_ds, void* grad_pos, void* grad_box, void* stream) {
+  if (npairs == 0 || nframes == 0) return ADMP_OK;
+  if (nframes < 0 || nframes > 65535 || npairs < 0 || !pairs || !pos || !grad_ds || (pbc && !box))
+    return fail(ADMP_ERR_BAD_ARG, "admp_pair_distances_frames_backward: args");
+  cudaStream_t st = (cudaStream_t)stream;
+  DevError* err = scratch_error(st);
+  if (!err) return ADMP_ERR_CUDA;
+  return pair_dist_bwd(dtype, pbc, nframes, natoms, npairs, pairs, pos, box, grad_ds, grad_pos, grad_box, err, st);
 }

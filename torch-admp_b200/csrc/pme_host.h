@@ -46,24 +46,81 @@ struct RecipPlan {
 };
 
 // The per-system table as one by-value parameter: the only launch of a call
-// that carries it.
+// that carries it (a small one for calls of a few systems).
+template <int M>
 struct SysTable {
-  SysDesc s[kMaxBatch];
+  SysDesc s[M];
+};
+constexpr int kFewSys = 8;
+
+template <int M>
+static __global__ void sys_table_kernel(SysTable<M> t, int n, SysDesc* __restrict__ dst) {
+  for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = t.s[i];
+}
+
+// The table upload and every zero-filled buffer of an energy evaluation in one
+// launch (they were up to ten).
+struct ZeroSpans {
+  void* p[6];
+  unsigned long long words[6];  // 4-byte words
+  int n;
+  void add(void* q, size_t bytes) {
+    if (!q || !bytes) return;
+    p[n] = q;
+    words[n++] = bytes / 4;
+  }
 };
 
-static __global__ void sys_table_kernel(SysTable t, int n, SysDesc* __restrict__ dst) {
-  for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = t.s[i];
+template <int M>
+static __global__ void __launch_bounds__(256) prep_kernel(SysTable<M> t, int nsys, SysDesc* __restrict__ dst,
+                                                          ZeroSpans z) {
+  if (blockIdx.x == 0)
+    for (int i = threadIdx.x; i < nsys; i += blockDim.x) dst[i] = t.s[i];
+  const unsigned long long i0 = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x,
+                           step = (unsigned long long)gridDim.x * blockDim.x;
+  for (int k = 0; k < z.n; ++k) {
+    uint32_t* p = (uint32_t*)z.p[k];
+    const unsigned long long n = z.words[k], n4 = ((uintptr_t)p & 15) ? 0 : n / 4;
+    for (unsigned long long i = i0; i < n4; i += step) reinterpret_cast<uint4*>(p)[i] = make_uint4(0, 0, 0, 0);
+    for (unsigned long long i = 4 * n4 + i0; i < n; i += step) p[i] = 0;
+  }
 }
 
 // Upload the plan's system table to `dev` (kMaxBatch entries of device
 // memory owned by the caller's workspace or pools) on stream `st`; the
 // launches that follow on the same stream read it through b.s.
+template <int M, typename T>
+inline SysTable<M> plan_table(const RecipPlan<T>& p) {
+  SysTable<M> t;
+  for (int s = 0; s < p.b.nsys; ++s) t.s[s] = p.hs[s];
+  return t;
+}
+
 template <typename T>
 inline int bind_plan(RecipPlan<T>& p, SysDesc* dev, cudaStream_t st) {
   if (!dev) return fail(ADMP_ERR_WORKSPACE, "no device memory for the system table");
-  SysTable t;
-  for (int s = 0; s < p.b.nsys; ++s) t.s[s] = p.hs[s];
-  sys_table_kernel<<<1, 128, 0, st>>>(t, p.b.nsys, dev);
+  if (p.b.nsys <= kFewSys)
+    sys_table_kernel<kFewSys><<<1, 32, 0, st>>>(plan_table<kFewSys>(p), p.b.nsys, dev);
+  else
+    sys_table_kernel<kMaxBatch><<<1, 128, 0, st>>>(plan_table<kMaxBatch>(p), p.b.nsys, dev);
+  count_launches(1);
+  ADMP_CUDA_TRY(cudaGetLastError());
+  p.b.s = dev;
+  return ADMP_OK;
+}
+
+// bind_plan and the zeroing of `z` in one launch
+template <typename T>
+inline int prep_plan(RecipPlan<T>& p, SysDesc* dev, const ZeroSpans& z, cudaStream_t st) {
+  if (!dev) return fail(ADMP_ERR_WORKSPACE, "no device memory for the system table");
+  unsigned long long words = 0;
+  for (int k = 0; k < z.n; ++k) words += z.words[k];
+  const unsigned long long want = (words / 4 + 255) / 256;
+  const int blocks = want < 1 ? 1 : (want > 2048 ? 2048 : (int)want);
+  if (p.b.nsys <= kFewSys)
+    prep_kernel<kFewSys><<<blocks, 256, 0, st>>>(plan_table<kFewSys>(p), p.b.nsys, dev, z);
+  else
+    prep_kernel<kMaxBatch><<<blocks, 256, 0, st>>>(plan_table<kMaxBatch>(p), p.b.nsys, dev, z);
   count_launches(1);
   ADMP_CUDA_TRY(cudaGetLastError());
   p.b.s = dev;
@@ -313,48 +370,54 @@ inline double plan_atoms(const RecipPlan<T>& p) {
 
 template <typename T>
 inline int launch_spread(const RecipPlan<T>& p, const T* pos, const T* box, const T* q, T* mesh, const int* order,
-                         cudaStream_t st) {
+                         cudaStream_t st, const TermArgs& terms = TermArgs{}) {
   if (!p.b.nblk_st) return ADMP_OK;
   constexpr size_t sm = kStWarps * WarpStencil<T, false>::bytes();
-  ADMP_CUDA_TRY(ensure_smem(spread_kernel<T>, sm));
-  spread_kernel<T><<<p.b.nblk_st, kStWarps * 32, sm, st>>>(family_batch(p, F_ST), pos, box, q, mesh, order);
+  auto* k = terms.flags ? spread_kernel<T, true> : spread_kernel<T, false>;
+  ADMP_CUDA_TRY(ensure_smem(k, sm));
+  k<<<p.b.nblk_st, kStWarps * 32, sm, st>>>(family_batch(p, F_ST), pos, box, q, mesh, order, terms);
   return ADMP_OK;
 }
 
-template <typename T, bool F, bool V>
+// F: energies' gradients and (virial) dE/dbox too, else the potential only.
+template <typename T, bool F>
 inline int launch_gather(const RecipPlan<T>& p, const T* pos, const T* box, const T* q, const T* phi, T* dE_dq,
-                         T* dE_dpos, double* acc, const int* order, cudaStream_t st) {
+                         T* dE_dpos, double* acc, const int* order, cudaStream_t st, bool virial = false,
+                         const TermArgs& terms = TermArgs{}) {
   if (!p.b.nblk_st) return ADMP_OK;
   const bool run = !F && plan_atoms(p) > kGatherRun;
   const int nw = run ? 8 : kStWarps;
   const size_t sm = nw * WarpStencil<T, F>::bytes();
-  ADMP_CUDA_TRY(ensure_smem(gather_kernel<T, F, V>, sm));
+  auto* k = gather_kernel<T, F, false, false>;
+  if constexpr (F)
+    k = terms.flags ? (virial ? gather_kernel<T, F, true, true> : gather_kernel<T, F, false, true>)
+                    : (virial ? gather_kernel<T, F, true, false> : gather_kernel<T, F, false, false>);
+  ADMP_CUDA_TRY(ensure_smem(k, sm));
   Batch b = family_batch(p, run ? F_ATOM : F_ST);
   if (run) b.aps = b.apb;
-  gather_kernel<T, F, V><<<run ? b.nblk_atom : b.nblk_st, nw * 32, sm, st>>>(b, pos, box, q, phi, dE_dq, dE_dpos, acc,
-                                                                            order);
+  k<<<run ? b.nblk_atom : b.nblk_st, nw * 32, sm, st>>>(b, pos, box, q, phi, dE_dq, dE_dpos, acc, order, terms);
   return ADMP_OK;
 }
 
 // Full reciprocal evaluation: spread q, FFT/Green, gather.
 // `dE_dq` receives the potential (dE/dq), `dE_dpos` the gradient; both accumulate.
-// `virial`: the accumulators get the virial terms too (dE/dbox is asked for).
+// `virial`: the accumulators get the virial terms too (dE/dbox is asked for).  With `terms` the caller has
+// zeroed the mesh and the accumulators (prep_kernel).
 template <typename T>
 inline int launch_recip(const RecipPlan<T>& p, const T* pos, const T* box, const T* q, T* mesh, Cplx<T>* spec,
                         double* acc, double ke, T* dE_dq, T* dE_dpos, cudaStream_t st, bool virial,
-                        const int* order = nullptr) {
+                        const int* order = nullptr, const TermArgs& terms = TermArgs{}) {
   const double na = plan_atoms(p), mb = (double)p.mesh_elems * sizeof(T);
-  ADMP_CUDA_TRY(cudaMemsetAsync(mesh, 0, p.mesh_elems * sizeof(T), st));
+  if (!terms.flags) ADMP_CUDA_TRY(cudaMemsetAsync(mesh, 0, p.mesh_elems * sizeof(T), st));
   int h = prof_begin(st);
-  int s = launch_spread<T>(p, pos, box, q, mesh, order, st);
+  int s = launch_spread<T>(p, pos, box, q, mesh, order, st, terms);
   if (s) return s;
   prof_end(h, PK_SPREAD, na * 4 * sizeof(T) + mb, st);
   count_launches(1);
   s = launch_fft_green<T>(p, mesh, spec, box, acc, ke, st, nullptr, virial);
   if (s) return s;
   h = prof_begin(st);
-  s = virial ? launch_gather<T, true, true>(p, pos, box, q, mesh, dE_dq, dE_dpos, acc, order, st)
-             : launch_gather<T, true, false>(p, pos, box, q, mesh, dE_dq, dE_dpos, acc, order, st);
+  s = launch_gather<T, true>(p, pos, box, q, mesh, dE_dq, dE_dpos, acc, order, st, virial, terms);
   if (s) return s;
   prof_end(h, PK_GATHER, mb + na * 4 * sizeof(T) + na * 3 * sizeof(T), st);
   count_launches(1);
@@ -376,7 +439,7 @@ inline int launch_recip_potential(const RecipPlan<T>& p, const T* pos, const T* 
   s = launch_fft_green<T>(p, mesh, spec, box, acc, ke, st, green);
   if (s) return s;
   h = prof_begin(st);
-  s = launch_gather<T, false, false>(p, pos, box, v, mesh, pot, nullptr, acc, order, st);
+  s = launch_gather<T, false>(p, pos, box, v, mesh, pot, nullptr, acc, order, st);
   if (s) return s;
   prof_end(h, PK_GATHER, mb + na * 4 * sizeof(T) + na * sizeof(T), st);
   count_launches(2);

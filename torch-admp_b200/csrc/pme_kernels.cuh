@@ -65,7 +65,8 @@ constexpr int kAccStride = 32;  // doubles per system in the accumulator array
 constexpr int kAccErec = 0;     // reciprocal energy
 constexpr int kAccVk = 1;       // 9: dE/dB (B = box^-1) through k vectors
 constexpr int kAccWf = 10;      // 9: dE/dB through fractional coordinates
-constexpr int kAccSlots = 19;
+constexpr int kAccQ = 19;       // 4: sums of q, q^2, q z and q z^2 (self, non-neutral and slab terms)
+constexpr int kAccSlots = 23;
 
 enum SysField { F_ATOM = 0, F_Z = 1, F_Y = 2, F_X = 3, F_SLAB = 4, F_XT = 5, F_YT = 6, F_ZT = 7, F_ST = 8 };
 
@@ -251,12 +252,25 @@ __device__ __forceinline__ void warp_build_stencil(WarpStencil<T, DERIV>& ws, co
   __syncwarp();
 }
 
-// spread: q -> mesh (zeroed), atomic adds
-template <typename T>
+// The terms an energy evaluation needs beside the mesh: self and non-neutral
+// (kTermEwald, pme.py:448-493) and slab correction along `axis` (kTermSlab,
+// pme.py:495-527).  The spread sums what they need, the gather adds their
+// per-atom gradients, coulomb_finalize_kernel the rest.
+enum { kTermEwald = 1, kTermSlab = 2 };
+struct TermArgs {
+  int flags;
+  int axis;
+  double ke;
+  double* acc;
+};
+
+// spread: q -> mesh (zeroed), atomic adds.  SUMS: also the charge sums of
+// `terms` into its accumulators.
+template <typename T, bool SUMS>
 __global__ void __launch_bounds__(256) spread_kernel(Batch b, const T* __restrict__ pos,
                                                      const T* __restrict__ box,
                                                      const T* __restrict__ q, T* __restrict__ mesh,
-                                                     const int* __restrict__ order) {
+                                                     const int* __restrict__ order, TermArgs terms) {
   extern __shared__ __align__(16) unsigned char dsm[];
   __shared__ Geom g;
   const int s = find_sys<F_ST>(b, blockIdx.x);
@@ -291,6 +305,32 @@ __global__ void __launch_bounds__(256) spread_kernel(Batch b, const T* __restric
       const int oyz = wrap_up(ws.byz[2 * jt] + 5, d.K1) * d.K2 + wrap_up(ws.byz[2 * jt + 1] + zt, d.K2);
 #pragma unroll
       for (int dx = 0; dx < 6; ++dx) atomicAdd(M + ox[dx] + oyz, w[dx] * wyz);
+    }
+  }
+  if constexpr (SUMS) {
+    __shared__ double red[8][4];
+    double v[4] = {0, 0, 0, 0};
+    if (lane < na) {
+      const double qa = ws.q[lane];
+      v[0] = qa;
+      v[1] = qa * qa;
+      if (terms.flags & kTermSlab) {
+        const double z = pos[3 * (size_t)ws.atom[lane] + terms.axis];
+        v[2] = qa * z;
+        v[3] = qa * z * z;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+#pragma unroll
+      for (int m = 1; m < kPw; m <<= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], m);
+      if (lane == 0) red[warp][k] = v[k];
+    }
+    __syncthreads();
+    if (threadIdx.x < 4) {
+      double t = 0.0;
+      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w][threadIdx.x];
+      if (t != 0.0) atomicAdd(terms.acc + (size_t)s * kAccStride + kAccQ + threadIdx.x, t);
     }
   }
 }
@@ -823,13 +863,14 @@ __device__ __forceinline__ T warp_sum_each(T (&v)[NV], int lane) {
 // 192,000 atoms (FP32, forces) took 17.5 / 19.4 / 19.9 / 76.2 us, now 6.2 / 6.2 /
 // 10.3 / 51.6.
 // ---------------------------------------------------------------------------
-template <typename T, bool FORCES, bool VIRIAL>
+template <typename T, bool FORCES, bool VIRIAL, bool TERMS>
 __global__ void __launch_bounds__(256) gather_kernel(Batch b, const T* __restrict__ pos,
                                                      const T* __restrict__ box,
                                                      const T* __restrict__ q,
                                                      const T* __restrict__ phi,
                                                      T* __restrict__ dE_dq, T* __restrict__ dE_dpos,
-                                                     double* __restrict__ acc, const int* __restrict__ order) {
+                                                     double* __restrict__ acc, const int* __restrict__ order,
+                                                     TermArgs terms) {
   extern __shared__ __align__(16) unsigned char dsm[];
   __shared__ Geom g;
   __shared__ double red[VIRIAL ? 8 : 1][9];
@@ -923,7 +964,25 @@ __global__ void __launch_bounds__(256) gather_kernel(Batch b, const T* __restric
       mine += (od ? k1 : k0) + __shfl_xor_sync(0xffffffffu, od ? k0 : k1, 1);
       const bool live = jt < na;
       const int c = lane & 3, ga = live ? ws.atom[jt] : 0;
-      if (live && c == 0 && dE_dq) dE_dq[ga] += mine;
+      if constexpr (TERMS) {
+        const double qa = live ? ws.q[jt] : T(0);
+        const double *S = terms.acc + (size_t)s * kAccStride + kAccQ, *bz = g.box + 3 * terms.axis;
+        const bool slab = (terms.flags & kTermSlab) != 0;
+        const double pre = 2.0 * kPi / g.vol * terms.ke, z = live && slab ? (double)pos[3 * (size_t)ga + terms.axis] : 0.0;
+        if (live && c == 0 && dE_dq) {
+          double t = 0.0;
+          if (terms.flags & kTermEwald)
+            t = -2.0 * terms.ke * d.kappa / kSqrtPi * qa - kPi / (g.vol * d.kappa * d.kappa) * terms.ke * S[0];
+          if (slab)
+            t += pre * (2.0 * S[2] * z - S[3] - S[0] * z * z -
+                        S[0] * (bz[0] * bz[0] + bz[1] * bz[1] + bz[2] * bz[2]) / 6.0);
+          dE_dq[ga] += (T)((double)mine + t);
+        }
+        if (live && slab && c == 1 + terms.axis && dE_dpos)
+          dE_dpos[3 * (size_t)ga + terms.axis] += (T)(pre * (2.0 * S[2] * qa - 2.0 * S[0] * qa * z));
+      } else if (live && c == 0 && dE_dq) {
+        dE_dq[ga] += mine;
+      }
       // u = m0 - x + 3  ->  dE/dx_d = -q * dE/du_d ; x_d = K_d (r @ B)_d
       const int Kc = c == 1 ? d.K0 : c == 2 ? d.K1 : d.K2;
       const double gc = live ? -(double)ws.q[jt] * mine * Kc : 0.0;
@@ -963,6 +1022,25 @@ __global__ void __launch_bounds__(256) gather_kernel(Batch b, const T* __restric
 // ---------------------------------------------------------------------------
 // finalize: energy and dE/dbox = -B^T (dE/dB) B^T - E B^T   (one thread / system)
 // ---------------------------------------------------------------------------
+// dE/dbox of the mesh energy E with accumulators a, box inverse bi
+__device__ __forceinline__ void recip_dbox(const double* a, double E, const double* bi, double* g) {
+  double dB[9];
+#pragma unroll
+  for (int k = 0; k < 9; ++k) dB[k] = a[kAccVk + k] + a[kAccWf + k];
+  // M = B^T dB B^T ; out = -M - E B^T
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      double m = 0.0;
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+#pragma unroll
+        for (int l = 0; l < 3; ++l) m += bi[k * 3 + i] * dB[k * 3 + l] * bi[j * 3 + l];
+      g[i * 3 + j] = -m - E * bi[j * 3 + i];
+    }
+}
+
 template <typename T>
 __global__ void recip_finalize_kernel(Batch b, const T* __restrict__ box, const double* __restrict__ acc,
                                       double* __restrict__ energy, T* __restrict__ dE_dbox) {
@@ -977,21 +1055,46 @@ __global__ void recip_finalize_kernel(Batch b, const T* __restrict__ box, const 
   const int o = d.box_idx;
   if (energy) energy[o] += E;
   if (dE_dbox) {
-    double dB[9];
+    double g[9];
+    recip_dbox(a, E, bi, g);
 #pragma unroll
-    for (int k = 0; k < 9; ++k) dB[k] = a[kAccVk + k] + a[kAccWf + k];
-    // M = B^T dB B^T ; out = -M - E B^T
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-      for (int j = 0; j < 3; ++j) {
-        double m = 0.0;
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-#pragma unroll
-          for (int l = 0; l < 3; ++l) m += bi[k * 3 + i] * dB[k * 3 + l] * bi[j * 3 + l];
-        dE_dbox[(size_t)o * 9 + i * 3 + j] += (T)(-m - E * bi[j * 3 + i]);
-      }
+    for (int k = 0; k < 9; ++k) dE_dbox[(size_t)o * 9 + k] += (T)g[k];
+  }
+}
+
+// The whole Coulomb energy of each system: comps[5] = real (summed by the pair
+// kernel), reciprocal, self, non-neutral, slab; E their sum; dE/dbox of all but
+// the pair distances (written, not added).
+template <typename T>
+__global__ void coulomb_finalize_kernel(Batch b, const T* __restrict__ box, TermArgs terms, double* __restrict__ comps,
+                                        T* __restrict__ energy, T* __restrict__ dE_dbox) {
+  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= b.nsys) return;
+  const SysDesc d = b.s[s];
+  const int o = d.box_idx;
+  double bx[9], bi[9];
+  load_box(box + (size_t)o * 9, bx);
+  const double V = inv3(bx, bi), kappa = d.kappa, ke = terms.ke;
+  const double *a = terms.acc + (size_t)s * kAccStride, *S = a + kAccQ, *bz = bx + 3 * terms.axis;
+  const double Q = S[0], Lz2 = bz[0] * bz[0] + bz[1] * bz[1] + bz[2] * bz[2];
+  const double pre = 2.0 * kPi / V * ke;
+  const bool slab = (terms.flags & kTermSlab) != 0;
+  const double Enn = -kPi / (2.0 * V * kappa * kappa) * ke * Q * Q;
+  const double Eslab = slab ? pre * (S[2] * S[2] - Q * S[3] - Q * Q * Lz2 / 12.0) : 0.0;
+  double* c = comps + (size_t)o * 5;
+  c[1] = a[kAccErec];
+  c[2] = -ke * kappa / kSqrtPi * S[1];
+  c[3] = Enn;
+  c[4] = Eslab;
+  energy[o] = (T)(c[0] + c[1] + c[2] + c[3] + c[4]);
+  if (dE_dbox) {
+    double g[9];
+    recip_dbox(a, a[kAccErec], bi, g);
+    for (int i = 0; i < 3; ++i)  // both scale as 1/V: dE/dbox = -E B^T
+      for (int j = 0; j < 3; ++j) g[i * 3 + j] -= (Enn + Eslab) * bi[j * 3 + i];
+    if (slab)
+      for (int j = 0; j < 3; ++j) g[terms.axis * 3 + j] += pre * (-Q * Q / 6.0) * bz[j];
+    for (int k = 0; k < 9; ++k) dE_dbox[(size_t)o * 9 + k] = (T)g[k];
   }
 }
 

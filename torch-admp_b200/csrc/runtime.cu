@@ -96,10 +96,14 @@ DevError* scratch_error(cudaStream_t) {
   return g_err_ptr[dev];
 }
 
-// The thread's page-locked staging buffer: kept while the thread lives.
+// The thread's page-locked staging buffer (read_back's part, then the probed
+// error word) and the probe's event: kept while the thread lives.
 struct PinnedBuf {
   void* p = nullptr;
+  cudaEvent_t ev = nullptr;
+  int ev_dev = -1;
   ~PinnedBuf() {
+    if (ev) cudaEventDestroy(ev);
     if (p) cudaFreeHost(p);
   }
 };
@@ -107,7 +111,7 @@ static thread_local PinnedBuf g_pin;
 
 static void* pinned() {
   if (!g_pin.p) {
-    cudaError_t e = cudaHostAlloc(&g_pin.p, kReadBack, cudaHostAllocPortable);
+    cudaError_t e = cudaHostAlloc(&g_pin.p, kReadBack + sizeof(DevError), cudaHostAllocPortable);
     if (e != cudaSuccess) {
       g_pin.p = nullptr;
       set_last_cuda_error(e, "cudaHostAlloc", __FILE__, __LINE__);
@@ -126,6 +130,30 @@ const void* read_back(const void* dev, size_t bytes, cudaStream_t st) {
     return nullptr;
   }
   return p;
+}
+
+int probe_error(DevError* err, cudaStream_t st) {
+  if (!g_sync) return ADMP_OK;
+  char* p = (char*)pinned();
+  if (!p) return ADMP_ERR_CUDA;
+  int dev = 0;
+  ADMP_CUDA_TRY(cudaGetDevice(&dev));
+  if (g_pin.ev_dev != dev) {
+    if (g_pin.ev) cudaEventDestroy(g_pin.ev);
+    g_pin.ev = nullptr;
+    g_pin.ev_dev = -1;
+    ADMP_CUDA_TRY(cudaEventCreateWithFlags(&g_pin.ev, cudaEventDisableTiming));
+    g_pin.ev_dev = dev;
+  }
+  ADMP_CUDA_TRY(cudaMemcpyAsync(p + kReadBack, err, sizeof(DevError), cudaMemcpyDeviceToHost, st));
+  ADMP_CUDA_TRY(cudaEventRecord(g_pin.ev, st));
+  return ADMP_OK;
+}
+
+int probed_error(DevError* err, cudaStream_t st) {
+  if (!g_sync) return ADMP_OK;
+  ADMP_CUDA_TRY(cudaEventSynchronize(g_pin.ev));
+  return ((const DevError*)((const char*)g_pin.p + kReadBack))->code ? check_error(err, st) : ADMP_OK;
 }
 
 static const char* where_name(int w) {

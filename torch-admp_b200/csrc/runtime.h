@@ -20,6 +20,12 @@ int check_error(DevError* err, cudaStream_t st);
 // thread's next call.  nullptr on a CUDA error.
 constexpr size_t kReadBack = 64 * 1024;
 const void* read_back(const void* dev, size_t bytes, cudaStream_t st);
+// check_error() without making the host wait for more than it must: probe_error
+// copies the error word on `st` behind the launches that may set it, and
+// probed_error (after the rest of a call has been launched) waits for that copy
+// only.  One probe per thread at a time.
+int probe_error(DevError* err, cudaStream_t st);
+int probed_error(DevError* err, cudaStream_t st);
 // Record a message and return `code`.
 int fail(int code, const char* fmt, ...);
 bool sync_checks();

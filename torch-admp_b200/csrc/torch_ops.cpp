@@ -8,6 +8,8 @@
 //   coulomb_pbc(pos, box, pairs, ds, bs, q, kappa, kmesh, spacing, ethresh,
 //               ke, rspace, kspace, slab, axis) -> [E, comps, kmesh]
 //                 pme.py:261-310 (real, reciprocal, self, non-neutral, slab)
+//   neighbor_list(pos, box, cutoff, nframes) -> status, pairs, scales, ds
+//                 nblist.py:304-445, 517-551
 //   coulomb_obc(pairs, ds, bs, q, ke) -> E                     pme.py:529-561
 //   damping(ds, q, eta, pairs, bs, ke) -> E                    qeq.py:60-129
 //   site(q, chi, hardness) -> E                                qeq.py:159-209
@@ -64,15 +66,30 @@ std::vector<int> kmesh_per_frame(const Tensor& box, double kappa, const std::vec
   const int64_t nf = box.size(0);
   std::vector<int> km(3 * nf);
   Tensor diag;
-  if (kmesh.empty()) diag = torch::diagonal(box.detach(), 0, 1, 2).to(torch::kCPU, torch::kDouble).contiguous();
+  std::vector<double> L(3 * nf);
+  if (kmesh.empty()) {
+    // the raw boxes through page-locked staging: one copy, no conversion kernels
+    const size_t bytes = (size_t)nf * 9 * box.element_size();
+    if (bytes <= 64 * 1024) {
+      std::vector<char> h(bytes);
+      check(admp_read_back(box.data_ptr(), bytes, h.data(), stream_of(box)), "box");
+      for (int64_t k = 0; k < 3 * nf; ++k) {
+        const int64_t e = (k / 3) * 9 + (k % 3) * 4;
+        L[k] = box.scalar_type() == torch::kDouble ? ((const double*)h.data())[e] : ((const float*)h.data())[e];
+      }
+    } else {
+      diag = torch::diagonal(box.detach(), 0, 1, 2).to(torch::kCPU, torch::kDouble).contiguous();
+      for (int64_t k = 0; k < 3 * nf; ++k) L[k] = diag.data_ptr<double>()[k];
+    }
+  }
   for (int64_t f = 0; f < nf; ++f)
     for (int d = 0; d < 3; ++d) {
       if (!kmesh.empty()) {
         km[3 * f + d] = (int)kmesh[d];
       } else {
-        const double L = diag.data_ptr<double>()[3 * f + d];
-        km[3 * f + d] = spacing.empty() ? (int)std::ceil(2 * kappa * L / (3.0 * std::pow(ethresh, 1.0 / 5.0)))
-                                        : (int)std::ceil(L / spacing[d]);
+        const double l = L[3 * f + d];
+        km[3 * f + d] = spacing.empty() ? (int)std::ceil(2 * kappa * l / (3.0 * std::pow(ethresh, 1.0 / 5.0)))
+                                        : (int)std::ceil(l / spacing[d]);
       }
     }
   return km;
@@ -86,43 +103,50 @@ class CoulombPBC : public torch::autograd::Function<CoulombPBC> {
     const int dt = dtype_code(pos);
     void* st = stream_of(pos);
     const int64_t nf = pos.size(0), N = pos.size(1), P = pairs.size(1);
-    const bool need = pos.requires_grad() || box.requires_grad() || ds.requires_grad() || q.requires_grad();
-    Tensor E_real = f64(nf, pos), E_recip = f64(nf, pos);
-    Tensor terms = torch::zeros({nf, 5}, pos.options().dtype(torch::kDouble));
+    ctx->set_materialize_grads(false);
+    // gradients of the inputs that need one, produced with the energy
     Tensor gpos, gbox, gds, gq;
-    if (need) {
-      gpos = torch::zeros_like(pos);
-      if (box.requires_grad()) gbox = torch::zeros_like(box);
-      gds = torch::zeros_like(ds);
-      gq = torch::zeros_like(q);
-    }
     std::vector<int> km = kspace ? kmesh_per_frame(box, kappa, kmesh, spacing, ethresh)
                                  : std::vector<int>(3 * nf, 1);
+    Tensor kmt = torch::tensor(std::vector<int64_t>(km.begin(), km.end()), torch::kLong).reshape({nf, 3});
+    if (kspace && N > 0 && nf > 0) {
+      if (pos.requires_grad()) gpos = torch::empty_like(pos);
+      if (box.requires_grad()) gbox = torch::empty_like(box);
+      if (ds.requires_grad()) gds = torch::empty_like(ds);
+      if (q.requires_grad()) gq = torch::empty_like(q);
+      Tensor E = torch::empty({nf}, pos.options());
+      Tensor comps = torch::empty({nf, 5}, pos.options().dtype(torch::kDouble));
+      const size_t nbytes = admp_pme_recip_workspace_size(dt, (int)nf, km.data());
+      TORCH_CHECK(nbytes > 0, "reciprocal workspace: ", admp_last_error_message());
+      Tensor ws = torch::empty({(int64_t)nbytes}, pos.options().dtype(torch::kUInt8));
+      const int flags = ADMP_QEQ_KSPACE | (rspace ? ADMP_QEQ_RSPACE : 0) | (slab ? ADMP_QEQ_SLAB | ((int)axis << 8) : 0);
+      check(admp_coulomb_pbc(dt, flags, (int)nf, (int)N, km.data(), ptr<void>(pos), ptr<void>(box), P,
+                             ptr<const long long>(pairs), ptr<void>(ds), ptr<void>(bs), ptr<void>(q), kappa, ke,
+                             ptr<void>(E), ptr<double>(comps), ptr<void>(gpos), ptr<void>(gq), ptr<void>(gbox),
+                             ptr<void>(gds), ptr<void>(ws), nbytes, st),
+            "Coulomb energy");
+      ctx->save_for_backward({gpos, gbox, gds, gq});
+      ctx->mark_non_differentiable({comps, kmt});
+      return {E, comps, kmt};
+    }
+    Tensor E_real = f64(nf, pos), E_recip = f64(nf, pos);
+    Tensor terms = torch::zeros({nf, 5}, pos.options().dtype(torch::kDouble));
+    if (pos.requires_grad()) gpos = torch::zeros_like(pos);
+    if (box.requires_grad()) gbox = torch::zeros_like(box);
+    if (ds.requires_grad()) gds = torch::zeros_like(ds);
+    if (q.requires_grad()) gq = torch::zeros_like(q);
     if (rspace && P > 0)
       check(admp_pair_energy(dt, ADMP_PAIR_EWALD, (int)nf, (int)N, P, ptr<const long long>(pairs), ptr<void>(ds),
                              ptr<void>(bs), ptr<void>(q), nullptr, kappa, ke, ptr<double>(E_real), ptr<void>(gds),
                              ptr<void>(gq), nullptr, st),
             "real-space pair energy");
-    if (kspace && N > 0) {
-      const size_t nbytes = admp_pme_recip_workspace_size(dt, (int)nf, km.data());
-      TORCH_CHECK(nbytes > 0, "reciprocal workspace: ", admp_last_error_message());
-      Tensor ws = torch::empty({(int64_t)nbytes}, pos.options().dtype(torch::kUInt8));
-      check(admp_pme_recip(dt, (int)nf, (int)N, km.data(), ptr<void>(pos), ptr<void>(box), ptr<void>(q), kappa, ke,
-                           ptr<double>(E_recip), ptr<void>(gpos), ptr<void>(gq), ptr<void>(gbox), ptr<void>(ws),
-                           nbytes, st),
-            "reciprocal PME");
-    }
-    int flags = 0;
-    if (kspace) flags |= ADMP_TERM_SELF | ADMP_TERM_NON_NEUTRAL;
-    if (slab) flags |= ADMP_TERM_SLAB | ((int)axis << 8);
-    if (flags && N > 0)
-      check(admp_atom_terms(dt, flags, (int)nf, (int)N, ptr<void>(pos), ptr<void>(box), ptr<void>(q), nullptr,
-                            nullptr, nullptr, kappa, ke, nullptr, ptr<double>(terms), ptr<void>(gq), ptr<void>(gpos),
-                            ptr<void>(gbox), nullptr, nullptr, nullptr, st),
-            "self / non-neutral / slab terms");
+    if (slab && N > 0)
+      check(admp_atom_terms(dt, ADMP_TERM_SLAB | ((int)axis << 8), (int)nf, (int)N, ptr<void>(pos), ptr<void>(box),
+                            ptr<void>(q), nullptr, nullptr, nullptr, kappa, ke, nullptr, ptr<double>(terms),
+                            ptr<void>(gq), ptr<void>(gpos), ptr<void>(gbox), nullptr, nullptr, nullptr, st),
+            "slab term");
     Tensor comps = torch::stack({E_real, E_recip, terms.select(1, 0), terms.select(1, 1), terms.select(1, 2)}, 1);
     Tensor E = comps.sum(1).to(q.scalar_type());
-    Tensor kmt = torch::tensor(std::vector<int64_t>(km.begin(), km.end()), torch::kLong).reshape({nf, 3});
     ctx->save_for_backward({gpos, gbox, gds, gq});
     ctx->mark_non_differentiable({comps, kmt});
     return {E, comps, kmt};
@@ -132,15 +156,57 @@ class CoulombPBC : public torch::autograd::Function<CoulombPBC> {
     auto s = ctx->get_saved_variables();
     const Tensor& gE = g[0];
     Tensor out_pos, out_box, out_ds, out_q;
-    if (gE.defined() && s[3].defined()) {
-      const Tensor w = gE.to(s[3].scalar_type());
-      out_pos = s[0] * w.view({-1, 1, 1});
-      if (s[1].defined()) out_box = s[1] * w.view({-1, 1, 1});
-      out_ds = s[2] * w.view({-1, 1});
-      out_q = s[3] * w.view({-1, 1});
+    if (gE.defined()) {
+      if (s[0].defined()) out_pos = s[0] * gE.view({-1, 1, 1});
+      if (s[1].defined()) out_box = s[1] * gE.view({-1, 1, 1});
+      if (s[2].defined()) out_ds = s[2] * gE.view({-1, 1});
+      if (s[3].defined()) out_q = s[3] * gE.view({-1, 1});
     }
     return {out_pos, out_box, out_ds, out_q, Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor(),
             Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+  }
+};
+
+// Full pair list of nf frames of N atoms (nblist.py:304-445), rows of a frame
+// padded to the longest frame's count, and its pair distances, differentiable
+// in positions and box (nblist.py:517-551; an empty box: open boundaries).  The counts come from
+// admp_nblist_frames_count on the same workspace.
+class NeighborList : public torch::autograd::Function<NeighborList> {
+ public:
+  static variable_list forward(AutogradContext* ctx, Tensor pos, Tensor box, Tensor ws, double cutoff, int64_t nf,
+                               int64_t N, int64_t P) {
+    const auto lo = pos.options().dtype(torch::kLong);
+    Tensor pairs = torch::empty({nf * P, 2}, lo), bs = torch::empty({nf * P}, lo);
+    Tensor ds = torch::empty({nf * P}, pos.options());
+    check(admp_nblist_frames_fill(dtype_code(pos), box.numel() ? 1 : 0, (int)nf, (int)N, ptr<void>(pos), cutoff,
+                                  ptr<void>(ws), (size_t)ws.numel(), P, ptr<long long>(pairs), ptr<long long>(bs),
+                                  ptr<void>(ds), stream_of(pos)),
+          "neighbour list fill");
+    ctx->save_for_backward({pos, box, pairs});
+    ctx->saved_data["nf"] = nf;
+    ctx->saved_data["N"] = N;
+    ctx->mark_non_differentiable({pairs, bs});
+    ctx->set_materialize_grads(false);  // else zeros as large as the pair list are made for them
+    return {pairs, bs, ds};
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    auto s = ctx->get_saved_variables();
+    Tensor gpos, gbox;
+    if (g[2].defined()) {
+      const Tensor &pos = s[0], &box = s[1];
+      const int64_t nf = ctx->saved_data["nf"].toInt(), N = ctx->saved_data["N"].toInt();
+      if (ctx->needs_input_grad(0)) gpos = torch::zeros_like(pos);
+      if (box.numel() && ctx->needs_input_grad(1)) gbox = torch::zeros_like(box);
+      const Tensor gds = g[2].contiguous();
+      if (gpos.defined() || gbox.defined())
+        check(admp_pair_distances_frames_backward(dtype_code(pos), box.numel() ? 1 : 0, (int)nf, (int)N,
+                                                  nf > 0 ? s[2].size(0) / nf : 0, ptr<const long long>(s[2]),
+                                                  ptr<void>(pos), box.numel() ? ptr<void>(box) : nullptr, ptr<void>(gds), ptr<void>(gpos),
+                                                  ptr<void>(gbox), stream_of(pos)),
+              "pair distances backward");
+    }
+    return {gpos, gbox, Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
   }
 };
 
@@ -253,6 +319,25 @@ class Site : public torch::autograd::Function<Site> {
   }
 };
 
+// Status and (when it is 0) pairs [nf P, 2], scales [nf P], distances [nf P] of positions [nf N, 3].
+std::tuple<int64_t, Tensor, Tensor, Tensor> neighbor_list(Tensor pos, std::optional<Tensor> box, double cutoff,
+                                                          int64_t nf) {
+  Tensor p = pos.contiguous(), b = box.has_value() ? box->contiguous() : torch::empty({0}, p.options());
+  const int dt = dtype_code(p);
+  void* st = stream_of(p);
+  const int64_t N = nf > 0 ? p.size(0) / nf : 0;
+  const size_t nbytes = admp_nblist_frames_workspace_size((int)nf, (int)N);
+  Tensor ws = torch::empty({(int64_t)nbytes}, p.options().dtype(torch::kUInt8));
+  std::vector<long long> np(nf > 0 ? nf : 1, 0);
+  const int status = admp_nblist_frames_count(dt, b.numel() ? 1 : 0, (int)nf, (int)N, ptr<void>(p), ptr<void>(b),
+                                              cutoff, ptr<void>(ws), nbytes, np.data(), st);
+  if (status != ADMP_OK) return {status, Tensor(), Tensor(), Tensor()};
+  long long P = 0;
+  for (long long n : np) P = n > P ? n : P;
+  auto r = NeighborList::apply(p, b, ws, cutoff, nf, N, (int64_t)P);
+  return {0, r[0], r[1], r[2]};
+}
+
 std::vector<Tensor> coulomb_pbc(Tensor pos, Tensor box, Tensor pairs, Tensor ds, Tensor bs, Tensor q, double kappa,
                                 std::vector<int64_t> kmesh, std::vector<double> spacing, double ethresh, double ke,
                                 bool rspace, bool kspace, bool slab, int64_t axis) {
@@ -285,6 +370,8 @@ TORCH_LIBRARY(admp_b200, m) {
         "int[] kmesh, float[] spacing, float ethresh, float ke, bool rspace, bool kspace, bool slab, int axis) "
         "-> Tensor[]",
         &coulomb_pbc);
+  m.def("neighbor_list(Tensor pos, Tensor? box, float cutoff, int nframes) -> (int, Tensor, Tensor, Tensor)",
+        &neighbor_list);
   m.def("coulomb_obc(Tensor pairs, Tensor ds, Tensor bs, Tensor q, float ke) -> Tensor", &coulomb_obc);
   m.def("damping(Tensor ds, Tensor q, Tensor eta, Tensor pairs, Tensor bs, float ke) -> Tensor", &damping);
   m.def("site(Tensor q, Tensor chi, Tensor hardness) -> Tensor", &site);
