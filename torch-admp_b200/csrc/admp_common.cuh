@@ -42,6 +42,48 @@ __device__ __forceinline__ T warp_sum(T v) {
   return v;
 }
 
+// Row p of an int64 pair list.  The list may start on any 8-byte boundary (a
+// view), so 16-byte accesses are taken only where it is aligned to them.
+__device__ __forceinline__ longlong2 load_pair(const long long* __restrict__ pairs, long long p) {
+  return make_longlong2(pairs[2 * p], pairs[2 * p + 1]);
+}
+__device__ __forceinline__ void store_pair(long long* __restrict__ pairs, size_t p, long long i, long long j) {
+  if (((uintptr_t)pairs & 15) == 0) {
+    reinterpret_cast<longlong2*>(pairs)[p] = make_longlong2(i, j);
+  } else {
+    pairs[2 * p] = i;
+    pairs[2 * p + 1] = j;
+  }
+}
+
+// Runs of equal keys among the lanes of a warp (pair lists come sorted by their
+// first atom, so a warp sees one or two): sum() leaves each run's total in the
+// lane where the run opens, so one atomic serves the run.  Keys may repeat in
+// later runs.
+struct WarpRuns {
+  unsigned same;  // bit k: the lane 2^k further on belongs to this lane's run
+  bool opens;
+  __device__ __forceinline__ WarpRuns(int key, int lane) {
+    const int prev = __shfl_up_sync(0xffffffffu, key, 1);
+    opens = lane == 0 || prev != key;
+    const unsigned heads = __ballot_sync(0xffffffffu, opens);
+    const unsigned later = lane < 31 ? heads >> (lane + 1) : 0u;
+    const int reach = later ? __ffs(later) - 1 : 31 - lane;  // lanes of the run after this one
+    same = 0;
+#pragma unroll
+    for (int k = 0; k < 5; ++k) same |= (reach >= (1 << k)) ? 1u << k : 0u;
+  }
+  template <typename T>
+  __device__ __forceinline__ T sum(T v) const {
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+      const T u = __shfl_down_sync(0xffffffffu, v, 1 << k);
+      if (same & (1u << k)) v += u;
+    }
+    return v;
+  }
+};
+
 // Block-wide sum of `n` doubles per thread into `out` (atomic add); `sh`
 // must hold n * 32 doubles.
 template <int NV>

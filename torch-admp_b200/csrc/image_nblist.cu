@@ -247,7 +247,7 @@ __global__ void __launch_bounds__(32 * kImgWarps)
     if (in) {
       const unsigned below = (1u << lane) - 1u;
       const long long p = j == i ? pii + __popc(self & below) : pij + __popc(other & below);
-      reinterpret_cast<longlong2*>(pairs)[p] = make_longlong2(i, j);
+      store_pair(pairs, p, i, j);
       // relative to the caller's unwrapped positions: n + k_i - k_j
       shifts[3 * p] = na + k0 - cell[3 * (size_t)j];
       shifts[3 * p + 1] = nb + k1 - cell[3 * (size_t)j + 1];

@@ -577,7 +577,7 @@ __global__ void __launch_bounds__(256) nb_fill_kernel(int pbc, int N, int mc, do
     for (long long k = r->npairs + blockIdx.x * (long long)blockDim.x + threadIdx.x; k < o.stride;
          k += (long long)gridDim.x * blockDim.x) {
       const size_t p = (size_t)f * o.stride + k;
-      reinterpret_cast<longlong2*>(o.pairs)[p] = make_longlong2(0, 0);
+      store_pair(o.pairs, p, 0, 0);
       if (o.bscale) o.bscale[p] = 0;
       if (o.ds) reinterpret_cast<T*>(o.ds)[p] = T(1);
     }
@@ -597,7 +597,7 @@ __global__ void __launch_bounds__(256) nb_fill_kernel(int pbc, int N, int mc, do
   if (o.ds)
     for (int e = 0; e < 3; ++e) ri[e] = (double)ps[3 * (size_t)i + e];
   auto emit = [&](int k, int j) {
-    reinterpret_cast<longlong2*>(o.pairs)[out + k] = make_longlong2(i, j);
+    store_pair(o.pairs, out + k, i, j);
     if (o.bscale) o.bscale[out + k] = i < j ? 1 : 0;
     if (o.ds) {
       double dr[3], n[3];

@@ -26,53 +26,79 @@ __global__ void __launch_bounds__(256)
   if (dE_dq) dE_dq += (size_t)f * N;
   if (dE_deta) dE_deta += (size_t)f * N;
   const T two_over_sqrtpi = T(2.0 / kSqrtPi);
+  const int lane = threadIdx.x & 31;
   double e = 0.0;
-  for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < P;
-       p += (long long)gridDim.x * blockDim.x) {
-    const long long i = pairs[2 * p], j = pairs[2 * p + 1];
-    if (i < 0 || i >= N || j < 0 || j >= N) {
-      report_error(err, ADMP_ERR_BAD_INDEX, 1, p);
-      if (put && dE_dds) dE_dds[p] = T(0);
-      continue;
-    }
-    const T d = ds[p], s = bs[p];
-    const T qi = q[i], qj = q[j];
-    const T thr = MODE == ADMP_PAIR_OBC ? T(1e-8) : T(1e-4);
-    const bool valid = fabs((double)d) > (double)thr;
-    const T inv = valid ? T(1) / d : T(0);
-    T ep, dd, c;
-    if (MODE == ADMP_PAIR_EWALD) {
-      const T x = kappa * d;
-      const T er = erfc_t(x);
-      ep = er * qi * qj * inv * s * ke;
-      dd = valid ? (-two_over_sqrtpi * kappa * exp_t(-x * x) * inv - er * inv * inv) * qi * qj * s * ke : T(0);
-      c = er * inv * s * ke;
-    } else if (MODE == ADMP_PAIR_OBC) {
-      ep = qi * qj * ke * inv * s;
-      dd = valid ? -qi * qj * ke * inv * inv * s : T(0);
-      c = ke * inv * s;
-    } else {
-      const T ei = eta[i], ej = eta[j];
-      const T eij = sqrt_t((ei * ei + ej * ej) / T(2));
-      const bool zero = eij == T(0);
-      const T eijs = zero ? T(1e-10) : eij;
-      const T x = d / (T(2) * eijs);
-      const T er = erfc_t(x);
-      const T ge = two_over_sqrtpi * exp_t(-x * x);
-      ep = -er * qi * qj * inv * s * ke;
-      dd = valid ? (ge / (T(2) * eijs) * inv + er * inv * inv) * qi * qj * s * ke : T(0);
-      c = -er * inv * s * ke;
-      if (dE_deta && !zero) {
-        const T deij = -ge * d / (T(2) * eijs * eijs) * qi * qj * inv * s * ke;
-        atomicAdd(dE_deta + i, deij * ei / (T(2) * eijs));
-        atomicAdd(dE_deta + j, deij * ej / (T(2) * eijs));
+  for (long long p0 = blockIdx.x * (long long)blockDim.x + (threadIdx.x & ~31); p0 < P;
+       p0 += (long long)gridDim.x * blockDim.x) {
+    const long long p = p0 + lane;
+    long long i = 0, j = 0;
+    bool ok = p < P;
+    if (ok) {
+      const longlong2 ij = load_pair(pairs, p);
+      i = ij.x;
+      j = ij.y;
+      if (i < 0 || i >= N || j < 0 || j >= N) {
+        report_error(err, ADMP_ERR_BAD_INDEX, 1, p);
+        if (put && dE_dds) dE_dds[p] = T(0);
+        ok = false;
       }
     }
-    e += (double)ep;
-    if (dE_dds) dE_dds[p] = put ? dd : dE_dds[p] + dd;
-    if (dE_dq && c != T(0)) {
-      atomicAdd(dE_dq + i, c * qj);
-      atomicAdd(dE_dq + j, c * qi);
+    const T d = ok ? ds[p] : T(1), s = ok ? bs[p] : T(0);
+    const T qi = ok ? q[i] : T(0), qj = ok ? q[j] : T(0);
+    T ei = T(0), ej = T(0);
+    if (MODE == ADMP_PAIR_DAMPING && ok) {
+      ei = eta[i];
+      ej = eta[j];
+    }
+    // a full list has scale 0 on half of its pairs: nothing to evaluate there unless a value is not finite
+    const bool skip = !ok || (s == T(0) && isfinite(d + qi * qj + ei + ej));
+    T ep = T(0), dd = T(0), c = T(0), gi = T(0), gj = T(0);
+    if (!skip) {
+      const T thr = MODE == ADMP_PAIR_OBC ? T(1e-8) : T(1e-4);
+      const bool valid = fabs((double)d) > (double)thr;
+      const T inv = valid ? T(1) / d : T(0);
+      if (MODE == ADMP_PAIR_EWALD) {
+        const T x = kappa * d;
+        const T er = erfc_t(x);
+        ep = er * qi * qj * inv * s * ke;
+        dd = valid ? (-two_over_sqrtpi * kappa * exp_t(-x * x) * inv - er * inv * inv) * qi * qj * s * ke : T(0);
+        c = er * inv * s * ke;
+      } else if (MODE == ADMP_PAIR_OBC) {
+        ep = qi * qj * ke * inv * s;
+        dd = valid ? -qi * qj * ke * inv * inv * s : T(0);
+        c = ke * inv * s;
+      } else {
+        const T eij = sqrt_t((ei * ei + ej * ej) / T(2));
+        const bool zero = eij == T(0);
+        const T eijs = zero ? T(1e-10) : eij;
+        const T x = d / (T(2) * eijs);
+        const T er = erfc_t(x);
+        const T ge = two_over_sqrtpi * exp_t(-x * x);
+        ep = -er * qi * qj * inv * s * ke;
+        dd = valid ? (ge / (T(2) * eijs) * inv + er * inv * inv) * qi * qj * s * ke : T(0);
+        c = -er * inv * s * ke;
+        if (dE_deta && !zero) {
+          const T deij = -ge * d / (T(2) * eijs * eijs) * qi * qj * inv * s * ke;
+          gi = deij * ei / (T(2) * eijs);
+          gj = deij * ej / (T(2) * eijs);
+        }
+      }
+      e += (double)ep;
+    }
+    if (ok && dE_dds) dE_dds[p] = put ? dd : dE_dds[p] + dd;
+    if ((dE_dq || (MODE == ADMP_PAIR_DAMPING && dE_deta)) && __any_sync(0xffffffffu, !skip)) {
+      // one atomic per run of pairs with the same first atom, one per pair for the second
+      const WarpRuns runs(ok ? (int)i : -1, lane);
+      if (dE_dq) {
+        const T a = runs.sum(c != T(0) ? c * qj : T(0));
+        if (runs.opens && a != T(0)) atomicAdd(dE_dq + i, a);
+        if (c != T(0)) atomicAdd(dE_dq + j, c * qi);
+      }
+      if (MODE == ADMP_PAIR_DAMPING && dE_deta) {
+        const T a = runs.sum(gi);
+        if (runs.opens && a != T(0)) atomicAdd(dE_deta + i, a);
+        if (gj != T(0)) atomicAdd(dE_deta + j, gj);
+      }
     }
   }
   double v[1] = {e};
@@ -241,31 +267,50 @@ __global__ void __launch_bounds__(256)
   }
   __syncthreads();
   double vb[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < P;
-       p += (long long)gridDim.x * blockDim.x) {
-    const long long i = pairs[2 * p], j = pairs[2 * p + 1];
-    if (i < 0 || i >= N || j < 0 || j >= N) {
-      report_error(err, ADMP_ERR_BAD_INDEX, 3, p);
+  const int lane = threadIdx.x & 31;
+  for (long long p0 = blockIdx.x * (long long)blockDim.x + (threadIdx.x & ~31); p0 < P;
+       p0 += (long long)gridDim.x * blockDim.x) {
+    const long long p = p0 + lane;
+    const double gp = p < P ? (double)g[p] : 0.0;
+    if (!__any_sync(0xffffffffu, p < P && gp != 0.0)) {
+      if (p >= P) continue;
+      const longlong2 ij = load_pair(pairs, p);
+      if (ij.x < 0 || ij.x >= N || ij.y < 0 || ij.y >= N) report_error(err, ADMP_ERR_BAD_INDEX, 3, p);
       continue;
     }
-    const double gp = g[p];
-    if (gp == 0.0) continue;
-    double dr[3], n[3] = {0, 0, 0};
-    if (pbc) {
-      for (int e = 0; e < 3; ++e) dr[e] = (double)pos[3 * i + e] - (double)pos[3 * j + e];
-      min_image(geo, geo + 9, dr, n);
-    } else {
-      for (int e = 0; e < 3; ++e) dr[e] = (double)pos[3 * j + e] - (double)pos[3 * i + e];
+    long long i = 0, j = 0;
+    bool ok = p < P;
+    if (ok) {
+      const longlong2 ij = load_pair(pairs, p);
+      i = ij.x;
+      j = ij.y;
+      if (i < 0 || i >= N || j < 0 || j >= N) {
+        report_error(err, ADMP_ERR_BAD_INDEX, 3, p);
+        ok = false;
+      }
     }
-    const double d = sqrt(dr[0] * dr[0] + dr[1] * dr[1] + dr[2] * dr[2]);
-    if (d == 0.0) continue;
-    const double s = gp / d;
-    const long long a = pbc ? i : j, c = pbc ? j : i;
+    const bool live = ok && gp != 0.0;
+    double dr[3] = {0, 0, 0}, n[3] = {0, 0, 0}, s = 0.0;
+    if (live) {
+      if (pbc) {
+        for (int e = 0; e < 3; ++e) dr[e] = (double)pos[3 * i + e] - (double)pos[3 * j + e];
+        min_image(geo, geo + 9, dr, n);
+      } else {
+        for (int e = 0; e < 3; ++e) dr[e] = (double)pos[3 * j + e] - (double)pos[3 * i + e];
+      }
+      const double d = sqrt(dr[0] * dr[0] + dr[1] * dr[1] + dr[2] * dr[2]);
+      s = d == 0.0 ? 0.0 : gp / d;
+    }
+    // dr points from j to i with a box and from i to j without: the first atom gets +v or -v; its share is summed
+    // over the run of pairs that start with it
+    const WarpRuns runs(ok ? (int)i : -1, lane);
+#pragma unroll
     for (int e = 0; e < 3; ++e) {
-      const double v = s * dr[e];
+      const double v = s == 0.0 ? 0.0 : s * dr[e];
       if (gpos) {
-        atomicAdd(gpos + 3 * a + e, (T)v);
-        atomicAdd(gpos + 3 * c + e, (T)(-v));
+        const T w = (T)(pbc ? v : -v), a = runs.sum(w);
+        if (runs.opens && a != T(0)) atomicAdd(gpos + 3 * i + e, a);
+        if (w != T(0)) atomicAdd(gpos + 3 * j + e, -w);
       }
       if (pbc)
         for (int k = 0; k < 3; ++k) vb[k * 3 + e] -= n[k] * v;

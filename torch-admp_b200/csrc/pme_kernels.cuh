@@ -252,6 +252,34 @@ __device__ __forceinline__ void warp_build_stencil(WarpStencil<T, DERIV>& ws, co
   __syncwarp();
 }
 
+// Lane mapping of a group: columns 0..31 of one atom at a time (lane = 6 y + z), then the last four columns
+// of all eight atoms (lane -> atom lane / 4, z 2 + lane % 4).
+template <typename T>
+__device__ __forceinline__ void spread_group(const WarpStencil<T, false>& ws, int na, int K1, int K2, T* M, int lane) {
+  const int y0 = lane / 6, z0 = lane % 6, jt = lane >> 2, zt = 2 + (lane & 3);
+  for (int j = 0; j < na; ++j) {
+    const T qa = ws.q[j];
+    if (qa == T(0)) continue;
+    const T* w = ws.w + j * 18;
+    const int* ox = ws.ox + j * 6;
+    const T wyz = qa * w[6 + y0] * w[12 + z0];
+    const int oyz = wrap_up(ws.byz[2 * j] + y0, K1) * K2 + wrap_up(ws.byz[2 * j + 1] + z0, K2);
+#pragma unroll
+    for (int dx = 0; dx < 6; ++dx) atomicAdd(M + ox[dx] + oyz, w[dx] * wyz);
+  }
+  if (jt < na) {
+    const T qa = ws.q[jt];
+    if (qa != T(0)) {
+      const T* w = ws.w + jt * 18;
+      const int* ox = ws.ox + jt * 6;
+      const T wyz = qa * w[6 + 5] * w[12 + zt];
+      const int oyz = wrap_up(ws.byz[2 * jt] + 5, K1) * K2 + wrap_up(ws.byz[2 * jt + 1] + zt, K2);
+#pragma unroll
+      for (int dx = 0; dx < 6; ++dx) atomicAdd(M + ox[dx] + oyz, w[dx] * wyz);
+    }
+  }
+}
+
 // The terms an energy evaluation needs beside the mesh: self and non-neutral
 // (kTermEwald, pme.py:448-493) and slab correction along `axis` (kTermSlab,
 // pme.py:495-527).  The spread sums what they need, the gather adds their
@@ -284,29 +312,8 @@ __global__ void __launch_bounds__(256) spread_kernel(Batch b, const T* __restric
   T* M = mesh + d.mesh_off;
   WarpStencil<T, false> ws;
   ws.carve(dsm + warp * WarpStencil<T, false>::bytes());
-  const int y0 = lane / 6, z0 = lane % 6, jt = lane >> 2, zt = 2 + (lane & 3);
   warp_build_stencil<T, false>(ws, d, g, pos, q, order, a0, d.natoms, lane);
-  for (int j = 0; j < na; ++j) {
-    const T qa = ws.q[j];
-    if (qa == T(0)) continue;
-    const T* w = ws.w + j * 18;
-    const int* ox = ws.ox + j * 6;
-    const T wyz = qa * w[6 + y0] * w[12 + z0];
-    const int oyz = wrap_up(ws.byz[2 * j] + y0, d.K1) * d.K2 + wrap_up(ws.byz[2 * j + 1] + z0, d.K2);
-#pragma unroll
-    for (int dx = 0; dx < 6; ++dx) atomicAdd(M + ox[dx] + oyz, w[dx] * wyz);
-  }
-  if (jt < na) {
-    const T qa = ws.q[jt];
-    if (qa != T(0)) {
-      const T* w = ws.w + jt * 18;
-      const int* ox = ws.ox + jt * 6;
-      const T wyz = qa * w[6 + 5] * w[12 + zt];
-      const int oyz = wrap_up(ws.byz[2 * jt] + 5, d.K1) * d.K2 + wrap_up(ws.byz[2 * jt + 1] + zt, d.K2);
-#pragma unroll
-      for (int dx = 0; dx < 6; ++dx) atomicAdd(M + ox[dx] + oyz, w[dx] * wyz);
-    }
-  }
+  spread_group<T>(ws, na, d.K1, d.K2, M, lane);
   if constexpr (SUMS) {
     __shared__ double red[8][4];
     double v[4] = {0, 0, 0, 0};
@@ -849,6 +856,88 @@ __device__ __forceinline__ T warp_sum_each(T (&v)[NV], int lane) {
   return r;
 }
 
+// Potential (and with FORCES the three stencil derivatives) of a group's atoms: all lanes get the potential of
+// atom lane / 4, or with FORCES lane l quantity l % 4 of atom l / 4.
+template <typename T, bool FORCES>
+__device__ __forceinline__ T gather_group(const WarpStencil<T, FORCES>& ws, int na, int K1, int K2, const T* M,
+                                          int lane) {
+  const int y0 = lane / 6, z0 = lane % 6, jt = lane >> 2, zt = 2 + (lane & 3);
+  constexpr int NQ = FORCES ? 4 : 1;                                    // quantities per atom
+  constexpr int GU = (sizeof(T) == 8 ? 2 : 4) * (FORCES ? 1 : 2);       // atoms per group
+  constexpr int kLanes = 32 / (GU * NQ);                                // lanes that share a group sum
+  T mine = T(0);
+#pragma unroll
+  for (int jb = 0; jb < kPw; jb += GU) {
+    if (jb >= na) break;
+    T fm[GU][6];
+#pragma unroll
+    for (int u = 0; u < GU; ++u) {
+      const int j = min(jb + u, na - 1);
+      const int* ox = ws.ox + j * 6;
+      const int oyz = wrap_up(ws.byz[2 * j] + y0, K1) * K2 + wrap_up(ws.byz[2 * j + 1] + z0, K2);
+#pragma unroll
+      for (int dx = 0; dx < 6; ++dx) fm[u][dx] = M[ox[dx] + oyz];
+    }
+    T v[GU * NQ];
+#pragma unroll
+    for (int u = 0; u < GU; ++u) {
+      const int j = min(jb + u, na - 1);
+      const T* w = ws.w + j * 18;
+      const T wy = w[6 + y0], wz = w[12 + z0];
+      T sw = 0, sdw = 0;
+#pragma unroll
+      for (int dx = 0; dx < 6; ++dx) {
+        sw += fm[u][dx] * w[dx];
+        if (FORCES) sdw += fm[u][dx] * ws.dw[j * 18 + dx];
+      }
+      v[u * NQ] = sw * wy * wz;
+      if (FORCES) {
+        v[u * NQ + 1] = sdw * wy * wz;
+        v[u * NQ + 2] = sw * ws.dw[j * 18 + 6 + y0] * wz;
+        v[u * NQ + 3] = sw * wy * ws.dw[j * 18 + 12 + z0];
+      }
+    }
+    const T sum = warp_sum_each<GU * NQ>(v, lane);
+    // to the lanes of the group's atoms: lane l takes quantity l % 4 of atom l / 4
+    const int want = FORCES ? lane - 4 * jb : jt - jb;
+    const T got = __shfl_sync(0xffffffffu, sum, (want * kLanes) & 31);
+    if (want >= 0 && want < GU * NQ) mine = got;
+  }
+  // the last four columns of atom lane / 4
+  T left[NQ] = {};
+  if (jt < na) {
+    const T* w = ws.w + jt * 18;
+    const int* ox = ws.ox + jt * 6;
+    const T wy = w[6 + 5], wz = w[12 + zt];
+    const int oyz = wrap_up(ws.byz[2 * jt] + 5, K1) * K2 + wrap_up(ws.byz[2 * jt + 1] + zt, K2);
+    T sw = 0, sdw = 0;
+#pragma unroll
+    for (int dx = 0; dx < 6; ++dx) {
+      const T f = M[ox[dx] + oyz];
+      sw += f * w[dx];
+      if (FORCES) sdw += f * ws.dw[jt * 18 + dx];
+    }
+    left[0] = sw * wy * wz;
+    if constexpr (FORCES) {
+      left[1] = sdw * wy * wz;
+      left[2] = sw * ws.dw[jt * 18 + 6 + 5] * wz;
+      left[3] = sw * wy * ws.dw[jt * 18 + 12 + zt];
+    }
+  }
+  if constexpr (!FORCES) {
+    left[0] += __shfl_xor_sync(0xffffffffu, left[0], 1);
+    left[0] += __shfl_xor_sync(0xffffffffu, left[0], 2);
+    return mine + left[0];
+  } else {
+    // four quantities over four lanes: lane c of the four ends with quantity c
+    const bool hi = (lane & 2) != 0, od = (lane & 1) != 0;
+    const T s0 = hi ? left[0] : left[2], s1 = hi ? left[1] : left[3];
+    const T k0 = (hi ? left[2] : left[0]) + __shfl_xor_sync(0xffffffffu, s0, 2);
+    const T k1 = (hi ? left[3] : left[1]) + __shfl_xor_sync(0xffffffffu, s1, 2);
+    return mine + (od ? k1 : k0) + __shfl_xor_sync(0xffffffffu, od ? k0 : k1, 1);
+  }
+}
+
 // ---------------------------------------------------------------------------
 // gather: pot_i = sum phi theta; dE/du_d = q sum phi dtheta/du_d (warp-cooperative)
 //
@@ -884,84 +973,15 @@ __global__ void __launch_bounds__(256) gather_kernel(Batch b, const T* __restric
   const T* M = phi + d.mesh_off;
   WarpStencil<T, FORCES> ws;
   ws.carve(dsm + warp * WarpStencil<T, FORCES>::bytes());
-  const int y0 = lane / 6, z0 = lane % 6, jt = lane >> 2, zt = 2 + (lane & 3);
-  constexpr int NQ = FORCES ? 4 : 1;                                    // quantities per atom
-  constexpr int GU = (sizeof(T) == 8 ? 2 : 4) * (FORCES ? 1 : 2);       // atoms per group
-  constexpr int kLanes = 32 / (GU * NQ);                                // lanes that share a group sum
+  const int jt = lane >> 2;
   double wf[3] = {0, 0, 0};  // virial row of this lane's component
   for (int a0 = a_begin + warp * kPw; a0 < a_end; a0 += (blockDim.x >> 5) * kPw) {
     const int na = min(kPw, a_end - a0);
     warp_build_stencil<T, FORCES>(ws, d, g, pos, FORCES ? q : nullptr, order, a0, a_end, lane);
-    T mine = T(0);
-#pragma unroll
-    for (int jb = 0; jb < kPw; jb += GU) {
-      if (jb >= na) break;
-      T fm[GU][6];
-#pragma unroll
-      for (int u = 0; u < GU; ++u) {
-        const int j = min(jb + u, na - 1);
-        const int* ox = ws.ox + j * 6;
-        const int oyz = wrap_up(ws.byz[2 * j] + y0, d.K1) * d.K2 + wrap_up(ws.byz[2 * j + 1] + z0, d.K2);
-#pragma unroll
-        for (int dx = 0; dx < 6; ++dx) fm[u][dx] = M[ox[dx] + oyz];
-      }
-      T v[GU * NQ];
-#pragma unroll
-      for (int u = 0; u < GU; ++u) {
-        const int j = min(jb + u, na - 1);
-        const T* w = ws.w + j * 18;
-        const T wy = w[6 + y0], wz = w[12 + z0];
-        T sw = 0, sdw = 0;
-#pragma unroll
-        for (int dx = 0; dx < 6; ++dx) {
-          sw += fm[u][dx] * w[dx];
-          if (FORCES) sdw += fm[u][dx] * ws.dw[j * 18 + dx];
-        }
-        v[u * NQ] = sw * wy * wz;
-        if (FORCES) {
-          v[u * NQ + 1] = sdw * wy * wz;
-          v[u * NQ + 2] = sw * ws.dw[j * 18 + 6 + y0] * wz;
-          v[u * NQ + 3] = sw * wy * ws.dw[j * 18 + 12 + z0];
-        }
-      }
-      const T sum = warp_sum_each<GU * NQ>(v, lane);
-      // to the lanes of the group's atoms: lane l takes quantity l % 4 of atom l / 4
-      const int want = FORCES ? lane - 4 * jb : jt - jb;
-      const T got = __shfl_sync(0xffffffffu, sum, (want * kLanes) & 31);
-      if (want >= 0 && want < GU * NQ) mine = got;
-    }
-    // the last four columns of atom lane / 4
-    T left[NQ] = {};
-    if (jt < na) {
-      const T* w = ws.w + jt * 18;
-      const int* ox = ws.ox + jt * 6;
-      const T wy = w[6 + 5], wz = w[12 + zt];
-      const int oyz = wrap_up(ws.byz[2 * jt] + 5, d.K1) * d.K2 + wrap_up(ws.byz[2 * jt + 1] + zt, d.K2);
-      T sw = 0, sdw = 0;
-#pragma unroll
-      for (int dx = 0; dx < 6; ++dx) {
-        const T f = M[ox[dx] + oyz];
-        sw += f * w[dx];
-        if (FORCES) sdw += f * ws.dw[jt * 18 + dx];
-      }
-      left[0] = sw * wy * wz;
-      if constexpr (FORCES) {
-        left[1] = sdw * wy * wz;
-        left[2] = sw * ws.dw[jt * 18 + 6 + 5] * wz;
-        left[3] = sw * wy * ws.dw[jt * 18 + 12 + zt];
-      }
-    }
+    const T mine = gather_group<T, FORCES>(ws, na, d.K1, d.K2, M, lane);
     if constexpr (!FORCES) {
-      left[0] += __shfl_xor_sync(0xffffffffu, left[0], 1);
-      left[0] += __shfl_xor_sync(0xffffffffu, left[0], 2);
-      if (jt < na && (lane & 3) == 0 && dE_dq) dE_dq[ws.atom[jt]] += mine + left[0];
+      if (jt < na && (lane & 3) == 0 && dE_dq) dE_dq[ws.atom[jt]] += mine;
     } else {
-      // four quantities over four lanes: lane c of the four ends with quantity c
-      const bool hi = (lane & 2) != 0, od = (lane & 1) != 0;
-      const T s0 = hi ? left[0] : left[2], s1 = hi ? left[1] : left[3];
-      const T k0 = (hi ? left[2] : left[0]) + __shfl_xor_sync(0xffffffffu, s0, 2);
-      const T k1 = (hi ? left[3] : left[1]) + __shfl_xor_sync(0xffffffffu, s1, 2);
-      mine += (od ? k1 : k0) + __shfl_xor_sync(0xffffffffu, od ? k0 : k1, 1);
       const bool live = jt < na;
       const int c = lane & 3, ga = live ? ws.atom[jt] : 0;
       if constexpr (TERMS) {

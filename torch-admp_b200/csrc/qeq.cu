@@ -4,6 +4,7 @@
 #include <vector>
 
 #include "pme_host.h"
+#include "qeq_cg.cuh"
 #include "qeq_kernels.cuh"
 
 namespace admp {
@@ -17,8 +18,10 @@ struct QEqWS {
   T* green;
   double* acc;
   double *x, *r, *diag, *zc, *chi_eff, *hx;
-  T *p, *Hp, *coef;
+  T *p, *Hp;
+  PairList<T> list;
   CGScal* sc;
+  CgShared* cg;
   size_t bytes;
 };
 
@@ -53,8 +56,11 @@ static int qeq_carve(QEqWS<T>& w, void* ws, size_t bytes, int nf, int N, long lo
   w.hx = c.take<double>(NT);
   w.p = c.take<T>(NT);
   w.Hp = c.take<T>(NT);
-  w.coef = c.take<T>(P > 0 ? P : 0);
+  w.list.ij = c.take<int2>(P > 0 ? P : 0);
+  w.list.coef = c.take<T>(P > 0 ? P : 0);
+  w.list.n = c.take<unsigned long long>(1);
   w.sc = c.take<CGScal>(nf);
+  w.cg = c.take<CgShared>(1);
   w.bytes = c.off;
   return ADMP_OK;
 }
@@ -85,14 +91,102 @@ static int qeq_matvec(QEqCtx<T>& c, const T* v, T* Hv, double* hv_out) {
     if (s) return s;
   }
   if (c.Pn > 0 && (c.P.flags & (ADMP_QEQ_RSPACE | ADMP_QEQ_DAMPING))) {
-    long long blocks = (c.Pn + 255) / 256;
+    long long blocks = (c.Pn + 511) / 512;  // about half of a full list's pairs are kept
     if (blocks > 4096) blocks = 4096;
-    qeq_coo_spmv_kernel<T><<<(unsigned)blocks, 256, 0, c.st>>>(c.Pn, c.pairs, c.w.coef, v, Hv, c.w.sc, c.N);
+    qeq_coo_spmv_kernel<T><<<(unsigned)blocks, 256, 0, c.st>>>(c.w.list, v, Hv, c.w.sc, c.N, c.nf);
   }
   qeq_finish_kernel<T><<<b.nblk_atom, 256, 0, c.st>>>(b, c.P, v, Hv, c.w.diag, c.w.zc, c.C, (long long)c.N,
                                                      c.w.sc, hv_out);
   ADMP_CUDA_TRY(cudaGetLastError());
   return ADMP_OK;
+}
+
+// Set-up of the persistent solve (qeq_cg.cuh) of one system: false where its
+// line buffers do not fit a block's shared memory.
+template <typename T>
+static bool cg_plan(const QEqCtx<T>& c, int sms, CgArgs<T>& a, size_t& smem) {
+  const SysDesc& d = c.w.plan.hs[0];
+  const size_t budget = 200 * 1024, cs = sizeof(Cplx<T>);
+  const int cap = (int)(64 * 1024 / cs);  // complex values in a line buffer
+  a.N = c.N;
+  a.K0 = d.K0;
+  a.K1 = d.K1;
+  a.K2 = d.K2;
+  a.buf = 0;
+  a.lz = a.ly = a.lx = 1;
+  if (c.P.flags & ADMP_QEQ_KSPACE) {
+    auto lines = [&](long long total, int K) {
+      long long l = (total + sms - 1) / sms;
+      const int most = cap / K < kCgMaxLines ? cap / K : kCgMaxLines;
+      l = l < most ? l : most;
+      return (int)(l < 1 ? 1 : l);
+    };
+    a.lz = lines(((long long)a.K0 * a.K1 + 1) / 2, a.K2);
+    a.ly = lines((long long)a.K0 * d.K2h, a.K1);
+    a.lx = lines((long long)a.K1 * d.K2h, a.K0);
+    a.buf = a.lz * a.K2 > a.ly * a.K1 ? a.lz * a.K2 : a.ly * a.K1;
+    a.buf = a.buf > a.lx * a.K0 ? a.buf : a.lx * a.K0;
+  }
+  const size_t fft = ((size_t)a.K0 + a.K1 + a.K2 + 2 * (size_t)a.buf) * cs;
+  const size_t st = (WarpStencil<T, false>::bytes() + 15) / 16 * 16 * kCgWarps;
+  const int groups = (c.N + kPw - 1) / kPw, per_warp = (groups + sms * kCgWarps - 1) / (sms * kCgWarps);
+  a.kept = fft + st * per_warp <= budget ? per_warp : 0;
+  smem = fft + st * (a.kept ? a.kept : 1);
+  return smem <= budget;
+}
+
+// The CG iterations by the persistent kernel; `used` is false (and nothing
+// launched) where the multi-kernel loop has to take the solve.
+template <typename T>
+static int cg_persistent(QEqCtx<T>& c, CGScal* h, bool& used) {
+  used = false;
+  if (c.nf != 1) return ADMP_OK;
+  int dev = 0, sms = 0, coop = 0;
+  ADMP_CUDA_TRY(cudaGetDevice(&dev));
+  ADMP_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  ADMP_CUDA_TRY(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+  CgArgs<T> a{};
+  size_t smem = 0;
+  if (!coop || !cg_plan<T>(c, sms, a, smem)) return ADMP_OK;
+  ADMP_CUDA_TRY(ensure_smem(qeq_cg_kernel<T>, smem));
+  int per_sm = 0;
+  ADMP_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, qeq_cg_kernel<T>, kCgThreads, smem));
+  if (per_sm < 1) return ADMP_OK;
+  a.kappa = c.w.plan.hs[0].kappa;
+  a.P = c.P;
+  a.pos = c.pos;
+  a.box = c.box;
+  a.C = c.C;
+  a.green = c.w.green;
+  a.diag = c.w.diag;
+  a.zc = c.w.zc;
+  a.mesh = c.w.mesh;
+  a.p = c.w.p;
+  a.Hp = c.w.Hp;
+  a.spec = c.w.spec;
+  a.x = c.w.x;
+  a.r = c.w.r;
+  a.list = c.w.list;
+  a.have_pairs = c.Pn > 0 && (c.P.flags & (ADMP_QEQ_RSPACE | ADMP_QEQ_DAMPING));
+  a.sc = c.w.sc;
+  a.sh = c.w.cg;
+  used = true;
+  // the mesh holds the potential of the initial charges
+  if (c.P.flags & ADMP_QEQ_KSPACE)
+    ADMP_CUDA_TRY(cudaMemsetAsync(c.w.mesh, 0, sizeof(T) * (size_t)a.K0 * a.K1 * a.K2, c.st));
+  ADMP_CUDA_TRY(cudaMemsetAsync(c.w.cg, 0, sizeof(CgShared), c.st));
+  for (a.k0 = 0;; a.k0 = h->iter) {
+    a.k1 = a.k0 + kCgLaunch;
+    if (a.k0) ADMP_CUDA_TRY(cudaMemsetAsync(&c.w.cg->arrived, 0, sizeof(unsigned), c.st));
+    void* args[] = {&a};
+    ADMP_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)qeq_cg_kernel<T>, dim3(sms), dim3(kCgThreads), args, smem,
+                                              c.st));
+    count_launches(1);
+    const void* p = read_back(c.w.sc, sizeof(CGScal), c.st);
+    if (!p) return ADMP_ERR_CUDA;
+    *h = *(const CGScal*)p;
+    if (h->done || h->status || h->iter >= c.P.max_iter + kCgLaunch) return ADMP_OK;
+  }
 }
 
 template <typename T>
@@ -115,8 +209,9 @@ static int qeq_prepare(QEqCtx<T>& c, const T* chi, const T* hard, const T* eta, 
     DevError* err = scratch_error(c.st);
     long long blocks = (c.Pn + 255) / 256;
     if (blocks > 4096) blocks = 4096;
+    ADMP_CUDA_TRY(cudaMemsetAsync(c.w.list.n, 0, sizeof(*c.w.list.n), c.st));
     qeq_pair_coef_kernel<T><<<(unsigned)blocks, 256, 0, c.st>>>(c.N * c.nf, c.Pn, c.P.flags, kappa, c.P.ke, c.pairs,
-                                                                ds, bs, eta, c.w.coef, err);
+                                                                ds, bs, eta, c.w.list, err);
   }
   ADMP_CUDA_TRY(cudaGetLastError());
   return ADMP_OK;
@@ -187,7 +282,10 @@ static int qeq_solve_impl(int flags, int nf, int N, const int* kmesh, const T* p
   const int chunk = 8;
   int it = 0;
   std::vector<CGScal> h(nf);
-  while (true) {
+  bool persistent = false;
+  s = cg_persistent<T>(c, h.data(), persistent);
+  if (s) return s;
+  while (!persistent) {
     for (int k = 0; k < chunk; ++k) {
       qeq_rotate_kernel<<<(nf + 31) / 32, 32, 0, st>>>(b, c.w.sc);
       s = qeq_matvec<T>(c, c.w.p, c.w.Hp, nullptr);
@@ -209,7 +307,7 @@ static int qeq_solve_impl(int flags, int nf, int N, const int* kmesh, const T* p
   for (int f = 0; f < nf; ++f) {
     if (iters) iters[f] = h[f].iter;
     if (resid) resid[f] = sqrt(h[f].rr_new > 0 ? h[f].rr_new : h[f].rr) / (N > 0 ? N : 1);
-    const int stf = h[f].done ? h[f].status : ADMP_ERR_NOT_CONVERGED;
+    const int stf = h[f].done || h[f].status ? h[f].status : ADMP_ERR_NOT_CONVERGED;
     if (stf && (worst == ADMP_OK || worst == ADMP_ERR_NOT_CONVERGED)) {
       worst = stf;
       worst_f = f;

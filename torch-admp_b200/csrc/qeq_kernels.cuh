@@ -183,48 +183,98 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// COO pair coefficients of J (drop-in list; pairs with scale 0 get 0).
+// The non-zero pair entries of J, compacted: (i, j) as 32-bit indices over the
+// frames' atoms and the coefficient.  A caller's full list has scale 0 on half
+// of its pairs and 16 bytes of indices on each; the CG reads the list once per
+// iteration.  A block's entries stay in the list's order, so that pairs with
+// the same first atom follow each other.
+template <typename T>
+struct PairList {
+  int2* ij;
+  T* coef;
+  unsigned long long* n;  // entries
+};
+
 template <typename T>
 __global__ void __launch_bounds__(256)
     qeq_pair_coef_kernel(int N, long long Pn, int flags, double kappa, double ke, const long long* __restrict__ pairs,
                          const T* __restrict__ ds, const T* __restrict__ bs, const T* __restrict__ eta,
-                         T* __restrict__ coef, DevError* err) {
-  for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < Pn; p += (long long)gridDim.x * blockDim.x) {
-    const long long i = pairs[2 * p], j = pairs[2 * p + 1];
+                         PairList<T> out, DevError* err) {
+  __shared__ int wsum[8];
+  __shared__ unsigned long long base;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (long long p0 = blockIdx.x * (long long)blockDim.x; p0 < Pn; p0 += (long long)gridDim.x * blockDim.x) {
+    const long long p = p0 + threadIdx.x;
+    long long i = 0, j = 0;
     double c = 0.0;
-    if (i < 0 || i >= N || j < 0 || j >= N) {
-      report_error(err, ADMP_ERR_BAD_INDEX, 5, p);
-    } else {
-      const double dd = ds[p], s = bs[p];
-      const double inv = fabs(dd) > 1e-4 ? 1.0 / dd : 0.0;
-      if (s != 0.0 && inv != 0.0) {
-        if (flags & ADMP_QEQ_RSPACE) c += erfc(kappa * dd);
-        if (flags & ADMP_QEQ_DAMPING) {
-          const double ei = eta[i], ej = eta[j];
-          double eij = sqrt((ei * ei + ej * ej) / 2.0);
-          if (eij == 0.0) eij = 1e-10;
-          c -= erfc(dd / (2.0 * eij));
+    if (p < Pn) {
+      const longlong2 ij = load_pair(pairs, p);
+      i = ij.x;
+      j = ij.y;
+      if (i < 0 || i >= N || j < 0 || j >= N) {
+        report_error(err, ADMP_ERR_BAD_INDEX, 5, p);
+      } else {
+        const double dd = ds[p], s = bs[p];
+        const double inv = fabs(dd) > 1e-4 ? 1.0 / dd : 0.0;
+        if (s != 0.0 && inv != 0.0) {
+          if (flags & ADMP_QEQ_RSPACE) c += erfc(kappa * dd);
+          if (flags & ADMP_QEQ_DAMPING) {
+            const double ei = eta[i], ej = eta[j];
+            double eij = sqrt((ei * ei + ej * ej) / 2.0);
+            if (eij == 0.0) eij = 1e-10;
+            c -= erfc(dd / (2.0 * eij));
+          }
+          c *= ke * s * inv;
         }
-        c *= ke * s * inv;
       }
     }
-    coef[p] = (T)c;
+    const T ct = (T)c;
+    const unsigned have = __ballot_sync(0xffffffffu, ct != T(0));
+    if (lane == 0) wsum[warp] = __popc(have);
+    __syncthreads();
+    int before = 0, total = 0;
+    for (int w = 0; w < 8; ++w) {
+      before += w < warp ? wsum[w] : 0;
+      total += wsum[w];
+    }
+    if (threadIdx.x == 0 && total) base = atomicAdd(out.n, (unsigned long long)total);
+    __syncthreads();
+    if (ct != T(0)) {
+      const size_t k = base + before + __popc(have & ((1u << lane) - 1u));
+      out.ij[k] = make_int2((int)i, (int)j);
+      out.coef[k] = ct;
+    }
   }
 }
 
-// Hv[i] += c_p v[j], Hv[j] += c_p v[i]  (COO over the frames of a batch:
-// atom i belongs to frame i / natoms, whose CG state is sc[i / natoms])
+// Hv[i] += c v[j], Hv[j] += c v[i] over the compacted entries of all frames
+// (atom i belongs to frame i / natoms, whose CG state is sc[i / natoms]).  The
+// first atom's share is summed over its run of entries, one atomic a run.
+//
+// With two atomics an entry over the caller's list, 64 frames of 3,000 atoms
+// (17 M pairs, half of them scale 0; FP32) took 150 us, now 44 us.
 template <typename T>
 __global__ void __launch_bounds__(256)
-    qeq_coo_spmv_kernel(long long Pn, const long long* __restrict__ pairs, const T* __restrict__ coef,
-                        const T* __restrict__ v, T* __restrict__ Hv, const CGScal* __restrict__ sc, int natoms) {
-  for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < Pn; p += (long long)gridDim.x * blockDim.x) {
-    const T c = coef[p];
-    if (c == T(0)) continue;
-    const long long i = pairs[2 * p], j = pairs[2 * p + 1];
-    if (sc[i / natoms].done) continue;
-    atomicAdd(Hv + i, c * v[j]);
-    atomicAdd(Hv + j, c * v[i]);
+    qeq_coo_spmv_kernel(PairList<T> list, const T* __restrict__ v, T* __restrict__ Hv, const CGScal* __restrict__ sc,
+                        int natoms, int nf) {
+  const long long n = (long long)*list.n;
+  const int lane = threadIdx.x & 31;
+  if (nf == 1 && sc[0].done) return;
+  for (long long p0 = blockIdx.x * (long long)blockDim.x + (threadIdx.x & ~31); p0 < n;
+       p0 += (long long)gridDim.x * blockDim.x) {
+    const long long p = p0 + lane;
+    int2 ij = make_int2(-1, -1);
+    T c = T(0);
+    if (p < n) {
+      ij = list.ij[p];
+      c = list.coef[p];
+      if (nf > 1 && sc[ij.x / natoms].done) c = T(0);
+    }
+    const bool on = c != T(0);
+    const WarpRuns runs(ij.x, lane);
+    const T a = runs.sum(on ? c * v[ij.y] : T(0));
+    if (runs.opens && a != T(0)) atomicAdd(Hv + ij.x, a);
+    if (on) atomicAdd(Hv + ij.y, c * v[ij.x]);
   }
 }
 
