@@ -165,6 +165,16 @@ int admp_coulomb_pbc(int dtype, int flags, int nframes, int natoms, const int* k
                      double ke, void* energy, double* comps, void* dE_dpos, void* dE_dq,
                      void* dE_dbox, void* dE_dds, void* workspace, size_t workspace_bytes,
                      void* stream);
+/* Gaussian damping energy, pairs and self part (qeq.py:60-129), and chemical */
+/* site energy (qeq.py:159-209) of nframes systems.  As admp_coulomb_pbc they */
+/* WRITE their outputs: energy [nframes] double and the gradients not NULL.   */
+int admp_damping_energy(int dtype, int nframes, int natoms, long long npairs,
+                        const long long* pairs, const void* ds, const void* buffer_scales,
+                        const void* q, const void* eta, double ke, double* energy, void* dE_dds,
+                        void* dE_dq, void* dE_deta, void* stream);
+int admp_site_energy(int dtype, int nframes, int natoms, const void* q, const void* chi,
+                     const void* hardness, double* energy, void* dE_dq, void* dE_dchi,
+                     void* dE_dhard, void* stream);
 /* Copies up to 64 KiB of device memory to `host` through page-locked staging */
 /* and waits for it.                                                          */
 int admp_read_back(const void* dev, size_t bytes, void* host, void* stream);
@@ -269,6 +279,7 @@ int admp_image_pair_distances_backward(int dtype, int natoms, long long npairs,
 #define ADMP_QEQ_DAMPING 4
 #define ADMP_QEQ_SLAB 8         /* slab axis in bits 8..9 */
 #define ADMP_QEQ_PROJECT_Q0 16  /* project the initial guess onto C q = b first */
+#define ADMP_QEQ_DEVICE_B 32    /* b is DEVICE memory (the host need not wait for it) */
 size_t admp_qeq_workspace_size(int dtype, int natoms, long long npairs, const int* kmesh,
                                int n_const);
 int admp_qeq_solve(int dtype, int flags, int natoms, const int* kmesh, const void* pos,

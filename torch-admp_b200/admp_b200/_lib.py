@@ -36,6 +36,7 @@ F64, F32 = 0, 1
 PAIR_EWALD, PAIR_OBC, PAIR_DAMPING = 0, 1, 2
 TERM_SELF, TERM_NON_NEUTRAL, TERM_SLAB, TERM_DAMP_SELF, TERM_SITE = 1, 2, 4, 8, 16
 QEQ_KSPACE, QEQ_RSPACE, QEQ_DAMPING, QEQ_SLAB, QEQ_PROJECT_Q0 = 1, 2, 4, 8, 16
+QEQ_DEVICE_B = 32
 
 EXPORTS = [
     "admp_abi_version", "admp_status_string", "admp_last_error_message", "admp_set_sync_checks",
@@ -50,6 +51,7 @@ EXPORTS = [
     "admp_image_nblist_fill", "admp_image_pair_distances", "admp_image_pair_distances_backward",
     "admp_nblist_frames_workspace_size", "admp_nblist_frames_count", "admp_nblist_frames_fill",
     "admp_pair_distances_frames_backward", "admp_coulomb_pbc", "admp_read_back",
+    "admp_damping_energy", "admp_site_energy",
 ]
 PROFILE_KERNELS = ["spread", "fft_z_fwd", "fft_y_fwd", "fft_x_green", "fft_y_inv", "fft_z_inv", "gather", "pair_ef",
                    "csr_spmv", "neighbors", "cg_vector", "tc_z_fwd", "tc_y_fwd", "tc_x", "tc_y_inv", "tc_z_inv"]
@@ -79,6 +81,8 @@ _SIGS = {
     "admp_pair_distances_frames_backward": (_i, [_i, _i, _i, _i, _ll, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
     "admp_coulomb_pbc": (_i, [_i, _i, _i, _i, _ip, _vp, _vp, _ll, _vp, _vp, _vp, _vp, _d, _d, _vp, _vp, _vp, _vp, _vp,
                               _vp, _vp, _sz, _vp]),
+    "admp_damping_energy": (_i, [_i, _i, _i, _ll, _vp, _vp, _vp, _vp, _vp, _d, _vp, _vp, _vp, _vp, _vp]),
+    "admp_site_energy": (_i, [_i, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
     "admp_read_back": (_i, [_vp, _sz, _vp, _vp]),
     "admp_nblist_count": (_i, [_i, _i, _i, _vp, _vp, _d, _vp, _sz, _llp, _vp]),
     "admp_nblist_fill": (_i, [_i, _i, _i, _vp, _vp, _d, _vp, _sz, _vp, _vp, _ll, _vp]),
@@ -195,6 +199,21 @@ def profile_read() -> dict:
 
 def workspace(nbytes: int, device) -> torch.Tensor:
     return torch.empty(max(int(nbytes), 1), dtype=torch.uint8, device=device)
+
+
+def constraint_values(b, n_const: int):
+    """(flag, pointer, keep-alive) of the n_const constraint values of a QEq
+    call: device values stay on the device, so that the host need not wait."""
+    if n_const == 0:
+        arr = (ctypes.c_double * 1)(0.0)
+        return 0, arr, arr
+    if b.is_cuda:
+        t = b.detach().reshape(-1).to(torch.float64).contiguous()
+        if t.numel() < n_const:
+            raise IndexError(f"{n_const} constraints need as many values, got {t.numel()}")
+        return QEQ_DEVICE_B, ctypes.cast(t.data_ptr(), _dp), t
+    arr = (ctypes.c_double * n_const)(*[float(v) for v in b.detach().reshape(-1).tolist()])
+    return 0, arr, arr
 
 
 def int3(vals):

@@ -151,7 +151,7 @@ def infer(calculator: PolarizableElectrode, positions, box, charges, pairs, ds, 
                                      eta, chi, hardness, constraint_matrix, constraint_vals, ffield_electrode_mask,
                                      ffield_potential, method)
     q_opt = charges.detach().clone()
-    q_opt[electrode_mask] = _q.detach().to(q_opt.dtype)
+    q_opt.masked_scatter_(electrode_mask, _q.detach().to(q_opt.dtype))
     energy, forces = calculator.coulomb_calculator(positions=positions, box=box, charges=q_opt, eta=eta, pairs=pairs,
                                                    ds=ds, buffer_scales=buffer_scales, efield=efield)
     return energy, forces, q_opt
@@ -162,13 +162,14 @@ def charge_optimization(calculator: PolarizableElectrode, positions, box, charge
                         ffield_electrode_mask, ffield_potential, method: str = "lbfgs"):
     """QEq on the electrode sub-system (electrode.py:456-560)."""
     device, dtype = positions.device, positions.dtype
-    if electrode_mask.sum() == 0:
+    idx = torch.nonzero(electrode_mask).reshape(-1)
+    if idx.numel() == 0:
         return charges[electrode_mask], None
     if ffield_electrode_mask is not None and calculator.slab_corr:
         raise ValueError("Slab correction and finite field cannot be used together.")
     chi_elec, _ = calculator.calc_coulomb_potential(electrode_mask, positions, box, eta, charges, pairs, ds,
                                                     buffer_scales)
-    chi_t = (chi + chi_elec.detach())[electrode_mask]
+    chi_t = (chi + chi_elec.detach())[idx]
     efield = None
     if ffield_electrode_mask is not None:
         chi_ff, _ef = finite_field_add_chi(positions.detach(), box.detach(), ffield_electrode_mask, ffield_potential,
@@ -176,14 +177,15 @@ def charge_optimization(calculator: PolarizableElectrode, positions, box, charge
         chi_t = chi_t + chi_ff
         efield = torch.zeros(3, dtype=dtype, device=device)
         efield[calculator.slab_axis] = _ef
-    pair_mask = electrode_mask[pairs[:, 0]] & electrode_mask[pairs[:, 1]]
-    idx = torch.nonzero(electrode_mask).reshape(-1)
-    mapping = torch.zeros(electrode_mask.size(0), dtype=torch.long, device=device)
+    # rows with both atoms on the electrodes, in electrode indices (index lists are made once: every boolean
+    # mask would count its elements on the device and wait for the count)
+    mapping = torch.full((electrode_mask.size(0),), -1, dtype=torch.long, device=device)
     mapping[idx] = torch.arange(idx.numel(), device=device, dtype=torch.long)
-    sub_pairs = torch.stack([mapping[pairs[pair_mask][:, 0]], mapping[pairs[pair_mask][:, 1]]], dim=1)
-    kw = dict(module=calculator, positions=positions.detach()[electrode_mask], box=box.detach(), chi=chi_t,
-              hardness=hardness[electrode_mask], eta=eta[electrode_mask], pairs=sub_pairs,
-              ds=ds.detach()[pair_mask], buffer_scales=buffer_scales[pair_mask],
+    local = mapping[pairs]
+    rows = torch.nonzero((local >= 0).all(1)).reshape(-1)
+    kw = dict(module=calculator, positions=positions.detach()[idx], box=box.detach(), chi=chi_t,
+              hardness=hardness[idx], eta=eta[idx], pairs=local[rows],
+              ds=ds.detach()[rows], buffer_scales=buffer_scales[rows],
               constraint_matrix=constraint_matrix if constraint_matrix is not None and constraint_matrix.shape[0] > 0
               else None,
               constraint_vals=constraint_vals if constraint_matrix is not None and constraint_matrix.shape[0] > 0
@@ -191,5 +193,5 @@ def charge_optimization(calculator: PolarizableElectrode, positions, box, charge
     if method == "matinv":
         _e, q = matinv_optimize(**kw)
     else:
-        _e, q = pgrad_optimize(q0=charges.detach()[electrode_mask].reshape(-1), method=method, reinit_q=True, **kw)
+        _e, q = pgrad_optimize(q0=charges.detach()[idx].reshape(-1), method=method, reinit_q=True, **kw)
     return q, efield

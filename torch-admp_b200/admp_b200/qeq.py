@@ -40,7 +40,11 @@ class GaussianDampingForceModule(BaseForceModule):
         nf, na = positions.size(0), positions.size(1)
         dt = positions.dtype
         q = params["charge"].reshape(nf, na).to(dt)
-        eta = (params["eta"].reshape(nf, na) * self.const_lib.length_coeff).to(dt)
+        eta = params["eta"].reshape(nf, na)
+        lc = self.const_lib.length_coeff
+        if lc != 1.0:
+            eta = eta * lc
+        eta = eta.to(dt)
         return torch.ops.admp_b200.damping(ds.to(dt), q, eta, pairs, buffer_scales.to(dt), self.const_lib.dielectric)
 
 
@@ -56,8 +60,13 @@ class SiteForceModule(BaseForceModule):
         nf, na = positions.size(0), positions.size(1)
         dt = positions.dtype
         ec = self.const_lib.energy_coeff
-        chi = (params["chi"].reshape(nf, na) * ec).to(dt)
-        hard = (params["hardness"].reshape(nf, na) * ec).to(dt)
+        chi = params["chi"].reshape(nf, na)
+        hard = params["hardness"].reshape(nf, na)
+        if ec != 1.0:
+            chi = chi * ec
+            hard = hard * ec
+        chi = chi.to(dt)
+        hard = hard.to(dt)
         q = params["charge"].reshape(nf, na).to(dt)
         return torch.ops.admp_b200.site(q, chi, hard)
 
@@ -190,14 +199,19 @@ def _kkt(hessian, chi, C, b):
     return torch.linalg.solve(A, rhs.reshape(-1, 1)).reshape(-1)[:n]
 
 
+def _times(t, c: float):
+    """t * c without a kernel for unit coefficients (Angstrom / eV, the default units)."""
+    return t if t is None or c == 1.0 else t * c
+
+
 def _std_inputs(module, positions, box, pairs, ds, buffer_scales, *vecs):
     dt = positions.dtype
     L.require_cuda(positions, "positions")
     lc = module.const_lib.length_coeff
-    pos = prep_float(positions.detach() * lc, dt)
-    bx = prep_float(box.detach() * lc, dt)
+    pos = prep_float(_times(positions.detach(), lc), dt)
+    bx = prep_float(_times(box.detach(), lc), dt)
     pr = pairs.to(torch.long).contiguous()
-    dsc = prep_float(ds.detach() * lc, dt)
+    dsc = prep_float(_times(ds.detach(), lc), dt)
     bsc = prep_float(buffer_scales, dt)
     out = [None if v is None else prep_float(v.detach().reshape(-1), dt) for v in vecs]
     return pos, bx, pr, dsc, bsc, out
@@ -219,8 +233,8 @@ def _qeq_solve_raw(module, q0, positions, box, chi, hardness, eta, pairs, ds, bu
         raise ValueError("admp_b200 QEq solve needs a periodic box")
     ec = module.const_lib.energy_coeff
     pos, bx, pr, dsc, bsc, (chi_c, hard_c, eta_c, sh, qv) = _std_inputs(
-        module, positions, box, pairs, ds, buffer_scales, chi * ec, hardness * ec,
-        eta * module.const_lib.length_coeff if eta is not None else None, shift, q0)
+        module, positions, box, pairs, ds, buffer_scales, _times(chi.detach(), ec), _times(hardness.detach(), ec),
+        _times(eta.detach(), module.const_lib.length_coeff) if eta is not None else None, shift, q0)
     n = pos.shape[0]
     dt = pos.dtype
     dev = pos.device
@@ -235,7 +249,8 @@ def _qeq_solve_raw(module, q0, positions, box, chi, hardness, eta, pairs, ds, bu
     P = pr.shape[0]
     nc = 0 if C is None else int(C.shape[0])
     Cc = prep_float(C.detach().reshape(nc, n), dt) if nc else None
-    bvals = (ctypes.c_double * max(nc, 1))(*([float(v) for v in b.detach().reshape(-1).tolist()] if nc else [0.0]))
+    bflag, bvals, _keep_b = L.constraint_values(b, nc)
+    flags |= bflag
     nbytes = lib.admp_qeq_workspace_size(L.dtype_code(dt), n, P, kp if c.kspace_flag else None, nc)
     ws = L.workspace(nbytes, dev)
     q = qv.clone()
@@ -260,8 +275,8 @@ def _hessian(module, positions, box, hardness, eta, pairs, ds, buffer_scales, ma
     lib = L.load()
     ec = module.const_lib.energy_coeff
     pos, bx, pr, dsc, bsc, (hard_c, eta_c) = _std_inputs(
-        module, positions, box, pairs, ds, buffer_scales, hardness * ec,
-        eta * module.const_lib.length_coeff if eta is not None else None)
+        module, positions, box, pairs, ds, buffer_scales, _times(hardness.detach(), ec),
+        _times(eta.detach(), module.const_lib.length_coeff) if eta is not None else None)
     n = pos.shape[0]
     dt, dev = pos.dtype, pos.device
     if eta_c is None:
@@ -451,16 +466,16 @@ def _qeq_solve_frames_raw(module, q0, positions, box, chi, hardness, eta, pairs,
     dev = positions.device
     ec = module.const_lib.energy_coeff
     lc = module.const_lib.length_coeff
-    pos = prep_float(positions.detach() * lc, dt)
-    bx = prep_float(box.detach().reshape(nf, 3, 3) * lc, dt)
+    pos = prep_float(_times(positions.detach(), lc), dt)
+    bx = prep_float(_times(box.detach().reshape(nf, 3, 3), lc), dt)
     P = int(pairs.shape[1])
     offs = (torch.arange(nf, device=dev, dtype=torch.long) * n).view(nf, 1, 1)
     prg = (pairs.to(torch.long) + offs).reshape(-1, 2).contiguous()
-    dsc = prep_float(ds.detach() * lc, dt).reshape(-1)
+    dsc = prep_float(_times(ds.detach(), lc), dt).reshape(-1)
     bsc = prep_float(buffer_scales.reshape(nf, P), dt).reshape(-1)
-    chi_c = _frames_vec(chi * ec, nf, n, dt)
-    hard_c = _frames_vec(hardness * ec, nf, n, dt)
-    eta_c = _frames_vec(eta * lc, nf, n, dt) if eta is not None else torch.zeros(nf * n, dtype=dt, device=dev)
+    chi_c = _frames_vec(_times(chi.detach(), ec), nf, n, dt)
+    hard_c = _frames_vec(_times(hardness.detach(), ec), nf, n, dt)
+    eta_c = _frames_vec(_times(eta.detach(), lc), nf, n, dt) if eta is not None else torch.zeros(nf * n, dtype=dt, device=dev)
     sh = _frames_vec(shift, nf, n, dt) if shift is not None else None
     q = _frames_vec(q0, nf, n, dt).clone()
     flags = module._flags()
@@ -474,7 +489,8 @@ def _qeq_solve_frames_raw(module, q0, positions, box, chi, hardness, eta, pairs,
     kp, _keep = L.int3([k for row in km for k in row])
     nc = 0 if C is None else int(C.shape[0])
     Cc = prep_float(C.detach().reshape(nc, n), dt) if nc else None
-    bvals = (ctypes.c_double * max(nc, 1))(*([float(v) for v in b.detach().reshape(-1).tolist()] if nc else [0.0]))
+    bflag, bvals, _keep_b = L.constraint_values(b, nc)
+    flags |= bflag
     nbytes = lib.admp_qeq_frames_workspace_size(L.dtype_code(dt), nf, n, nf * P, kp if c.kspace_flag else None, nc)
     if nbytes == 0:
         L.check(L.BAD_ARG, f"QEq workspace for {nf} frames")

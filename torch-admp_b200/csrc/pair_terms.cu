@@ -217,6 +217,38 @@ __global__ void __launch_bounds__(512)
   }
 }
 
+// Damping self energies (DAMP: q, eta) or chemical site energies (q, chi,
+// hardness) of every atom: gradients are written, energies summed into
+// energy[frame].  A block per 256 atoms (one block a frame, two passes over the
+// atoms, took 20 us at 20,000 atoms).
+template <typename T, bool DAMP>
+__global__ void __launch_bounds__(256)
+    atom_energy_kernel(int N, const T* __restrict__ q, const T* __restrict__ u, const T* __restrict__ w, double ke,
+                       double* __restrict__ energy, T* __restrict__ dq, T* __restrict__ du, T* __restrict__ dw) {
+  __shared__ double red[32];
+  const int f = blockIdx.y, i = blockIdx.x * blockDim.x + threadIdx.x;
+  double v[1] = {0.0};
+  if (i < N) {
+    const size_t a = (size_t)f * N + i;
+    const double qi = q[a];
+    if (DAMP) {
+      const double e = u[a];
+      const bool ok = fabs(e) > 1e-4;
+      const double einv = ok ? 1.0 / e : 0.0;
+      v[0] = ke * einv / (2.0 * kSqrtPi) * qi * qi;
+      if (dq) dq[a] = (T)(ke * qi * einv / kSqrtPi);
+      if (du) du[a] = (T)(ok ? -ke * qi * qi / (2.0 * kSqrtPi) * einv * einv : 0.0);
+    } else {
+      const double chi = u[a], hard = w[a];
+      v[0] = chi * qi + hard * qi * qi;
+      if (dq) dq[a] = (T)(chi + 2.0 * hard * qi);
+      if (du) du[a] = (T)qi;
+      if (dw) dw[a] = (T)(qi * qi);
+    }
+  }
+  block_atomic_sum<1>(v, energy + f, red);
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256)
     pair_dist_kernel(int pbc, int N, long long P, const long long* __restrict__ pairs,
@@ -477,4 +509,56 @@ extern "C" int admp_pair_distances_frames_backward(int dtype, int pbc, int nfram
   DevError* err = scratch_error(st);
   if (!err) return ADMP_ERR_CUDA;
   return pair_dist_bwd(dtype, pbc, nframes, natoms, npairs, pairs, pos, box, grad_ds, grad_pos, grad_box, err, st);
+}
+
+extern "C" int admp_damping_energy(int dtype, int nframes, int natoms, long long npairs, const long long* pairs,
+                                   const void* ds, const void* buffer_scales, const void* q, const void* eta, double ke,
+                                   double* energy, void* dE_dds, void* dE_dq, void* dE_deta, void* stream) {
+  if (nframes <= 0 || nframes > 65535 || natoms <= 0 || npairs < 0 || !q || !eta || !energy)
+    return fail(ADMP_ERR_BAD_ARG, "admp_damping_energy: args");
+  if (npairs > 0 && (!pairs || !ds || !buffer_scales)) return fail(ADMP_ERR_BAD_ARG, "admp_damping_energy: pairs");
+  if (dtype != ADMP_F64 && dtype != ADMP_F32) return fail(ADMP_ERR_BAD_ARG, "bad dtype");
+  cudaStream_t st = (cudaStream_t)stream;
+  DevError* err = scratch_error(st);
+  if (!err) return ADMP_ERR_CUDA;
+  ADMP_CUDA_TRY(cudaMemsetAsync(energy, 0, sizeof(double) * nframes, st));
+  const dim3 grid((natoms + 255) / 256, nframes);
+  int s;
+  if (dtype == ADMP_F64) {
+    atom_energy_kernel<double, true><<<grid, 256, 0, st>>>(natoms, (const double*)q, (const double*)eta, nullptr, ke,
+                                                           energy, (double*)dE_dq, (double*)dE_deta, nullptr);
+    s = launch_pair_energy<double>(ADMP_PAIR_DAMPING, nframes, natoms, npairs, pairs, (const double*)ds,
+                                   (const double*)buffer_scales, (const double*)q, (const double*)eta, 0.0, ke, energy,
+                                   1, true, (double*)dE_dds, (double*)dE_dq, (double*)dE_deta, err, st);
+  } else {
+    atom_energy_kernel<float, true><<<grid, 256, 0, st>>>(natoms, (const float*)q, (const float*)eta, nullptr, ke,
+                                                          energy, (float*)dE_dq, (float*)dE_deta, nullptr);
+    s = launch_pair_energy<float>(ADMP_PAIR_DAMPING, nframes, natoms, npairs, pairs, (const float*)ds,
+                                  (const float*)buffer_scales, (const float*)q, (const float*)eta, 0.0, ke, energy, 1,
+                                  true, (float*)dE_dds, (float*)dE_dq, (float*)dE_deta, err, st);
+  }
+  ADMP_CUDA_TRY(cudaGetLastError());
+  return s || npairs == 0 ? s : check_error(err, st);
+}
+
+extern "C" int admp_site_energy(int dtype, int nframes, int natoms, const void* q, const void* chi,
+                                const void* hardness, double* energy, void* dE_dq, void* dE_dchi, void* dE_dhard,
+                                void* stream) {
+  if (nframes <= 0 || nframes > 65535 || natoms <= 0 || !q || !chi || !hardness || !energy)
+    return fail(ADMP_ERR_BAD_ARG, "admp_site_energy: args");
+  cudaStream_t st = (cudaStream_t)stream;
+  ADMP_CUDA_TRY(cudaMemsetAsync(energy, 0, sizeof(double) * nframes, st));
+  const dim3 grid((natoms + 255) / 256, nframes);
+  if (dtype == ADMP_F64)
+    atom_energy_kernel<double, false><<<grid, 256, 0, st>>>(natoms, (const double*)q, (const double*)chi,
+                                                            (const double*)hardness, 0.0, energy, (double*)dE_dq,
+                                                            (double*)dE_dchi, (double*)dE_dhard);
+  else if (dtype == ADMP_F32)
+    atom_energy_kernel<float, false><<<grid, 256, 0, st>>>(natoms, (const float*)q, (const float*)chi,
+                                                           (const float*)hardness, 0.0, energy, (float*)dE_dq,
+                                                           (float*)dE_dchi, (float*)dE_dhard);
+  else
+    return fail(ADMP_ERR_BAD_ARG, "bad dtype");
+  ADMP_CUDA_TRY(cudaGetLastError());
+  return ADMP_OK;
 }

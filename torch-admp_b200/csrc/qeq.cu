@@ -249,8 +249,9 @@ static int qeq_solve_impl(int flags, int nf, int N, const int* kmesh, const T* p
   s = qeq_prepare<T>(c, chi, hard, eta, shift, ds, bs, kappa);
   if (s) return s;
   double bv[4] = {0, 0, 0, 0};
-  for (int k = 0; k < nc; ++k) bv[k] = bvals[k];
-  qeq_set_b_kernel<<<sb, 64, 0, st>>>(nf, c.w.sc, nc, bv[0], bv[1], bv[2], bv[3]);
+  const bool dev_b = (flags & ADMP_QEQ_DEVICE_B) != 0;
+  for (int k = 0; k < nc && !dev_b; ++k) bv[k] = bvals[k];
+  qeq_set_b_kernel<<<sb, 64, 0, st>>>(nf, c.w.sc, nc, bv[0], bv[1], bv[2], bv[3], dev_b ? bvals : nullptr);
   // x0 (optionally projected onto C x = b)
   const int cb = (int)((NT + 255) / 256 < 2048 ? (NT + 255) / 256 : 2048);
   cast_kernel<T><<<cb > 0 ? cb : 1, 256, 0, st>>>(NT, q, c.w.x);

@@ -476,13 +476,11 @@ __global__ void __launch_bounds__(256)
 
 // Constraint values b (shared by every system of the batch) and their count.
 static __global__ void qeq_set_b_kernel(int nsys, CGScal* __restrict__ sc, int nc, double b0, double b1, double b2,
-                                        double b3) {
+                                        double b3, const double* __restrict__ dev) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= nsys) return;
-  sc[s].b[0] = b0;
-  sc[s].b[1] = b1;
-  sc[s].b[2] = b2;
-  sc[s].b[3] = b3;
+  const double b[kMaxConst] = {b0, b1, b2, b3};
+  for (int c = 0; c < kMaxConst; ++c) sc[s].b[c] = dev ? (c < nc ? dev[c] : 0.0) : b[c];
   sc[s].n_const = nc;
 }
 

@@ -250,37 +250,32 @@ class Damping : public torch::autograd::Function<Damping> {
     const int dt = dtype_code(q);
     void* st = stream_of(q);
     const int64_t nf = q.size(0), N = q.size(1), P = pairs.size(1);
-    const bool need = ds.requires_grad() || q.requires_grad() || eta.requires_grad();
-    Tensor E = f64(nf, q), gds, gq, geta;
-    if (need) {
-      gds = torch::zeros_like(ds);
-      gq = torch::zeros_like(q);
-      geta = torch::zeros_like(eta);
-    }
-    if (P > 0)
-      check(admp_pair_energy(dt, ADMP_PAIR_DAMPING, (int)nf, (int)N, P, ptr<const long long>(pairs), ptr<void>(ds),
-                             ptr<void>(bs), ptr<void>(q), ptr<void>(eta), 0.0, ke, ptr<double>(E), ptr<void>(gds),
-                             ptr<void>(gq), ptr<void>(geta), st),
-            "damping pair energy");
-    if (N > 0)
-      check(admp_atom_terms(dt, ADMP_TERM_DAMP_SELF, (int)nf, (int)N, nullptr, nullptr, ptr<void>(q), ptr<void>(eta),
-                            nullptr, nullptr, 0.0, ke, ptr<double>(E), nullptr, ptr<void>(gq), nullptr, nullptr,
-                            ptr<void>(geta), nullptr, nullptr, st),
-            "damping self energy");
+    Tensor gds, gq, geta;
+    const bool any = nf > 0 && N > 0;
+    // gradients of the inputs that need one; the call writes them
+    auto grad = [&](const Tensor& x) {
+      return !x.requires_grad() ? Tensor() : any ? torch::empty_like(x) : torch::zeros_like(x);
+    };
+    gds = grad(ds);
+    gq = grad(q);
+    geta = grad(eta);
+    Tensor E = any ? torch::empty({nf}, q.options().dtype(torch::kDouble)) : f64(nf, q);
+    if (any)
+      check(admp_damping_energy(dt, (int)nf, (int)N, P, ptr<const long long>(pairs), ptr<void>(ds), ptr<void>(bs),
+                                ptr<void>(q), ptr<void>(eta), ke, ptr<double>(E), ptr<void>(gds), ptr<void>(gq),
+                                ptr<void>(geta), st),
+            "damping energy");
     ctx->save_for_backward({gds, gq, geta});
     return {E.to(q.scalar_type())};
   }
 
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     auto s = ctx->get_saved_variables();
-    Tensor a, b, c;
-    if (g[0].defined() && s[1].defined()) {
-      const Tensor w = g[0].to(s[1].scalar_type()).view({-1, 1});
-      a = s[0] * w;
-      b = s[1] * w;
-      c = s[2] * w;
-    }
-    return {a, b, c, Tensor(), Tensor(), Tensor()};
+    variable_list out(6);
+    if (g[0].defined())
+      for (int k = 0; k < 3; ++k)
+        if (s[k].defined()) out[k] = s[k] * g[0].view({-1, 1});
+    return out;
   }
 };
 
@@ -290,17 +285,15 @@ class Site : public torch::autograd::Function<Site> {
     const int dt = dtype_code(q);
     void* st = stream_of(q);
     const int64_t nf = q.size(0), N = q.size(1);
-    const bool need = q.requires_grad() || chi.requires_grad() || hard.requires_grad();
-    Tensor E = f64(nf, q), gq, gc, gh;
-    if (need) {
-      gq = torch::zeros_like(q);
-      gc = torch::zeros_like(chi);
-      gh = torch::zeros_like(hard);
-    }
-    if (N > 0)
-      check(admp_atom_terms(dt, ADMP_TERM_SITE, (int)nf, (int)N, nullptr, nullptr, ptr<void>(q), nullptr,
-                            ptr<void>(chi), ptr<void>(hard), 0.0, 0.0, ptr<double>(E), nullptr, ptr<void>(gq), nullptr,
-                            nullptr, nullptr, ptr<void>(gc), ptr<void>(gh), st),
+    const bool any = nf > 0 && N > 0;
+    auto grad = [&](const Tensor& x) {
+      return !x.requires_grad() ? Tensor() : any ? torch::empty_like(x) : torch::zeros_like(x);
+    };
+    Tensor gq = grad(q), gc = grad(chi), gh = grad(hard);
+    Tensor E = any ? torch::empty({nf}, q.options().dtype(torch::kDouble)) : f64(nf, q);
+    if (any)
+      check(admp_site_energy(dt, (int)nf, (int)N, ptr<void>(q), ptr<void>(chi), ptr<void>(hard), ptr<double>(E),
+                             ptr<void>(gq), ptr<void>(gc), ptr<void>(gh), st),
             "site energy");
     ctx->save_for_backward({gq, gc, gh});
     return {E.to(q.scalar_type())};
@@ -308,14 +301,11 @@ class Site : public torch::autograd::Function<Site> {
 
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     auto s = ctx->get_saved_variables();
-    Tensor a, b, c;
-    if (g[0].defined() && s[0].defined()) {
-      const Tensor w = g[0].to(s[0].scalar_type()).view({-1, 1});
-      a = s[0] * w;
-      b = s[1] * w;
-      c = s[2] * w;
-    }
-    return {a, b, c};
+    variable_list out(3);
+    if (g[0].defined())
+      for (int k = 0; k < 3; ++k)
+        if (s[k].defined()) out[k] = s[k] * g[0].view({-1, 1});
+    return out;
   }
 };
 
