@@ -330,6 +330,17 @@ int admp_qeq_hvp_frames(int dtype, int flags, int nframes, int natoms, const int
                         const void* hardness, const void* eta, double kappa, double ke,
                         const void* p, void* out, void* workspace, size_t workspace_bytes,
                         void* stream);
+/* Dense Hessian d2E/dq2 [N, N] (qeq.py:460-515) of one system, written and   */
+/* symmetric: one geometry, Green's function and pair list for all columns,   */
+/* `cols` (1..256) columns of the reciprocal part at a time.                  */
+size_t admp_qeq_hessian_workspace_size(int dtype, int natoms, long long npairs, const int* kmesh,
+                                       int cols);
+int admp_qeq_hessian(int dtype, int flags, int natoms, const int* kmesh, const void* pos,
+                     const void* box, long long npairs, const long long* pairs, const void* ds,
+                     const void* buffer_scales, const void* hardness, const void* eta,
+                     double kappa, double ke, int cols, void* H, void* workspace,
+                     size_t workspace_bytes, void* stream);
+
 
 /* ------------------------------------------------------------------------ */
 /* Batched serving.  Many independent systems (PME energy+forces requests or */

@@ -35,18 +35,63 @@ def test_recip_energy_and_gradients(cuda, n, dtype, tol):
         assert err < 10 * tol * max(np.abs(r).max(), 1.0), (name, err)
 
 
-@pytest.mark.parametrize("frames", [63, 64, 65])
-def test_hessian_products_on_both_sides_of_the_gather_rule(cuda, frames):
-    """1,000 atoms a frame: 63,000 and 64,000 atoms take one group a warp, 65,000 several;
-    equal frames have equal products either way."""
-    from admp_b200 import synthetic
+@pytest.mark.parametrize("dtype,tol", [(torch.float64, 1e-12), (torch.float32, 2e-5)])
+@pytest.mark.parametrize("slab", [False, True])
+def test_hessian_equals_hessian_vector_products(cuda, slab, dtype, tol):
+    """The dense matrix (chunks of 7, 60 and all columns) against unit-vector
+    products, which go through the matvec kernels."""
+    import ctypes  # noqa: F401
+    from admp_b200 import _lib as L, synthetic
     from admp_b200.nblist import TorchNeighborList
     from admp_b200.qeq import QEqForceModule, _hessian
-    pos, box, chi, hard, eta, _ = synthetic.water_system(20, 13.0, 3)
-    m = QEqForceModule(6.0, 5e-4, kmesh=14)
+    pos, box, chi, hard, eta, _ = synthetic.water_system(30, 13.0, 3)
+    n = len(pos)
+    m = QEqForceModule(6.0, 5e-4, kmesh=15, slab_corr=slab)
     nb = TorchNeighborList(6.0)
-    p, b = T(pos, cuda), T(box, cuda)
+    p, b = T(pos, cuda, dtype), T(box, cuda, dtype)
+    h, e = T(hard, cuda, dtype), T(eta, cuda, dtype)
     pairs = nb(p, b)
-    one = _hessian(m, p, b, T(hard, cuda), T(eta, cuda), pairs, nb.get_ds(), nb.get_buffer_scales(), max_cols=1)
-    many = _hessian(m, p, b, T(hard, cuda), T(eta, cuda), pairs, nb.get_ds(), nb.get_buffer_scales(), max_cols=frames)
-    assert rel(many, one) < 1e-12
+    ds, bs = nb.get_ds(), nb.get_buffer_scales().to(dtype)
+    lib = L.load()
+    kp, _k = L.int3([15, 15, 15])
+    c = m.submodels["coulomb"]
+    ws = L.workspace(lib.admp_qeq_workspace_size(L.dtype_code(dtype), n, pairs.shape[0], kp, 0), cuda)
+    ref = torch.empty(n, n, dtype=dtype, device=cuda)
+    for k in range(n):
+        v, out = torch.zeros(n, dtype=dtype, device=cuda), torch.empty(n, dtype=dtype, device=cuda)
+        v[k] = 1
+        L.check(lib.admp_qeq_hvp(L.dtype_code(dtype), m._flags(), n, kp, L.ptr(p), L.ptr(b), pairs.shape[0],
+                                 L.ptr(pairs), L.ptr(ds), L.ptr(bs), L.ptr(h), L.ptr(e), c.kappa,
+                                 m.const_lib.dielectric, L.ptr(v), L.ptr(out), L.ptr(ws), ws.numel(),
+                                 L.stream_of(cuda)))
+        ref[:, k] = out
+    for cols in (7, 60, 256):
+        got = _hessian(m, p, b, h, e, pairs, ds, bs, max_cols=cols)
+        # the same terms in another order (FP32: two different single-precision transforms, ~1e-6 of the largest)
+        assert rel(got, 0.5 * (ref + ref.T)) < tol, cols
+
+
+@pytest.mark.parametrize("frames", [63, 64, 65])
+def test_hessian_products_on_both_sides_of_the_gather_rule(cuda, frames):
+    """63,000 and 64,000 atoms take one group a warp, 65,000 several: the products
+    of equal frames agree with each other and across the rule."""
+    from admp_b200 import _lib as L
+    rng = np.random.default_rng(5)
+    n, K = 1000, 12
+    pos = rng.random((n, 3)) * 22.0
+    v = rng.normal(size=n)
+    lib = L.load()
+
+    def product(nf):
+        kp, _k = L.int3([K] * 3 * nf)
+        rep = lambda x: T(np.repeat(x[None], nf, 0), cuda)  # noqa: E731
+        p, b, h, q = rep(pos), rep(np.diag([22.0] * 3)), rep(np.full(n, 10.0)), rep(v)
+        out = torch.empty(nf, n, dtype=torch.float64, device=cuda)
+        ws = L.workspace(lib.admp_qeq_frames_workspace_size(L.F64, nf, n, 0, kp, 0), cuda)
+        L.check(lib.admp_qeq_hvp_frames(L.F64, L.QEQ_KSPACE, nf, n, kp, L.ptr(p), L.ptr(b), 0, None, None, None,
+                                        L.ptr(h), None, 0.4, 14.4, L.ptr(q), L.ptr(out), L.ptr(ws), ws.numel(),
+                                        L.stream_of(cuda)))
+        return out
+
+    one, many = product(1), product(frames)
+    assert float((many - one).abs().max() / one.abs().max()) < 1e-12

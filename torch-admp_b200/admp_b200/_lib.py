@@ -51,7 +51,7 @@ EXPORTS = [
     "admp_image_nblist_fill", "admp_image_pair_distances", "admp_image_pair_distances_backward",
     "admp_nblist_frames_workspace_size", "admp_nblist_frames_count", "admp_nblist_frames_fill",
     "admp_pair_distances_frames_backward", "admp_coulomb_pbc", "admp_read_back",
-    "admp_damping_energy", "admp_site_energy",
+    "admp_damping_energy", "admp_site_energy", "admp_qeq_hessian_workspace_size", "admp_qeq_hessian",
 ]
 PROFILE_KERNELS = ["spread", "fft_z_fwd", "fft_y_fwd", "fft_x_green", "fft_y_inv", "fft_z_inv", "gather", "pair_ef",
                    "csr_spmv", "neighbors", "cg_vector", "tc_z_fwd", "tc_y_fwd", "tc_x", "tc_y_inv", "tc_z_inv"]
@@ -83,6 +83,8 @@ _SIGS = {
                               _vp, _vp, _sz, _vp]),
     "admp_damping_energy": (_i, [_i, _i, _i, _ll, _vp, _vp, _vp, _vp, _vp, _d, _vp, _vp, _vp, _vp, _vp]),
     "admp_site_energy": (_i, [_i, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
+    "admp_qeq_hessian_workspace_size": (_sz, [_i, _i, _ll, _ip, _i]),
+    "admp_qeq_hessian": (_i, [_i, _i, _i, _ip, _vp, _vp, _ll, _vp, _vp, _vp, _vp, _vp, _d, _d, _i, _vp, _vp, _sz, _vp]),
     "admp_read_back": (_i, [_vp, _sz, _vp, _vp]),
     "admp_nblist_count": (_i, [_i, _i, _i, _vp, _vp, _d, _vp, _sz, _llp, _vp]),
     "admp_nblist_fill": (_i, [_i, _i, _i, _vp, _vp, _d, _vp, _sz, _vp, _vp, _ll, _vp]),

@@ -4,8 +4,8 @@ The charge solve runs as a matrix-free projected conjugate gradient on the
 GPU (admp_qeq_solve) for every ``method`` the reference accepts ("lbfgs",
 "quadratic"): E(q) is quadratic, so all of them reach the same minimiser,
 stopped by the reference's criterion ||P grad||_2 / N < eps (qeq.py:1516).
-``matinv`` builds the dense Hessian column by column from GPU
-Hessian-vector products and solves the KKT system (qeq.py:1530-1617).
+``matinv`` builds the dense Hessian on the GPU (admp_qeq_hessian) and solves
+the KKT system (qeq.py:1530-1617).
 
 ``qeq_solve`` additionally returns charges that are differentiable with
 respect to positions, box, chi, hardness, eta and a right-hand-side shift
@@ -267,11 +267,10 @@ def _qeq_solve_raw(module, q0, positions, box, chi, hardness, eta, pairs, ds, bu
     return q, int(iters.value), float(resid.value), st
 
 
-def _hessian(module, positions, box, hardness, eta, pairs, ds, buffer_scales, max_cols: int = 64,
-             max_pair_rows: int = 16_000_000):
-    """Dense d2E/dq2 from batched GPU Hessian-vector products: columns in
-    chunks, each chunk one admp_qeq_hvp_frames call on unit vectors (the
-    geometry repeated per column), with one workspace for all chunks."""
+def _hessian(module, positions, box, hardness, eta, pairs, ds, buffer_scales, max_cols: int = 256,
+             max_mesh_bytes: int = 1 << 30):
+    """Dense d2E/dq2 by admp_qeq_hessian: the reciprocal part in chunks of up to
+    ``max_cols`` columns whose meshes take at most ``max_mesh_bytes``."""
     lib = L.load()
     ec = module.const_lib.energy_coeff
     pos, bx, pr, dsc, bsc, (hard_c, eta_c) = _std_inputs(
@@ -282,36 +281,23 @@ def _hessian(module, positions, box, hardness, eta, pairs, ds, buffer_scales, ma
     if eta_c is None:
         eta_c = torch.zeros(n, dtype=dt, device=dev)
     P = int(pr.shape[0])
-    nv = max(1, min(max_cols, n, max_pair_rows // max(P, 1)))
     c = module.submodels["coulomb"]
     km = _kmesh_of(module, bx)
-    flags = module._flags()
-    kp, _keep = L.int3(km * nv)
-    nbytes = lib.admp_qeq_frames_workspace_size(L.dtype_code(dt), nv, n, P * nv, kp if c.kspace_flag else None, 0)
+    per_col = 2 * km[0] * km[1] * (km[2] + 2) * pos.element_size()
+    cols = max(1, min(max_cols, n, max_mesh_bytes // per_col))
+    kp, _keep = L.int3(km)
+    H = torch.empty(n, n, dtype=dt, device=dev)
+    if n == 0:
+        return H
+    nbytes = lib.admp_qeq_hessian_workspace_size(L.dtype_code(dt), n, P, kp if c.kspace_flag else None, cols)
     if nbytes == 0:
         L.check(L.BAD_ARG, "QEq Hessian workspace")
     ws = L.workspace(nbytes, dev)
-    offs = (torch.arange(nv, device=dev, dtype=torch.long) * n).view(nv, 1, 1)
-    pos_r = pos.reshape(1, n, 3).expand(nv, n, 3).contiguous()
-    box_r = bx.reshape(1, 3, 3).expand(nv, 3, 3).contiguous()
-    pr_r = (pr.reshape(1, P, 2) + offs).reshape(-1, 2).contiguous()
-    ds_r = dsc.reshape(1, P).expand(nv, P).contiguous()
-    bs_r = bsc.reshape(1, P).expand(nv, P).contiguous()
-    hard_r = hard_c.reshape(1, n).expand(nv, n).contiguous()
-    eta_r = eta_c.reshape(1, n).expand(nv, n).contiguous()
-    H = torch.empty(n, n, dtype=dt, device=dev)
-    E = torch.zeros(nv, n, dtype=dt, device=dev)
-    out = torch.empty(nv, n, dtype=dt, device=dev)
-    for k0 in range(0, n, nv):
-        m = min(nv, n - k0)
-        E.zero_()
-        E[torch.arange(m, device=dev), torch.arange(k0, k0 + m, device=dev)] = 1.0
-        L.check(lib.admp_qeq_hvp_frames(L.dtype_code(dt), flags, m, n, kp, L.ptr(pos_r), L.ptr(box_r), P * m,
-                                        L.ptr(pr_r), L.ptr(ds_r), L.ptr(bs_r), L.ptr(hard_r), L.ptr(eta_r),
-                                        float(c.kappa) or 1.0, module.const_lib.dielectric, L.ptr(E), L.ptr(out),
-                                        L.ptr(ws), nbytes, L.stream_of(dev)), "QEq Hessian-vector products")
-        H[:, k0:k0 + m] = out[:m].T
-    return 0.5 * (H + H.T)
+    L.check(lib.admp_qeq_hessian(L.dtype_code(dt), module._flags(), n, kp, L.ptr(pos), L.ptr(bx), P, L.ptr(pr),
+                                 L.ptr(dsc), L.ptr(bsc), L.ptr(hard_c), L.ptr(eta_c), float(c.kappa) or 1.0,
+                                 module.const_lib.dielectric, cols, L.ptr(H), L.ptr(ws), nbytes, L.stream_of(dev)),
+            "QEq Hessian")
+    return H
 
 
 def pgrad_optimize(module: QEqForceModule, q0, positions, box, chi, hardness, eta, pairs, ds, buffer_scales,

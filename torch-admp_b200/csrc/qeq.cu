@@ -360,6 +360,126 @@ static int qeq_hvp_impl(int flags, int nf, int N, const int* kmesh, const T* pos
   return err ? check_error(err, st) : ADMP_OK;
 }
 
+// ------------------------------------------------------------ dense Hessian
+template <typename T>
+struct HessWS {
+  RecipPlan<T> one, unit, all;  // geometry, one atom per column, all atoms per column
+  SysDesc *t_one, *t_unit, *t_all;
+  T *mesh, *green, *rep, *ones;
+  Cplx<T>* spec;
+  double *acc, *diag, *zc, *chi;
+  PairList<T> list;
+  CGScal* sc;
+  size_t bytes;
+};
+
+template <typename T>
+static int hess_plan(RecipPlan<T>& p, int n, int natoms, int stride, const int* K, double kappa) {
+  SysSpec sys[kMaxBatch];
+  for (int c = 0; c < n; ++c) {
+    sys[c].natoms = natoms;
+    sys[c].atom_off = c * stride;
+    for (int d = 0; d < 3; ++d) sys[c].K[d] = K[d];
+    sys[c].kappa = kappa;
+    sys[c].box_idx = 0;
+    sys[c].green_off = 0;
+  }
+  return build_recip_plan<T>(sys, n, p);
+}
+
+template <typename T>
+static int hess_carve(HessWS<T>& w, void* ws, size_t bytes, int N, long long P, const int* kmesh, double kappa,
+                      int flags, int cols) {
+  const int one[3] = {1, 1, 1};
+  const int* K = (flags & ADMP_QEQ_KSPACE) ? kmesh : one;
+  int s = hess_plan<T>(w.one, 1, N, 0, K, kappa);
+  if (!s) s = hess_plan<T>(w.unit, cols, 1, 1, K, kappa);
+  if (!s) s = hess_plan<T>(w.all, cols, N, N, K, kappa);
+  if (s) return s;
+  const bool ks = (flags & ADMP_QEQ_KSPACE) != 0;
+  Carver c(ws, bytes);
+  w.t_one = reinterpret_cast<SysDesc*>(c.take<unsigned char>(sys_table_bytes()));
+  w.t_unit = reinterpret_cast<SysDesc*>(c.take<unsigned char>(sys_table_bytes()));
+  w.t_all = reinterpret_cast<SysDesc*>(c.take<unsigned char>(sys_table_bytes()));
+  w.mesh = c.take<T>(ks ? w.all.mesh_elems : 0);
+  w.spec = c.take<Cplx<T>>(ks ? w.all.spec_elems : 0);
+  w.green = c.take<T>(ks ? w.one.spec_elems : 0);
+  w.rep = c.take<T>(ks ? 3 * (size_t)N * cols : 0);
+  w.ones = c.take<T>(cols);
+  w.acc = c.take<double>((size_t)kAccStride * cols);
+  w.diag = c.take<double>(N);
+  w.zc = c.take<double>(N);
+  w.chi = c.take<double>(N);
+  w.list.ij = c.take<int2>(P > 0 ? P : 0);
+  w.list.coef = c.take<T>(P > 0 ? P : 0);
+  w.list.n = c.take<unsigned long long>(1);
+  w.sc = c.take<CGScal>(1);
+  w.bytes = c.off;
+  return ADMP_OK;
+}
+
+template <typename T>
+static int qeq_hessian_impl(int flags, int N, const int* kmesh, const T* pos, const T* box, long long Pn,
+                            const long long* pairs, const T* ds, const T* bs, const T* hard, const T* eta, double kappa,
+                            double ke, int cols, T* H, void* ws, size_t bytes, cudaStream_t st) {
+  HessWS<T> w;
+  int s = hess_carve<T>(w, ws, bytes, N, Pn, kmesh, kappa > 0 ? kappa : 1.0, flags, cols);
+  if (s) return s;
+  if (!ws || w.bytes > bytes) return fail(ADMP_ERR_WORKSPACE, "Hessian workspace: need %zu bytes, got %zu", w.bytes, bytes);
+  QEqParams P{flags, (flags >> 8) & 3, 0, 0.0, ke};
+  DevError* err = scratch_error(st);
+  if (!err) return ADMP_ERR_CUDA;
+  ADMP_CUDA_TRY(cudaMemsetAsync(w.sc, 0, sizeof(CGScal), st));
+  ADMP_CUDA_TRY(cudaMemsetAsync(H, 0, sizeof(T) * (size_t)N * N, st));
+  s = bind_plan<T>(w.one, w.t_one, st);
+  if (s) return s;
+  qeq_setup_kernel<T><<<w.one.b.nblk_atom, 256, 0, st>>>(w.one.b, P, pos, box, (const T*)nullptr, hard, eta,
+                                                         (const T*)nullptr, w.diag, w.zc, w.chi, w.sc);
+  const bool pair = Pn > 0 && (flags & (ADMP_QEQ_RSPACE | ADMP_QEQ_DAMPING));
+  if (pair) {
+    long long blocks = (Pn + 255) / 256;
+    if (blocks > 4096) blocks = 4096;
+    ADMP_CUDA_TRY(cudaMemsetAsync(w.list.n, 0, sizeof(*w.list.n), st));
+    qeq_pair_coef_kernel<T><<<(unsigned)blocks, 256, 0, st>>>(N, Pn, flags, kappa, ke, pairs, ds, bs, eta, w.list, err);
+    s = probe_error(err, st);
+    if (s) return s;
+  }
+  if (flags & ADMP_QEQ_KSPACE) {
+    s = launch_green_build<T>(w.one, box, w.green, ke, st);
+    if (s) return s;
+    const long long rep = 3LL * N * cols;
+    hess_repeat_kernel<T><<<(unsigned)((rep + 255) / 256), 256, 0, st>>>(N, cols, pos, w.rep, w.ones);
+    for (int c0 = 0; c0 < N; c0 += cols) {
+      const int n = N - c0 < cols ? N - c0 : cols;
+      if (c0 == 0 || n != cols) {
+        if (n != cols) {  // the last columns
+          s = hess_plan<T>(w.unit, n, 1, 1, kmesh, kappa);
+          if (!s) s = hess_plan<T>(w.all, n, N, N, kmesh, kappa);
+          if (s) return s;
+        }
+        s = bind_plan<T>(w.unit, w.t_unit, st);
+        if (!s) s = bind_plan<T>(w.all, w.t_all, st);
+        if (s) return s;
+      }
+      ADMP_CUDA_TRY(cudaMemsetAsync(w.mesh, 0, w.all.mesh_elems * sizeof(T), st));
+      s = launch_spread<T>(w.unit, pos + 3 * (size_t)c0, box, w.ones, w.mesh, nullptr, st);
+      if (!s) s = launch_fft_green<T>(w.all, w.mesh, w.spec, box, w.acc, ke, st, w.green);
+      if (!s)
+        s = launch_gather<T, false>(w.all, w.rep, box, w.ones, w.mesh, H + (size_t)c0 * N, nullptr, w.acc, nullptr, st);
+      if (s) return s;
+    }
+  }
+  if (pair) {
+    long long blocks = (Pn + 511) / 512;
+    if (blocks > 4096) blocks = 4096;
+    hess_pairs_kernel<T><<<(unsigned)blocks, 256, 0, st>>>(w.list, N, H);
+  }
+  const int tiles = (N + 15) / 16;
+  hess_finish_kernel<T><<<dim3(tiles, tiles), 256, 0, st>>>(N, P, w.diag, w.zc, w.sc, H);
+  ADMP_CUDA_TRY(cudaGetLastError());
+  return pair ? probed_error(err, st) : ADMP_OK;
+}
+
 }  // namespace admp
 
 using namespace admp;
@@ -467,4 +587,36 @@ extern "C" int admp_qeq_hvp(int dtype, int flags, int natoms, const int* kmesh, 
                             void* workspace, size_t workspace_bytes, void* stream) {
   return admp_qeq_hvp_frames(dtype, flags, 1, natoms, kmesh, pos, box, npairs, pairs, ds, buffer_scales, hardness,
                              eta, kappa, ke, p, out, workspace, workspace_bytes, stream);
+}
+
+extern "C" size_t admp_qeq_hessian_workspace_size(int dtype, int natoms, long long npairs, const int* kmesh, int cols) {
+  if (natoms <= 0 || cols <= 0 || cols > kMaxBatch) return 0;
+  const int fl = kmesh ? ADMP_QEQ_KSPACE : 0;
+  if (dtype == ADMP_F32) {
+    HessWS<float> w;
+    return hess_carve<float>(w, nullptr, 0, natoms, npairs, kmesh, 1.0, fl, cols) ? 0 : w.bytes;
+  }
+  HessWS<double> w;
+  return hess_carve<double>(w, nullptr, 0, natoms, npairs, kmesh, 1.0, fl, cols) ? 0 : w.bytes;
+}
+
+extern "C" int admp_qeq_hessian(int dtype, int flags, int natoms, const int* kmesh, const void* pos, const void* box,
+                                long long npairs, const long long* pairs, const void* ds, const void* buffer_scales,
+                                const void* hardness, const void* eta, double kappa, double ke, int cols, void* H,
+                                void* workspace, size_t workspace_bytes, void* stream) {
+  if (natoms <= 0 || cols <= 0 || cols > kMaxBatch || !pos || !box || !hardness || !H)
+    return fail(ADMP_ERR_BAD_ARG, "admp_qeq_hessian: args");
+  if ((flags & ADMP_QEQ_KSPACE) && (!kmesh || !(kappa > 0))) return fail(ADMP_ERR_BAD_ARG, "admp_qeq_hessian: kspace needs kmesh and kappa");
+  if ((flags & ADMP_QEQ_DAMPING) && !eta) return fail(ADMP_ERR_BAD_ARG, "admp_qeq_hessian: damping needs eta");
+  if (npairs > 0 && (!pairs || !ds || !buffer_scales)) return fail(ADMP_ERR_BAD_ARG, "admp_qeq_hessian: pairs");
+  cudaStream_t st = (cudaStream_t)stream;
+  if (dtype == ADMP_F64)
+    return qeq_hessian_impl<double>(flags, natoms, kmesh, (const double*)pos, (const double*)box, npairs, pairs,
+                                    (const double*)ds, (const double*)buffer_scales, (const double*)hardness,
+                                    (const double*)eta, kappa, ke, cols, (double*)H, workspace, workspace_bytes, st);
+  if (dtype == ADMP_F32)
+    return qeq_hessian_impl<float>(flags, natoms, kmesh, (const float*)pos, (const float*)box, npairs, pairs,
+                                   (const float*)ds, (const float*)buffer_scales, (const float*)hardness,
+                                   (const float*)eta, kappa, ke, cols, (float*)H, workspace, workspace_bytes, st);
+  return fail(ADMP_ERR_BAD_ARG, "bad dtype");
 }

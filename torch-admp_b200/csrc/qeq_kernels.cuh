@@ -278,6 +278,53 @@ __global__ void __launch_bounds__(256)
   }
 }
 
+// ---------------------------------------------------------------------------
+// Dense Hessian (qeq.py:460-515).  Column c of the reciprocal part is the
+// potential of a unit charge on atom c: a one-atom spread, the transforms and a
+// gather over all atoms, with one geometry, one Green's function and one pair
+// list for all columns; the pair entries go into the matrix directly.
+// ---------------------------------------------------------------------------
+// pos repeated n times, and n ones
+template <typename T>
+__global__ void hess_repeat_kernel(int N, int n, const T* __restrict__ pos, T* __restrict__ rep, T* __restrict__ ones) {
+  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (t < (long long)3 * N * n) rep[t] = pos[t % (3 * N)];
+  if (t < n) ones[t] = T(1);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) hess_pairs_kernel(PairList<T> list, int N, T* __restrict__ H) {
+  const long long n = (long long)*list.n;
+  for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x) {
+    const int2 ij = list.ij[p];
+    const T c = list.coef[p];
+    atomicAdd(H + (size_t)ij.x * N + ij.y, c);
+    atomicAdd(H + (size_t)ij.y * N + ij.x, c);
+  }
+}
+
+// diagonal and rank-one terms, and the mean of the matrix and its transpose
+template <typename T>
+__global__ void __launch_bounds__(256) hess_finish_kernel(int N, QEqParams P, const double* __restrict__ diag,
+                                                          const double* __restrict__ zc,
+                                                          const CGScal* __restrict__ sc, T* __restrict__ H) {
+  const int i = blockIdx.x * 16 + (threadIdx.x & 15), c = blockIdx.y * 16 + (threadIdx.x >> 4);
+  if (i > c || c >= N) return;
+  double t = i == c ? diag[i] : 0.0;
+  t += sc->nn;
+  double ab = t, ba = t;
+  if (P.flags & ADMP_QEQ_SLAB) {
+    const double zi = zc[i], zj = zc[c];
+    const double s = sc->pre * (2.0 * zi * zj - zj * zj - zi * zi - sc->Lz2 / 6.0);
+    ab += s;
+    ba += s;
+  }
+  const T a = (T)((double)H[(size_t)i * N + c] + ab), b = (T)((double)H[(size_t)c * N + i] + ba);
+  const T m = T(0.5) * (a + b);
+  H[(size_t)i * N + c] = m;
+  H[(size_t)c * N + i] = m;
+}
+
 // Hv += diag v + rank-1 terms; accumulate p^T Hv and C Hv.
 template <typename T>
 __global__ void __launch_bounds__(256)
