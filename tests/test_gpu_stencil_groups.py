@@ -95,3 +95,24 @@ def test_hessian_products_on_both_sides_of_the_gather_rule(cuda, frames):
 
     one, many = product(1), product(frames)
     assert float((many - one).abs().max() / one.abs().max()) < 1e-12
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.float64, 1e-12), (torch.float32, 1e-4)])
+@pytest.mark.parametrize("definite", [True, False])
+@pytest.mark.parametrize("m", [None, 0, 1, 2])
+def test_kkt_solves_definite_and_indefinite_systems(cuda, m, definite, dtype, tol):
+    """Every route of the dense solve against numpy's solution of the bordered system."""
+    from admp_b200.qeq import _kkt
+    rng = np.random.default_rng(11)
+    n = 37
+    a = rng.normal(size=(n, n))
+    h = a @ a.T / n + 3 * np.eye(n)
+    if not definite:
+        h[5, 5] -= 20.0
+    chi, k = rng.normal(size=n), m or 0
+    c, b = np.abs(rng.normal(size=(k, n))), rng.normal(size=k)
+    full = np.block([[h, c.T], [c, np.zeros((k, k))]])
+    want = np.linalg.solve(full, np.concatenate([-chi, b]))[:n]
+    got = _kkt(T(h, cuda, dtype), T(chi, cuda, dtype), None if m is None else T(c, cuda, dtype), T(b, cuda, dtype))
+    # condition numbers below 100: a few hundred ulp
+    assert rel(got, want) < tol
