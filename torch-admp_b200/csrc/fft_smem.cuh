@@ -79,6 +79,18 @@ __device__ __forceinline__ void make_twiddles(Cplx<T>* W, int n) {
   }
 }
 
+// The threads that run a transform together: the whole block, or the first
+// nthr threads of a block whose others do something else meanwhile (named
+// barrier 1).
+enum { kSyncBlock = 0, kSyncPart = 1 };
+template <int SYNC>
+__device__ __forceinline__ void group_sync(int nthr) {
+  if constexpr (SYNC == kSyncPart)
+    asm volatile("bar.sync 1, %0;" ::"r"(nthr) : "memory");
+  else
+    __syncthreads();
+}
+
 // Shared-memory offsets in these stages are 32-bit ints: a block never holds
 // more than 227 KB, i.e. fewer than 2^16 complex values.
 //
@@ -94,7 +106,7 @@ __device__ __forceinline__ void make_twiddles(Cplx<T>* W, int n) {
 // ones.  Step 1 twiddles and folds the inputs (in -> out, in the butterfly's
 // own output slots), step 2 forms the output pairs (out -> in), so the result
 // of this stage is left in `in`.
-template <typename T, bool LINE_FAST, bool WARP, bool INV, int NL>
+template <typename T, bool LINE_FAST, int SYNC, bool INV, int NL>
 __device__ __forceinline__ void stockham_odd(Cplx<T>* __restrict__ in, Cplx<T>* __restrict__ out,
                                              int nl, int n, int ls, int es, int Ns, int r,
                                              const Cplx<T>* __restrict__ W, int tid, int nthr) {
@@ -135,10 +147,7 @@ __device__ __forceinline__ void stockham_odd(Cplx<T>* __restrict__ in, Cplx<T>* 
       dst[(int)(base + (h + u) * Ns) * es] = dv;
     }
   }
-  if (WARP)
-    __syncwarp();
-  else
-    __syncthreads();
+  group_sync<SYNC>(nthr);
   // step 2 items: class 0 forms X_0, class c >= 1 the output pairs
   // kk = 1 + QK (c - 1) .. QK c, which share each load of s_t and d_t
   // (4 and 8 pairs per item measured slower on the serving stream: fewer items per stage, more registers)
@@ -368,10 +377,9 @@ __device__ __forceinline__ void stockham_r2(const Cplx<T>* __restrict__ in, Cplx
 }
 
 // One pass of all stages over nl lines with threads tid, tid + nthr, ...;
-// WARP: the calling threads are one warp (synchronised with __syncwarp),
-// otherwise the whole block (__syncthreads).  Returns the buffer holding the
-// result (a or b).
-template <typename T, bool LINE_FAST, bool WARP, bool INV, int NL = 0>
+// SYNC: who the calling threads are (group_sync).  Returns the buffer holding
+// the result (a or b).
+template <typename T, bool LINE_FAST, int SYNC, bool INV, int NL = 0>
 __device__ __forceinline__ Cplx<T>* fft_run(const Radices& R, Cplx<T>* a, Cplx<T>* b, int nl, int n, int ls, int es,
                                             const Cplx<T>* W, int tid, int nthr) {
   int Ns = 1;
@@ -388,11 +396,8 @@ __device__ __forceinline__ Cplx<T>* fft_run(const Radices& R, Cplx<T>* a, Cplx<T
     else if (r == 5)
       stockham_r35<T, LINE_FAST, 5, INV, NL>(in, out, nl, n, ls, es, Ns, W, tid, nthr);
     else
-      stockham_odd<T, LINE_FAST, WARP, INV, NL>(in, out, nl, n, ls, es, Ns, r, W, tid, nthr);
-    if (WARP)
-      __syncwarp();
-    else
-      __syncthreads();
+      stockham_odd<T, LINE_FAST, SYNC, INV, NL>(in, out, nl, n, ls, es, Ns, r, W, tid, nthr);
+    group_sync<SYNC>(nthr);
     Ns *= r;
     if (r <= 5) {  // the odd-radix stage leaves its result in `in`
       Cplx<T>* tmp = in;
@@ -412,7 +417,7 @@ template <typename T, bool LINE_FAST, bool INV, int NL = 0>
 __device__ Cplx<T>* fft_lines(Cplx<T>* a, Cplx<T>* b, int nl, int n, int ls, int es, const Cplx<T>* W) {
   Radices R;
   factor_radices(n, R);
-  return fft_run<T, LINE_FAST, false, INV, NL>(R, a, b, nl, n, ls, es, W, threadIdx.x, blockDim.x);
+  return fft_run<T, LINE_FAST, kSyncBlock, INV, NL>(R, a, b, nl, n, ls, es, W, threadIdx.x, blockDim.x);
 }
 
 }  // namespace admp

@@ -872,7 +872,12 @@ __device__ __forceinline__ T gather_group(const WarpStencil<T, FORCES>& ws, int 
     T fm[GU][6];
 #pragma unroll
     for (int u = 0; u < GU; ++u) {
-      const int j = min(jb + u, na - 1);
+      if (jb + u >= na) {  // the sums of absent atoms are not used
+#pragma unroll
+        for (int dx = 0; dx < 6; ++dx) fm[u][dx] = T(0);
+        continue;
+      }
+      const int j = jb + u;
       const int* ox = ws.ox + j * 6;
       const int oyz = wrap_up(ws.byz[2 * j] + y0, K1) * K2 + wrap_up(ws.byz[2 * j + 1] + z0, K2);
 #pragma unroll

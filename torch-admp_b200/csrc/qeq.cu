@@ -129,7 +129,14 @@ static bool cg_plan(const QEqCtx<T>& c, int sms, CgArgs<T>& a, size_t& smem) {
   }
   const size_t fft = ((size_t)a.K0 + a.K1 + a.K2 + 2 * (size_t)a.buf) * cs;
   const size_t st = (WarpStencil<T, false>::bytes() + 15) / 16 * 16 * kCgWarps;
-  const int groups = (c.N + kPw - 1) / kPw, per_warp = (groups + sms * kCgWarps - 1) / (sms * kCgWarps);
+  // the smallest group that still gives every warp one at most; eight atoms above that
+  a.group = kPw;
+  for (int s = 2; s < kPw; s <<= 1)
+    if ((c.N + s - 1) / s <= sms * kCgWarps) {
+      a.group = s;
+      break;
+    }
+  const int groups = (c.N + a.group - 1) / a.group, per_warp = (groups + sms * kCgWarps - 1) / (sms * kCgWarps);
   a.kept = fft + st * per_warp <= budget ? per_warp : 0;
   smem = fft + st * (a.kept ? a.kept : 1);
   return smem <= budget;

@@ -7,12 +7,15 @@
 // iteration are separated by a barrier over the grid, every transform spreads
 // its lines over all blocks, the twiddles and (while they fit) the atoms'
 // stencils are built once per launch, and the host reads the result once.
+// Now 41 us (3,000 atoms, 48^3, FP32), 55 (10,701, 64^3, FP64; 110 before) and
+// 49 (2,304 electrode atoms, 64 x 64 x 160, FP32; 100 before): eight barriers
+// take 14-16 of them, the five transforms 16-26, spread and gather 8-15.
 //
 //   A   direction p = r + beta p of the group's atoms, spread
-//   Z   z transform of the mesh lines; real-space matrix times p
-//   Y   y transform
+//   Z   z transform of the mesh lines,  Y  y transform
 //   X   x transform, Green's function, inverse x transform
 //   Y'  inverse y,  Z' inverse z
+//       (a quarter of the warps multiply p by the pair matrix meanwhile)
 //   E   gather, rest of the matvec, p.Hp and C.Hp
 //   F   x += alpha p, r -= alpha P(Hp), |r|^2; zero Hp and the mesh
 //
@@ -28,10 +31,11 @@
 
 namespace admp {
 
-constexpr int kCgThreads = 256;
-constexpr int kCgWarps = kCgThreads / 32;
+constexpr int kCgThreads = 512;
+constexpr int kCgWarps = kCgThreads / 32;  // cg_block_sum counts on 16
+constexpr int kCgFft = 384;                // threads of the transforms; the others multiply by the pair matrix
 constexpr long long kCgSpin = 1LL << 23;
-constexpr int kCgMaxLines = kCgThreads;  // lines of a block's y transform
+constexpr int kCgMaxLines = kCgFft;      // lines of a block's y transform
 constexpr int kCgLaunch = 128;           // iterations per launch
 
 struct CgSlot {
@@ -63,14 +67,17 @@ struct CgArgs {
   int k0, k1;        // iterations of this launch: k0 <= k < k1
   int lz, ly, lx;    // lines (z: pairs of lines) a block transforms at a time
   int buf;           // complex values in each of the two line buffers
+  int group;         // atoms of a warp's group (at most kPw)
   int kept;          // stencil groups a warp keeps, 0: built anew every time
 };
 
-// Barrier over the grid; false when it ran out of polls.
-__device__ __forceinline__ bool cg_barrier(CgShared* sh, unsigned& target) {
+// Barrier over the grid; false when it ran out of polls.  Called by the whole
+// block, or (kSyncPart) by its first nthr threads.
+template <int SYNC>
+__device__ __forceinline__ bool cg_barrier(CgShared* sh, unsigned& target, int nthr) {
   __shared__ int ok;
   target += gridDim.x;
-  __syncthreads();
+  group_sync<SYNC>(nthr);
   if (threadIdx.x == 0) {
     unsigned seen;
     __threadfence();
@@ -82,8 +89,33 @@ __device__ __forceinline__ bool cg_barrier(CgShared* sh, unsigned& target) {
     ok = seen >= target;
     __threadfence();
   }
-  __syncthreads();
+  group_sync<SYNC>(nthr);
   return ok != 0;
+}
+
+// Sums of NV <= 4 values over the block, added to out[0 .. NV): the warp sums
+// are taken together and one warp adds the 16 warps' results.
+template <int NV>
+__device__ __forceinline__ void cg_block_sum(const double (&in)[NV], double* out, double (*sh)[kCgWarps]) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double v[4] = {0, 0, 0, 0};
+#pragma unroll
+  for (int k = 0; k < NV; ++k) v[k] = in[k];
+  if (NV == 1) {
+    v[0] = warp_sum(v[0]);
+    if (lane == 0) sh[0][warp] = v[0];
+  } else {
+    const double s = warp_sum_each<4>(v, lane);  // lane l: value l / 8
+    if ((lane & 7) == 0) sh[lane >> 3][warp] = s;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    const int q = lane >> 3, w = lane & 7;
+    double s = q < NV ? sh[q][w] + sh[q][w + 8] : 0.0;
+#pragma unroll
+    for (int m = 4; m >= 1; m >>= 1) s += __shfl_xor_sync(0xffffffffu, s, m);
+    if (w == 0 && q < NV && s != 0.0) atomicAdd(out + q, s);
+  }
 }
 
 template <typename T>
@@ -98,7 +130,7 @@ __device__ void cg_z_pass(const CgArgs<T>& a, const CgFft<T>& f, const Radices& 
   const FastDiv fdK2 = fast_div(K2), fdK2h = fast_div(K2h);
   for (int p0 = blockIdx.x * a.lz; p0 < npair; p0 += gridDim.x * a.lz) {
     const int np = min(a.lz, npair - p0);
-    for (int idx = threadIdx.x; idx < np * K2; idx += kCgThreads) {
+    for (int idx = threadIdx.x; idx < np * K2; idx += kCgFft) {
       const int p = fdiv(idx, fdK2), t = idx - p * K2;
       const size_t l0 = 2 * (size_t)(p0 + p);
       const bool two = l0 + 1 < (size_t)L;
@@ -121,10 +153,10 @@ __device__ void cg_z_pass(const CgArgs<T>& a, const CgFft<T>& f, const Radices& 
       }
       f.A[idx] = z;
     }
-    __syncthreads();
-    Cplx<T>* R2 = fft_run<T, false, false, INV>(R, f.A, f.B, np, K2, K2, 1, f.W2, threadIdx.x, kCgThreads);
+    group_sync<kSyncPart>(kCgFft);
+    Cplx<T>* R2 = fft_run<T, false, kSyncPart, INV>(R, f.A, f.B, np, K2, K2, 1, f.W2, threadIdx.x, kCgFft);
     if (!INV) {
-      for (int idx = threadIdx.x; idx < np * K2h; idx += kCgThreads) {
+      for (int idx = threadIdx.x; idx < np * K2h; idx += kCgFft) {
         const int p = fdiv(idx, fdK2h), k = idx - p * K2h;
         const Cplx<T> Z = R2[p * K2 + k], Zm = R2[p * K2 + (k == 0 ? 0 : K2 - k)];
         const size_t l0 = 2 * (size_t)(p0 + p);
@@ -137,7 +169,7 @@ __device__ void cg_z_pass(const CgArgs<T>& a, const CgFft<T>& f, const Radices& 
         if (l0 + 1 < (size_t)L) a.spec[(l0 + 1) * K2h + k] = v;
       }
     } else {
-      for (int idx = threadIdx.x; idx < np * K2; idx += kCgThreads) {
+      for (int idx = threadIdx.x; idx < np * K2; idx += kCgFft) {
         const int p = fdiv(idx, fdK2), t = idx - p * K2;
         const size_t l0 = 2 * (size_t)(p0 + p);
         const Cplx<T> z = R2[idx];
@@ -145,7 +177,7 @@ __device__ void cg_z_pass(const CgArgs<T>& a, const CgFft<T>& f, const Radices& 
         if (l0 + 1 < (size_t)L) a.mesh[(l0 + 1) * K2 + t] = z.y;
       }
     }
-    __syncthreads();
+    group_sync<kSyncPart>(kCgFft);
   }
 }
 
@@ -161,18 +193,18 @@ __device__ void cg_y_pass(const CgArgs<T>& a, const CgFft<T>& f, const Radices& 
       const int c = c0 + threadIdx.x, xx = c / K2h;
       off[threadIdx.x] = (long long)xx * K1 * K2h + (c - xx * K2h);
     }
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < K1 * n; idx += kCgThreads) {
+    group_sync<kSyncPart>(kCgFft);
+    for (int idx = threadIdx.x; idx < K1 * n; idx += kCgFft) {
       const int y = fdiv(idx, fdn), c = idx - y * n;
       f.A[idx] = a.spec[off[c] + (long long)y * K2h];
     }
-    __syncthreads();
-    Cplx<T>* R1 = fft_run<T, true, false, INV>(R, f.A, f.B, n, K1, 1, n, f.W1, threadIdx.x, kCgThreads);
-    for (int idx = threadIdx.x; idx < K1 * n; idx += kCgThreads) {
+    group_sync<kSyncPart>(kCgFft);
+    Cplx<T>* R1 = fft_run<T, true, kSyncPart, INV>(R, f.A, f.B, n, K1, 1, n, f.W1, threadIdx.x, kCgFft);
+    for (int idx = threadIdx.x; idx < K1 * n; idx += kCgFft) {
       const int y = fdiv(idx, fdn), c = idx - y * n;
       a.spec[off[c] + (long long)y * K2h] = R1[idx];
     }
-    __syncthreads();
+    group_sync<kSyncPart>(kCgFft);
   }
 }
 
@@ -183,26 +215,58 @@ __device__ void cg_x_pass(const CgArgs<T>& a, const CgFft<T>& f, const Radices& 
   for (int c0 = blockIdx.x * a.lx; c0 < L; c0 += gridDim.x * a.lx) {
     const int n = min(a.lx, L - c0);
     const FastDiv fdn = fast_div(n);
-    for (int idx = threadIdx.x; idx < K0 * n; idx += kCgThreads) {
+    for (int idx = threadIdx.x; idx < K0 * n; idx += kCgFft) {
       const int x = fdiv(idx, fdn), c = c0 + idx - x * n;
       f.A[idx] = a.spec[(size_t)x * L + c];
     }
-    __syncthreads();
-    Cplx<T>* F = fft_run<T, true, false, false>(R, f.A, f.B, n, K0, 1, n, f.W0, threadIdx.x, kCgThreads);
+    group_sync<kSyncPart>(kCgFft);
+    Cplx<T>* F = fft_run<T, true, kSyncPart, false>(R, f.A, f.B, n, K0, 1, n, f.W0, threadIdx.x, kCgFft);
     Cplx<T>* O = F == f.A ? f.B : f.A;
-    for (int idx = threadIdx.x; idx < K0 * n; idx += kCgThreads) {
+    for (int idx = threadIdx.x; idx < K0 * n; idx += kCgFft) {
       const int x = fdiv(idx, fdn), c = c0 + idx - x * n;
       const T g = a.green[(size_t)x * L + c];
       F[idx].x *= g;
       F[idx].y *= g;
     }
-    __syncthreads();
-    Cplx<T>* I = fft_run<T, true, false, true>(R, F, O, n, K0, 1, n, f.W0, threadIdx.x, kCgThreads);
-    for (int idx = threadIdx.x; idx < K0 * n; idx += kCgThreads) {
+    group_sync<kSyncPart>(kCgFft);
+    Cplx<T>* I = fft_run<T, true, kSyncPart, true>(R, F, O, n, K0, 1, n, f.W0, threadIdx.x, kCgFft);
+    for (int idx = threadIdx.x; idx < K0 * n; idx += kCgFft) {
       const int x = fdiv(idx, fdn), c = c0 + idx - x * n;
       a.spec[(size_t)x * L + c] = I[idx];
     }
-    __syncthreads();
+    group_sync<kSyncPart>(kCgFft);
+  }
+}
+
+// Hp += real-space matrix times p by the block's threads t0, t0 + 1, ...: four
+// entries a thread in flight, the first atom's share summed over its run.
+template <typename T>
+__device__ void cg_pairs(const CgArgs<T>& a, int t0, int nthr) {
+  constexpr int U = 4;
+  const int lane = threadIdx.x & 31;
+  const long long n = (long long)*a.list.n, step = (long long)gridDim.x * nthr;
+  for (long long p0 = blockIdx.x * (long long)nthr + ((threadIdx.x - t0) & ~31); p0 < n; p0 += U * step) {
+    int2 ij[U];
+    T c[U], vi[U], vj[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const long long p = p0 + u * step + lane;
+      ij[u] = p < n ? a.list.ij[p] : make_int2(-1, -1);
+      c[u] = p < n ? a.list.coef[p] : T(0);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const bool on = c[u] != T(0);
+      vi[u] = on ? a.p[ij[u].x] : T(0);
+      vj[u] = on ? a.p[ij[u].y] : T(0);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const WarpRuns runs(ij[u].x, lane);
+      const T w = runs.sum(c[u] != T(0) ? c[u] * vj[u] : T(0));
+      if (runs.opens && w != T(0)) atomicAdd(a.Hp + ij[u].x, w);
+      if (c[u] != T(0)) atomicAdd(a.Hp + ij[u].y, c[u] * vi[u]);
+    }
   }
 }
 
@@ -211,7 +275,8 @@ __global__ void __launch_bounds__(kCgThreads) qeq_cg_kernel(CgArgs<T> a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ Geom g;
   __shared__ Radices R0, R1, R2;
-  __shared__ double red[5 * 32];
+  __shared__ double red[4][kCgWarps], red2[4][kCgWarps];
+  __shared__ int broken;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const bool kspace = (a.P.flags & ADMP_QEQ_KSPACE) != 0, slab = (a.P.flags & ADMP_QEQ_SLAB) != 0;
   CgFft<T> f;
@@ -230,6 +295,7 @@ __global__ void __launch_bounds__(kCgThreads) qeq_cg_kernel(CgArgs<T> a) {
   d.K1 = a.K1;
   d.K2 = a.K2;
   load_geom(a.box, 0, &g);
+  if (threadIdx.x == 0) broken = 0;
   if (kspace) {
     make_twiddles(f.W0, a.K0);
     make_twiddles(f.W1, a.K1);
@@ -239,23 +305,28 @@ __global__ void __launch_bounds__(kCgThreads) qeq_cg_kernel(CgArgs<T> a) {
     if (threadIdx.x == 96) factor_radices(a.K2, R2);
   }
   __syncthreads();
-  // warp w of block b takes the groups of eight atoms w G + b, + G kCgWarps, ...
-  const int ng = (a.N + kPw - 1) / kPw, g0 = warp * gridDim.x + blockIdx.x, gstep = gridDim.x * kCgWarps;
+  // warp w of block b takes the groups of a.group atoms w G + b, + G kCgWarps, ...
+  const int ng = (a.N + a.group - 1) / a.group, g0 = warp * gridDim.x + blockIdx.x, gstep = gridDim.x * kCgWarps;
+  auto atoms = [&](int gi) { return min(a.group, a.N - gi * a.group); };
   auto stencil = [&](int u) {
     WarpStencil<T, false> ws;
     ws.carve(st_base + (size_t)(warp * nkeep + (a.kept ? u : 0)) * kStBytes);
     return ws;
   };
+  auto build = [&](WarpStencil<T, false>& ws, int gi) {
+    warp_build_stencil<T, false>(ws, d, g, a.pos, nullptr, nullptr, gi * a.group, gi * a.group + atoms(gi), lane);
+  };
   if (kspace && a.kept) {
     int u = 0;
     for (int gi = g0; gi < ng; gi += gstep, ++u) {
       WarpStencil<T, false> ws = stencil(u);
-      warp_build_stencil<T, false>(ws, d, g, a.pos, nullptr, nullptr, gi * kPw, a.N, lane);
+      build(ws, gi);
     }
   }
   CGScal* sc = a.sc;
   if (sc->done) return;  // the same for every block: only phase A writes it, behind the first barrier
-  const double rr0 = sc->rr;
+  const double rr0 = sc->rr, nn = sc->nn, pre = sc->pre, Lz2 = sc->Lz2;
+  const double few = a.P.tol * (double)a.N, few2 = few * few;
   const int nc = sc->n_const;
   unsigned target = 0;
   auto stop = [&]() {
@@ -264,14 +335,26 @@ __global__ void __launch_bounds__(kCgThreads) qeq_cg_kernel(CgArgs<T> a) {
       atomicExch(&sc->status, ADMP_ERR_CUDA);
     }
   };
+  auto meet = [&]() { return cg_barrier<kSyncBlock>(a.sh, target, kCgThreads); };
   for (int k = a.k0;; ++k) {
     CgSlot& S = a.sh->slot[k % 3];
     volatile CgSlot& S1 = a.sh->slot[(k + 2) % 3];  // iteration k - 1
     volatile CgSlot& S2 = a.sh->slot[(k + 1) % 3];  // iteration k - 2
-    const double rr = k == 0 ? rr0 : S1.rr_new;
-    // ---- A: convergence of the last iterate, direction, spread
+    // ---- A: convergence of the last iterate, direction, spread (the first group's values are asked for before
+    // the scalars are worked out)
+    double rv = 0.0, zv = 0.0;
+    T pv = T(0);
+    if (g0 < ng && lane < atoms(g0)) {
+      const int i = g0 * a.group + lane;
+      rv = a.r[i];
+      pv = a.p[i];
+      zv = a.zc[i];
+    }
+    const double rr = k == 0 ? rr0 : S1.rr_new, rp = k == 0 ? 0.0 : (k == 1 ? rr0 : S2.rr_new);
     if (k > 0) {
-      const bool conv = sqrt(rr) / (double)a.N < a.P.tol;
+      // sqrt(rr) / N < tol; the square root and the division only where rounding could decide
+      bool conv = rr < few2 * (1.0 - 1e-9);
+      if (!conv && rr <= few2 * (1.0 + 1e-9)) conv = sqrt(rr) / (double)a.N < a.P.tol;
       if (conv || k >= a.P.max_iter) {
         if (blockIdx.x == 0 && threadIdx.x == 0) {
           sc->rr_new = rr;
@@ -290,88 +373,78 @@ __global__ void __launch_bounds__(kCgThreads) qeq_cg_kernel(CgArgs<T> a) {
       return;
     }
     {
-      const double rp = k == 0 ? 0.0 : (k == 1 ? rr0 : S2.rr_new);
       const double beta = rp != 0.0 ? rr / rp : 0.0;
       double acc[3] = {0, 0, 0};
       int u = 0;
       for (int gi = g0; gi < ng; gi += gstep, ++u) {
         WarpStencil<T, false> ws = stencil(u);
-        const int na = min(kPw, a.N - gi * kPw);
-        if (kspace && !a.kept) warp_build_stencil<T, false>(ws, d, g, a.pos, nullptr, nullptr, gi * kPw, a.N, lane);
+        const int na = atoms(gi);
+        if (kspace && !a.kept) build(ws, gi);
         if (lane < na) {
-          const int i = gi * kPw + lane;
-          T pt = a.p[i];
-          double pn = (double)pt;
-          if (k > 0) {
-            pn = a.r[i] + beta * pn;
-            pt = (T)pn;
-            a.p[i] = pt;
-          } else {
-            pn = a.r[i];  // the first direction is the residual
+          const int i = gi * a.group + lane;
+          if (u > 0) {
+            rv = a.r[i];
+            pv = a.p[i];
+            zv = a.zc[i];
           }
-          if (kspace) ws.q[lane] = pt;
-          const double z = a.zc[i];
+          double pn = rv;  // the first direction is the residual
+          if (k > 0) {
+            pn = rv + beta * (double)pv;
+            pv = (T)pn;
+            a.p[i] = pv;
+          }
+          if (kspace) ws.q[lane] = pv;
           acc[0] += pn;
-          acc[1] += pn * z;
-          acc[2] += pn * z * z;
+          acc[1] += pn * zv;
+          acc[2] += pn * zv * zv;
         }
         __syncwarp();
         if (kspace) spread_group<T>(ws, na, a.K1, a.K2, a.mesh, lane);
         __syncwarp();
       }
-      block_atomic_sum<3>(acc, &S.sp, red);
+      cg_block_sum<3>(acc, &S.sp, red);
     }
-    if (!cg_barrier(a.sh, target)) return stop();
-    // ---- Z .. Z': the mesh part; the pairs need only p and Hp
-    if (kspace) cg_z_pass<T, false>(a, f, R2);
-    if (a.have_pairs) {
-      const long long n = (long long)*a.list.n;
-      for (long long p0 = blockIdx.x * (long long)kCgThreads + (threadIdx.x & ~31); p0 < n;
-           p0 += (long long)gridDim.x * kCgThreads) {
-        const long long p = p0 + lane;
-        int2 ij = make_int2(-1, -1);
-        T c = T(0);
-        if (p < n) {
-          ij = a.list.ij[p];
-          c = a.list.coef[p];
-        }
-        const bool on = c != T(0);
-        const WarpRuns runs(ij.x, lane);
-        const T w = runs.sum(on ? c * a.p[ij.y] : T(0));
-        if (runs.opens && w != T(0)) atomicAdd(a.Hp + ij.x, w);
-        if (on) atomicAdd(a.Hp + ij.y, c * a.p[ij.x]);
+    if (!meet()) return stop();
+    // ---- Z .. Z': the mesh part by the first kCgFft threads; the pairs, which need only p and Hp, by the others
+    if (threadIdx.x < kCgFft) {
+      if (kspace) {
+        unsigned t = target;
+        bool ok = true;
+        auto pass = [&]() { return cg_barrier<kSyncPart>(a.sh, t, kCgFft); };
+        cg_z_pass<T, false>(a, f, R2);
+        if ((ok = pass())) cg_y_pass<T, false>(a, f, R1);
+        if (ok && (ok = pass())) cg_x_pass<T>(a, f, R0);
+        if (ok && (ok = pass())) cg_y_pass<T, true>(a, f, R1);
+        if (ok && (ok = pass())) cg_z_pass<T, true>(a, f, R2);
+        if (!ok && threadIdx.x == 0) broken = 1;
       }
+    } else if (a.have_pairs) {
+      cg_pairs<T>(a, kCgFft, kCgThreads - kCgFft);
     }
-    if (kspace) {
-      if (!cg_barrier(a.sh, target)) return stop();
-      cg_y_pass<T, false>(a, f, R1);
-      if (!cg_barrier(a.sh, target)) return stop();
-      cg_x_pass<T>(a, f, R0);
-      if (!cg_barrier(a.sh, target)) return stop();
-      cg_y_pass<T, true>(a, f, R1);
-      if (!cg_barrier(a.sh, target)) return stop();
-      cg_z_pass<T, true>(a, f, R2);
-    }
-    if (!cg_barrier(a.sh, target)) return stop();
+    if (kspace) target += 4 * gridDim.x;
+    __syncthreads();
+    if (broken) return stop();
+    if (!meet()) return stop();
     // ---- E: potential, diagonal and rank-one terms, p.Hp and C.Hp
     {
       volatile CgSlot& V = S;
-      const double sp = V.sp, spz = V.spz, spz2 = V.spz2, nn = sc->nn, pre = sc->pre, Lz2 = sc->Lz2;
+      const double sp = V.sp, spz = V.spz, spz2 = V.spz2;
       double acc[5] = {0, 0, 0, 0, 0};
       int u = 0;
       for (int gi = g0; gi < ng; gi += gstep, ++u) {
-        const int na = min(kPw, a.N - gi * kPw);
+        const int na = atoms(gi), i = gi * a.group + (lane >> 2);
+        const bool mine = (lane & 3) == 0 && (lane >> 2) < na;
+        const double x = mine ? (double)a.p[i] : 0.0, dg = mine ? a.diag[i] : 0.0;
+        const T hp = mine ? a.Hp[i] : T(0);
         T pot = T(0);
         if (kspace) {
           WarpStencil<T, false> ws = stencil(u);
-          if (!a.kept) warp_build_stencil<T, false>(ws, d, g, a.pos, nullptr, nullptr, gi * kPw, a.N, lane);
+          if (!a.kept) build(ws, gi);
           pot = gather_group<T, false>(ws, na, a.K1, a.K2, a.mesh, lane);
           __syncwarp();
         }
-        if ((lane & 3) == 0 && (lane >> 2) < na) {
-          const int i = gi * kPw + (lane >> 2);
-          const double x = (double)a.p[i];
-          double h = (double)(T)(a.Hp[i] + pot) + a.diag[i] * x + nn * sp;
+        if (mine) {
+          double h = (double)(T)(hp + pot) + dg * x + nn * sp;
           if (slab) {
             const double z = a.zc[i];
             h += pre * (2.0 * z * spz - spz2 - z * z * sp - Lz2 / 6.0 * sp);
@@ -381,40 +454,56 @@ __global__ void __launch_bounds__(kCgThreads) qeq_cg_kernel(CgArgs<T> a) {
           for (int c = 0; c < nc; ++c) acc[1 + c] += cval(a.C, c, (long long)a.N, i) * h;
         }
       }
-      double a1[1] = {acc[0]};
-      block_atomic_sum<1>(a1, &S.pHp, red);
-      if (nc > 0) {
-        double a4[4] = {acc[1], acc[2], acc[3], acc[4]};
-        block_atomic_sum<4>(a4, S.Cv, red);
+      // p.Hp and the first three of C.Hp are next to each other in the slot
+      const double a4[4] = {acc[0], acc[1], acc[2], acc[3]};
+      cg_block_sum<4>(a4, &S.pHp, red2);
+      if (nc == kMaxConst) {
+        __syncthreads();
+        const double a1[1] = {acc[4]};
+        cg_block_sum<1>(a1, &S.Cv[kMaxConst - 1], red);
       }
     }
-    if (!cg_barrier(a.sh, target)) return stop();
+    if (!meet()) return stop();
     // ---- F: iterate and residual; zero what the next iteration accumulates into
     {
+      const int tid = blockIdx.x * kCgThreads + threadIdx.x, nthr = gridDim.x * kCgThreads;
+      T hv = T(0), pw = T(0);
+      double xv = 0.0, rw = 0.0;
+      if (tid < a.N) {
+        hv = a.Hp[tid];
+        pw = a.p[tid];
+        xv = a.x[tid];
+        rw = a.r[tid];
+      }
       volatile CgSlot& V = S;
       const double pHp = V.pHp, alpha = pHp != 0.0 ? rr / pHp : 0.0;
       double lam[kMaxConst] = {0, 0, 0, 0};
       for (int r0 = 0; r0 < nc; ++r0)
         for (int c = 0; c < nc; ++c) lam[r0] += sc->Ginv[r0 * kMaxConst + c] * V.Cv[c];
       double acc[1] = {0.0};
-      const int tid = blockIdx.x * kCgThreads + threadIdx.x, nthr = gridDim.x * kCgThreads;
       for (int i = tid; i < a.N; i += nthr) {
-        double w = (double)a.Hp[i];
+        if (i != tid) {
+          hv = a.Hp[i];
+          pw = a.p[i];
+          xv = a.x[i];
+          rw = a.r[i];
+        }
+        double w = (double)hv;
         a.Hp[i] = T(0);
         for (int c = 0; c < nc; ++c) w -= cval(a.C, c, (long long)a.N, i) * lam[c];
-        a.x[i] += alpha * (double)a.p[i];
-        const double rn = a.r[i] - alpha * w;
+        a.x[i] = xv + alpha * (double)pw;
+        const double rn = rw - alpha * w;
         a.r[i] = rn;
         acc[0] += rn * rn;
       }
-      block_atomic_sum<1>(acc, &S.rr_new, red);
       if (kspace) {
         const size_t M = (size_t)a.K0 * a.K1 * a.K2;
         for (size_t i = tid; i < M; i += nthr) a.mesh[i] = T(0);
       }
       if (blockIdx.x == 0 && threadIdx.x == 0) a.sh->slot[(k + 1) % 3] = CgSlot{};
+      cg_block_sum<1>(acc, &S.rr_new, red);
     }
-    if (!cg_barrier(a.sh, target)) return stop();
+    if (!meet()) return stop();
   }
 }
 
