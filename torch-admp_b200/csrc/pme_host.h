@@ -16,6 +16,8 @@ namespace admp {
 constexpr int kStWarps = 4;
 constexpr int kGatherRun = 64000;
 
+constexpr int kFillBlocks = 296;  // two blocks on each of 148 SMs
+
 struct SysSpec {
   int natoms;
   int atom_off;
@@ -151,6 +153,14 @@ inline Batch family_batch(const RecipPlan<T>& p, int F) {
 // device bytes of a system table (kept 256-byte aligned for what follows it)
 inline size_t sys_table_bytes() { return align_up(sizeof(SysDesc) * kMaxBatch, 256); }
 
+// Lines per block of a transform pass of `total` lines: at most `most`, fewer
+// (two at least) where that would leave SMs without a block.  79^3, FP32, one
+// system: x pass with the Green's function 27.4 -> 21.5 us, 42^3 15.9 -> 11.6.
+inline int few_lines(long long total, int most) {
+  const long long per = (total + kFillBlocks - 1) / kFillBlocks;
+  return per < most ? (per < 2 ? 2 : (int)per) : most;
+}
+
 template <typename T>
 inline int build_recip_plan(const SysSpec* sys, int nsys, RecipPlan<T>& p) {
   if (nsys <= 0 || nsys > kMaxBatch) return fail(ADMP_ERR_BAD_ARG, "batch of %d systems (max %d)", nsys, kMaxBatch);
@@ -174,12 +184,19 @@ inline int build_recip_plan(const SysSpec* sys, int nsys, RecipPlan<T>& p) {
   b.maxK2 = maxK[2];
   const size_t cs = sizeof(Cplx<T>);
   const size_t budget = 150 * 1024;
+  long long pairs = 0, cols = 0, planes = 0;  // z line pairs, x columns and x planes of the launch
+  for (int s = 0; s < nsys; ++s) {
+    pairs += ((long long)sys[s].K[0] * sys[s].K[1] + 1) / 2;
+    cols += (long long)sys[s].K[1] * (sys[s].K[2] / 2 + 1);
+    planes += sys[s].K[0];
+  }
   // z passes: lp line pairs of length K2 per block, two buffers
   int lp = (int)((sizeof(T) == 4 ? 4096 : 2048) / maxK[2]);
   lp = lp < 1 ? 1 : (lp > 64 ? 64 : lp);
+  lp = few_lines(pairs, lp);
   while (lp > 1 && (2 * (size_t)lp + 1) * maxK[2] * cs > budget) --lp;
   b.lp = lp;
-  int zb = sizeof(T) == 4 ? 32 : 16;
+  int zb = few_lines(cols, sizeof(T) == 4 ? 32 : 16);
   const int mk01 = maxK[0] > maxK[1] ? maxK[0] : maxK[1];
   while (zb > 1 && (2 * (size_t)zb + 1) * mk01 * cs + (mk01 + 2 * zb) * 8 + zb * 16 > budget) zb >>= 1;
   b.zb = zb;
@@ -236,23 +253,29 @@ inline int build_recip_plan(const SysSpec* sys, int nsys, RecipPlan<T>& p) {
   b.nblk_x = bx;
   p.mesh_elems = mo;
   p.spec_elems = so;
-  // fused slab passes: two buffers of at least one plane (max(ceil(K1/2) K2, K1 (K2/2+1)) complex) and at
-  // least kSlabTarget complex values, so that small meshes take several planes per block; plus twiddles
+  // Fused slab passes: two buffers of at least one plane (max(ceil(K1/2) K2, K1 (K2/2+1)) complex).  With
+  // enough planes to fill the chip small meshes take several planes a block (at least kSlabTarget complex
+  // values); with fewer, one plane a block (17^3 / 32^3, one system, FP32: 11.7 / 11.2 -> 6.9 / 7.0 us).
   const int kSlabTarget = sizeof(T) == 4 ? 3072 : 1536;
-  int be = kSlabTarget;
+  int plane = 1;
   for (int s = 0; s < nsys; ++s) {
     const int a = slab_plane_elems(sys[s].K[1], sys[s].K[2]);
-    be = be > a ? be : a;
+    plane = plane > a ? plane : a;
   }
+  const int be = planes >= 2 * kFillBlocks && plane < kSlabTarget ? kSlabTarget : plane;
   p.buf_elems = be;
   p.smem_slab = (2 * (size_t)be + maxK[1] + maxK[2]) * cs;
-  p.slab = p.smem_slab <= 200 * 1024;
   b.nblk_slab = 0;
   for (int s = 0; s < nsys; ++s) {
     p.hs[s].blk_slab = b.nblk_slab;
     const int ppb = slab_ppb(be, slab_plane_elems(sys[s].K[1], sys[s].K[2]), sys[s].K[0]);
     b.nblk_slab += (sys[s].K[0] + ppb - 1) / ppb;
   }
+  // Few large planes leave SMs idle for long: separate z and y passes, split by lines, take two launches more
+  // but fill the chip (both transforms and the x pass, one system: 79^3 FP32 81 -> 67, FP64 102 -> 91 us,
+  // 64 x 64 x 160 FP32 51 -> 45; equal at 64^3, and slower from four systems of 79^3 on).
+  constexpr int kSplitPlane = 2304;
+  p.slab = p.smem_slab <= 200 * 1024 && !(plane > kSplitPlane && b.nblk_slab < kFillBlocks);
   b.fam = F_ATOM;
   for (int s = 0; s < nsys; ++s) b.blk[s] = p.hs[s].blk_atom;
   return ADMP_OK;

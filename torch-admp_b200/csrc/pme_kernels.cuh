@@ -440,13 +440,27 @@ __global__ void __launch_bounds__(256) fft_x_green_kernel(Batch b, Cplx<T>* __re
   Cplx<T>* W = reinterpret_cast<Cplx<T>*>(smem_raw);
   Cplx<T>* A = W + b.maxK0;
   Cplx<T>* B = A + (size_t)zb * b.maxK0;
-  double* thx = reinterpret_cast<double*>(B + (size_t)zb * b.maxK0);
-  double* thyz = thx + b.maxK0;   // theta_y theta_z per column
-  double* wcol = thyz + zb;       // half-spectrum weight per column
+  // 1 / theta^2 per x and per column, times exp(-k^2 / 4 kappa^2) of that axis (axes) where the cell is
+  // orthorhombic and the exponential factorises
+  double* gx = reinterpret_cast<double*>(B + (size_t)zb * b.maxK0);
+  double* gyz = gx + b.maxK0;
+  double* wcol = gyz + zb;        // half-spectrum weight per column
   int* lab = reinterpret_cast<int*>(wcol + zb);  // per column: ny, mirror ny, nz, mirror nz
   make_twiddles(W, K0);
   load_geom(box, d.box_idx, &g);
-  for (int i = threadIdx.x; i < K0; i += blockDim.x) thx[i] = theta_1d(signed_k(i, K0), K0);
+  __syncthreads();
+  const double kappa = d.kappa;
+  const double inv4k2 = 1.0 / (4.0 * kappa * kappa);
+  const bool ortho = g.binv[1] == 0.0 && g.binv[2] == 0.0 && g.binv[3] == 0.0 && g.binv[5] == 0.0 &&
+                     g.binv[6] == 0.0 && g.binv[7] == 0.0;
+  auto decay = [&](int n, int axis) {
+    const double k = 2.0 * kPi * n * g.binv[4 * axis];
+    return ortho ? exp(-k * k * inv4k2) : 1.0;
+  };
+  for (int i = threadIdx.x; i < K0; i += blockDim.x) {
+    const double th = theta_1d(signed_k(i, K0), K0);
+    gx[i] = decay(signed_k(i, K0), 0) / (th * th);
+  }
   for (int i = threadIdx.x; i < nz; i += blockDim.x) {
     const int c = c0 + i, y = c / K2h, kz = c - y * K2h;
     // labels of the mirror indices -y, -kz (the reference labels K/2 as -K/2,
@@ -456,7 +470,8 @@ __global__ void __launch_bounds__(256) fft_x_green_kernel(Batch b, Cplx<T>* __re
     lab[4 * i + 1] = signed_k(y == 0 ? 0 : K1 - y, K1);
     lab[4 * i + 2] = n2;
     lab[4 * i + 3] = signed_k(kz == 0 ? 0 : K2 - kz, K2);
-    thyz[i] = theta_1d(ny, K1) * theta_1d(n2, K2);
+    const double th = theta_1d(ny, K1) * theta_1d(n2, K2);
+    gyz[i] = decay(ny, 1) * decay(n2, 2) / (th * th);
     wcol[i] = (kz == 0 || (2 * kz == K2)) ? 1.0 : 2.0;
   }
   Cplx<T>* H = spec + d.spec_off + c0;
@@ -474,8 +489,6 @@ __global__ void __launch_bounds__(256) fft_x_green_kernel(Batch b, Cplx<T>* __re
   __syncthreads();
   Cplx<T>* R = fft_lines<T, true, false>(A, B, nz, K0, 1, zb, W);
   Cplx<T>* F = (R == A) ? B : A;
-  const double kappa = d.kappa;
-  const double inv4k2 = 1.0 / (4.0 * kappa * kappa);
   const double pref = ke * 2.0 * kPi / g.vol;
   double v[NV];
 #pragma unroll
@@ -489,8 +502,7 @@ __global__ void __launch_bounds__(256) fft_x_green_kernel(Batch b, Cplx<T>* __re
     // kz = 0 and kz = K2/2 planes, whose mirrors are separate entries).
     const int ny = lab[4 * c], nyb = lab[4 * c + 1], n2 = lab[4 * c + 2], n2b = lab[4 * c + 3];
     const int n0 = signed_k(x, K0), n0b = signed_k(x == 0 ? 0 : K0 - x, K0);
-    const double th = thx[x] * thyz[c];
-    const double inv_th2 = 1.0 / (th * th);
+    const double gxyz = pref * gx[x] * gyz[c];
     const double w = wcol[c];
     Cplx<T> S = R[x * zb + c];
     const double s2 = (double)S.x * (double)S.x + (double)S.y * (double)S.y;
@@ -509,7 +521,7 @@ __global__ void __launch_bounds__(256) fft_x_green_kernel(Batch b, Cplx<T>* __re
       for (int e = 0; e < 3; ++e)
         kv[e] = 2.0 * kPi * (a0 * g.binv[0 * 3 + e] + a1 * g.binv[1 * 3 + e] + a2 * g.binv[2 * 3 + e]);
       const double ksq = kv[0] * kv[0] + kv[1] * kv[1] + kv[2] * kv[2];
-      const double G = pref / ksq * exp(-ksq * inv4k2) * inv_th2;
+      const double G = gxyz / ksq * (ortho ? 1.0 : exp(-ksq * inv4k2));
       Gs += 0.5 * mult * G;
       const double Ek = 0.5 * mult * w * G * s2;
       v[0] += Ek;
