@@ -168,13 +168,18 @@ int admp_coulomb_pbc(int dtype, int flags, int nframes, int natoms, const int* k
 /* Gaussian damping energy, pairs and self part (qeq.py:60-129), and chemical */
 /* site energy (qeq.py:159-209) of nframes systems.  As admp_coulomb_pbc they */
 /* WRITE their outputs: energy [nframes] double and the gradients not NULL.   */
-int admp_damping_energy(int dtype, int nframes, int natoms, long long npairs,
+/* flags: 0 or ADMP_PAIR_INT64_SCALES.                                        */
+int admp_damping_energy(int dtype, int flags, int nframes, int natoms, long long npairs,
                         const long long* pairs, const void* ds, const void* buffer_scales,
                         const void* q, const void* eta, double ke, double* energy, void* dE_dds,
                         void* dE_dq, void* dE_deta, void* stream);
 int admp_site_energy(int dtype, int nframes, int natoms, const void* q, const void* chi,
                      const void* hardness, double* energy, void* dE_dq, void* dE_dchi,
                      void* dE_dhard, void* stream);
+/* out[k][f, :] = in[k][f, :] * w[f w_stride] for up to four arrays (host      */
+/* arrays of device pointers, per_frame[k] values a frame) in one launch.      */
+int admp_scale_frames(int dtype, int nframes, int narrays, const void* const* in, void* const* out,
+                      const long long* per_frame, const void* w, long long w_stride, void* stream);
 /* Copies up to 64 KiB of device memory to `host` through page-locked staging */
 /* and waits for it.                                                          */
 int admp_read_back(const void* dev, size_t bytes, void* host, void* stream);
@@ -192,6 +197,7 @@ int admp_pair_distances_backward(int dtype, int pbc, int natoms, long long npair
 
 /* The backward over nframes frames of one atom count (pairs [nframes,       */
 /* npairs, 2] with frame-local indices); rows with i == j contribute nothing. */
+/* Outputs are written.                                                       */
 /* It does not wait for the device: a bad index is skipped and left in the    */
 /* error word for the next checked call or admp_check_errors.                 */
 int admp_pair_distances_frames_backward(int dtype, int pbc, int nframes, int natoms,
@@ -280,6 +286,7 @@ int admp_image_pair_distances_backward(int dtype, int natoms, long long npairs,
 #define ADMP_QEQ_SLAB 8         /* slab axis in bits 8..9 */
 #define ADMP_QEQ_PROJECT_Q0 16  /* project the initial guess onto C q = b first */
 #define ADMP_QEQ_DEVICE_B 32    /* b is DEVICE memory (the host need not wait for it) */
+#define ADMP_PAIR_INT64_SCALES 64 /* admp_coulomb_pbc, admp_damping_energy: buffer_scales is int64 */
 size_t admp_qeq_workspace_size(int dtype, int natoms, long long npairs, const int* kmesh,
                                int n_const);
 int admp_qeq_solve(int dtype, int flags, int natoms, const int* kmesh, const void* pos,

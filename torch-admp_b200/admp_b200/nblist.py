@@ -51,9 +51,8 @@ class TorchNeighborList(torch.nn.Module):
         if status == L.CUTOFF:
             check_cutoff(box, self.cutoff)
         L.check(status, "neighbour list")
-        self.pairs = pairs
-        self.buffer_scales = bs
-        self.ds = ds
+        # plain attributes: Module.__setattr__ looks for parameters, buffers and modules first
+        self.__dict__.update(pairs=pairs, buffer_scales=bs, ds=ds)
         return pairs
 
     @staticmethod

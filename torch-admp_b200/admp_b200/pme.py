@@ -118,7 +118,7 @@ class CoulombForceModule(BaseForceModule):
                              + str(positions.device))
         dt = positions.dtype
         charges = params["charge"].reshape(nf, na).to(dt)
-        bs = buffer_scales.to(dt)
+        bs = buffer_scales  # int64 scales are taken as they are, others converted by the operators
         dsc = ds.to(dt)
         ke = self.const_lib.dielectric
         if box is None:

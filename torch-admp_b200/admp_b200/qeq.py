@@ -45,7 +45,7 @@ class GaussianDampingForceModule(BaseForceModule):
         if lc != 1.0:
             eta = eta * lc
         eta = eta.to(dt)
-        return torch.ops.admp_b200.damping(ds.to(dt), q, eta, pairs, buffer_scales.to(dt), self.const_lib.dielectric)
+        return torch.ops.admp_b200.damping(ds.to(dt), q, eta, pairs, buffer_scales, self.const_lib.dielectric)
 
 
 class SiteForceModule(BaseForceModule):

@@ -12,14 +12,17 @@ namespace admp {
 template <typename T, int MODE>
 __global__ void __launch_bounds__(256)
     pair_list_kernel(int N, long long P, const long long* __restrict__ pairs, const T* __restrict__ ds,
-                     const T* __restrict__ bs, const T* __restrict__ q, const T* __restrict__ eta, T kappa,
+                     const void* __restrict__ scales, int int_scales, const T* __restrict__ q,
+                     const T* __restrict__ eta, T kappa,
                      T ke, double* __restrict__ energy, int estride, int put, T* __restrict__ dE_dds,
                      T* __restrict__ dE_dq, T* __restrict__ dE_deta, DevError* err) {
   __shared__ double red[32];
   const int f = blockIdx.y;
   pairs += (size_t)f * P * 2;
   ds += (size_t)f * P;
-  bs += (size_t)f * P;
+  // buffer scales of the working type, or int64 as the neighbour list makes them
+  const T* bs = int_scales ? nullptr : (const T*)scales + (size_t)f * P;
+  const long long* ibs = int_scales ? (const long long*)scales + (size_t)f * P : nullptr;
   q += (size_t)f * N;
   if (eta) eta += (size_t)f * N;
   if (dE_dds) dE_dds += (size_t)f * P;
@@ -43,7 +46,7 @@ __global__ void __launch_bounds__(256)
         ok = false;
       }
     }
-    const T d = ok ? ds[p] : T(1), s = ok ? bs[p] : T(0);
+    const T d = ok ? ds[p] : T(1), s = ok ? (ibs ? (T)ibs[p] : bs[p]) : T(0);
     const T qi = ok ? q[i] : T(0), qj = ok ? q[j] : T(0);
     T ei = T(0), ej = T(0);
     if (MODE == ADMP_PAIR_DAMPING && ok) {
@@ -330,8 +333,8 @@ __global__ void __launch_bounds__(256)
       } else {
         for (int e = 0; e < 3; ++e) dr[e] = (double)pos[3 * j + e] - (double)pos[3 * i + e];
       }
-      const double d = sqrt(dr[0] * dr[0] + dr[1] * dr[1] + dr[2] * dr[2]);
-      s = d == 0.0 ? 0.0 : gp / d;
+      const double r2 = dr[0] * dr[0] + dr[1] * dr[1] + dr[2] * dr[2];
+      s = r2 == 0.0 ? 0.0 : gp * rsqrt(r2);
     }
     // dr points from j to i with a box and from i to j without: the first atom gets +v or -v; its share is summed
     // over the run of pairs that start with it
@@ -344,7 +347,7 @@ __global__ void __launch_bounds__(256)
         if (runs.opens && a != T(0)) atomicAdd(gpos + 3 * i + e, a);
         if (w != T(0)) atomicAdd(gpos + 3 * j + e, -w);
       }
-      if (pbc)
+      if (pbc && gbox)
         for (int k = 0; k < 3; ++k) vb[k * 3 + e] -= n[k] * v;
     }
   }
@@ -357,12 +360,32 @@ __global__ void __launch_bounds__(256)
   }
 }
 
+// out[f][k] = in[f][k] * w[f] for up to four arrays in one launch
+struct ScaleArgs {
+  const void* in[4];
+  void* out[4];
+  long long n[4];  // values per frame
+};
+template <typename T>
+__global__ void __launch_bounds__(256) scale_frames_kernel(ScaleArgs a, const T* __restrict__ w, long long wstride) {
+  const int f = blockIdx.y;
+  const T x = w[f * wstride];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const T* in = (const T*)a.in[k] + (size_t)f * a.n[k];
+    T* out = (T*)a.out[k] + (size_t)f * a.n[k];
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < a.n[k];
+         i += (long long)gridDim.x * blockDim.x)
+      out[i] = in[i] * x;
+  }
+}
+
 // ------------------------------------------------------------------ host side
 // energy[f estride] += E of frame f; dE/dds is added to, or with `put` written.
 template <typename T>
-int launch_pair_energy(int mode, int nf, int N, long long P, const long long* pairs, const T* ds, const T* bs,
-                       const T* q, const T* eta, double kappa, double ke, double* energy, int estride, bool put, T* dds,
-                       T* dq, T* deta, DevError* err, cudaStream_t st) {
+int launch_pair_energy(int mode, int nf, int N, long long P, const long long* pairs, const T* ds, const void* bs,
+                       bool int_scales, const T* q, const T* eta, double kappa, double ke, double* energy, int estride,
+                       bool put, T* dds, T* dq, T* deta, DevError* err, cudaStream_t st) {
   if (P == 0 || nf == 0) return ADMP_OK;
   long long blocks = (P + 255) / 256;
   if (blocks > 4096) blocks = 4096;
@@ -370,15 +393,15 @@ int launch_pair_energy(int mode, int nf, int N, long long P, const long long* pa
   auto* k = mode == ADMP_PAIR_EWALD ? pair_list_kernel<T, ADMP_PAIR_EWALD>
             : mode == ADMP_PAIR_OBC ? pair_list_kernel<T, ADMP_PAIR_OBC>
                                     : pair_list_kernel<T, ADMP_PAIR_DAMPING>;
-  k<<<grid, 256, 0, st>>>(N, P, pairs, ds, bs, q, eta, (T)kappa, (T)ke, energy, estride, put ? 1 : 0, dds, dq, deta,
-                          err);
+  k<<<grid, 256, 0, st>>>(N, P, pairs, ds, bs, int_scales ? 1 : 0, q, eta, (T)kappa, (T)ke, energy, estride,
+                          put ? 1 : 0, dds, dq, deta, err);
   ADMP_CUDA_TRY(cudaGetLastError());
   return ADMP_OK;
 }
-template int launch_pair_energy<float>(int, int, int, long long, const long long*, const float*, const float*,
+template int launch_pair_energy<float>(int, int, int, long long, const long long*, const float*, const void*, bool,
                                        const float*, const float*, double, double, double*, int, bool, float*, float*,
                                        float*, DevError*, cudaStream_t);
-template int launch_pair_energy<double>(int, int, int, long long, const long long*, const double*, const double*,
+template int launch_pair_energy<double>(int, int, int, long long, const long long*, const double*, const void*, bool,
                                         const double*, const double*, double, double, double*, int, bool, double*,
                                         double*, double*, DevError*, cudaStream_t);
 
@@ -389,7 +412,7 @@ static int pair_energy_impl(int mode, int nf, int N, long long P, const long lon
   if (P == 0 || nf == 0) return ADMP_OK;
   DevError* err = scratch_error(st);
   if (!err) return ADMP_ERR_CUDA;
-  const int s = launch_pair_energy<T>(mode, nf, N, P, pairs, (const T*)ds, (const T*)bs, (const T*)q, (const T*)eta,
+  const int s = launch_pair_energy<T>(mode, nf, N, P, pairs, (const T*)ds, bs, false, (const T*)q, (const T*)eta,
                                       kappa, ke, energy, 1, false, (T*)dds, (T*)dq, (T*)deta, err, st);
   return s ? s : check_error(err, st);
 }
@@ -502,16 +525,21 @@ extern "C" int admp_pair_distances_backward(int dtype, int pbc, int natoms, long
 extern "C" int admp_pair_distances_frames_backward(int dtype, int pbc, int nframes, int natoms, long long npairs,
                                                    const long long* pairs, const void* pos, const void* box,
                                                    const void* grad_ds, void* grad_pos, void* grad_box, void* stream) {
-  if (npairs == 0 || nframes == 0) return ADMP_OK;
-  if (nframes < 0 || nframes > 65535 || npairs < 0 || !pairs || !pos || !grad_ds || (pbc && !box))
+  if (nframes < 0 || nframes > 65535 || natoms < 0 || npairs < 0 || (dtype != ADMP_F64 && dtype != ADMP_F32))
     return fail(ADMP_ERR_BAD_ARG, "admp_pair_distances_frames_backward: args");
   cudaStream_t st = (cudaStream_t)stream;
+  const size_t size = dtype == ADMP_F64 ? 8 : 4;
+  if (grad_pos) ADMP_CUDA_TRY(cudaMemsetAsync(grad_pos, 0, size * 3 * natoms * nframes, st));
+  if (grad_box) ADMP_CUDA_TRY(cudaMemsetAsync(grad_box, 0, size * 9 * nframes, st));
+  if (npairs == 0 || nframes == 0) return ADMP_OK;
+  if (!pairs || !pos || !grad_ds || (pbc && !box))
+    return fail(ADMP_ERR_BAD_ARG, "admp_pair_distances_frames_backward: args");
   DevError* err = scratch_error(st);
   if (!err) return ADMP_ERR_CUDA;
   return pair_dist_bwd(dtype, pbc, nframes, natoms, npairs, pairs, pos, box, grad_ds, grad_pos, grad_box, err, st);
 }
 
-extern "C" int admp_damping_energy(int dtype, int nframes, int natoms, long long npairs, const long long* pairs,
+extern "C" int admp_damping_energy(int dtype, int flags, int nframes, int natoms, long long npairs, const long long* pairs,
                                    const void* ds, const void* buffer_scales, const void* q, const void* eta, double ke,
                                    double* energy, void* dE_dds, void* dE_dq, void* dE_deta, void* stream) {
   if (nframes <= 0 || nframes > 65535 || natoms <= 0 || npairs < 0 || !q || !eta || !energy)
@@ -523,19 +551,20 @@ extern "C" int admp_damping_energy(int dtype, int nframes, int natoms, long long
   if (!err) return ADMP_ERR_CUDA;
   ADMP_CUDA_TRY(cudaMemsetAsync(energy, 0, sizeof(double) * nframes, st));
   const dim3 grid((natoms + 255) / 256, nframes);
+  const bool ints = (flags & ADMP_PAIR_INT64_SCALES) != 0;
   int s;
   if (dtype == ADMP_F64) {
     atom_energy_kernel<double, true><<<grid, 256, 0, st>>>(natoms, (const double*)q, (const double*)eta, nullptr, ke,
                                                            energy, (double*)dE_dq, (double*)dE_deta, nullptr);
     s = launch_pair_energy<double>(ADMP_PAIR_DAMPING, nframes, natoms, npairs, pairs, (const double*)ds,
-                                   (const double*)buffer_scales, (const double*)q, (const double*)eta, 0.0, ke, energy,
-                                   1, true, (double*)dE_dds, (double*)dE_dq, (double*)dE_deta, err, st);
+                                   buffer_scales, ints, (const double*)q, (const double*)eta, 0.0, ke, energy, 1, true,
+                                   (double*)dE_dds, (double*)dE_dq, (double*)dE_deta, err, st);
   } else {
     atom_energy_kernel<float, true><<<grid, 256, 0, st>>>(natoms, (const float*)q, (const float*)eta, nullptr, ke,
                                                           energy, (float*)dE_dq, (float*)dE_deta, nullptr);
     s = launch_pair_energy<float>(ADMP_PAIR_DAMPING, nframes, natoms, npairs, pairs, (const float*)ds,
-                                  (const float*)buffer_scales, (const float*)q, (const float*)eta, 0.0, ke, energy, 1,
-                                  true, (float*)dE_dds, (float*)dE_dq, (float*)dE_deta, err, st);
+                                  buffer_scales, ints, (const float*)q, (const float*)eta, 0.0, ke, energy, 1, true,
+                                  (float*)dE_dds, (float*)dE_dq, (float*)dE_deta, err, st);
   }
   ADMP_CUDA_TRY(cudaGetLastError());
   return s || npairs == 0 ? s : check_error(err, st);
@@ -557,6 +586,32 @@ extern "C" int admp_site_energy(int dtype, int nframes, int natoms, const void* 
     atom_energy_kernel<float, false><<<grid, 256, 0, st>>>(natoms, (const float*)q, (const float*)chi,
                                                            (const float*)hardness, 0.0, energy, (float*)dE_dq,
                                                            (float*)dE_dchi, (float*)dE_dhard);
+  else
+    return fail(ADMP_ERR_BAD_ARG, "bad dtype");
+  ADMP_CUDA_TRY(cudaGetLastError());
+  return ADMP_OK;
+}
+
+extern "C" int admp_scale_frames(int dtype, int nframes, int narrays, const void* const* in, void* const* out,
+                                 const long long* per_frame, const void* w, long long w_stride, void* stream) {
+  if (nframes <= 0 || nframes > 65535 || narrays < 0 || narrays > 4 || !w)
+    return nframes == 0 ? ADMP_OK : fail(ADMP_ERR_BAD_ARG, "admp_scale_frames: args");
+  ScaleArgs a{};
+  long long most = 0;
+  for (int k = 0; k < narrays; ++k) {
+    a.in[k] = in[k];
+    a.out[k] = out[k];
+    a.n[k] = per_frame[k];
+    most = most > per_frame[k] ? most : per_frame[k];
+  }
+  if (most == 0) return ADMP_OK;
+  long long blocks = (most + 255) / 256;
+  if (blocks > 2048) blocks = 2048;
+  const dim3 grid((unsigned)blocks, nframes);
+  if (dtype == ADMP_F64)
+    scale_frames_kernel<double><<<grid, 256, 0, (cudaStream_t)stream>>>(a, (const double*)w, w_stride);
+  else if (dtype == ADMP_F32)
+    scale_frames_kernel<float><<<grid, 256, 0, (cudaStream_t)stream>>>(a, (const float*)w, w_stride);
   else
     return fail(ADMP_ERR_BAD_ARG, "bad dtype");
   ADMP_CUDA_TRY(cudaGetLastError());

@@ -18,6 +18,12 @@ constexpr int kGatherRun = 64000;
 
 constexpr int kFillBlocks = 296;  // two blocks on each of 148 SMs
 
+constexpr int kMaxMesh = 4096;  // longest axis of the shared-memory transforms
+
+// places a system's mesh and half spectrum take in the packed buffers
+inline size_t mesh_elems_of(const int* K) { return align_up((size_t)K[0] * K[1] * K[2], 64); }
+inline size_t spec_elems_of(const int* K) { return align_up((size_t)K[0] * K[1] * (K[2] / 2 + 1), 32); }
+
 struct SysSpec {
   int natoms;
   int atom_off;
@@ -175,8 +181,8 @@ inline int build_recip_plan(const SysSpec* sys, int nsys, RecipPlan<T>& p) {
   int maxK[3] = {1, 1, 1};
   for (int s = 0; s < nsys; ++s)
     for (int d = 0; d < 3; ++d) {
-      if (sys[s].K[d] <= 0 || sys[s].K[d] > 4096)
-        return fail(ADMP_ERR_MESH, "mesh size %d out of range [1, 4096]", sys[s].K[d]);
+      if (sys[s].K[d] <= 0 || sys[s].K[d] > kMaxMesh)
+        return fail(ADMP_ERR_MESH, "mesh size %d out of range [1, %d]", sys[s].K[d], kMaxMesh);
       maxK[d] = maxK[d] > sys[s].K[d] ? maxK[d] : sys[s].K[d];
     }
   b.maxK0 = maxK[0];
@@ -238,8 +244,8 @@ inline int build_recip_plan(const SysSpec* sys, int nsys, RecipPlan<T>& p) {
     bxt += (d.K1 * d.K2h + kTcRows - 1) / kTcRows;
     byt += (d.K0 * d.K2h + kTcRows - 1) / kTcRows;
     bzt += (d.K0 * d.K1 + kTcRows - 1) / kTcRows;
-    mo += align_up((size_t)d.K0 * d.K1 * d.K2, 64);
-    so += align_up((size_t)d.K0 * d.K1 * d.K2h, 32);
+    mo += mesh_elems_of(sys[s].K);
+    so += spec_elems_of(sys[s].K);
   }
   b.nblk_atom = ba;
   b.nblk_st = bst;

@@ -22,24 +22,31 @@ static int recip_chunk_plan(int c0, int nsys, int N, const int* kmesh, double ka
 }
 
 template <typename T>
-static size_t recip_ws_bytes(const RecipPlan<T>& p) {
+static size_t recip_ws_bytes(size_t mesh_elems, size_t spec_elems, int nsys) {
   Carver c(nullptr, 0);
   c.take<unsigned char>(sys_table_bytes());
-  c.take<T>(p.mesh_elems);
-  c.take<Cplx<T>>(p.spec_elems);
-  c.take<double>((size_t)p.b.nsys * kAccStride);
+  c.take<T>(mesh_elems);
+  c.take<Cplx<T>>(spec_elems);
+  c.take<double>((size_t)nsys * kAccStride);
   return c.off;
 }
 
+// Workspace of the largest chunk, from the mesh sizes alone (as build_recip_plan
+// lays the meshes out; every mesh within its range fits the passes).
 template <typename T>
 static int recip_ws_size(int nf, const int* kmesh, size_t* out) {
   size_t best = 0;
   for (int c0 = 0; c0 < nf; c0 += kMaxBatch) {
     const int ns = nf - c0 < kMaxBatch ? nf - c0 : kMaxBatch;
-    RecipPlan<T> p;
-    int s = recip_chunk_plan<T>(c0, ns, 1, kmesh, 1.0, p);
-    if (s) return s;
-    size_t b = recip_ws_bytes(p);
+    size_t mesh = 0, spec = 0;
+    for (int s = 0; s < ns; ++s) {
+      const int* K = kmesh + 3 * (c0 + s);
+      for (int d = 0; d < 3; ++d)
+        if (K[d] <= 0 || K[d] > kMaxMesh) return fail(ADMP_ERR_MESH, "mesh size %d out of range [1, %d]", K[d], kMaxMesh);
+      mesh += mesh_elems_of(K);
+      spec += spec_elems_of(K);
+    }
+    const size_t b = recip_ws_bytes<T>(mesh, spec, ns);
     best = b > best ? b : best;
   }
   *out = best;
@@ -82,7 +89,7 @@ static int pme_recip_impl(int nf, int N, const int* kmesh, const T* pos, const T
 // the pair kernel's error word, after the rest has been launched.
 template <typename T>
 static int coulomb_impl(int flags, int nf, int N, const int* kmesh, const T* pos, const T* box, long long P,
-                        const long long* pairs, const T* ds, const T* bs, const T* q, double kappa, double ke, T* energy,
+                        const long long* pairs, const T* ds, const void* bs, const T* q, double kappa, double ke, T* energy,
                         double* comps, T* dpos, T* dq, T* dbox, T* dds, void* ws, size_t bytes, cudaStream_t st) {
   DevError* err = scratch_error(st);
   if (!err) return ADMP_ERR_CUDA;
@@ -110,8 +117,8 @@ static int coulomb_impl(int flags, int nf, int N, const int* kmesh, const T* pos
     s = prep_plan<T>(p, table, z, st);
     if (s) return s;
     if (c0 == 0 && pair) {
-      s = launch_pair_energy<T>(ADMP_PAIR_EWALD, nf, N, P, pairs, ds, bs, q, nullptr, kappa, ke, comps, 5, true, dds,
-                                dq, nullptr, err, st);
+      s = launch_pair_energy<T>(ADMP_PAIR_EWALD, nf, N, P, pairs, ds, bs, (flags & ADMP_PAIR_INT64_SCALES) != 0, q,
+                                nullptr, kappa, ke, comps, 5, true, dds, dq, nullptr, err, st);
       if (!s) s = probe_error(err, st);
       if (s) return s;
     }
@@ -170,12 +177,12 @@ extern "C" int admp_coulomb_pbc(int dtype, int flags, int nframes, int natoms, c
   cudaStream_t st = (cudaStream_t)stream;
   if (dtype == ADMP_F64)
     return coulomb_impl<double>(flags, nframes, natoms, kmesh, (const double*)pos, (const double*)box, npairs, pairs,
-                                (const double*)ds, (const double*)buffer_scales, (const double*)q, kappa, ke,
+                                (const double*)ds, buffer_scales, (const double*)q, kappa, ke,
                                 (double*)energy, comps, (double*)dE_dpos, (double*)dE_dq, (double*)dE_dbox,
                                 (double*)dE_dds, workspace, workspace_bytes, st);
   if (dtype == ADMP_F32)
     return coulomb_impl<float>(flags, nframes, natoms, kmesh, (const float*)pos, (const float*)box, npairs, pairs,
-                               (const float*)ds, (const float*)buffer_scales, (const float*)q, kappa, ke,
+                               (const float*)ds, buffer_scales, (const float*)q, kappa, ke,
                                (float*)energy, comps, (float*)dE_dpos, (float*)dE_dq, (float*)dE_dbox, (float*)dE_dds,
                                workspace, workspace_bytes, st);
   return fail(ADMP_ERR_BAD_ARG, "bad dtype");

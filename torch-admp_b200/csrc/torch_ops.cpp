@@ -55,6 +55,46 @@ X* ptr(const Tensor& t) {
   return t.defined() ? (X*)t.data_ptr() : nullptr;
 }
 
+// Buffer scales as a call takes them: int64 (as the neighbour list makes them) or the working type.
+Tensor scales_of(const Tensor& bs, const Tensor& like) {
+  return (bs.scalar_type() == torch::kLong ? bs : bs.to(like.scalar_type())).contiguous();
+}
+int scale_flag(const Tensor& bs) { return bs.scalar_type() == torch::kLong ? ADMP_PAIR_INT64_SCALES : 0; }
+
+// Saved gradients times the incoming dL/dE of each frame, all in one launch;
+// by torch operators where the product itself is to be differentiated
+// (create_graph with a dL/dE that needs a gradient).
+variable_list scaled(const variable_list& saved, const Tensor& gE) {
+  if (at::GradMode::is_enabled() && gE.requires_grad()) {
+    variable_list r(saved.size());
+    for (size_t i = 0; i < saved.size(); ++i)
+      if (saved[i].defined()) {
+        std::vector<int64_t> shape(saved[i].dim(), 1);
+        shape[0] = gE.numel();
+        r[i] = saved[i] * gE.reshape(shape);
+      }
+    return r;
+  }
+  const void* in[4];
+  void* out[4];
+  long long n[4];
+  int k = 0;
+  variable_list r(saved.size());
+  const int64_t nf = gE.numel();
+  for (size_t i = 0; i < saved.size(); ++i) {
+    if (!saved[i].defined()) continue;
+    r[i] = torch::empty_like(saved[i]);
+    in[k] = saved[i].data_ptr();
+    out[k] = r[i].data_ptr();
+    n[k++] = nf > 0 ? saved[i].numel() / nf : 0;
+  }
+  if (k && nf > 0)
+    check(admp_scale_frames(dtype_code(gE), (int)nf, k, in, out, n, gE.data_ptr(), nf > 1 ? gE.stride(0) : 0,
+                            stream_of(gE)),
+          "gradient scaling");
+  return r;
+}
+
 Tensor f64(int64_t n, const Tensor& like) {
   return torch::zeros({n}, like.options().dtype(torch::kDouble));
 }
@@ -108,7 +148,8 @@ class CoulombPBC : public torch::autograd::Function<CoulombPBC> {
     Tensor gpos, gbox, gds, gq;
     std::vector<int> km = kspace ? kmesh_per_frame(box, kappa, kmesh, spacing, ethresh)
                                  : std::vector<int>(3 * nf, 1);
-    Tensor kmt = torch::tensor(std::vector<int64_t>(km.begin(), km.end()), torch::kLong).reshape({nf, 3});
+    Tensor kmt = torch::empty({nf, 3}, torch::kLong);
+    for (int64_t k = 0; k < 3 * nf; ++k) kmt.data_ptr<int64_t>()[k] = km[k];
     if (kspace && N > 0 && nf > 0) {
       if (pos.requires_grad()) gpos = torch::empty_like(pos);
       if (box.requires_grad()) gbox = torch::empty_like(box);
@@ -119,7 +160,8 @@ class CoulombPBC : public torch::autograd::Function<CoulombPBC> {
       const size_t nbytes = admp_pme_recip_workspace_size(dt, (int)nf, km.data());
       TORCH_CHECK(nbytes > 0, "reciprocal workspace: ", admp_last_error_message());
       Tensor ws = torch::empty({(int64_t)nbytes}, pos.options().dtype(torch::kUInt8));
-      const int flags = ADMP_QEQ_KSPACE | (rspace ? ADMP_QEQ_RSPACE : 0) | (slab ? ADMP_QEQ_SLAB | ((int)axis << 8) : 0);
+      const int flags = ADMP_QEQ_KSPACE | (rspace ? ADMP_QEQ_RSPACE : 0) |
+                        (slab ? ADMP_QEQ_SLAB | ((int)axis << 8) : 0) | scale_flag(bs);
       check(admp_coulomb_pbc(dt, flags, (int)nf, (int)N, km.data(), ptr<void>(pos), ptr<void>(box), P,
                              ptr<const long long>(pairs), ptr<void>(ds), ptr<void>(bs), ptr<void>(q), kappa, ke,
                              ptr<void>(E), ptr<double>(comps), ptr<void>(gpos), ptr<void>(gq), ptr<void>(gbox),
@@ -135,9 +177,10 @@ class CoulombPBC : public torch::autograd::Function<CoulombPBC> {
     if (box.requires_grad()) gbox = torch::zeros_like(box);
     if (ds.requires_grad()) gds = torch::zeros_like(ds);
     if (q.requires_grad()) gq = torch::zeros_like(q);
+    const Tensor bst = bs.to(pos.scalar_type());
     if (rspace && P > 0)
       check(admp_pair_energy(dt, ADMP_PAIR_EWALD, (int)nf, (int)N, P, ptr<const long long>(pairs), ptr<void>(ds),
-                             ptr<void>(bs), ptr<void>(q), nullptr, kappa, ke, ptr<double>(E_real), ptr<void>(gds),
+                             ptr<void>(bst), ptr<void>(q), nullptr, kappa, ke, ptr<double>(E_real), ptr<void>(gds),
                              ptr<void>(gq), nullptr, st),
             "real-space pair energy");
     if (slab && N > 0)
@@ -153,17 +196,12 @@ class CoulombPBC : public torch::autograd::Function<CoulombPBC> {
   }
 
   static variable_list backward(AutogradContext* ctx, variable_list g) {
-    auto s = ctx->get_saved_variables();
-    const Tensor& gE = g[0];
-    Tensor out_pos, out_box, out_ds, out_q;
-    if (gE.defined()) {
-      if (s[0].defined()) out_pos = s[0] * gE.view({-1, 1, 1});
-      if (s[1].defined()) out_box = s[1] * gE.view({-1, 1, 1});
-      if (s[2].defined()) out_ds = s[2] * gE.view({-1, 1});
-      if (s[3].defined()) out_q = s[3] * gE.view({-1, 1});
+    variable_list out(15);
+    if (g[0].defined()) {
+      const variable_list s = scaled(ctx->get_saved_variables(), g[0]);
+      for (int k = 0; k < 4; ++k) out[k] = s[k];
     }
-    return {out_pos, out_box, out_ds, out_q, Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor(),
-            Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+    return out;
   }
 };
 
@@ -196,8 +234,8 @@ class NeighborList : public torch::autograd::Function<NeighborList> {
     if (g[2].defined()) {
       const Tensor &pos = s[0], &box = s[1];
       const int64_t nf = ctx->saved_data["nf"].toInt(), N = ctx->saved_data["N"].toInt();
-      if (ctx->needs_input_grad(0)) gpos = torch::zeros_like(pos);
-      if (box.numel() && ctx->needs_input_grad(1)) gbox = torch::zeros_like(box);
+      if (ctx->needs_input_grad(0)) gpos = torch::empty_like(pos);
+      if (box.numel() && ctx->needs_input_grad(1)) gbox = torch::empty_like(box);
       const Tensor gds = g[2].contiguous();
       if (gpos.defined() || gbox.defined())
         check(admp_pair_distances_frames_backward(dtype_code(pos), box.numel() ? 1 : 0, (int)nf, (int)N,
@@ -261,7 +299,7 @@ class Damping : public torch::autograd::Function<Damping> {
     geta = grad(eta);
     Tensor E = any ? torch::empty({nf}, q.options().dtype(torch::kDouble)) : f64(nf, q);
     if (any)
-      check(admp_damping_energy(dt, (int)nf, (int)N, P, ptr<const long long>(pairs), ptr<void>(ds), ptr<void>(bs),
+      check(admp_damping_energy(dt, scale_flag(bs), (int)nf, (int)N, P, ptr<const long long>(pairs), ptr<void>(ds), ptr<void>(bs),
                                 ptr<void>(q), ptr<void>(eta), ke, ptr<double>(E), ptr<void>(gds), ptr<void>(gq),
                                 ptr<void>(geta), st),
             "damping energy");
@@ -272,9 +310,10 @@ class Damping : public torch::autograd::Function<Damping> {
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     auto s = ctx->get_saved_variables();
     variable_list out(6);
-    if (g[0].defined())
-      for (int k = 0; k < 3; ++k)
-        if (s[k].defined()) out[k] = s[k] * g[0].view({-1, 1});
+    if (g[0].defined()) {
+      const variable_list r = scaled(s, g[0]);
+      for (int k = 0; k < 3; ++k) out[k] = r[k];
+    }
     return out;
   }
 };
@@ -301,11 +340,7 @@ class Site : public torch::autograd::Function<Site> {
 
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     auto s = ctx->get_saved_variables();
-    variable_list out(3);
-    if (g[0].defined())
-      for (int k = 0; k < 3; ++k)
-        if (s[k].defined()) out[k] = s[k] * g[0].view({-1, 1});
-    return out;
+    return g[0].defined() ? scaled(s, g[0]) : variable_list(3);
   }
 };
 
@@ -334,19 +369,19 @@ std::vector<Tensor> coulomb_pbc(Tensor pos, Tensor box, Tensor pairs, Tensor ds,
   TORCH_CHECK(kmesh.empty() || kmesh.size() == 3, "kmesh: 3 values or none");
   TORCH_CHECK(spacing.empty() || spacing.size() == 3, "spacing: 3 values or none");
   auto r = CoulombPBC::apply(pos.contiguous(), box.contiguous(), ds.contiguous(), q.contiguous(),
-                             pairs.to(torch::kLong).contiguous(), bs.contiguous(), kappa, kmesh, spacing, ethresh, ke,
+                             pairs.to(torch::kLong).contiguous(), scales_of(bs, q), kappa, kmesh, spacing, ethresh, ke,
                              rspace, kspace, slab, axis);
   return {r[0], r[1], r[2]};
 }
 
 Tensor coulomb_obc(Tensor pairs, Tensor ds, Tensor bs, Tensor q, double ke) {
-  return CoulombOBC::apply(ds.contiguous(), q.contiguous(), pairs.to(torch::kLong).contiguous(), bs.contiguous(),
-                           ke)[0];
+  return CoulombOBC::apply(ds.contiguous(), q.contiguous(), pairs.to(torch::kLong).contiguous(),
+                           bs.to(q.scalar_type()).contiguous(), ke)[0];
 }
 
 Tensor damping(Tensor ds, Tensor q, Tensor eta, Tensor pairs, Tensor bs, double ke) {
   return Damping::apply(ds.contiguous(), q.contiguous(), eta.contiguous(), pairs.to(torch::kLong).contiguous(),
-                        bs.contiguous(), ke)[0];
+                        scales_of(bs, q), ke)[0];
 }
 
 Tensor site(Tensor q, Tensor chi, Tensor hard) {
