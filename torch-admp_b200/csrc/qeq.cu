@@ -112,7 +112,7 @@ static bool cg_plan(const QEqCtx<T>& c, int sms, CgArgs<T>& a, size_t& smem) {
   a.K0 = d.K0;
   a.K1 = d.K1;
   a.K2 = d.K2;
-  a.buf = 0;
+  a.buf = a.planes = 0;
   a.lz = a.ly = a.lx = 1;
   if (c.P.flags & ADMP_QEQ_KSPACE) {
     auto lines = [&](long long total, int K) {
@@ -124,7 +124,10 @@ static bool cg_plan(const QEqCtx<T>& c, int sms, CgArgs<T>& a, size_t& smem) {
     a.lz = lines(((long long)a.K0 * a.K1 + 1) / 2, a.K2);
     a.ly = lines((long long)a.K0 * d.K2h, a.K1);
     a.lx = lines((long long)a.K1 * d.K2h, a.K0);
+    const int plane = slab_plane_elems(a.K1, a.K2);
+    a.planes = a.K0 <= sms && plane <= kCgPlane;
     a.buf = a.lz * a.K2 > a.ly * a.K1 ? a.lz * a.K2 : a.ly * a.K1;
+    if (a.planes) a.buf = plane;
     a.buf = a.buf > a.lx * a.K0 ? a.buf : a.lx * a.K0;
   }
   const size_t fft = ((size_t)a.K0 + a.K1 + a.K2 + 2 * (size_t)a.buf) * cs;

@@ -7,14 +7,15 @@
 // iteration are separated by a barrier over the grid, every transform spreads
 // its lines over all blocks, the twiddles and (while they fit) the atoms'
 // stencils are built once per launch, and the host reads the result once.
-// Now 41 us (3,000 atoms, 48^3, FP32), 55 (10,701, 64^3, FP64; 110 before) and
-// 49 (2,304 electrode atoms, 64 x 64 x 160, FP32; 100 before): eight barriers
-// take 14-16 of them, the five transforms 16-26, spread and gather 8-15.
+// Now 37 us (3,000 atoms, 48^3, FP32), 52 (10,701, 64^3, FP64; 110 before) and
+// 49 (2,304 electrode atoms, 64 x 64 x 160, FP32; 100 before): a barrier takes
+// 1.8 of them, there are six (eight in the last case).
 //
 //   A   direction p = r + beta p of the group's atoms, spread
 //   Z   z transform of the mesh lines,  Y  y transform
 //   X   x transform, Green's function, inverse x transform
 //   Y'  inverse y,  Z' inverse z
+//       (Z with Y and Y' with Z' in one block's shared memory while the planes are small)
 //       (a quarter of the warps multiply p by the pair matrix meanwhile)
 //   E   gather, rest of the matvec, p.Hp and C.Hp
 //   F   x += alpha p, r -= alpha P(Hp), |r|^2; zero Hp and the mesh
@@ -37,6 +38,10 @@ constexpr int kCgFft = 384;                // threads of the transforms; the oth
 constexpr long long kCgSpin = 1LL << 23;
 constexpr int kCgMaxLines = kCgFft;      // lines of a block's y transform
 constexpr int kCgLaunch = 128;           // iterations per launch
+// Complex values of the largest x plane that one block transforms in z and y by itself: two barriers and a trip of
+// the spectrum through L2 less in each direction, for fewer blocks at work.  18 iterations of 48^3 (FP32) 776 -> 690
+// us, 56 of 64^3 (FP64) 3,090 -> 2,895; with 64 x 160 values a plane both ways take the same (1,732 and 1,738).
+constexpr int kCgPlane = 4096;
 
 struct CgSlot {
   double rr_new, pHp, Cv[kMaxConst], sp, spz, spz2;
@@ -66,6 +71,7 @@ struct CgArgs {
   CgShared* sh;
   int k0, k1;        // iterations of this launch: k0 <= k < k1
   int lz, ly, lx;    // lines (z: pairs of lines) a block transforms at a time
+  int planes;        // a block transforms whole x planes in z and y
   int buf;           // complex values in each of the two line buffers
   int group;         // atoms of a warp's group (at most kPw)
   int kept;          // stencil groups a warp keeps, 0: built anew every time
@@ -203,6 +209,81 @@ __device__ void cg_y_pass(const CgArgs<T>& a, const CgFft<T>& f, const Radices& 
     for (int idx = threadIdx.x; idx < K1 * n; idx += kCgFft) {
       const int y = fdiv(idx, fdn), c = idx - y * n;
       a.spec[off[c] + (long long)y * K2h] = R1[idx];
+    }
+    group_sync<kSyncPart>(kCgFft);
+  }
+}
+
+// z and y passes of whole x planes: the half spectrum of a plane goes from the one to the other in shared memory.
+template <typename T>
+__device__ void cg_plane_fwd(const CgArgs<T>& a, const CgFft<T>& f, const Radices& R1, const Radices& R2) {
+  const int K1 = a.K1, K2 = a.K2, K2h = K2 / 2 + 1, np = (K1 + 1) / 2;
+  const FastDiv fdK2 = fast_div(K2), fdK2h = fast_div(K2h);
+  for (int x = blockIdx.x; x < a.K0; x += gridDim.x) {
+    const T* Q = a.mesh + (size_t)x * K1 * K2;
+    for (int idx = threadIdx.x; idx < np * K2; idx += kCgFft) {
+      const int p = fdiv(idx, fdK2), t = idx - p * K2;
+      Cplx<T> z;
+      z.x = Q[2 * p * K2 + t];
+      z.y = 2 * p + 1 < K1 ? Q[(2 * p + 1) * K2 + t] : T(0);
+      f.A[idx] = z;
+    }
+    group_sync<kSyncPart>(kCgFft);
+    Cplx<T>* Z = fft_run<T, false, kSyncPart, false>(R2, f.A, f.B, np, K2, K2, 1, f.W2, threadIdx.x, kCgFft);
+    Cplx<T>* U = Z == f.A ? f.B : f.A;
+    for (int idx = threadIdx.x; idx < np * K2h; idx += kCgFft) {
+      const int p = fdiv(idx, fdK2h), k = idx - p * K2h;
+      const Cplx<T> z = Z[p * K2 + k], zm = Z[p * K2 + (k == 0 ? 0 : K2 - k)];
+      Cplx<T> u, v;
+      u.x = (z.x + zm.x) * T(0.5);
+      u.y = (z.y - zm.y) * T(0.5);
+      v.x = (z.y + zm.y) * T(0.5);
+      v.y = (zm.x - z.x) * T(0.5);
+      U[2 * p * K2h + k] = u;
+      if (2 * p + 1 < K1) U[(2 * p + 1) * K2h + k] = v;
+    }
+    group_sync<kSyncPart>(kCgFft);
+    const Cplx<T>* V = fft_run<T, true, kSyncPart, false>(R1, U, Z, K2h, K1, 1, K2h, f.W1, threadIdx.x, kCgFft);
+    Cplx<T>* H = a.spec + (size_t)x * K1 * K2h;
+    for (int idx = threadIdx.x; idx < K1 * K2h; idx += kCgFft) H[idx] = V[idx];
+    group_sync<kSyncPart>(kCgFft);
+  }
+}
+
+template <typename T>
+__device__ void cg_plane_inv(const CgArgs<T>& a, const CgFft<T>& f, const Radices& R1, const Radices& R2) {
+  const int K1 = a.K1, K2 = a.K2, K2h = K2 / 2 + 1, np = (K1 + 1) / 2;
+  const FastDiv fdK2 = fast_div(K2);
+  for (int x = blockIdx.x; x < a.K0; x += gridDim.x) {
+    const Cplx<T>* H = a.spec + (size_t)x * K1 * K2h;
+    for (int idx = threadIdx.x; idx < K1 * K2h; idx += kCgFft) f.A[idx] = H[idx];
+    group_sync<kSyncPart>(kCgFft);
+    Cplx<T>* V = fft_run<T, true, kSyncPart, true>(R1, f.A, f.B, K2h, K1, 1, K2h, f.W1, threadIdx.x, kCgFft);
+    Cplx<T>* Z = V == f.A ? f.B : f.A;
+    for (int idx = threadIdx.x; idx < np * K2; idx += kCgFft) {
+      const int p = fdiv(idx, fdK2), t = idx - p * K2;
+      const bool lo = t < K2h;
+      const int tt = lo ? t : K2 - t;
+      Cplx<T> u = V[2 * p * K2h + tt], v;
+      v.x = v.y = T(0);
+      if (2 * p + 1 < K1) v = V[(2 * p + 1) * K2h + tt];
+      if (!lo) {
+        u.y = -u.y;
+        v.y = -v.y;
+      }
+      Cplx<T> z;
+      z.x = u.x - v.y;
+      z.y = u.y + v.x;
+      Z[idx] = z;
+    }
+    group_sync<kSyncPart>(kCgFft);
+    const Cplx<T>* R = fft_run<T, false, kSyncPart, true>(R2, Z, V, np, K2, K2, 1, f.W2, threadIdx.x, kCgFft);
+    T* Q = a.mesh + (size_t)x * K1 * K2;
+    for (int idx = threadIdx.x; idx < np * K2; idx += kCgFft) {
+      const int p = fdiv(idx, fdK2), t = idx - p * K2;
+      const Cplx<T> z = R[idx];
+      Q[2 * p * K2 + t] = z.x;
+      if (2 * p + 1 < K1) Q[(2 * p + 1) * K2 + t] = z.y;
     }
     group_sync<kSyncPart>(kCgFft);
   }
@@ -411,17 +492,23 @@ __global__ void __launch_bounds__(kCgThreads) qeq_cg_kernel(CgArgs<T> a) {
         unsigned t = target;
         bool ok = true;
         auto pass = [&]() { return cg_barrier<kSyncPart>(a.sh, t, kCgFft); };
-        cg_z_pass<T, false>(a, f, R2);
-        if ((ok = pass())) cg_y_pass<T, false>(a, f, R1);
-        if (ok && (ok = pass())) cg_x_pass<T>(a, f, R0);
-        if (ok && (ok = pass())) cg_y_pass<T, true>(a, f, R1);
-        if (ok && (ok = pass())) cg_z_pass<T, true>(a, f, R2);
+        if (a.planes) {
+          cg_plane_fwd<T>(a, f, R1, R2);
+          if ((ok = pass())) cg_x_pass<T>(a, f, R0);
+          if (ok && (ok = pass())) cg_plane_inv<T>(a, f, R1, R2);
+        } else {
+          cg_z_pass<T, false>(a, f, R2);
+          if ((ok = pass())) cg_y_pass<T, false>(a, f, R1);
+          if (ok && (ok = pass())) cg_x_pass<T>(a, f, R0);
+          if (ok && (ok = pass())) cg_y_pass<T, true>(a, f, R1);
+          if (ok && (ok = pass())) cg_z_pass<T, true>(a, f, R2);
+        }
         if (!ok && threadIdx.x == 0) broken = 1;
       }
     } else if (a.have_pairs) {
       cg_pairs<T>(a, kCgFft, kCgThreads - kCgFft);
     }
-    if (kspace) target += 4 * gridDim.x;
+    if (kspace) target += (a.planes ? 2 : 4) * gridDim.x;
     __syncthreads();
     if (broken) return stop();
     if (!meet()) return stop();
