@@ -228,6 +228,7 @@ static __global__ void __launch_bounds__(256)
                            const int* __restrict__ col, const T* __restrict__ coef, const T* __restrict__ v,
                            T* __restrict__ Hv, const double* __restrict__ diag, const double* __restrict__ zc,
                            CGScal* __restrict__ sc, double* __restrict__ hv_out) {
+  constexpr int kUnroll = kSpmvUnroll<T>;
   __shared__ double red[5 * 32];
   const int s0 = find_sys<F_ATOM>(b, blockIdx.x);
   const SysDesc d = b.s[s0];
@@ -259,21 +260,21 @@ static __global__ void __launch_bounds__(256)
       n_next = pcnt[i + ngrp];
     }
     T acc = 0;
-    for (int k0 = 0; k0 < n; k0 += kSpmvLanes * kSpmvUnroll) {
-      int c[kSpmvUnroll];
-      T w[kSpmvUnroll];
+    for (int k0 = 0; k0 < n; k0 += kSpmvLanes * kUnroll) {
+      int c[kUnroll];
+      T w[kUnroll];
 #pragma unroll
-      for (int u = 0; u < kSpmvUnroll; ++u) {
+      for (int u = 0; u < kUnroll; ++u) {
         const int k = k0 + sub + u * kSpmvLanes;
         const bool ok = k < n;
-        c[u] = ok ? col[st + k] : -1;
-        w[u] = ok ? coef[st + k] : T(0);
+        c[u] = ok ? spmv_load<T>(col + st + k) : -1;
+        w[u] = ok ? spmv_load<T>(coef + st + k) : T(0);
       }
-      T vv[kSpmvUnroll];
+      T vv[kUnroll];
 #pragma unroll
-      for (int u = 0; u < kSpmvUnroll; ++u) vv[u] = c[u] >= 0 ? v[c[u]] : T(0);
+      for (int u = 0; u < kUnroll; ++u) vv[u] = c[u] >= 0 ? v[c[u]] : T(0);
 #pragma unroll
-      for (int u = 0; u < kSpmvUnroll; ++u) acc += w[u] * vv[u];
+      for (int u = 0; u < kUnroll; ++u) acc += w[u] * vv[u];
     }
 #pragma unroll
     for (int o = kSpmvLanes / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);

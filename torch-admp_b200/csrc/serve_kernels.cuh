@@ -617,8 +617,18 @@ static __global__ void __launch_bounds__(256)
 // of its row before using any of them, so a row costs about three dependent
 // memory latencies (row start, entries, gathered p) instead of three per 32
 // entries: the SpMV is bound by the latency of those chains, not by bytes.
+// In double precision twelve entries cost so many registers that fewer rows
+// are in flight; six, read past L1 so that p stays there, are the better
+// split: 102,840 atoms 60.4 -> 43.3 us (six 51.1, streaming loads alone 54.3).
+// Single precision, 412,569 atoms: 100 us with twelve plain loads, 106 with
+// eight, 114 with six, 109 with six streaming ones.
 constexpr int kSpmvLanes = 8;
-constexpr int kSpmvUnroll = 12;
+template <typename T>
+constexpr int kSpmvUnroll = sizeof(T) == 8 ? 6 : 12;
+template <typename T, typename E>
+__device__ __forceinline__ E spmv_load(const E* p) {
+  return sizeof(T) == 8 ? __ldcs(p) : *p;
+}
 
 // block per system: self + non-neutral (+ damping self + site for QEq systems)
 template <typename T>
