@@ -200,7 +200,7 @@ static int serve_ef_impl(const admp_pools* P, const admp_sys* sys, int nsys, dou
   srv_table_kernel<<<(nsys + 63) / 64, 64, 0, st>>>(c.L, P->box, sizeof(T) == 8, P->slot_info, ss, 0);
   zero_atoms_kernel<T><<<b.nblk_atom, 256, 0, st>>>(b, (T*)P->force, P->energy);
   int h = prof_begin(st);
-  pair_ef_kernel<T><<<b.nblk_atom, 256, 0, st>>>(b, ss, (const V4*)P->frac,
+  pair_ef_kernel<T><<<b.nblk_st, kEfWarps * 32, 0, st>>>(family_batch(plan, F_ST), ss, (const V4*)P->frac,
                                                  P->pos64 ? (const double4*)P->frac64 : nullptr, (const T*)P->q,
                                                  (const T*)P->eta, P->pstart, P->pcnt, P->col, ke, (T*)P->force,
                                                  P->energy);

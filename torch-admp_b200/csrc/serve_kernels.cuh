@@ -460,23 +460,26 @@ __device__ __forceinline__ void disp(const V4& fi, const V4& fj, const double* b
   for (int e = 0; e < 3; ++e) dr[e] = df[0] * bx[e] + df[1] * bx[3 + e] + df[2] * bx[6 + e];
 }
 
-// warp per atom: real-space Ewald (+ damping for QEq systems) energy, gradient, potential
+// warp per atom: real-space Ewald (+ damping for QEq systems) energy, gradient, potential.  Blocks of 32 atoms: with
+// 256 an SM stood idle for a fifth of the launch behind the last ones (155,068 atoms, FP64, 352 -> 306 us; 619,264,
+// FP32, 753 -> 737).
+constexpr int kEfWarps = 4;
 template <typename T>
-static __global__ void __launch_bounds__(256)
+static __global__ void __launch_bounds__(kEfWarps * 32)
     pair_ef_kernel(Batch b, const SrvSys* __restrict__ ss, const typename Vec4<T>::type* __restrict__ frac,
                    const double4* __restrict__ frac64, const T* __restrict__ q, const T* __restrict__ eta,
                    const long long* __restrict__ pstart, const int* __restrict__ pcnt, const int* __restrict__ col,
                    double ke, T* __restrict__ grad, double* __restrict__ energy) {
   __shared__ double bx[9];
   __shared__ double red[32];
-  const int s = find_sys<F_ATOM>(b, blockIdx.x);
+  const int s = find_sys<F_ST>(b, blockIdx.x);
   const SysDesc d = b.s[s];
   const SrvSys& S = ss[s];
   if (threadIdx.x < 9) bx[threadIdx.x] = S.b[threadIdx.x];
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int a0 = (blockIdx.x - d.blk_atom) * b.apb;
-  const int a1 = min(a0 + b.apb, d.natoms);
+  const int a0 = (blockIdx.x - b.blk[s]) * b.aps;
+  const int a1 = min(a0 + b.aps, d.natoms);
   const T kappa = (T)S.kappa, kt = (T)ke;
   const T tsp = T(2.0 / kSqrtPi);
   const bool damp = S.kind == 1 && eta != nullptr;
