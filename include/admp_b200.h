@@ -347,6 +347,16 @@ int admp_qeq_hessian(int dtype, int flags, int natoms, const int* kmesh, const v
                      const void* buffer_scales, const void* hardness, const void* eta,
                      double kappa, double ke, int cols, void* H, void* workspace,
                      size_t workspace_bytes, void* stream);
+/* Charges of a dense Hessian: H q + C^T lam = -chi, C q = value              */
+/* (qeq.py:1530-1617) with one constraint row C [N] or none (NULL), by        */
+/* Cholesky in double precision.  *info: 0, or k + 1 where column k finds H   */
+/* not positive definite, or natoms + 1 where C H^-1 C^T is zero (q is then   */
+/* not written).  value: one device double.  Waits for the result.            */
+#define ADMP_QEQ_DENSE_MAX 1024
+size_t admp_qeq_dense_workspace_size(int natoms);
+int admp_qeq_dense_solve(int natoms, const double* H, const double* chi, const double* constraint,
+                         const double* value, double* q, int* info, void* workspace,
+                         size_t workspace_bytes, void* stream);
 
 
 /* ------------------------------------------------------------------------ */

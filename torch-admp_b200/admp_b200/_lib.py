@@ -52,6 +52,7 @@ EXPORTS = [
     "admp_nblist_frames_workspace_size", "admp_nblist_frames_count", "admp_nblist_frames_fill",
     "admp_pair_distances_frames_backward", "admp_coulomb_pbc", "admp_read_back",
     "admp_damping_energy", "admp_site_energy", "admp_qeq_hessian_workspace_size", "admp_qeq_hessian",
+    "admp_qeq_dense_workspace_size", "admp_qeq_dense_solve",
     "admp_scale_frames",
 ]
 PROFILE_KERNELS = ["spread", "fft_z_fwd", "fft_y_fwd", "fft_x_green", "fft_y_inv", "fft_z_inv", "gather", "pair_ef",
@@ -85,6 +86,8 @@ _SIGS = {
     "admp_scale_frames": (_i, [_i, _i, _i, _vp, _vp, _llp, _vp, _ll, _vp]),
     "admp_damping_energy": (_i, [_i, _i, _i, _i, _ll, _vp, _vp, _vp, _vp, _vp, _d, _vp, _vp, _vp, _vp, _vp]),
     "admp_site_energy": (_i, [_i, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
+    "admp_qeq_dense_workspace_size": (_sz, [_i]),
+    "admp_qeq_dense_solve": (_i, [_i, _vp, _vp, _vp, _vp, _vp, ctypes.POINTER(_i), _vp, _sz, _vp]),
     "admp_qeq_hessian_workspace_size": (_sz, [_i, _i, _ll, _ip, _i]),
     "admp_qeq_hessian": (_i, [_i, _i, _i, _ip, _vp, _vp, _ll, _vp, _vp, _vp, _vp, _vp, _d, _d, _i, _vp, _vp, _sz, _vp]),
     "admp_read_back": (_i, [_vp, _sz, _vp, _vp]),

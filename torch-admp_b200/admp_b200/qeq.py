@@ -192,15 +192,29 @@ def _kkt(hessian, chi, C, b):
     """Charges of H q = -chi under C q = b.
 
     H is positive definite for a stable charge model, so in double precision a
-    Cholesky factorisation and the n_const x n_const Schur complement solve it
-    (201 / 429 / 2,304 atoms: 0.34 / 0.51 / 2.2 ms, the pivoted LU of the bordered
-    matrix 0.56 / 1.15 / 8.6 ms, the same error); any other H takes the LU, as the
-    reference does, and so does single precision, where Cholesky was up to 1.3
-    times further off at 2,304 atoms."""
+    Cholesky factorisation and the n_const x n_const Schur complement solve it: up
+    to 1,024 atoms in one kernel (admp_qeq_dense_solve; 201 / 429 / 1,024 atoms:
+    0.13 / 0.22 / 0.57 ms, the library's Cholesky and triangular solves 0.33 / 0.52 /
+    1.02), above that by the library (2,304 atoms 2.2 ms, the pivoted LU of the
+    bordered matrix 8.6).  Any other H takes the LU, as the reference does, and so
+    does single precision, where Cholesky was up to 1.3 times further off at 2,304
+    atoms."""
     n = hessian.shape[0]
-    rhs = -chi.reshape(-1, 1).to(hessian.dtype)
     m = 0 if C is None else C.shape[0]
     if n > 0 and m <= 1 and hessian.dtype == torch.float64:
+        lib = L.load()
+        nbytes = lib.admp_qeq_dense_workspace_size(n)
+        if nbytes:
+            H, g = hessian.contiguous(), chi.reshape(-1).to(torch.float64).contiguous()
+            row = C.to(torch.float64).contiguous() if m else None
+            val = b.reshape(-1).to(H.device, torch.float64).contiguous() if m else None
+            q, info, ws = torch.empty_like(g), ctypes.c_int(0), L.workspace(nbytes, H.device)
+            L.check(lib.admp_qeq_dense_solve(n, L.ptr(H), L.ptr(g), L.ptr(row), L.ptr(val), L.ptr(q),
+                                             ctypes.byref(info), L.ptr(ws), nbytes, L.stream_of(H.device)), "QEq dense solve")
+            if info.value == 0:
+                return q
+    rhs = -chi.reshape(-1, 1).to(hessian.dtype)
+    if n > 0 and m <= 1 and hessian.dtype == torch.float64 and nbytes == 0:  # more atoms than that solve takes
         factor, bad = torch.linalg.cholesky_ex(hessian)
         Ct = hessian.new_zeros(n, 0) if m == 0 else C.T.to(hessian.dtype)
         x = torch.cholesky_solve(torch.cat([rhs, Ct], 1), factor)
