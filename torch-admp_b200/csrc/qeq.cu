@@ -170,6 +170,7 @@ static int cg_persistent(QEqCtx<T>& c, CGScal* h, bool& used) {
   a.green = c.w.green;
   a.diag = c.w.diag;
   a.zc = c.w.zc;
+  a.chi = c.w.chi_eff;
   a.mesh = c.w.mesh;
   a.p = c.w.p;
   a.Hp = c.w.Hp;
@@ -181,12 +182,12 @@ static int cg_persistent(QEqCtx<T>& c, CGScal* h, bool& used) {
   a.sc = c.w.sc;
   a.sh = c.w.cg;
   used = true;
-  // the mesh holds the potential of the initial charges
   if (c.P.flags & ADMP_QEQ_KSPACE)
     ADMP_CUDA_TRY(cudaMemsetAsync(c.w.mesh, 0, sizeof(T) * (size_t)a.K0 * a.K1 * a.K2, c.st));
   ADMP_CUDA_TRY(cudaMemsetAsync(c.w.cg, 0, sizeof(CgShared), c.st));
   for (a.k0 = 0;; a.k0 = h->iter) {
     a.k1 = a.k0 + kCgLaunch;
+    a.init = a.k0 == 0;
     if (a.k0) ADMP_CUDA_TRY(cudaMemsetAsync(&c.w.cg->arrived, 0, sizeof(unsigned), c.st));
     void* args[] = {&a};
     ADMP_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)qeq_cg_kernel<T>, dim3(sms), dim3(kCgThreads), args, smem,
@@ -271,31 +272,33 @@ static int qeq_solve_impl(int flags, int nf, int N, const int* kmesh, const T* p
     qeq_project_kernel<T><<<b.nblk_atom, 256, 0, st>>>(b, c.w.x, C, (long long)N, c.w.sc);
     qeq_clear_acc_kernel<<<sb, 64, 0, st>>>(nf, c.w.sc);
   }
-  // H x0 -> hx (double); the p buffer carries x0 in T for the matvec
-  qeq_sums_kernel<T, double><<<b.nblk_atom, 256, 0, st>>>(b, c.w.x, c.w.zc, C, (long long)N, nc, 0, c.w.sc, c.w.Hp,
-                                                          c.w.p);
-  s = qeq_matvec<T>(c, c.w.p, c.w.Hp, c.w.hx);
-  if (s) return s;
-  qeq_clear_acc_kernel<<<sb, 64, 0, st>>>(nf, c.w.sc);
-  ADMP_CUDA_TRY(cudaMemsetAsync(c.w.Hp, 0, sizeof(T) * NT, st));
-  qeq_resid_kernel<T><<<b.nblk_atom, 256, 0, st>>>(b, c.w.hx, c.w.chi_eff, C, (long long)N, c.w.zc, c.w.r, c.w.p,
-                                                   c.w.sc, 0);
-  qeq_resid_kernel<T><<<b.nblk_atom, 256, 0, st>>>(b, c.w.hx, c.w.chi_eff, C, (long long)N, c.w.zc, c.w.r, c.w.p,
-                                                   c.w.sc, 1);
-  qeq_init_done_kernel<<<(nf + 31) / 32, 32, 0, st>>>(b, c.P, c.w.sc);
-  ADMP_CUDA_TRY(cudaGetLastError());
-  // iterate; read the per-frame done flags every `chunk` iterations
-  RecipPlan<T> pl = c.w.plan;
-  pl.b.done = &c.w.sc->done;
-  pl.b.done_stride = (int)(sizeof(CGScal) / sizeof(int));
-  pl.b.status_off = (int)((offsetof(CGScal, status) - offsetof(CGScal, done)) / sizeof(int));
-  c.w.plan = pl;
-  const int chunk = 8;
-  int it = 0;
   std::vector<CGScal> h(nf);
   bool persistent = false;
   s = cg_persistent<T>(c, h.data(), persistent);
   if (s) return s;
+  if (!persistent) {
+    // H x0 -> hx (double); the p buffer carries x0 in T for the matvec
+    qeq_sums_kernel<T, double><<<b.nblk_atom, 256, 0, st>>>(b, c.w.x, c.w.zc, C, (long long)N, nc, 0, c.w.sc, c.w.Hp,
+                                                            c.w.p);
+    s = qeq_matvec<T>(c, c.w.p, c.w.Hp, c.w.hx);
+    if (s) return s;
+    qeq_clear_acc_kernel<<<sb, 64, 0, st>>>(nf, c.w.sc);
+    ADMP_CUDA_TRY(cudaMemsetAsync(c.w.Hp, 0, sizeof(T) * NT, st));
+    qeq_resid_kernel<T><<<b.nblk_atom, 256, 0, st>>>(b, c.w.hx, c.w.chi_eff, C, (long long)N, c.w.zc, c.w.r, c.w.p,
+                                                     c.w.sc, 0);
+    qeq_resid_kernel<T><<<b.nblk_atom, 256, 0, st>>>(b, c.w.hx, c.w.chi_eff, C, (long long)N, c.w.zc, c.w.r, c.w.p,
+                                                     c.w.sc, 1);
+    qeq_init_done_kernel<<<(nf + 31) / 32, 32, 0, st>>>(b, c.P, c.w.sc);
+    ADMP_CUDA_TRY(cudaGetLastError());
+    // iterate; read the per-frame done flags every `chunk` iterations
+    RecipPlan<T> pl = c.w.plan;
+    pl.b.done = &c.w.sc->done;
+    pl.b.done_stride = (int)(sizeof(CGScal) / sizeof(int));
+    pl.b.status_off = (int)((offsetof(CGScal, status) - offsetof(CGScal, done)) / sizeof(int));
+    c.w.plan = pl;
+  }
+  const int chunk = 8;
+  int it = 0;
   while (!persistent) {
     for (int k = 0; k < chunk; ++k) {
       qeq_rotate_kernel<<<(nf + 31) / 32, 32, 0, st>>>(b, c.w.sc);

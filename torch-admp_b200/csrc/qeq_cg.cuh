@@ -20,6 +20,10 @@
 //   E   gather, rest of the matvec, p.Hp and C.Hp
 //   F   x += alpha p, r -= alpha P(Hp), |r|^2; zero Hp and the mesh
 //
+// Iteration -1 takes the initial charges in the direction's place and leaves
+// r = -P(chi + H x) and p = r: a pass of these phases instead of seventeen
+// launches (a solve of 3,000 atoms 1,660 -> 1,563 us, of 10,701 4,119 -> 4,013).
+//
 // Arithmetic, scalars and stopping rule are those of the kernels in
 // qeq_kernels.cuh.  The scalars of iteration k live in slot k % 3, so that a
 // slot is zeroed (phase F of the iteration before) two barriers after its last
@@ -61,7 +65,7 @@ struct CgArgs {
   double kappa;
   QEqParams P;
   const T *pos, *box, *C, *green;
-  const double *diag, *zc;
+  const double *diag, *zc, *chi;
   T *mesh, *p, *Hp;
   Cplx<T>* spec;
   double *x, *r;
@@ -70,6 +74,7 @@ struct CgArgs {
   CGScal* sc;
   CgShared* sh;
   int k0, k1;        // iterations of this launch: k0 <= k < k1
+  int init;          // iteration -1 first: r = -P(chi + H x), p = r
   int lz, ly, lx;    // lines (z: pairs of lines) a block transforms at a time
   int planes;        // a block transforms whole x planes in z and y
   int buf;           // complex values in each of the two line buffers
@@ -357,6 +362,7 @@ __global__ void __launch_bounds__(kCgThreads) qeq_cg_kernel(CgArgs<T> a) {
   __shared__ Geom g;
   __shared__ Radices R0, R1, R2;
   __shared__ double red[4][kCgWarps], red2[4][kCgWarps];
+  __shared__ double Ginv[kMaxConst * kMaxConst];
   __shared__ int broken;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const bool kspace = (a.P.flags & ADMP_QEQ_KSPACE) != 0, slab = (a.P.flags & ADMP_QEQ_SLAB) != 0;
@@ -377,6 +383,7 @@ __global__ void __launch_bounds__(kCgThreads) qeq_cg_kernel(CgArgs<T> a) {
   d.K2 = a.K2;
   load_geom(a.box, 0, &g);
   if (threadIdx.x == 0) broken = 0;
+  if (threadIdx.x < kMaxConst * kMaxConst) Ginv[threadIdx.x] = a.sc->Ginv[threadIdx.x];
   if (kspace) {
     make_twiddles(f.W0, a.K0);
     make_twiddles(f.W1, a.K1);
@@ -406,7 +413,8 @@ __global__ void __launch_bounds__(kCgThreads) qeq_cg_kernel(CgArgs<T> a) {
   }
   CGScal* sc = a.sc;
   if (sc->done) return;  // the same for every block: only phase A writes it, behind the first barrier
-  const double rr0 = sc->rr, nn = sc->nn, pre = sc->pre, Lz2 = sc->Lz2;
+  double rr0 = sc->rr;
+  const double nn = sc->nn, pre = sc->pre, Lz2 = sc->Lz2;
   const double few = a.P.tol * (double)a.N, few2 = few * few;
   const int nc = sc->n_const;
   unsigned target = 0;
@@ -417,10 +425,11 @@ __global__ void __launch_bounds__(kCgThreads) qeq_cg_kernel(CgArgs<T> a) {
     }
   };
   auto meet = [&]() { return cg_barrier<kSyncBlock>(a.sh, target, kCgThreads); };
-  for (int k = a.k0;; ++k) {
-    CgSlot& S = a.sh->slot[k % 3];
+  for (int k = a.init ? -1 : a.k0;; ++k) {
+    const bool init = k < 0;  // the matvec of the initial charges in the direction's place
+    CgSlot& S = a.sh->slot[(k + 3) % 3];
     volatile CgSlot& S1 = a.sh->slot[(k + 2) % 3];  // iteration k - 1
-    volatile CgSlot& S2 = a.sh->slot[(k + 1) % 3];  // iteration k - 2
+    volatile CgSlot& S2 = a.sh->slot[(k + 4) % 3];  // iteration k - 2
     // ---- A: convergence of the last iterate, direction, spread (the first group's values are asked for before
     // the scalars are worked out)
     double rv = 0.0, zv = 0.0;
@@ -469,8 +478,8 @@ __global__ void __launch_bounds__(kCgThreads) qeq_cg_kernel(CgArgs<T> a) {
             zv = a.zc[i];
           }
           double pn = rv;  // the first direction is the residual
-          if (k > 0) {
-            pn = rv + beta * (double)pv;
+          if (k != 0) {
+            pn = init ? a.x[i] : rv + beta * (double)pv;
             pv = (T)pn;
             a.p[i] = pv;
           }
@@ -536,9 +545,14 @@ __global__ void __launch_bounds__(kCgThreads) qeq_cg_kernel(CgArgs<T> a) {
             const double z = a.zc[i];
             h += pre * (2.0 * z * spz - spz2 - z * z * sp - Lz2 / 6.0 * sp);
           }
-          a.Hp[i] = (T)h;
+          if (init)
+            a.r[i] = h += a.chi[i];
+          else
+            a.Hp[i] = (T)h;
           acc[0] += x * h;
-          for (int c = 0; c < nc; ++c) acc[1 + c] += cval(a.C, c, (long long)a.N, i) * h;
+#pragma unroll
+          for (int c = 0; c < kMaxConst; ++c)
+            if (c < nc) acc[1 + c] += cval(a.C, c, (long long)a.N, i) * h;
         }
       }
       // p.Hp and the first three of C.Hp are next to each other in the slot
@@ -564,9 +578,21 @@ __global__ void __launch_bounds__(kCgThreads) qeq_cg_kernel(CgArgs<T> a) {
       }
       volatile CgSlot& V = S;
       const double pHp = V.pHp, alpha = pHp != 0.0 ? rr / pHp : 0.0;
-      double lam[kMaxConst] = {0, 0, 0, 0};
-      for (int r0 = 0; r0 < nc; ++r0)
-        for (int c = 0; c < nc; ++c) lam[r0] += sc->Ginv[r0 * kMaxConst + c] * V.Cv[c];
+      double lam[kMaxConst];
+#pragma unroll
+      for (int c = 0; c < kMaxConst; ++c) lam[c] = c < nc ? V.Cv[c] : 0.0;
+      {
+        double t[kMaxConst];
+#pragma unroll
+        for (int r0 = 0; r0 < kMaxConst; ++r0) {
+          t[r0] = 0.0;
+#pragma unroll
+          for (int c = 0; c < kMaxConst; ++c)
+            if (r0 < nc && c < nc) t[r0] += Ginv[r0 * kMaxConst + c] * lam[c];
+        }
+#pragma unroll
+        for (int c = 0; c < kMaxConst; ++c) lam[c] = t[c];
+      }
       double acc[1] = {0.0};
       for (int i = tid; i < a.N; i += nthr) {
         if (i != tid) {
@@ -575,11 +601,16 @@ __global__ void __launch_bounds__(kCgThreads) qeq_cg_kernel(CgArgs<T> a) {
           xv = a.x[i];
           rw = a.r[i];
         }
-        double w = (double)hv;
+        double w = init ? rw : (double)hv;
         a.Hp[i] = T(0);
-        for (int c = 0; c < nc; ++c) w -= cval(a.C, c, (long long)a.N, i) * lam[c];
-        a.x[i] = xv + alpha * (double)pw;
-        const double rn = rw - alpha * w;
+#pragma unroll
+        for (int c = 0; c < kMaxConst; ++c)
+          if (c < nc) w -= cval(a.C, c, (long long)a.N, i) * lam[c];
+        const double rn = init ? -w : rw - alpha * w;
+        if (init)
+          a.p[i] = (T)rn;
+        else
+          a.x[i] = xv + alpha * (double)pw;
         a.r[i] = rn;
         acc[0] += rn * rn;
       }
@@ -591,6 +622,19 @@ __global__ void __launch_bounds__(kCgThreads) qeq_cg_kernel(CgArgs<T> a) {
       cg_block_sum<1>(acc, &S.rr_new, red);
     }
     if (!meet()) return stop();
+    if (init) {
+      volatile CgSlot& V = S;
+      rr0 = V.rr_new;
+      const bool conv = sqrt(rr0) / (double)a.N < a.P.tol, stay = !conv && a.P.max_iter > 0;
+      if (blockIdx.x == 0 && threadIdx.x == 0) {
+        sc->rr = sc->rr_new = rr0;
+        if (!stay) {
+          sc->status = conv ? ADMP_OK : ADMP_ERR_NOT_CONVERGED;
+          sc->done = 1;
+        }
+      }
+      if (!stay) return;
+    }
   }
 }
 
