@@ -36,8 +36,10 @@ CASES = [  # atoms, box length (None: open), rc, triclinic
     (700, 13.0, 6.0, False),     # ~285 neighbours a row: past the ordering buffer
     (257, 7.0, 3.4, False),      # two cells per axis, dense
     (900, 30.0, 4.0, True),      # seven cells per axis, triclinic
-    (8192, 44.0, 5.0, False),    # the largest frame of the one-block build
-    (8193, 44.0, 5.0, True),     # the smallest of the other
+    (2048, 28.0, 5.0, False),    # the largest frame of the one-block build
+    (2049, 28.0, 5.0, True),     # the smallest of the other
+    (8192, 44.0, 5.0, False),
+    (8193, 44.0, 5.0, True),
     (500, None, 4.0, False),
     (600, None, 30.0, False),    # everything within the cutoff: rows of 599
     (9000, None, 3.0, False),

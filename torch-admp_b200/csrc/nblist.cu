@@ -38,8 +38,9 @@ struct NbResult {
 // rows inside their own slice of the output.
 constexpr int kNbKeep = 128;
 constexpr int kNbRow = 256;
-// Atoms a single block bins by itself (one launch instead of four).
-constexpr int kNbOneBlock = 8192;
+// Atoms a single block bins by itself (one launch instead of four).  A list of 1,536 / 2,100 / 3,000 / 6,007 atoms
+// takes 60 / 68 / 71 / 100 us by one block and 66 / 66 / 66 / 84 by the four launches.
+constexpr int kNbOneBlock = 2048;
 
 // Device state of a build over nf frames of N atoms: per-atom arrays are
 // [nf][N], per-cell arrays [nf][mc + 1].  cs32 / cs64 / sorted hold the
@@ -261,8 +262,8 @@ __device__ void nb_block_scan(const TI* __restrict__ in, TO* __restrict__ out, i
 }
 
 // Geometry of every frame (a block per frame) and, with BIN, the whole cell
-// sort of it: bin, scan and placement by the one block.  A launch costs more
-// than 8 atoms a thread, so frames of up to kNbOneBlock atoms take this form.
+// sort of it: bin, scan and placement by the one block.  Three launches cost
+// more than 2 atoms a thread, so frames of up to kNbOneBlock atoms take this form.
 template <typename T, bool BIN>
 __global__ void __launch_bounds__(1024) nb_setup_kernel(int pbc, int N, int mc, const T* __restrict__ pos,
                                                         const T* __restrict__ box, double rc, NbWS w0,
