@@ -7,8 +7,8 @@
 // iteration are separated by a barrier over the grid, every transform spreads
 // its lines over all blocks, the twiddles and (while they fit) the atoms'
 // stencils are built once per launch, and the host reads the result once.
-// Now 37 us (3,000 atoms, 48^3, FP32), 52 (10,701, 64^3, FP64; 110 before) and
-// 49 (2,304 electrode atoms, 64 x 64 x 160, FP32; 100 before): a barrier takes
+// Now 36 us (3,000 atoms, 48^3, FP32), 52 (10,701, 64^3, FP64; 110 before) and
+// 50 (2,304 electrode atoms, 64 x 64 x 160, FP32; 100 before): a barrier takes
 // 1.8 of them, there are six (eight in the last case).
 //
 //   A   direction p = r + beta p of the group's atoms, spread
@@ -43,8 +43,8 @@ constexpr long long kCgSpin = 1LL << 23;
 constexpr int kCgMaxLines = kCgFft;      // lines of a block's y transform
 constexpr int kCgLaunch = 128;           // iterations per launch
 // Complex values of the largest x plane that one block transforms in z and y by itself: two barriers and a trip of
-// the spectrum through L2 less in each direction, for fewer blocks at work.  18 iterations of 48^3 (FP32) 776 -> 690
-// us, 56 of 64^3 (FP64) 3,090 -> 2,895; with 64 x 160 values a plane both ways take the same (1,732 and 1,738).
+// the spectrum through L2 less in each direction, for fewer blocks at work.  19 iterations of 48^3 (FP32) 776 -> 690
+// us, 58 of 64^3 (FP64) 3,090 -> 2,895; with 64 x 160 values a plane both ways take the same (1,732 and 1,738).
 constexpr int kCgPlane = 4096;
 
 struct CgSlot {
