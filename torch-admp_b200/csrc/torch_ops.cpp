@@ -344,9 +344,19 @@ class Site : public torch::autograd::Function<Site> {
   }
 };
 
-// Status and (when it is 0) pairs [nf P, 2], scales [nf P], distances [nf P] of positions [nf N, 3].
+// Status and (when it is 0) pairs [nf P, 2], scales [nf P], distances [nf P] of positions [nf N, 3].  The kernels
+// index a box a frame and three coordinates an atom, so both counts are checked before a pointer is taken.
 std::tuple<int64_t, Tensor, Tensor, Tensor> neighbor_list(Tensor pos, std::optional<Tensor> box, double cutoff,
                                                           int64_t nf) {
+  TORCH_CHECK_VALUE(nf >= 0 && pos.dim() >= 1, "neighbour list: positions [frames x atoms, 3]");
+  const int64_t rows = pos.size(0);
+  TORCH_CHECK_INDEX((nf > 0 ? rows % nf == 0 : rows == 0) && pos.numel() >= 3 * rows, "neighbour list: positions ",
+                    pos.sizes(), " for ", nf, " frame(s) of atoms with three coordinates");
+  if (box.has_value()) {
+    TORCH_CHECK_INDEX(nf == 1 ? box->numel() >= 9 : box->numel() == 9 * nf, "neighbour list: box ", box->sizes(), " for ", nf, " frame(s)");
+    TORCH_CHECK_TYPE(box->scalar_type() == pos.scalar_type(), "neighbour list: box and positions of one type");
+    TORCH_CHECK(box->device() == pos.device(), "neighbour list: box on ", box->device(), ", positions on ", pos.device());
+  }
   Tensor p = pos.contiguous(), b = box.has_value() ? box->contiguous() : torch::empty({0}, p.options());
   const int dt = dtype_code(p);
   void* st = stream_of(p);
