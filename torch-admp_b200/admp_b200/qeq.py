@@ -200,38 +200,58 @@ def _kkt(hessian, chi, C, b):
     does single precision, where Cholesky was up to 1.3 times further off at 2,304
     atoms."""
     n = hessian.shape[0]
-    m = 0 if C is None else C.shape[0]
-    if n > 0 and m <= 1 and hessian.dtype == torch.float64:
-        lib = L.load()
-        nbytes = lib.admp_qeq_dense_workspace_size(n)
-        if nbytes:
-            H, g = hessian.contiguous(), chi.reshape(-1).to(torch.float64).contiguous()
-            row = C.to(torch.float64).contiguous() if m else None
-            val = b.reshape(-1).to(H.device, torch.float64).contiguous() if m else None
-            q, info, ws = torch.empty_like(g), ctypes.c_int(0), L.workspace(nbytes, H.device)
-            L.check(lib.admp_qeq_dense_solve(n, L.ptr(H), L.ptr(g), L.ptr(row), L.ptr(val), L.ptr(q),
-                                             ctypes.byref(info), L.ptr(ws), nbytes, L.stream_of(H.device)), "QEq dense solve")
-            if info.value == 0:
-                return q
-    rhs = -chi.reshape(-1, 1).to(hessian.dtype)
-    if n > 0 and m <= 1 and hessian.dtype == torch.float64 and nbytes == 0:  # more atoms than that solve takes
-        factor, bad = torch.linalg.cholesky_ex(hessian)
-        Ct = hessian.new_zeros(n, 0) if m == 0 else C.T.to(hessian.dtype)
-        x = torch.cholesky_solve(torch.cat([rhs, Ct], 1), factor)
-        if m == 1:
-            schur = Ct.T @ x[:, 1:]
-            bad = bad + (schur == 0).sum()
-        if int(bad) == 0:
-            if m == 0:
-                return x.reshape(-1)
-            lam = (Ct.T @ x[:, :1] - b.reshape(-1, 1).to(hessian.dtype)) / schur
-            return (x[:, :1] - x[:, 1:] * lam).reshape(-1)
-    if m == 0 and C is None:
-        return torch.linalg.solve(hessian, rhs).reshape(-1)
+    q = _kkt_cholesky(hessian, chi, C, b) if _cholesky_takes(hessian, chi, C, b) else None
+    if q is not None:
+        return q
+    if C is None:
+        return torch.linalg.solve(hessian, -chi.reshape(-1, 1)).reshape(-1)
+    m = C.shape[0]
     A = torch.cat([torch.cat([hessian, C.T.to(hessian.dtype)], 1),
                    torch.cat([C.to(hessian.dtype), torch.zeros(m, m, device=hessian.device, dtype=hessian.dtype)], 1)], 0)
-    rhs = torch.cat([rhs.reshape(-1), b.reshape(-1).to(hessian.dtype)])
+    rhs = torch.cat([-chi.reshape(-1).to(hessian.dtype), b.reshape(-1).to(hessian.dtype)])
     return torch.linalg.solve(A, rhs.reshape(-1, 1)).reshape(-1)[:n]
+
+
+def _cholesky_takes(hessian, chi, C, b) -> bool:
+    """Whether the arrays are what _kkt_cholesky indexes; the bordered system refuses
+    or takes every other form as torch does."""
+    n = hessian.shape[0]
+    m = 0 if C is None else C.shape[0]
+    if n == 0 or m > 1 or hessian.dtype != torch.float64 or not hessian.is_cuda or hessian.shape != (n, n):
+        return False
+    if chi.numel() != n or chi.device != hessian.device or (C is None and chi.dtype != hessian.dtype):
+        return False
+    return C is None or (C.shape == (m, n) and b.numel() == m and C.device == b.device == hessian.device)
+
+
+def _kkt_cholesky(hessian, chi, C, b):
+    """_kkt of a positive definite double-precision H with at most one constraint, or
+    None where a pivot or the Schur complement says that it is not."""
+    n = hessian.shape[0]
+    m = 0 if C is None else C.shape[0]
+    lib = L.load()
+    nbytes = lib.admp_qeq_dense_workspace_size(n)
+    if nbytes:
+        H, g = hessian.contiguous(), chi.reshape(-1).to(torch.float64).contiguous()
+        row = C.to(torch.float64).contiguous() if m else None
+        val = b.reshape(-1).to(torch.float64).contiguous() if m else None
+        q, info, ws = torch.empty_like(g), ctypes.c_int(0), L.workspace(nbytes, H.device)
+        L.check(lib.admp_qeq_dense_solve(n, L.ptr(H), L.ptr(g), L.ptr(row), L.ptr(val), L.ptr(q),
+                                         ctypes.byref(info), L.ptr(ws), nbytes, L.stream_of(H.device)), "QEq dense solve")
+        return q if info.value == 0 else None
+    rhs = -chi.reshape(-1, 1).to(hessian.dtype)
+    factor, bad = torch.linalg.cholesky_ex(hessian)
+    Ct = hessian.new_zeros(n, 0) if m == 0 else C.T.to(hessian.dtype)
+    x = torch.cholesky_solve(torch.cat([rhs, Ct], 1), factor)
+    if m == 1:
+        schur = Ct.T @ x[:, 1:]
+        bad = bad + (schur == 0).sum()
+    if int(bad) != 0:
+        return None
+    if m == 0:
+        return x.reshape(-1)
+    lam = (Ct.T @ x[:, :1] - b.reshape(-1, 1).to(hessian.dtype)) / schur
+    return (x[:, :1] - x[:, 1:] * lam).reshape(-1)
 
 
 def _times(t, c: float):
