@@ -63,3 +63,37 @@ def test_mixed_devices_are_refused(cuda, k):
         _kkt(*a)
     a = _arrays(cuda)
     assert rel(_kkt(*a), _kkt(*_arrays("cpu"))) < 1e-11
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("constrained", [True, False])
+def test_charges_and_fermi_level_differentiate(cuda, constrained):
+    """dq/dchi, dq/db and dE_fermi/dchi of solve_matrix_inversion against the inverse
+    of the bordered matrix (condition number below 1e4: relative 1e-9)."""
+    from admp_b200 import synthetic
+    from admp_b200.nblist import TorchNeighborList
+    from admp_b200.qeq import QEqForceModule
+    pos, box, chi, hard, eta, _ = synthetic.water_system(11, 12.5, 3)
+    t = lambda x: torch.tensor(x, dtype=torch.float64, device=cuda)  # noqa: E731
+    p, bx, c, h, e = t(pos), t(box), t(chi).requires_grad_(True), t(hard), t(eta)
+    n = len(pos)
+    C = torch.linspace(0.5, 1.5, n, dtype=torch.float64, device=cuda)[None] if constrained else None
+    b = t([0.3]).requires_grad_(True) if constrained else None
+    nb = TorchNeighborList(6.0)
+    pairs = nb(p, bx)
+    m = QEqForceModule(6.0, 5e-4, kmesh=14)
+    args = (p, bx, c, h, e, pairs, nb.get_ds(), nb.get_buffer_scales())
+    _, q, _, fermi = m.solve_matrix_inversion(*args, C, b)
+    w = torch.linspace(-1, 1, n, dtype=torch.float64, device=cuda)
+    got = torch.autograd.grad((w * q).sum() + fermi, [c, b] if constrained else [c])
+    H = m.calc_hessian(*args)
+    k = 1 if constrained else 0
+    A = torch.zeros(n + k, n + k, dtype=torch.float64, device=cuda)
+    A[:n, :n] = H
+    if constrained:
+        A[n:, :n], A[:n, n:] = C, C.T
+    inv = torch.linalg.inv(A)
+    dq = w + H.sum(0) / n  # d(w.q + fermi)/dq
+    assert rel(got[0], 1.0 / n - inv[:n, :n].T @ dq) < 1e-9
+    if constrained:
+        assert rel(got[1], inv[:n, n:].T @ dq) < 1e-9

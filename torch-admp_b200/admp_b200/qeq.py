@@ -213,10 +213,13 @@ def _kkt(hessian, chi, C, b):
 
 
 def _cholesky_takes(hessian, chi, C, b) -> bool:
-    """Whether the arrays are what _kkt_cholesky indexes; the bordered system refuses
-    or takes every other form as torch does."""
+    """Whether the arrays are what _kkt_cholesky indexes and none asks for a gradient
+    (its kernel has no backward); the bordered system differentiates, and refuses or
+    takes every other form as torch does."""
     n = hessian.shape[0]
     m = 0 if C is None else C.shape[0]
+    if torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in (hessian, chi, C, b)):
+        return False
     if n == 0 or m > 1 or hessian.dtype != torch.float64 or not hessian.is_cuda or hessian.shape != (n, n):
         return False
     if chi.numel() != n or chi.device != hessian.device or (C is None and chi.dtype != hessian.dtype):
