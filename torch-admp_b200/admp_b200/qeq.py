@@ -329,16 +329,19 @@ def _hessian(module, positions, box, hardness, eta, pairs, ds, buffer_scales, ma
              max_mesh_bytes: int = 1 << 30):
     """Dense d2E/dq2 by admp_qeq_hessian: the reciprocal part in chunks of up to
     ``max_cols`` columns whose meshes take at most ``max_mesh_bytes``."""
+    # the kernels index n atoms and P pairs whatever the arrays hold: any other length is refused here
+    n, P = positions.shape[0], pairs.shape[0]
+    positions, box, pairs = positions.reshape(n, 3), box.reshape(3, 3), pairs.reshape(P, 2)
+    ds, buffer_scales, hardness = ds.reshape(P), buffer_scales.reshape(P), hardness.reshape(n)
+    eta = eta.reshape(n) if eta is not None else None
     lib = L.load()
     ec = module.const_lib.energy_coeff
     pos, bx, pr, dsc, bsc, (hard_c, eta_c) = _std_inputs(
         module, positions, box, pairs, ds, buffer_scales, _times(hardness.detach(), ec),
         _times(eta.detach(), module.const_lib.length_coeff) if eta is not None else None)
-    n = pos.shape[0]
     dt, dev = pos.dtype, pos.device
     if eta_c is None:
         eta_c = torch.zeros(n, dtype=dt, device=dev)
-    P = int(pr.shape[0])
     c = module.submodels["coulomb"]
     km = _kmesh_of(module, bx)
     per_col = 2 * km[0] * km[1] * (km[2] + 2) * pos.element_size()
