@@ -142,7 +142,10 @@ __device__ void nb_setup(int pbc, const T* __restrict__ box, double rc, int maxc
   } else {
     for (int d = 0; d < 3; ++d) {
       double ext = m->hi[d] - m->lo[d];
-      if (!isfinite(ext)) status = ADMP_ERR_NONFINITE;
+      if (!(ext >= 0.0) || !isfinite(ext)) {  // no finite coordinate on this axis leaves the bounds crossed
+        status = ADMP_ERR_NONFINITE;
+        ext = 0.0;
+      }
       m->cs[d] = rc;
       double r = ext / rc;
       nc[d] = r < 1e6 ? (int)floor(r) + 1 : 1;
