@@ -20,12 +20,16 @@ struct ImgGeom {
   double b[9], bi[9];
   int m[3];
   int pbc;
+  int bad;  // more images than an atom's counts hold
 };
 
 // Open boundaries (pbc == 0, box unused): identity cell, no wrap, no images.
+// A singular box, or a cutoff of more than 2^19 - 1 cells along an axis or 2^31
+// images in all (the packed image vectors and the counts), has no image walked.
 template <typename T>
 __device__ __forceinline__ void img_geom(const T* box, int pbc, double rc, ImgGeom& g) {
   g.pbc = pbc;
+  g.bad = 0;
   if (!pbc) {
     for (int k = 0; k < 9; ++k) g.b[k] = g.bi[k] = (k % 4 == 0) ? 1.0 : 0.0;
     g.m[0] = g.m[1] = g.m[2] = 0;
@@ -33,12 +37,20 @@ __device__ __forceinline__ void img_geom(const T* box, int pbc, double rc, ImgGe
   }
   load_box(box, g.b);
   const double V = fabs(inv3(g.b, g.bi));
+  double images = 1.0, most = 0.0;
   for (int d = 0; d < 3; ++d) {
     const double* u = g.b + ((d + 1) % 3) * 3;
     const double* v = g.b + ((d + 2) % 3) * 3;
     const double cx = u[1] * v[2] - u[2] * v[1], cy = u[2] * v[0] - u[0] * v[2], cz = u[0] * v[1] - u[1] * v[0];
     const double h = V / sqrt(cx * cx + cy * cy + cz * cz);
-    g.m[d] = min((int)ceil(rc / h), (1 << 19) - 1);
+    const double m = ceil(rc / h);
+    g.m[d] = (int)m;
+    images *= 2.0 * m + 1.0;
+    most = fmax(most, m);
+  }
+  if (images > 2147483647.0 || most > (double)((1 << 19) - 1)) {
+    g.bad = 1;
+    g.m[0] = g.m[1] = g.m[2] = 0;
   }
 }
 
@@ -49,7 +61,7 @@ __global__ void __launch_bounds__(256) img_frac_kernel(int N, const T* __restric
                                                        int* __restrict__ cell, int* __restrict__ ntrunc) {
   __shared__ ImgGeom g;
   if (threadIdx.x == 0) img_geom<T>(box, pbc, rc, g);
-  if (blockIdx.x == 0 && threadIdx.x == 0) *ntrunc = 0;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *ntrunc = g.bad ? -1 : 0;
   __syncthreads();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
@@ -168,6 +180,11 @@ __global__ void __launch_bounds__(32 * kImgWarps)
   if (threadIdx.x == 0) nkept = 0;
   img_block<T>(b, box, pbc, rc);
   const int i = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (b.g.bad) {
+    if (lane == 0) cnt_ij[i * kImgWarps + warp] = cnt_ii[i * kImgWarps + warp] = 0;
+    if (threadIdx.x == 0) thr[i] = -1.0;
+    return;
+  }
   const double rc2 = rc * rc;
   const long long all = (long long)N * b.nimg;
   long long t0, t1;
@@ -410,6 +427,8 @@ static int img_count_impl(int pbc, int N, const T* pos, const T* box, double rc,
   ADMP_CUDA_TRY(cudaGetLastError());
   const ImgResult* h = (const ImgResult*)read_back(w.res, sizeof(ImgResult), st);
   if (!h) return ADMP_ERR_CUDA;
+  if (h->ntrunc < 0)
+    return fail(ADMP_ERR_BAD_ARG, "image neighbour list: cutoff %g takes too many images of the box (or it is singular)", rc);
   *n_ij = h->n_ij;
   *n_ii = h->n_ii;
   if (n_truncated) *n_truncated = h->ntrunc;
