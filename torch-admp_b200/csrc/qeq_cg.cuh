@@ -415,7 +415,7 @@ __global__ void __launch_bounds__(kCgThreads) qeq_cg_kernel(CgArgs<T> a) {
   if (sc->done) return;  // the same for every block: only phase A writes it, behind the first barrier
   double rr0 = sc->rr;
   const double nn = sc->nn, pre = sc->pre, Lz2 = sc->Lz2;
-  const double few = a.P.tol * (double)a.N, few2 = few * few;
+  const double few = a.P.tol > 0.0 ? a.P.tol * (double)a.N : 0.0, few2 = few * few;
   const int nc = sc->n_const;
   unsigned target = 0;
   auto stop = [&]() {
