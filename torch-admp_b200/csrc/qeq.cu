@@ -196,7 +196,8 @@ static int cg_persistent(QEqCtx<T>& c, CGScal* h, bool& used) {
     const void* p = read_back(c.w.sc, sizeof(CGScal), c.st);
     if (!p) return ADMP_ERR_CUDA;
     *h = *(const CGScal*)p;
-    if (h->done || h->status || h->iter >= c.P.max_iter + kCgLaunch) return ADMP_OK;
+    // another status is not the end: a singular Gram matrix left one, and the solve's own verdict replaces it
+    if (h->done || h->status == ADMP_ERR_CUDA || h->iter >= c.P.max_iter + kCgLaunch) return ADMP_OK;
   }
 }
 
@@ -321,7 +322,7 @@ static int qeq_solve_impl(int flags, int nf, int N, const int* kmesh, const T* p
   for (int f = 0; f < nf; ++f) {
     if (iters) iters[f] = h[f].iter;
     if (resid) resid[f] = sqrt(h[f].rr_new > 0 ? h[f].rr_new : h[f].rr) / (N > 0 ? N : 1);
-    const int stf = h[f].done || h[f].status ? h[f].status : ADMP_ERR_NOT_CONVERGED;
+    const int stf = h[f].done || h[f].status == ADMP_ERR_CUDA ? h[f].status : ADMP_ERR_NOT_CONVERGED;
     if (stf && (worst == ADMP_OK || worst == ADMP_ERR_NOT_CONVERGED)) {
       worst = stf;
       worst_f = f;
