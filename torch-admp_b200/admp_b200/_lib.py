@@ -208,16 +208,21 @@ def workspace(nbytes: int, device) -> torch.Tensor:
     return torch.empty(max(int(nbytes), 1), dtype=torch.uint8, device=device)
 
 
-def constraint_values(b, n_const: int):
-    """(flag, pointer, keep-alive) of the n_const constraint values of a QEq
-    call: device values stay on the device, so that the host need not wait."""
+def constraint_values(b, n_const: int, device):
+    """(flag, pointer, keep-alive) of the n_const constraint values of a QEq call
+    on ``device``: device values stay on the device, so that the host need not wait
+    (those of another device are copied to it).  As with host values, missing ones
+    are zero and more than n_const raise IndexError."""
     if n_const == 0:
         arr = (ctypes.c_double * 1)(0.0)
         return 0, arr, arr
     if b.is_cuda:
-        t = b.detach().reshape(-1).to(torch.float64).contiguous()
+        t = b.detach().reshape(-1).to(device, torch.float64)
+        if t.numel() > n_const:
+            raise IndexError(f"{n_const} constraints take as many values, got {t.numel()}")
         if t.numel() < n_const:
-            raise IndexError(f"{n_const} constraints need as many values, got {t.numel()}")
+            t = torch.cat([t, t.new_zeros(n_const - t.numel())])
+        t = t.contiguous()
         return QEQ_DEVICE_B, ctypes.cast(t.data_ptr(), _dp), t
     arr = (ctypes.c_double * n_const)(*[float(v) for v in b.detach().reshape(-1).tolist()])
     return 0, arr, arr

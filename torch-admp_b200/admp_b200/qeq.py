@@ -323,7 +323,7 @@ def _qeq_solve_raw(module, q0, positions, box, chi, hardness, eta, pairs, ds, bu
     P = pr.shape[0]
     nc = 0 if C is None else int(C.shape[0])
     Cc = prep_float(C.detach().reshape(nc, n), dt) if nc else None
-    bflag, bvals, _keep_b = L.constraint_values(b, nc)
+    bflag, bvals, _keep_b = L.constraint_values(b, nc, dev)
     flags |= bflag
     nbytes = lib.admp_qeq_workspace_size(L.dtype_code(dt), n, P, kp if c.kspace_flag else None, nc)
     ws = L.workspace(nbytes, dev)
@@ -558,7 +558,7 @@ def _qeq_solve_frames_raw(module, q0, positions, box, chi, hardness, eta, pairs,
     kp, _keep = L.int3([k for row in km for k in row])
     nc = 0 if C is None else int(C.shape[0])
     Cc = prep_float(C.detach().reshape(nc, n), dt) if nc else None
-    bflag, bvals, _keep_b = L.constraint_values(b, nc)
+    bflag, bvals, _keep_b = L.constraint_values(b, nc, dev)
     flags |= bflag
     nbytes = lib.admp_qeq_frames_workspace_size(L.dtype_code(dt), nf, n, nf * P, kp if c.kspace_flag else None, nc)
     if nbytes == 0:
