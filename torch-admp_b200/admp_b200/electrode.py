@@ -151,7 +151,7 @@ def infer(calculator: PolarizableElectrode, positions, box, charges, pairs, ds, 
                                      eta, chi, hardness, constraint_matrix, constraint_vals, ffield_electrode_mask,
                                      ffield_potential, method)
     q_opt = charges.detach().clone()
-    q_opt.masked_scatter_(electrode_mask, _q.detach().to(q_opt.dtype))
+    q_opt.masked_scatter_(electrode_mask != 0, _q.detach().to(q_opt.dtype))  # masks of bytes too
     energy, forces = calculator.coulomb_calculator(positions=positions, box=box, charges=q_opt, eta=eta, pairs=pairs,
                                                    ds=ds, buffer_scales=buffer_scales, efield=efield)
     return energy, forces, q_opt
