@@ -61,11 +61,24 @@ Tensor scales_of(const Tensor& bs, const Tensor& like) {
 }
 int scale_flag(const Tensor& bs) { return bs.scalar_type() == torch::kLong ? ADMP_PAIR_INT64_SCALES : 0; }
 
+// Whether admp_scale_frames may take a tensor's pointer: batched and other wrapped tensors have no memory of their own,
+// and a saved-tensor hook may return another layout.
+bool plain(const Tensor& t, const Tensor& like) {
+  return t.has_storage() && !t.unsafeGetTensorImpl()->key_set().has_any(c10::DispatchKeySet(
+                                {c10::DispatchKey::FuncTorchBatched, c10::DispatchKey::FuncTorchGradWrapper,
+                                 c10::DispatchKey::Python, c10::DispatchKey::Functionalize, c10::DispatchKey::Conjugate,
+                                 c10::DispatchKey::Negative})) &&
+         t.device() == like.device() && t.scalar_type() == like.scalar_type();
+}
+
 // Saved gradients times the incoming dL/dE of each frame, all in one launch;
 // by torch operators where the product itself is to be differentiated
-// (create_graph with a dL/dE that needs a gradient).
+// (create_graph with a dL/dE that needs a gradient) or a tensor is not plain
+// (is_grads_batched: one dL/dE for each of a batch of backward passes).
 variable_list scaled(const variable_list& saved, const Tensor& gE) {
-  if (at::GradMode::is_enabled() && gE.requires_grad()) {
+  bool direct = !(at::GradMode::is_enabled() && gE.requires_grad()) && plain(gE, gE);
+  for (const Tensor& t : saved) direct = direct && (!t.defined() || (plain(t, gE) && t.is_contiguous()));
+  if (!direct) {
     variable_list r(saved.size());
     for (size_t i = 0; i < saved.size(); ++i)
       if (saved[i].defined()) {
