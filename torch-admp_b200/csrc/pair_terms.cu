@@ -539,10 +539,26 @@ extern "C" int admp_pair_distances_frames_backward(int dtype, int pbc, int nfram
   return pair_dist_bwd(dtype, pbc, nframes, natoms, npairs, pairs, pos, box, grad_ds, grad_pos, grad_box, err, st);
 }
 
+// Frames are the y dimension of these grids; the entry points take more of them in several launches.
+constexpr int kGridFrames = 65535;
+static const void* frame_at(const void* p, long long elems, size_t size) { return p ? (const char*)p + elems * size : p; }
+static void* frame_at(void* p, long long elems, size_t size) { return p ? (char*)p + elems * size : p; }
+
+template <typename T>
+static int damping_frames(bool ints, int nf, int N, long long P, const long long* pairs, const void* ds, const void* bs,
+                          const void* q, const void* eta, double ke, double* energy, void* dds, void* dq, void* deta,
+                          DevError* err, cudaStream_t st) {
+  atom_energy_kernel<T, true><<<dim3((N + 255) / 256, nf), 256, 0, st>>>(N, (const T*)q, (const T*)eta, nullptr, ke,
+                                                                         energy, (T*)dq, (T*)deta, nullptr);
+  ADMP_CUDA_TRY(cudaGetLastError());
+  return launch_pair_energy<T>(ADMP_PAIR_DAMPING, nf, N, P, pairs, (const T*)ds, bs, ints, (const T*)q, (const T*)eta,
+                               0.0, ke, energy, 1, true, (T*)dds, (T*)dq, (T*)deta, err, st);
+}
+
 extern "C" int admp_damping_energy(int dtype, int flags, int nframes, int natoms, long long npairs, const long long* pairs,
                                    const void* ds, const void* buffer_scales, const void* q, const void* eta, double ke,
                                    double* energy, void* dE_dds, void* dE_dq, void* dE_deta, void* stream) {
-  if (nframes <= 0 || nframes > 65535 || natoms <= 0 || npairs < 0 || !q || !eta || !energy)
+  if (nframes <= 0 || natoms <= 0 || npairs < 0 || !q || !eta || !energy)
     return fail(ADMP_ERR_BAD_ARG, "admp_damping_energy: args");
   if (npairs > 0 && (!pairs || !ds || !buffer_scales)) return fail(ADMP_ERR_BAD_ARG, "admp_damping_energy: pairs");
   if (dtype != ADMP_F64 && dtype != ADMP_F32) return fail(ADMP_ERR_BAD_ARG, "bad dtype");
@@ -550,70 +566,73 @@ extern "C" int admp_damping_energy(int dtype, int flags, int nframes, int natoms
   DevError* err = scratch_error(st);
   if (!err) return ADMP_ERR_CUDA;
   ADMP_CUDA_TRY(cudaMemsetAsync(energy, 0, sizeof(double) * nframes, st));
-  const dim3 grid((natoms + 255) / 256, nframes);
   const bool ints = (flags & ADMP_PAIR_INT64_SCALES) != 0;
-  int s;
-  if (dtype == ADMP_F64) {
-    atom_energy_kernel<double, true><<<grid, 256, 0, st>>>(natoms, (const double*)q, (const double*)eta, nullptr, ke,
-                                                           energy, (double*)dE_dq, (double*)dE_deta, nullptr);
-    s = launch_pair_energy<double>(ADMP_PAIR_DAMPING, nframes, natoms, npairs, pairs, (const double*)ds,
-                                   buffer_scales, ints, (const double*)q, (const double*)eta, 0.0, ke, energy, 1, true,
-                                   (double*)dE_dds, (double*)dE_dq, (double*)dE_deta, err, st);
-  } else {
-    atom_energy_kernel<float, true><<<grid, 256, 0, st>>>(natoms, (const float*)q, (const float*)eta, nullptr, ke,
-                                                          energy, (float*)dE_dq, (float*)dE_deta, nullptr);
-    s = launch_pair_energy<float>(ADMP_PAIR_DAMPING, nframes, natoms, npairs, pairs, (const float*)ds,
-                                  buffer_scales, ints, (const float*)q, (const float*)eta, 0.0, ke, energy, 1, true,
-                                  (float*)dE_dds, (float*)dE_dq, (float*)dE_deta, err, st);
+  const size_t es = dtype == ADMP_F64 ? 8 : 4, ss = ints ? 8 : es;
+  for (int f = 0; f < nframes; f += kGridFrames) {
+    const int nf = nframes - f < kGridFrames ? nframes - f : kGridFrames;
+    const long long a = (long long)f * natoms, p = f * npairs;
+    auto* call = dtype == ADMP_F64 ? damping_frames<double> : damping_frames<float>;
+    const int s = call(ints, nf, natoms, npairs, pairs + 2 * p, frame_at(ds, p, es), frame_at(buffer_scales, p, ss),
+                       frame_at(q, a, es), frame_at(eta, a, es), ke, energy + f, frame_at(dE_dds, p, es),
+                       frame_at(dE_dq, a, es), frame_at(dE_deta, a, es), err, st);
+    if (s) return s;
   }
-  ADMP_CUDA_TRY(cudaGetLastError());
-  return s || npairs == 0 ? s : check_error(err, st);
+  return npairs == 0 ? ADMP_OK : check_error(err, st);
+}
+
+template <typename T>
+static void site_frames(int nf, int N, const void* q, const void* chi, const void* hard, double* energy, void* dq,
+                        void* dchi, void* dhard, cudaStream_t st) {
+  atom_energy_kernel<T, false><<<dim3((N + 255) / 256, nf), 256, 0, st>>>(N, (const T*)q, (const T*)chi, (const T*)hard,
+                                                                          0.0, energy, (T*)dq, (T*)dchi, (T*)dhard);
 }
 
 extern "C" int admp_site_energy(int dtype, int nframes, int natoms, const void* q, const void* chi,
                                 const void* hardness, double* energy, void* dE_dq, void* dE_dchi, void* dE_dhard,
                                 void* stream) {
-  if (nframes <= 0 || nframes > 65535 || natoms <= 0 || !q || !chi || !hardness || !energy)
+  if (nframes <= 0 || natoms <= 0 || !q || !chi || !hardness || !energy)
     return fail(ADMP_ERR_BAD_ARG, "admp_site_energy: args");
+  if (dtype != ADMP_F64 && dtype != ADMP_F32) return fail(ADMP_ERR_BAD_ARG, "bad dtype");
   cudaStream_t st = (cudaStream_t)stream;
   ADMP_CUDA_TRY(cudaMemsetAsync(energy, 0, sizeof(double) * nframes, st));
-  const dim3 grid((natoms + 255) / 256, nframes);
-  if (dtype == ADMP_F64)
-    atom_energy_kernel<double, false><<<grid, 256, 0, st>>>(natoms, (const double*)q, (const double*)chi,
-                                                            (const double*)hardness, 0.0, energy, (double*)dE_dq,
-                                                            (double*)dE_dchi, (double*)dE_dhard);
-  else if (dtype == ADMP_F32)
-    atom_energy_kernel<float, false><<<grid, 256, 0, st>>>(natoms, (const float*)q, (const float*)chi,
-                                                           (const float*)hardness, 0.0, energy, (float*)dE_dq,
-                                                           (float*)dE_dchi, (float*)dE_dhard);
-  else
-    return fail(ADMP_ERR_BAD_ARG, "bad dtype");
-  ADMP_CUDA_TRY(cudaGetLastError());
+  const size_t es = dtype == ADMP_F64 ? 8 : 4;
+  for (int f = 0; f < nframes; f += kGridFrames) {
+    const long long a = (long long)f * natoms;
+    auto* call = dtype == ADMP_F64 ? site_frames<double> : site_frames<float>;
+    call(nframes - f < kGridFrames ? nframes - f : kGridFrames, natoms, frame_at(q, a, es), frame_at(chi, a, es),
+         frame_at(hardness, a, es), energy + f, frame_at(dE_dq, a, es), frame_at(dE_dchi, a, es),
+         frame_at(dE_dhard, a, es), st);
+    ADMP_CUDA_TRY(cudaGetLastError());
+  }
   return ADMP_OK;
 }
 
 extern "C" int admp_scale_frames(int dtype, int nframes, int narrays, const void* const* in, void* const* out,
                                  const long long* per_frame, const void* w, long long w_stride, void* stream) {
-  if (nframes <= 0 || nframes > 65535 || narrays < 0 || narrays > 4 || !w)
+  if (nframes <= 0 || narrays < 0 || narrays > 4 || !w)
     return nframes == 0 ? ADMP_OK : fail(ADMP_ERR_BAD_ARG, "admp_scale_frames: args");
-  ScaleArgs a{};
-  long long most = 0;
-  for (int k = 0; k < narrays; ++k) {
-    a.in[k] = in[k];
-    a.out[k] = out[k];
-    a.n[k] = per_frame[k];
-    most = most > per_frame[k] ? most : per_frame[k];
+  if (dtype != ADMP_F64 && dtype != ADMP_F32) return fail(ADMP_ERR_BAD_ARG, "bad dtype");
+  const size_t es = dtype == ADMP_F64 ? 8 : 4;
+  cudaStream_t st = (cudaStream_t)stream;
+  for (int f = 0; f < nframes; f += kGridFrames) {
+    ScaleArgs a{};
+    long long most = 0;
+    for (int k = 0; k < narrays; ++k) {
+      a.in[k] = frame_at(in[k], f * per_frame[k], es);
+      a.out[k] = frame_at(out[k], f * per_frame[k], es);
+      a.n[k] = per_frame[k];
+      most = most > per_frame[k] ? most : per_frame[k];
+    }
+    if (most == 0) return ADMP_OK;
+    long long blocks = (most + 255) / 256;
+    if (blocks > 2048) blocks = 2048;
+    const dim3 grid((unsigned)blocks, nframes - f < kGridFrames ? nframes - f : kGridFrames);
+    const void* wf = frame_at(w, f * w_stride, es);
+    if (dtype == ADMP_F64)
+      scale_frames_kernel<double><<<grid, 256, 0, st>>>(a, (const double*)wf, w_stride);
+    else
+      scale_frames_kernel<float><<<grid, 256, 0, st>>>(a, (const float*)wf, w_stride);
+    ADMP_CUDA_TRY(cudaGetLastError());
   }
-  if (most == 0) return ADMP_OK;
-  long long blocks = (most + 255) / 256;
-  if (blocks > 2048) blocks = 2048;
-  const dim3 grid((unsigned)blocks, nframes);
-  if (dtype == ADMP_F64)
-    scale_frames_kernel<double><<<grid, 256, 0, (cudaStream_t)stream>>>(a, (const double*)w, w_stride);
-  else if (dtype == ADMP_F32)
-    scale_frames_kernel<float><<<grid, 256, 0, (cudaStream_t)stream>>>(a, (const float*)w, w_stride);
-  else
-    return fail(ADMP_ERR_BAD_ARG, "bad dtype");
-  ADMP_CUDA_TRY(cudaGetLastError());
   return ADMP_OK;
 }
