@@ -20,7 +20,9 @@ from . import _lib as L
 from .ops import ImagePairDistanceFn, PairDistanceFn, image_neighbor_pairs
 
 L.load_torch_ops()  # torch.ops.admp_b200.neighbor_list
-_MAX_FRAMES = 4096  # frames per call of the frame lists
+# Frames and atoms per call of the frame lists: the scratch of a call is some 650 B an atom (512 of them the
+# neighbours kept between the passes), 2.7 GB at the limit, where a list of 90 neighbours an atom takes 12.
+_MAX_FRAMES, _MAX_ATOMS = 4096, 4 << 20
 
 
 def check_cutoff(box: torch.Tensor, cutoff: float) -> None:
@@ -153,8 +155,9 @@ def frame_pair_lists(positions: torch.Tensor, box: torch.Tensor, cutoff: float):
         raise ValueError("frame_pair_lists needs at least one frame")
     b = box.to(positions.dtype)
     parts = []
-    for f0 in range(0, nf, _MAX_FRAMES):
-        n = min(_MAX_FRAMES, nf - f0)
+    step = max(1, min(_MAX_FRAMES, _MAX_ATOMS // max(na, 1)))
+    for f0 in range(0, nf, step):
+        n = min(step, nf - f0)
         status, *rows = torch.ops.admp_b200.neighbor_list(positions[f0:f0 + n].reshape(n * na, 3), b[f0:f0 + n],
                                                           float(cutoff), n)
         if status == L.CUTOFF:
