@@ -116,10 +116,10 @@ static bool cg_plan(const QEqCtx<T>& c, int sms, CgArgs<T>& a, size_t& smem) {
   a.lz = a.ly = a.lx = 1;
   if (c.P.flags & ADMP_QEQ_KSPACE) {
     auto lines = [&](long long total, int K) {
-      long long l = (total + sms - 1) / sms;
-      const int most = cap / K < kCgMaxLines ? cap / K : kCgMaxLines;
-      l = l < most ? l : most;
-      return (int)(l < 1 ? 1 : l);
+      int most = cap / K < kCgMaxLines ? cap / K : kCgMaxLines;
+      most = most < 1 ? 1 : most;
+      const long long rounds = (total + (long long)sms * most - 1) / ((long long)sms * most);
+      return (int)((total + sms * rounds - 1) / (sms * rounds));
     };
     a.lz = lines(((long long)a.K0 * a.K1 + 1) / 2, a.K2);
     a.ly = lines((long long)a.K0 * d.K2h, a.K1);
