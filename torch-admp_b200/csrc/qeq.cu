@@ -102,10 +102,20 @@ static int qeq_matvec(QEqCtx<T>& c, const T* v, T* Hv, double* hv_out) {
 }
 
 // Set-up of the persistent solve (qeq_cg.cuh) of one system: false where its
-// line buffers do not fit a block's shared memory.
+// line buffers do not fit a block's shared memory, and where it is too large.
+//
+// One block an SM hides less latency than the kernels of the multi-launch loop,
+// which pays off while launches and short kernels bound an iteration.  A solve
+// (ms, this / the loop) of 10,701 atoms, 64^3: 1.3 / 3.0 (FP32), 2.0 / 3.5 (FP64);
+// 42,000, 100^3: 3.4 / 4.4, 6.0 / 8.0; 90,000, 128^3: 7.7 / 8.4, 15.1 / 16.9;
+// 120,000, 144^3: 11.5 / 11.3, 21.0 / 21.3, 142^3: 14.4 / 15.4, 29.3 / 29.7;
+// 180,000, 160^3: 20.3 / 17.5, 33.6 / 31.5; 300,000, 192^3: 35.1 / 26.7, 61.4 / 53.5.
+constexpr long long kCgMesh = 3000000;
+constexpr int kCgAtoms = 150000;
 template <typename T>
 static bool cg_plan(const QEqCtx<T>& c, int sms, CgArgs<T>& a, size_t& smem) {
   const SysDesc& d = c.w.plan.hs[0];
+  if (c.N > kCgAtoms || ((c.P.flags & ADMP_QEQ_KSPACE) && (long long)d.K0 * d.K1 * d.K2 > kCgMesh)) return false;
   const size_t budget = 200 * 1024, cs = sizeof(Cplx<T>);
   const int cap = (int)(64 * 1024 / cs);  // complex values in a line buffer
   a.N = c.N;

@@ -56,7 +56,6 @@ struct CgSlot {
 struct CgShared {
   CgSlot slot[3];
   unsigned arrived;
-  int failed;
 };
 
 template <typename T>
@@ -419,10 +418,7 @@ __global__ void __launch_bounds__(kCgThreads) qeq_cg_kernel(CgArgs<T> a) {
   const int nc = sc->n_const;
   unsigned target = 0;
   auto stop = [&]() {
-    if (threadIdx.x == 0) {
-      atomicExch(&a.sh->failed, 1);
-      atomicExch(&sc->status, ADMP_ERR_CUDA);
-    }
+    if (threadIdx.x == 0) atomicExch(&sc->status, ADMP_ERR_CUDA);
   };
   auto meet = [&]() { return cg_barrier<kSyncBlock>(a.sh, target, kCgThreads); };
   for (int k = a.init ? -1 : a.k0;; ++k) {
