@@ -200,6 +200,7 @@ static int cg_persistent(QEqCtx<T>& c, CGScal* h, bool& used) {
     a.init = a.k0 == 0;
     if (a.k0) ADMP_CUDA_TRY(cudaMemsetAsync(&c.w.cg->arrived, 0, sizeof(unsigned), c.st));
     void* args[] = {&a};
+    std::lock_guard<std::mutex> alone(grid_mutex(dev));
     ADMP_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)qeq_cg_kernel<T>, dim3(sms), dim3(kCgThreads), args, smem,
                                               c.st));
     count_launches(1);

@@ -156,6 +156,11 @@ int probed_error(DevError* err, cudaStream_t st) {
   return ((const DevError*)((const char*)g_pin.p + kReadBack))->code ? check_error(err, st) : ADMP_OK;
 }
 
+std::mutex& grid_mutex(int dev) {
+  static std::mutex mu[64];
+  return mu[dev & 63];
+}
+
 static const char* where_name(int w) {
   switch (w) {
     case 1: return "pair energy";

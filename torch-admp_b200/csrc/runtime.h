@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stddef.h>
 
+#include <mutex>
+
 #include "admp_common.cuh"
 
 namespace admp {
@@ -26,6 +28,11 @@ const void* read_back(const void* dev, size_t bytes, cudaStream_t st);
 // only.  One probe per thread at a time.
 int probe_error(DevError* err, cudaStream_t st);
 int probed_error(DevError* err, cudaStream_t st);
+// Held from the launch of a kernel whose blocks wait for one another over the
+// whole device until it has ended.  A cooperative launch has all its blocks
+// resident, but two of them on the streams of two threads, each with a block
+// for every SM, are not promised to take turns.
+std::mutex& grid_mutex(int dev);
 // Record a message and return `code`.
 int fail(int code, const char* fmt, ...);
 bool sync_checks();

@@ -287,6 +287,7 @@ static int spd_kkt(int n, const double* H, const double* chi, const double* C, c
   ADMP_CUDA_TRY(cudaMemsetAsync(w.sh, 0, sizeof(CgShared), st));
   ADMP_CUDA_TRY(cudaMemsetAsync(w.info, 0, sizeof(int), st));
   void* args[] = {&a};
+  std::lock_guard<std::mutex> alone(grid_mutex(dev));
   ADMP_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)spd_kkt_kernel, dim3(grid), dim3(kSpdThreads), args, smem, st));
   count_launches(1);
   const void* p = read_back(w.info, sizeof(int), st);
