@@ -55,3 +55,17 @@ def test_threads_on_their_own_streams(cuda):
         for x, y in zip(g, _work(cuda, k)):
             # both solves within n eps (4e-10) over eigenvalues of 1 or more, of charges above 0.1
             assert rel(x[0], y[0]) < 1e-8 and rel(x[1], y[1]) < 1e-10
+
+
+def test_first_calls_of_a_process_from_several_threads(cuda):
+    """A fresh process whose first calls come from eight threads at once: each kernel's
+    shared-memory limit is set before any of them launches it."""
+    import os
+    import subprocess
+    import sys
+    here = os.path.dirname(os.path.abspath(__file__))
+    paths = [here, os.path.dirname(here), os.path.join(os.path.dirname(here), "torch-admp_b200")]
+    code = (f"import sys; sys.path[:0] = {paths!r}\nimport torch\nfrom test_gpu_threads import _threads\n"
+            "_threads(torch.device('cuda:0'), 8, 1)\nprint('all ran')\n")
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "all ran" in r.stdout, r.stderr[-2000:]

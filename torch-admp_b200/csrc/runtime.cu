@@ -23,14 +23,15 @@ bool sync_checks() { return g_sync; }
 static std::mutex g_smem_mu;
 static std::map<std::pair<const void*, int>, size_t> g_smem_set;
 
-bool smem_already(const void* fn, size_t bytes) {
+cudaError_t smem_limit(const void* fn, size_t bytes) {
   int dev = 0;
   cudaGetDevice(&dev);
-  std::lock_guard<std::mutex> lock(g_smem_mu);
+  std::lock_guard<std::mutex> lock(g_smem_mu);  // over the call too: another thread launches once this returns
   size_t& v = g_smem_set[std::make_pair(fn, dev)];
-  if (v >= bytes) return true;
-  v = bytes;
-  return false;
+  if (v >= bytes) return cudaSuccess;
+  const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e == cudaSuccess) v = bytes;
+  return e;
 }
 
 static long long g_launches = 0;

@@ -72,12 +72,11 @@ struct Carver {
 
 // Raises a kernel's dynamic shared-memory limit to `bytes` (static shared
 // memory counts against the default 48 KB too, so the limit is always set);
-// remembers the largest value set per kernel and device.
-bool smem_already(const void* fn, size_t bytes);
+// remembers the largest value set per kernel and device, once it is set.
+cudaError_t smem_limit(const void* fn, size_t bytes);
 template <typename K>
 inline cudaError_t ensure_smem(K kernel, size_t bytes) {
-  if (bytes == 0 || smem_already((const void*)kernel, bytes)) return cudaSuccess;
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  return bytes == 0 ? cudaSuccess : smem_limit((const void*)kernel, bytes);
 }
 
 }  // namespace admp
