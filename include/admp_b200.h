@@ -276,7 +276,8 @@ int admp_image_pair_distances_backward(int dtype, int natoms, long long npairs,
 /* E(q) = site + Coulomb(PME) + damping subject to C q = b with linear CG    */
 /* (E is quadratic in q); stops when ||P grad||_2 / N < tol (qeq.py:1516).   */
 /*   flags: ADMP_QEQ_* below; kmesh HOST [3]; C [n_const, N] dtype;           */
-/*   b HOST [n_const] (double); q in: initial guess, out: solution.           */
+/*   b HOST [n_const] (double; DEVICE with ADMP_QEQ_DEVICE_B); q in: initial  */
+/*   guess, out: solution.                                                    */
 /*   rhs_shift: optional [N] added to chi (electrode potential b-vector).     */
 /* Returns ADMP_ERR_NOT_CONVERGED (q still written) when max_iter is hit.    */
 /* ------------------------------------------------------------------------ */
@@ -304,7 +305,7 @@ int admp_qeq_solve(int dtype, int flags, int natoms, const int* kmesh, const voi
 /* same as admp_qeq_solve.  Frame f holds atoms [f N, (f+1) N) of pos, chi,   */
 /* hardness, eta, rhs_shift and q, box f, and mesh kmesh[3f .. 3f+2] (HOST    */
 /* [nframes, 3]); pairs index atoms over all frames (frame f's pairs use     */
-/* indices f N + i); C [n_const, N] and b (HOST [n_const]) are shared by      */
+/* indices f N + i); C [n_const, N] and b (as above) are shared by            */
 /* every frame.  iters, resid: HOST [nframes] or NULL.  nframes <= 256.       */
 size_t admp_qeq_frames_workspace_size(int dtype, int nframes, int natoms, long long npairs,
                                       const int* kmesh, int n_const);
@@ -318,7 +319,7 @@ int admp_qeq_solve_frames(int dtype, int flags, int nframes, int natoms, const i
                           void* stream);
 
 /* Hessian-vector product of the same quadratic form (dE/dq at p minus at   */
-/* 0): out [N] = H p.  Used by the implicit adjoint of the charge solve.      */
+/* 0): out [N] = H p.                                                         */
 int admp_qeq_hvp(int dtype, int flags, int natoms, const int* kmesh, const void* pos,
                  const void* box, long long npairs, const long long* pairs, const void* ds,
                  const void* buffer_scales, const void* hardness, const void* eta, double kappa,
@@ -327,10 +328,7 @@ int admp_qeq_hvp(int dtype, int flags, int natoms, const int* kmesh, const void*
 
 /* admp_qeq_hvp for nframes frames at once (the layout of                     */
 /* admp_qeq_solve_frames; workspace from admp_qeq_frames_workspace_size):    */
-/* out [nframes, N] = H_f p_f.  The dense Hessian of matinv_optimize /       */
-/* calc_hessian (qeq.py:460-515, 1620-1670) is built from these, one batch   */
-/* of unit vectors (frames of the same geometry) per call, instead of one    */
-/* autograd pass per column.                                                 */
+/* out [nframes, N] = H_f p_f.                                               */
 int admp_qeq_hvp_frames(int dtype, int flags, int nframes, int natoms, const int* kmesh,
                         const void* pos, const void* box, long long npairs,
                         const long long* pairs, const void* ds, const void* buffer_scales,

@@ -221,29 +221,6 @@ class PairDistanceFn(torch.autograd.Function):
         return gpos, gbox, None
 
 
-def neighbor_pairs(pos: torch.Tensor, box: Optional[torch.Tensor], cutoff: float):
-    """Cell-list pair build (nblist.py:304-445): returns pairs [P,2] int64, buffer_scales [P] int64."""
-    lib = L.load()
-    dev = pos.device
-    dt = L.dtype_code(pos.dtype)
-    N = pos.shape[0]
-    st = L.stream_of(dev)
-    nbytes = lib.admp_nblist_workspace_size(N)
-    ws = L.workspace(nbytes, dev)
-    import ctypes
-    npairs = ctypes.c_longlong(0)
-    pbc = 1 if box is not None else 0
-    L.check(lib.admp_nblist_count(dt, pbc, N, L.ptr(pos), L.ptr(box), float(cutoff), L.ptr(ws), nbytes,
-                                  ctypes.byref(npairs), st), "neighbour list")
-    P = int(npairs.value)
-    pairs = torch.empty((P, 2), dtype=torch.long, device=dev)
-    bs = torch.empty(P, dtype=torch.long, device=dev)
-    if P > 0:
-        L.check(lib.admp_nblist_fill(dt, pbc, N, L.ptr(pos), L.ptr(box), float(cutoff), L.ptr(ws), nbytes,
-                                     L.ptr(pairs), L.ptr(bs), P, st), "neighbour list fill")
-    return pairs, bs
-
-
 class ImagePairDistanceFn(torch.autograd.Function):
     """ds = |r_j - r_i + n.B| for pairs with integer image shifts n (make_ds, nblist.py:212-240)."""
 

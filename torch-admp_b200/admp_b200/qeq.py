@@ -155,7 +155,7 @@ class QEqForceModule(BaseForceModule):
                               constraint_matrix, constraint_vals, project_q0, tol, max_iter, shift)
 
     def calc_hessian(self, positions, box, chi, hardness, eta, pairs, ds, buffer_scales):
-        """Dense Hessian d2E/dq2 from GPU Hessian-vector products (qeq.py:460-515)."""
+        """Dense Hessian d2E/dq2 (qeq.py:460-515)."""
         return _hessian(self, positions, box, hardness, eta, pairs, ds, buffer_scales)
 
     def solve_matrix_inversion(self, positions, box, chi, hardness, eta, pairs, ds, buffer_scales,

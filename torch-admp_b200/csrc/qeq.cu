@@ -78,7 +78,6 @@ struct QEqCtx {
   const T* C;
   int nc;
   cudaStream_t st;
-  int atom_blocks;
 };
 
 // Hv = H v (Hv zeroed, sums of v already in sc); optional double copy.
