@@ -13,6 +13,7 @@ N = 2
 @pytest.mark.parametrize("dtype,tol", [(torch.float64, 1e-13), (torch.float32, 1e-5)])
 @pytest.mark.parametrize("nf", [65535, 65536, 70001])
 def test_site(cuda, nf, dtype, tol):
+    from admp_b200 import qeq  # noqa: F401  (loads the operators)
     g = torch.Generator().manual_seed(nf)
     q, chi, h = (torch.rand(nf, N, dtype=dtype, generator=g).to(cuda).requires_grad_(True) for _ in range(3))
     w = torch.rand(nf, dtype=dtype, generator=g).to(cuda)
@@ -25,6 +26,7 @@ def test_site(cuda, nf, dtype, tol):
 
 @pytest.mark.parametrize("pairs", [0, 1])
 def test_damping(cuda, pairs):
+    from admp_b200 import qeq  # noqa: F401
     from admp_b200.utils import DIELECTRIC
     nf = 70001
     g = torch.Generator().manual_seed(7)
@@ -41,3 +43,25 @@ def test_damping(cuda, pairs):
     wrt = [q, eta, ds] if pairs else [q, eta]
     for x, y in zip(torch.autograd.grad(e.sum(), wrt), torch.autograd.grad(want.sum(), wrt)):
         assert rel(x, y) < 1e-12
+
+
+@pytest.mark.parametrize("nf", [8, 9, 256, 257])
+def test_coulomb_frames(cuda, nf):
+    """Either form of the system table and several calls' worth of frames: each frame's
+    energy and gradients are those of the frame by itself (atomics in another order)."""
+    from admp_b200.pme import CoulombForceModule
+    g = torch.Generator().manual_seed(nf)
+    pos = (torch.rand(nf, 5, 3, dtype=torch.float64, generator=g) * 9).to(cuda).requires_grad_(True)
+    q = torch.rand(nf, 5, dtype=torch.float64, generator=g).to(cuda).requires_grad_(True)
+    box = (torch.eye(3, dtype=torch.float64) * torch.linspace(9, 11, nf, dtype=torch.float64)[:, None, None]).to(cuda)
+    ij = torch.tensor([[0, 1], [2, 3]], device=cuda).expand(nf, 2, 2)
+    ds = torch.full((nf, 2), 2.5, dtype=torch.float64, device=cuda)
+    bs = torch.ones(nf, 2, dtype=torch.long, device=cuda)
+    m = CoulombForceModule(4.0, 1e-4, kmesh=10, slab_corr=True)
+    e = m(pos, box, ij, ds, bs, {"charge": q})
+    gp, gq = torch.autograd.grad(e.sum(), [pos, q])
+    for f in {0, 1, nf // 2, nf - 2, nf - 1}:
+        p1, q1 = pos[f].detach().requires_grad_(True), q[f].detach().requires_grad_(True)
+        e1 = m(p1, box[f], ij[f], ds[f], bs[f], {"charge": q1})
+        g1 = torch.autograd.grad(e1.sum(), [p1, q1])
+        assert rel(e[f], e1) < 1e-12 and rel(gp[f], g1[0]) < 1e-11 and rel(gq[f], g1[1]) < 1e-11
