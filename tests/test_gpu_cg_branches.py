@@ -105,6 +105,24 @@ def test_sizes(cuda, n, kmesh, dtype):
     assert err < 2 * n * eps / 30 + (1e-12 if dtype == torch.float64 else 1e-5) * size
 
 
+@pytest.mark.parametrize("n,pairs,kspace", [(300, 10000000, True), (300, 10000001, True), (20000, 50000, False),
+                                            (20001, 50000, False)])
+def test_pair_lists(cuda, n, pairs, kspace):
+    """Both sides of the lines by listed pairs (nearly all of scale 0) and, without a mesh, by atoms."""
+    from admp_b200.qeq import QEqForceModule
+    a = _cloud(cuda, n, [20.0, 21.0, 22.0], torch.float64)
+    g = torch.Generator().manual_seed(2)
+    ij = torch.randint(0, n, (pairs, 2), generator=g).to(cuda)
+    ds = torch.rand(pairs, dtype=torch.float64, generator=g).to(cuda) * 3 + 3
+    bs = torch.zeros(pairs, dtype=torch.float64, device=cuda)
+    bs[:n] = 0.5
+    bs[-n:] = 0.5
+    m = QEqForceModule(6.0, 5e-4, kmesh=[20, 21, 22], kspace=kspace, damping=False)
+    _, err, size = _against_frames(cuda, a[:5] + (ij, ds, bs), m, 1e-14)
+    # couplings below ke erfc(1.3) / 3 of a few pairs an atom: eigenvalues stay above 20
+    assert err < 2 * n * 1e-14 / 20 + 1e-12 * size
+
+
 @pytest.mark.parametrize("dtype,eps,tol", [(torch.float64, 1e-13, 1e-9), (torch.float32, 1e-7, 1e-4)])
 @pytest.mark.parametrize("kspace", [True, False])
 @pytest.mark.parametrize("nc", [0, 1, 2, 3, 4])

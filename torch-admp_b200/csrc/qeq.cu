@@ -109,12 +109,22 @@ static int qeq_matvec(QEqCtx<T>& c, const T* v, T* Hv, double* hv_out) {
 // 42,000, 100^3: 3.4 / 4.4, 6.0 / 8.0; 90,000, 128^3: 7.7 / 8.4, 15.1 / 16.9;
 // 120,000, 144^3: 11.5 / 11.3, 21.0 / 21.3, 142^3: 14.4 / 15.4, 29.3 / 29.7;
 // 180,000, 160^3: 20.3 / 17.5, 33.6 / 31.5; 300,000, 192^3: 35.1 / 26.7, 61.4 / 53.5.
-constexpr long long kCgMesh = 3000000;
-constexpr int kCgAtoms = 150000;
+//
+// The pairs are a quarter of the warps' work, at four entries a lane, and fall
+// behind the mesh once their list outgrows the L2 (listed pairs; half of a full
+// list has scale 0 and is dropped).  8.0 M, 10,701 atoms at 12 A: 2.8 / 3.1, 3.9 /
+// 4.0; 9.1 M, 30,000 at 9 A: 4.4 / 4.6, 7.0 / 6.8; 12 M, 40,000 at 9 A: 5.9 / 5.2,
+// 10.2 / 7.7; 29 M, 40,000 at 12 A: 14.4 / 6.7, 20.0 / 9.1.  Without a mesh, 20,000
+// atoms 0.43 / 0.47, 0.53 / 0.50; 60,000 0.76 / 0.64, 0.95 / 0.70; 140,000 1.53 /
+// 0.99, 2.37 / 1.18.
+constexpr long long kCgMesh = 3000000, kCgPairs = 10000000;
+constexpr int kCgAtoms = 150000, kCgAtomsNoMesh = 20000;
 template <typename T>
 static bool cg_plan(const QEqCtx<T>& c, int sms, CgArgs<T>& a, size_t& smem) {
   const SysDesc& d = c.w.plan.hs[0];
-  if (c.N > kCgAtoms || ((c.P.flags & ADMP_QEQ_KSPACE) && (long long)d.K0 * d.K1 * d.K2 > kCgMesh)) return false;
+  const bool mesh = (c.P.flags & ADMP_QEQ_KSPACE) != 0;
+  if (c.N > (mesh ? kCgAtoms : kCgAtomsNoMesh) || c.Pn > kCgPairs) return false;
+  if (mesh && (long long)d.K0 * d.K1 * d.K2 > kCgMesh) return false;
   const size_t budget = 200 * 1024, cs = sizeof(Cplx<T>);
   const int cap = (int)(64 * 1024 / cs);  // complex values in a line buffer
   a.N = c.N;
@@ -123,7 +133,7 @@ static bool cg_plan(const QEqCtx<T>& c, int sms, CgArgs<T>& a, size_t& smem) {
   a.K2 = d.K2;
   a.buf = a.planes = 0;
   a.lz = a.ly = a.lx = 1;
-  if (c.P.flags & ADMP_QEQ_KSPACE) {
+  if (mesh) {
     auto lines = [&](long long total, int K) {
       int most = cap / K < kCgMaxLines ? cap / K : kCgMaxLines;
       most = most < 1 ? 1 : most;
