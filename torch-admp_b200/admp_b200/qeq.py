@@ -262,16 +262,16 @@ def _times(t, c: float):
     return t if t is None or c == 1.0 else t * c
 
 
-def _check_arrays(device, **arrays) -> None:
-    """name=(tensor or None, least count): refuse what a kernel would read out of range
+def _check_arrays(positions, *arrays) -> None:
+    """(name, tensor or None, least count): refuse what a kernel would read out of range
     or from another device.  Metadata only: no launch, no wait."""
-    for name, (t, least) in arrays.items():
-        if t is None:
+    dev = positions.get_device()
+    for name, t, least in arrays:
+        if t is None or (t.numel() >= least and t.get_device() == dev):
             continue
-        if t.device != device:
-            raise RuntimeError(f"admp_b200: {name} is on {t.device}, positions on {device}")
-        if t.numel() < least:
-            raise ValueError(f"admp_b200: {name} has {t.numel()} values, {least} are needed")
+        if t.get_device() != dev:
+            raise RuntimeError(f"admp_b200: {name} is on {t.device}, positions on {positions.device}")
+        raise ValueError(f"admp_b200: {name} has {t.numel()} values, {least} are needed")
 
 
 def _std_inputs(module, positions, box, pairs, ds, buffer_scales, *vecs):
@@ -302,9 +302,10 @@ def _qeq_solve_raw(module, q0, positions, box, chi, hardness, eta, pairs, ds, bu
     if box is None:
         raise ValueError("admp_b200 QEq solve needs a periodic box")
     na, np_ = positions.shape[0], pairs.shape[0]
-    _check_arrays(positions.device, positions=(positions, 3 * na), box=(box, 9), chi=(chi, na), hardness=(hardness, na),
-                  eta=(eta, na), shift=(shift, na), charges=(q0, na), pairs=(pairs, 2 * np_), ds=(ds, np_),
-                  buffer_scales=(buffer_scales, np_), constraint_matrix=(C, 0))
+    _check_arrays(positions, ("positions", positions, 3 * na), ("box", box, 9), ("chi", chi, na),
+                  ("hardness", hardness, na), ("eta", eta, na), ("shift", shift, na), ("charges", q0, na),
+                  ("pairs", pairs, 2 * np_), ("ds", ds, np_), ("buffer_scales", buffer_scales, np_),
+                  ("constraint_matrix", C, 0))
     ec = module.const_lib.energy_coeff
     pos, bx, pr, dsc, bsc, (chi_c, hard_c, eta_c, sh, qv) = _std_inputs(
         module, positions, box, pairs, ds, buffer_scales, _times(chi.detach(), ec), _times(hardness.detach(), ec),
@@ -350,8 +351,8 @@ def _hessian(module, positions, box, hardness, eta, pairs, ds, buffer_scales, ma
     positions, box, pairs = positions.reshape(n, 3), box.reshape(3, 3), pairs.reshape(P, 2)
     ds, buffer_scales, hardness = ds.reshape(P), buffer_scales.reshape(P), hardness.reshape(n)
     eta = eta.reshape(n) if eta is not None else None
-    _check_arrays(positions.device, box=(box, 9), hardness=(hardness, n), eta=(eta, n), pairs=(pairs, 2 * P), ds=(ds, P),
-                  buffer_scales=(buffer_scales, P))
+    _check_arrays(positions, ("box", box, 9), ("hardness", hardness, n), ("eta", eta, n), ("pairs", pairs, 2 * P),
+                  ("ds", ds, P), ("buffer_scales", buffer_scales, P))
     lib = L.load()
     ec = module.const_lib.energy_coeff
     pos, bx, pr, dsc, bsc, (hard_c, eta_c) = _std_inputs(
@@ -527,9 +528,10 @@ def _qeq_solve_frames_raw(module, q0, positions, box, chi, hardness, eta, pairs,
         raise ValueError("admp_b200 QEq solve needs a periodic box")
     nf, n = int(positions.shape[0]), int(positions.shape[1])
     rows = nf * int(pairs.shape[1])
-    _check_arrays(positions.device, positions=(positions, 3 * nf * n), box=(box, 9 * nf), chi=(chi, n),
-                  hardness=(hardness, n), eta=(eta, n), shift=(shift, n), charges=(q0, n), pairs=(pairs, 2 * rows),
-                  ds=(ds, rows), buffer_scales=(buffer_scales, rows), constraint_matrix=(C, 0))
+    _check_arrays(positions, ("positions", positions, 3 * nf * n), ("box", box, 9 * nf), ("chi", chi, n),
+                  ("hardness", hardness, n), ("eta", eta, n), ("shift", shift, n), ("charges", q0, n),
+                  ("pairs", pairs, 2 * rows), ("ds", ds, rows), ("buffer_scales", buffer_scales, rows),
+                  ("constraint_matrix", C, 0))
     L.require_cuda(positions, "positions")
     dt = positions.dtype
     dev = positions.device
