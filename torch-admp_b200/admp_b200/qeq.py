@@ -348,9 +348,9 @@ def _hessian(module, positions, box, hardness, eta, pairs, ds, buffer_scales, ma
     ``max_cols`` columns whose meshes take at most ``max_mesh_bytes``."""
     # the kernels index n atoms and P pairs whatever the arrays hold: any other length is refused here
     n, P = positions.shape[0], pairs.shape[0]
-    positions, box, pairs = positions.reshape(n, 3), box.reshape(3, 3), pairs.reshape(P, 2)
-    ds, buffer_scales, hardness = ds.reshape(P), buffer_scales.reshape(P), hardness.reshape(n)
-    eta = eta.reshape(n) if eta is not None else None
+    for t, size in ((positions, 3 * n), (box, 9), (pairs, 2 * P), (ds, P), (buffer_scales, P), (hardness, n), (eta, n)):
+        if t is not None and t.numel() != size:
+            t.reshape(size)  # raises
     _check_arrays(positions, ("box", box, 9), ("hardness", hardness, n), ("eta", eta, n), ("pairs", pairs, 2 * P),
                   ("ds", ds, P), ("buffer_scales", buffer_scales, P))
     lib = L.load()
