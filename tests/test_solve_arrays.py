@@ -51,3 +51,19 @@ def test_arrays_elsewhere_are_refused(cuda, frames, name):
     with pytest.raises(RuntimeError, match="positions on cuda"):
         _call(cuda, frames, elsewhere=name)
     assert _call(cuda, frames).numel() == (NF * N if frames else N)
+
+
+@pytest.mark.gpu
+def test_arrays_that_nothing_reads_may_be_short(cuda):
+    """Without damping the widths are not read, without pair terms the pair list."""
+    from admp_b200 import _lib as L
+    from admp_b200.qeq import QEqForceModule
+    r = lambda *s: torch.rand(*s, dtype=torch.float64, device=cuda)  # noqa: E731
+    pos, box, chi, hard = r(N, 3) * 10, torch.eye(3, dtype=torch.float64, device=cuda) * 12, r(N), r(N) + 10
+    pairs = torch.tensor([[0, 1], [2, 3]], device=cuda)
+    for rspace, ds in ((True, r(2) + 2), (False, r(1))):
+        m = QEqForceModule(4.0, 1e-4, kmesh=8, damping=False, rspace=rspace)
+        for eta in (r(1), torch.zeros(1, dtype=torch.float64), None):
+            q, _, _, st = m._solve(torch.zeros_like(chi), pos, box, chi, hard, eta, pairs, ds, torch.ones_like(ds), None,
+                                   None, False, 1e-10, 100)
+            assert st == L.OK and bool(torch.isfinite(q).all())

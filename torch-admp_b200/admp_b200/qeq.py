@@ -274,6 +274,19 @@ def _check_arrays(positions, *arrays) -> None:
         raise ValueError(f"admp_b200: {name} has {t.numel()} values, {least} are needed")
 
 
+def _read_arrays(flags, eta, n, pairs, ds, buffer_scales, rows, C=None):
+    """_check_arrays entries of the arrays that the terms in `flags` read: a model without
+    damping ignores eta, one without pair terms the pair list."""
+    out = []
+    if flags & L.QEQ_DAMPING:
+        out.append(("eta", eta, n))
+    if flags & (L.QEQ_DAMPING | L.QEQ_RSPACE):
+        out += [("pairs", pairs, 2 * rows), ("ds", ds, rows), ("buffer_scales", buffer_scales, rows)]
+    if C is not None and C.shape[0]:
+        out.append(("constraint_matrix", C, 0))
+    return out
+
+
 def _std_inputs(module, positions, box, pairs, ds, buffer_scales, *vecs):
     dt = positions.dtype
     L.require_cuda(positions, "positions")
@@ -301,11 +314,11 @@ def _qeq_solve_raw(module, q0, positions, box, chi, hardness, eta, pairs, ds, bu
     lib = L.load()
     if box is None:
         raise ValueError("admp_b200 QEq solve needs a periodic box")
+    flags = module._flags()
     na, np_ = positions.shape[0], pairs.shape[0]
     _check_arrays(positions, ("positions", positions, 3 * na), ("box", box, 9), ("chi", chi, na),
-                  ("hardness", hardness, na), ("eta", eta, na), ("shift", shift, na), ("charges", q0, na),
-                  ("pairs", pairs, 2 * np_), ("ds", ds, np_), ("buffer_scales", buffer_scales, np_),
-                  ("constraint_matrix", C, 0))
+                  ("hardness", hardness, na), ("shift", shift, na), ("charges", q0, na),
+                  *_read_arrays(flags, eta, na, pairs, ds, buffer_scales, np_, C))
     ec = module.const_lib.energy_coeff
     pos, bx, pr, dsc, bsc, (chi_c, hard_c, eta_c, sh, qv) = _std_inputs(
         module, positions, box, pairs, ds, buffer_scales, _times(chi.detach(), ec), _times(hardness.detach(), ec),
@@ -315,7 +328,6 @@ def _qeq_solve_raw(module, q0, positions, box, chi, hardness, eta, pairs, ds, bu
     dev = pos.device
     if eta_c is None:
         eta_c = torch.zeros(n, dtype=dt, device=dev)
-    flags = module._flags()
     if project_q0:
         flags |= L.QEQ_PROJECT_Q0
     c = module.submodels["coulomb"]
@@ -351,8 +363,9 @@ def _hessian(module, positions, box, hardness, eta, pairs, ds, buffer_scales, ma
     for t, size in ((positions, 3 * n), (box, 9), (pairs, 2 * P), (ds, P), (buffer_scales, P), (hardness, n), (eta, n)):
         if t is not None and t.numel() != size:
             t.reshape(size)  # raises
-    _check_arrays(positions, ("box", box, 9), ("hardness", hardness, n), ("eta", eta, n), ("pairs", pairs, 2 * P),
-                  ("ds", ds, P), ("buffer_scales", buffer_scales, P))
+    flags = module._flags()
+    _check_arrays(positions, ("box", box, 9), ("hardness", hardness, n),
+                  *_read_arrays(flags, eta, n, pairs, ds, buffer_scales, P))
     lib = L.load()
     ec = module.const_lib.energy_coeff
     pos, bx, pr, dsc, bsc, (hard_c, eta_c) = _std_inputs(
@@ -373,7 +386,7 @@ def _hessian(module, positions, box, hardness, eta, pairs, ds, buffer_scales, ma
     if nbytes == 0:
         L.check(L.BAD_ARG, "QEq Hessian workspace")
     ws = L.workspace(nbytes, dev)
-    L.check(lib.admp_qeq_hessian(L.dtype_code(dt), module._flags(), n, kp, L.ptr(pos), L.ptr(bx), P, L.ptr(pr),
+    L.check(lib.admp_qeq_hessian(L.dtype_code(dt), flags, n, kp, L.ptr(pos), L.ptr(bx), P, L.ptr(pr),
                                  L.ptr(dsc), L.ptr(bsc), L.ptr(hard_c), L.ptr(eta_c), float(c.kappa) or 1.0,
                                  module.const_lib.dielectric, cols, L.ptr(H), L.ptr(ws), nbytes, L.stream_of(dev)),
             "QEq Hessian")
@@ -527,11 +540,10 @@ def _qeq_solve_frames_raw(module, q0, positions, box, chi, hardness, eta, pairs,
     if box is None:
         raise ValueError("admp_b200 QEq solve needs a periodic box")
     nf, n = int(positions.shape[0]), int(positions.shape[1])
-    rows = nf * int(pairs.shape[1])
+    flags = module._flags()
     _check_arrays(positions, ("positions", positions, 3 * nf * n), ("box", box, 9 * nf), ("chi", chi, n),
-                  ("hardness", hardness, n), ("eta", eta, n), ("shift", shift, n), ("charges", q0, n),
-                  ("pairs", pairs, 2 * rows), ("ds", ds, rows), ("buffer_scales", buffer_scales, rows),
-                  ("constraint_matrix", C, 0))
+                  ("hardness", hardness, n), ("shift", shift, n), ("charges", q0, n),
+                  *_read_arrays(flags, eta, n, pairs, ds, buffer_scales, nf * int(pairs.shape[1]), C))
     L.require_cuda(positions, "positions")
     dt = positions.dtype
     dev = positions.device
@@ -549,7 +561,6 @@ def _qeq_solve_frames_raw(module, q0, positions, box, chi, hardness, eta, pairs,
     eta_c = _frames_vec(_times(eta.detach(), lc), nf, n, dt) if eta is not None else torch.zeros(nf * n, dtype=dt, device=dev)
     sh = _frames_vec(shift, nf, n, dt) if shift is not None else None
     q = _frames_vec(q0, nf, n, dt).clone()
-    flags = module._flags()
     if project_q0:
         flags |= L.QEQ_PROJECT_Q0
     c = module.submodels["coulomb"]
