@@ -86,7 +86,7 @@ static int pme_recip_impl(int nf, int N, const int* kmesh, const T* pos, const T
 // Real-space, reciprocal, self, non-neutral and slab energies and their
 // gradients: table and zeroing, pairs, spread, three FFT passes, gather,
 // finalize -- eight launches (ten where build_recip_plan splits the passes of
-// few large planes in two).  Outputs are written, and the host waits only for
+// few large planes in two, one more above eight systems).  Outputs are written, and the host waits only for
 // the pair kernel's error word, after the rest has been launched.
 template <typename T>
 static int coulomb_impl(int flags, int nf, int N, const int* kmesh, const T* pos, const T* box, long long P,
